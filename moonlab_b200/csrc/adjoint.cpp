@@ -7,10 +7,12 @@
 //
 // One evaluation of B parameter vectors:
 //   1. cos/sin(theta/2) table on the host (libm, as gate_ry / gate_rz do);
-//   2. psi[b] = |hf>; forward tile passes over the tape;
+//   2. psi[b] from |hf>; forward rotation passes (hea_plan.h: the ladders
+//      are relabelling, the index order throughout is that after the last
+//      layer, where lambda and the energies are taken);
 //   3. lambda = H psi in tile passes over the Pauli terms; the last pass also
 //      produces E_b = <psi_b|lambda_b> (per-tile partials, fixed-order sum);
-//   4. backward tile passes over the reversed tape on (psi, lambda) with the
+//   4. backward rotation passes on (psi, lambda) with the
 //      per-parameter partials of Im<lambda|G|psi>; fixed-order sums.
 // Checkpoints: the tape is planned in segments of s = ceil(sqrt(L)) layers.
 // The forward sweep keeps psi at every segment boundary, and the backward
@@ -30,6 +32,7 @@
 #include <vector>
 
 #include "fused.h"
+#include "hea_plan.h"
 #include "mlb_internal.h"
 #include "planner.h"
 
@@ -56,12 +59,6 @@ struct TapeOp {
   int p;
 };
 
-struct GatePass {
-  AdjPass P;
-  std::vector<AdjOp> ops;
-  std::vector<int> param_of_slot;
-  size_t ops_off = 0, slots_off = 0;  // offsets into the device arrays
-};
 struct TermPass {
   AdjPass P;
   std::vector<AdjTerm> terms;
@@ -72,12 +69,15 @@ struct TermPass {
 
 struct mlb_hea {
   uint32_t n = 0, layers = 0, P = 0;
+  uint32_t nr = 0;  // the problem's qubits (n is at least 3)
   uint64_t hf = 0;
   int dtype = MLB_C128, device = 0, num_sms = 148;
   std::vector<uint64_t> xm, zm;
   std::vector<double> coeff;
   std::vector<TapeOp> tape;
-  std::vector<GatePass> fwd, bwd;
+  std::vector<hea::Pass> fwd, bwd;
+  std::vector<uint32_t> bound;  // layers before segment k; the last entry is all layers
+  int num_slots = 0;            // gradient slots of all backward passes
   // segments: fwd passes [fwd_seg[k], fwd_seg[k+1]) run segment k; bwd
   // passes [bwd_seg[j], bwd_seg[j+1]) run segment C-1-j backwards
   std::vector<size_t> fwd_seg, bwd_seg;
@@ -99,9 +99,9 @@ struct mlb_hea {
   size_t part_cap = 0;
   double* d_epart = nullptr;
   size_t epart_cap = 0;
-  AdjOp* d_ops = nullptr;
+  HeaSeg* d_segs = nullptr;
   AdjTerm* d_terms = nullptr;
-  int* d_slots = nullptr;
+  int* d_slots = nullptr;  // slot of each parameter
   double* d_out = nullptr;  // [B] energies then [B][P] grads
   size_t out_cap = 0;
   unsigned char* d_gram = nullptr;  // geometry: Gram matrix, then the Gram kernel's scratch
@@ -175,119 +175,39 @@ mlb_op_t proxy(const TapeOp& t) {
   return o;
 }
 
-// Partition a tape (forward or reversed) into gate passes and lower them.
-void plan_gates(mlb_hea* h, const std::vector<TapeOp>& tape, bool backward, std::vector<GatePass>& out) {
-  const int TB = adj_tile_bits(h->dtype, backward);
-  Planner pl{h->n, h->dtype, Geo{TB, 3}};
-  pl.max_ops = std::min({kMaxAdjOps, kMaxAdjSlots, kMaxAdjSegs});
-  std::vector<mlb_op_t> px;
-  px.reserve(tape.size());
-  for (const auto& t : tape) px.push_back(proxy(t));
-  const int n = (int)h->n;
-  const int L = n <= TB ? n : 5;
-  std::vector<int> rem(tape.size());
-  for (size_t i = 0; i < tape.size(); i++) rem[i] = (int)i;
-  while (!rem.empty()) {
-    uint64_t SH = 0;
-    std::vector<int> taken;
-    if (n <= TB) taken.assign(rem.begin(), rem.begin() + std::min<size_t>(rem.size(), pl.max_ops));
-    else taken = pl.choose(px, rem, L, SH);
-    GatePass gp{};
-    AdjPass& P = gp.P;
-    P.n = n;
-    P.L = L;
-    int local_of[64];
-    for (int q = 0; q < 64; q++) local_of[q] = q < L ? q : -1;
-    int H = 0;
-    for (int q = L; q < n; q++)
-      if (SH >> q & 1ull) {
-        P.high[H] = q;
-        local_of[q] = L + H;
-        H++;
+// Plans one segment of layers [l0, l1) as rotation passes; the backward
+// sweep runs its rotations in reverse.
+void plan_rotations(mlb_hea* h, uint32_t l0, uint32_t l1, bool backward, std::vector<hea::Pass>& out) {
+  std::vector<hea::Rot> rots;
+  for (uint32_t l = l0; l < l1; l++)
+    for (uint32_t q = 0; q < h->nr; q++) {
+      hea::Rot r{(int)l, (int)q, (int)(2 * (l * h->nr + q)), 1ull << q, 1ull << q};
+      for (uint32_t k = l; k < h->layers; k++) {  // to the coordinates after the last layer
+        r.dir = hea::ladder(r.dir, (int)h->nr);
+        r.fun = hea::unladder_functional(r.fun, (int)h->nr);
       }
-    P.H = H;
-    const int m = L + H;
-    const uint64_t allm = (1ull << n) - 1ull;
-    P.tile_free_mask = allm & ~(((1ull << L) - 1ull) | SH);
-    P.tiles_per_state = 1ull << (n - m);
-    P.num_params = (int)h->P;
-    auto local_mask = [&](uint64_t gm, uint32_t& lm, uint64_t& om) {
-      lm = 0;
-      om = 0;
-      for (int b = 0; b < n; b++)
-        if (gm >> b & 1ull) {
-          if (local_of[b] >= 0) lm |= 1u << local_of[b];
-          else om |= 1ull << b;
-        }
-    };
-    const std::vector<int> order = pl.schedule_segments(px, taken, local_mask, 3);
-    // pack into segments of <= 3 register bits (padded with the lowest free bits)
-    size_t i = 0;
-    while (i < order.size()) {
-      uint32_t bits = 0;
-      size_t j = i;
-      for (; j < order.size(); j++) {
-        uint32_t tl;
-        uint64_t om;
-        local_mask(op_targets(px[order[j]]), tl, om);
-        if (__builtin_popcount(bits | tl) > 3) break;
-        bits |= tl;
-      }
-      for (int b = 0; b < m && __builtin_popcount(bits) < 3; b++) bits |= 1u << b;
-      AdjSeg& sg = P.segs[P.num_segments++];
-      int nb = 0;
-      for (int b = 0; b < m && nb < 3; b++)
-        if (bits >> b & 1u) sg.bits[nb++] = b;
-      for (; nb < 3; nb++) sg.bits[nb] = sg.bits[nb - 1];  // never reached for m >= 3
-      sg.op_begin = (int)gp.ops.size();
-      for (size_t k = i; k < j; k++) {
-        const TapeOp& t = tape[order[k]];
-        AdjOp a{};
-        a.kind = t.kind;
-        a.p = t.p;
-        a.slot = -1;
-        a.lt = -1;
-        a.qt = t.q;
-        a.rt = 0;
-        if (t.kind != ADJ_KIND_RZ) {
-          const int lb = local_of[t.q];
-          for (int r = 0; r < 3; r++)
-            if (sg.bits[r] == lb) a.rt = r;
-        } else {
-          a.lt = local_of[t.q];
-        }
-        if (t.ctrl >= 0) {
-          uint64_t om;
-          local_mask(1ull << t.ctrl, a.lcmask, om);
-          a.ocmask = om;
-        }
-        if (backward && t.p >= 0) {
-          a.slot = (int)gp.param_of_slot.size();
-          gp.param_of_slot.push_back(t.p);
-        }
-        gp.ops.push_back(a);
-      }
-      sg.op_end = (int)gp.ops.size();
-      i = j;
+      rots.push_back(r);
     }
-    P.num_ops = (int)gp.ops.size();
-    P.num_slots = (int)gp.param_of_slot.size();
-    out.push_back(std::move(gp));
-    std::vector<int> next;
-    size_t t = 0;
-    for (int idx : rem) {
-      if (t < taken.size() && taken[t] == idx) { t++; continue; }
-      next.push_back(idx);
-    }
-    rem.swap(next);
-  }
+  if (backward) std::reverse(rots.begin(), rots.end());
+  // rows of 64 bytes
+  hea::plan(rots, (int)h->n, hea_tile_bits(h->dtype, backward), h->dtype == MLB_C128 ? 2 : 3, h->dtype, out);
+}
+
+// A rotation pass's work items: runs of a state's tiles, at most 256 items a
+// state (the gradient partials' count), the same for every batch size.
+HeaPass pass_for_batch(const hea::Pass& p, size_t B) {
+  HeaPass P = p.dev;
+  P.tiles_per_item = (uint32_t)std::max<uint64_t>(1, P.tiles_per_state >> 8);
+  P.items_per_state = (uint32_t)(P.tiles_per_state / P.tiles_per_item);
+  P.num_items = (uint64_t)P.items_per_state * B;
+  return P;
 }
 
 // Partition the Pauli terms into lambda passes: a term fits a pass when its
 // X-part lies inside the tile (Z-part may lie anywhere).  Terms commute in
 // the sum, so no ordering constraint applies.
 void plan_terms(mlb_hea* h) {
-  const int TB = adj_tile_bits(h->dtype, false);
+  const int TB = adj_tile_bits(h->dtype);
   const int n = (int)h->n;
   const int L = n <= TB ? n : 5;
   const int Hmax = n <= TB ? 0 : TB - L;
@@ -399,26 +319,36 @@ bool plan_fused_forward(mlb_hea* h, const std::vector<size_t>& cut) {
 }
 
 int upload_programs(mlb_hea* h) {
-  std::vector<AdjOp> all_ops;
-  std::vector<int> all_slots;
+  std::vector<HeaSeg> all_segs;
   for (auto* vec : {&h->fwd, &h->bwd})
-    for (auto& gp : *vec) {
-      gp.ops_off = all_ops.size();
-      gp.slots_off = all_slots.size();
-      all_ops.insert(all_ops.end(), gp.ops.begin(), gp.ops.end());
-      all_slots.insert(all_slots.end(), gp.param_of_slot.begin(), gp.param_of_slot.end());
+    for (auto& p : *vec) {
+      p.segs_off = all_segs.size();
+      all_segs.insert(all_segs.end(), p.segs.begin(), p.segs.end());
     }
+  std::vector<int> slot_of_param(h->P, 0);
+  h->num_slots = 0;
+  for (auto& p : h->bwd) {
+    p.slots_off = (size_t)h->num_slots;
+    for (const HeaSeg& sg : p.segs) {
+      for (int i = 0; i < 3; i++)
+        if (sg.param[i] >= 0) {
+          slot_of_param[sg.param[i] + 1] = h->num_slots + i;  // RZ
+          slot_of_param[sg.param[i]] = h->num_slots + 3 + i;  // RY
+        }
+      h->num_slots += kHeaSlots;
+    }
+  }
   std::vector<AdjTerm> all_terms;
   for (auto& tp : h->lam) {
     tp.terms_off = all_terms.size();
     all_terms.insert(all_terms.end(), tp.terms.begin(), tp.terms.end());
   }
-  cudaError_t e = cudaMalloc((void**)&h->d_ops, std::max<size_t>(1, all_ops.size()) * sizeof(AdjOp));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_slots, std::max<size_t>(1, all_slots.size()) * sizeof(int));
+  cudaError_t e = cudaMalloc((void**)&h->d_segs, all_segs.size() * sizeof(HeaSeg));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_slots, slot_of_param.size() * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_terms, std::max<size_t>(1, all_terms.size()) * sizeof(AdjTerm));
   if (e != cudaSuccess) return cfail(e, "adjoint program upload");
-  cudaMemcpy(h->d_ops, all_ops.data(), all_ops.size() * sizeof(AdjOp), cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_slots, all_slots.data(), all_slots.size() * sizeof(int), cudaMemcpyHostToDevice);
+  cudaMemcpy(h->d_segs, all_segs.data(), all_segs.size() * sizeof(HeaSeg), cudaMemcpyHostToDevice);
+  cudaMemcpy(h->d_slots, slot_of_param.data(), slot_of_param.size() * sizeof(int), cudaMemcpyHostToDevice);
   e = cudaMemcpy(h->d_terms, all_terms.data(), all_terms.size() * sizeof(AdjTerm), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cfail(e, "adjoint program upload");
   if (h->fused_ok) {
@@ -480,15 +410,13 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
       h->ckpt_cap = need;
     }
   }
-  size_t max_slots_tiles = 1, max_tiles = 1;
-  for (auto& gp : h->bwd) max_slots_tiles = std::max(max_slots_tiles, gp.P.tiles_per_state * B * (size_t)gp.P.num_slots);
+  size_t max_tiles = 1;
   for (auto& tp : h->lam) max_tiles = std::max(max_tiles, tp.P.tiles_per_state * B);
-  if ((rc = grow(h->d_part, h->part_cap, max_slots_tiles))) return rc;
+  const uint32_t items = pass_for_batch(h->bwd[0], B).items_per_state;
+  if (h_G && (rc = grow(h->d_part, h->part_cap, (size_t)items * B * h->num_slots))) return rc;
   if ((rc = grow(h->d_epart, h->epart_cap, max_tiles))) return rc;
   if ((rc = grow(h->d_out, h->out_cap, B + B * h->P))) return rc;
   // 2. forward
-  // |0...0>: the tape itself starts with X on the hf_reference bits (vqe.c:1953-1959)
-  if ((rc = launch_adj_init(h->dtype, h->psi, (int)h->n, B, 0, h->stream))) return hfail(rc, "init kernel");
   const size_t nseg = h->fwd_seg.size() - 1;
   const size_t state_bytes = B * dim * ab;
   const bool fused = use_fused_forward(h, B);
@@ -507,6 +435,8 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
                                   h->stream)))
       return hfail(rc, "operand image build");
     cudaMemsetAsync(h->d_ferr, 0, sizeof(int), h->stream);
+    // |0...0>: the tape itself starts with X on the hf_reference bits (vqe.c:1953-1959)
+    if ((rc = launch_adj_init(h->dtype, h->psi, (int)h->n, B, 0, h->stream))) return hfail(rc, "init kernel");
   }
   for (size_t k = 0; k < nseg; k++) {
     if (fused) {
@@ -519,16 +449,19 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
           return hfail(rc, "fused forward pass");
       }
     } else {
+      // the segment's last pass writes the checkpoint, the next segment's
+      // first pass reads it back
       for (size_t i = h->fwd_seg[k]; i < h->fwd_seg[k + 1]; i++) {
-        const GatePass& gp = h->fwd[i];
-        AdjPass P = gp.P;
-        P.num_tiles = P.tiles_per_state * B;
-        if ((rc = launch_adj_gates(h->dtype, h->psi, nullptr, P, h->d_ops + gp.ops_off, h->d_cs, nullptr, false,
-                                   false, h->num_sms, h->stream)))
+        const bool from = use_ckpt && k > 0 && i == h->fwd_seg[k];
+        const bool to = use_ckpt && k + 1 < nseg && i + 1 == h->fwd_seg[k + 1];
+        if ((rc = launch_hea_pass(h->dtype, from ? (char*)h->ckpt + (k - 1) * state_bytes : h->psi,
+                                  to ? (char*)h->ckpt + k * state_bytes : h->psi, nullptr,
+                                  pass_for_batch(h->fwd[i], B), h->d_segs + h->fwd[i].segs_off, h->d_cs, nullptr, 0,
+                                  false, h->num_sms, h->stream)))
           return hfail(rc, "forward pass");
       }
     }
-    if (use_ckpt && k + 1 < nseg) {
+    if (fused && use_ckpt && k + 1 < nseg) {
       cudaError_t e = cudaMemcpyAsync((char*)h->ckpt + k * state_bytes, h->psi, state_bytes,
                                       cudaMemcpyDeviceToDevice, h->stream);
       if (e != cudaSuccess) return cfail(e, "checkpoint save");
@@ -549,31 +482,33 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
     if ((rc = launch_adj_pauli(h->dtype, h->psi, h->lamb, P, h->d_terms + h->lam[k].terms_off, k > 0, last,
                                h->d_epart, h->num_sms, h->stream)))
       return hfail(rc, "lambda pass");
-    if (last && (rc = launch_adj_reduce(h->d_epart, P.tiles_per_state, 1, B, nullptr, 1, h->d_out, h->stream)))
+    if (last && (rc = launch_adj_energy(h->d_epart, P.tiles_per_state, B, h->d_out, h->stream)))
       return hfail(rc, "energy reduce");
   }
   // 4. backward
   if (h_G) {
     for (size_t j = 0; j < nseg; j++) {
       const size_t k = nseg - 1 - j;  // segment swept backwards
+      const void* src = h->psi;
       if (use_ckpt && k + 1 < nseg) {  // psi at the end of segment k, as the forward sweep left it
-        cudaError_t e = cudaMemcpyAsync(h->psi, (char*)h->ckpt + k * state_bytes, state_bytes,
-                                        cudaMemcpyDeviceToDevice, h->stream);
-        if (e != cudaSuccess) return cfail(e, "checkpoint restore");
+        const void* c = (char*)h->ckpt + k * state_bytes;
+        if (!fused) {
+          src = c;
+        } else if ((rc = launch_unladder(c, h->psi, (int)h->n, (int)(h->layers - h->bound[k + 1]), B, h->num_sms,
+                                         h->stream))) {  // the tensor-core passes carry the ladders out
+          return hfail(rc, "checkpoint restore");
+        }
       }
-    for (size_t i = h->bwd_seg[j]; i < h->bwd_seg[j + 1]; i++) {
-      const GatePass& gp = h->bwd[i];
-      AdjPass P = gp.P;
-      P.num_tiles = P.tiles_per_state * B;
-      if ((rc = launch_adj_gates(h->dtype, h->psi, h->lamb, P, h->d_ops + gp.ops_off, h->d_cs, h->d_part, true,
-                                 true, h->num_sms, h->stream)))
-        return hfail(rc, "backward pass");
-      if (P.num_slots &&
-          (rc = launch_adj_reduce(h->d_part, P.tiles_per_state, P.num_slots, B, h->d_slots + gp.slots_off,
-                                  (int)h->P, h->d_out + B, h->stream)))
-        return hfail(rc, "gradient reduce");
+      for (size_t i = h->bwd_seg[j]; i < h->bwd_seg[j + 1]; i++) {
+        const hea::Pass& p = h->bwd[i];
+        if ((rc = launch_hea_pass(h->dtype, src, h->psi, h->lamb, pass_for_batch(p, B), h->d_segs + p.segs_off,
+                                  h->d_cs, h->d_part + p.slots_off, h->num_slots, true, h->num_sms, h->stream)))
+          return hfail(rc, "backward pass");
+        src = h->psi;
+      }
     }
-    }
+    if ((rc = launch_hea_reduce(h->d_part, items, h->num_slots, B, h->d_slots, (int)h->P, h->d_out + B, h->stream)))
+      return hfail(rc, "gradient reduce");
   }
   if (fused && (rc = launch_divide_by_norm(h->d_out, B, (int)h->P, h->d_norm, h->stream)))
     return hfail(rc, "norm correction");
@@ -627,14 +562,10 @@ int geometry(mlb_hea* h, const double* params, double* metric, double* curvature
   size_t cap = h->gram_cap;
   if ((rc = grow(h->d_gram, cap, (need + 255) / 256 * 256))) return rc;
   h->gram_cap = cap;
-  if ((rc = launch_adj_init(h->dtype, h->psi, (int)h->n, B, 0, h->stream))) return hfail(rc, "init kernel");
-  for (const GatePass& gp : h->fwd) {
-    AdjPass Pp = gp.P;
-    Pp.num_tiles = Pp.tiles_per_state * B;
-    if ((rc = launch_adj_gates(h->dtype, h->psi, nullptr, Pp, h->d_ops + gp.ops_off, h->d_cs, nullptr, false,
-                               false, h->num_sms, h->stream)))
+  for (const hea::Pass& p : h->fwd)
+    if ((rc = launch_hea_pass(h->dtype, h->psi, h->psi, nullptr, pass_for_batch(p, B), h->d_segs + p.segs_off, h->d_cs,
+                              nullptr, 0, false, h->num_sms, h->stream)))
       return hfail(rc, "forward pass");
-  }
   double2* d_G = reinterpret_cast<double2*>(h->d_gram);
   if ((rc = launch_gram(h->psi, dim, (int)B, d_G, h->d_gram + (gbytes + 255) / 256 * 256, h->num_sms, h->stream)))
     return hfail(rc, "Gram kernel");
@@ -707,6 +638,7 @@ int mlb_hea_create(uint32_t n, uint32_t layers, uint64_t hf, size_t num_terms, c
   // passes' register groups span 3 qubits.  Energies and gradients are those
   // of the n-qubit problem.
   h->n = n < 3 ? 3 : n;
+  h->nr = n;
   h->layers = layers;
   h->P = 2 * n * layers;
   h->hf = hf;
@@ -737,18 +669,28 @@ int mlb_hea_create(uint32_t n, uint32_t layers, uint64_t hf, size_t num_terms, c
   std::vector<size_t> cut{0};
   for (uint32_t l = h->seg_layers; l < layers; l += h->seg_layers) cut.push_back(prefix + l * per_layer);
   cut.push_back(h->tape.size());
+  for (uint32_t l = 0; l < layers; l += h->seg_layers) h->bound.push_back(l);
+  h->bound.push_back(layers);
   h->fwd_seg.push_back(0);
-  for (size_t k = 0; k + 1 < cut.size(); k++) {
-    std::vector<TapeOp> sub(h->tape.begin() + cut[k], h->tape.begin() + cut[k + 1]);
-    plan_gates(h, sub, false, h->fwd);
+  for (size_t k = 0; k + 1 < h->bound.size(); k++) {
+    plan_rotations(h, h->bound[k], h->bound[k + 1], false, h->fwd);
     h->fwd_seg.push_back(h->fwd.size());
   }
   h->bwd_seg.push_back(0);
-  for (size_t k = cut.size() - 1; k-- > 0;) {
-    std::vector<TapeOp> rev(h->tape.rend() - cut[k + 1], h->tape.rend() - cut[k]);
-    plan_gates(h, rev, true, h->bwd);
+  for (size_t k = h->bound.size() - 1; k-- > 0;) {
+    plan_rotations(h, h->bound[k], h->bound[k + 1], true, h->bwd);
     h->bwd_seg.push_back(h->bwd.size());
   }
+  {  // the first pass starts from |hf>
+    uint64_t at = hf;
+    for (uint32_t l = 0; l < layers; l++) at = hea::ladder(at, (int)n);
+    hea::Pass& p = h->fwd[0];
+    p.dev.init = 1;
+    p.dev.init_base = (uint32_t)p.basis.reduce(at);
+    p.dev.init_local = p.basis.coords(at);
+  }
+  for (auto* vec : {&h->fwd, &h->bwd})
+    for (auto& p : *vec) p.dev.num_params = (int)h->P;
   plan_terms(h);
   // the tensor-core forward sweep's plans (used by complex64 problems by default)
   if (dtype == MLB_C64 && h->n == n && n >= (uint32_t)fused::kTileBits) {
@@ -778,7 +720,7 @@ void mlb_hea_free(mlb_hea_t* h) {
   Guard g(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : {h->psi, h->lamb, h->ckpt, (void*)h->d_cs, (void*)h->d_part, (void*)h->d_epart,
-                  (void*)h->d_ops, (void*)h->d_terms, (void*)h->d_slots, (void*)h->d_out, (void*)h->d_gram,
+                  (void*)h->d_segs, (void*)h->d_terms, (void*)h->d_slots, (void*)h->d_out, (void*)h->d_gram,
                   (void*)h->d_fblocks, (void*)h->d_gblocks, (void*)h->d_gops, (void*)h->d_images,
                   (void*)h->d_ferr, (void*)h->d_norm})
     if (p) cudaFree(p);

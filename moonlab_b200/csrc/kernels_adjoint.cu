@@ -13,19 +13,20 @@
 // cos/sin of its own theta (table cs[b][p], computed once per call).
 //
 // Kernels (all tile passes, one HBM read + write of each array per pass):
-//   k_adj_gates : gate ops on psi (forward) or on psi and lambda together
+//   k_hea       : rotations on psi (forward) or on psi and lambda together
 //                 with the per-parameter partial inner products (backward).
-//                 Register groups of 2^3 amplitudes per thread, as in the
-//                 state engine's tile passes.
 //   k_adj_pauli : lambda (+)= sum_k c_k P_k psi for the Pauli terms whose
 //                 X-part lies inside the tile; the last pass also emits the
 //                 per-tile partial of Re<psi|lambda> (the energy).
-//   k_adj_reduce: fixed-order sums of the per-tile partials (deterministic).
+//   k_hea_reduce, k_adj_energy: fixed-order sums of the partials
+//                 (deterministic, and the same for every batch size).
+//   k_unladder  : a complex64 batch from the index order of a layer boundary
+//                 to the order after the last layer (hea_plan.h).
 // Tiles come into shared memory by asynchronous copies, all in flight at
-// once.  (Issuing the next tile's copies from the store loop, as the state
-// engine's tile passes do, measured no faster here.)
-#include <cstdio>
+// once.
+#include <vector>
 
+#include "hea_plan.h"
 #include "kernels_common.cuh"
 #include "mlb_internal.h"
 
@@ -36,7 +37,8 @@ namespace {
 template <typename Real> struct AdjCfg;
 template <> struct AdjCfg<double> { static constexpr int TB = 11, NT = 256, SW_SHIFT = 3, SW_MASK = 7; };
 template <> struct AdjCfg<float> { static constexpr int TB = 12, NT = 256, SW_SHIFT = 4, SW_MASK = 15; };
-constexpr int kRB = 3, kG = 1 << kRB;
+
+constexpr int kUnladderBits = 11, kUnladderLow = 4;  // tile of k_unladder, contiguous bits of its rows
 
 template <typename Real>
 __device__ __forceinline__ uint32_t aswz(uint32_t e) {
@@ -72,210 +74,296 @@ __device__ __forceinline__ void load_tile(typename Cplx<Real>::T* __restrict__ s
 __device__ __forceinline__ void tile_loads_wait() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
-template <typename Real>
-__device__ __forceinline__ void store_tile(const typename Cplx<Real>::T* __restrict__ sm,
-                                           typename Cplx<Real>::T* __restrict__ g, uint64_t tile_base,
-                                           const uint64_t* rowoff, int L, uint32_t amps) {
-  constexpr int NT = AdjCfg<Real>::NT;
-  const uint32_t lm = (1u << L) - 1u;
-  for (uint32_t e = threadIdx.x; e < amps; e += NT) __stcs(&g[tile_base | rowoff[e >> L] | (e & lm)], sm[aswz<Real>(e)]);
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
 }
 
 // ---------------------------------------------------------------------------
-// gate passes
+// rotation passes
 // ---------------------------------------------------------------------------
-template <typename A, int RT, bool DUAL>
-__device__ __forceinline__ void apply_x(A (&v)[kG], A (&w)[kG], uint32_t gb, const uint32_t (&bm)[kRB],
-                                        uint32_t lcmask) {
-#pragma unroll
-  for (int k = 0; k < kG; k++) {
-    if (k & (1 << RT)) continue;
-    uint32_t loc = gb;
-#pragma unroll
-    for (int b = 0; b < kRB; b++)
-      if (k >> b & 1) loc |= bm[b];
-    if ((loc & lcmask) != lcmask) continue;
-    const int k1 = k | (1 << RT);
-    A t = v[k]; v[k] = v[k1]; v[k1] = t;
-    if (DUAL) { t = w[k]; w[k] = w[k1]; w[k1] = t; }
-  }
-}
+// One tile per step and CTA: 2^m amplitudes base ^ span(basis), whose local
+// index bits 0.. are contiguous amplitudes.  Four warps; the 16-byte units of
+// a tile (one complex128 or two complex64 amplitudes) come by cp.async, all
+// in flight at once.  A segment's thread holds groups of 8 amplitudes whose
+// register index is the segment's three target bits, so every rotation is
+// compile-time code: no per-gate dispatch, no CNOTs (they are relabelling,
+// hea_plan.h).  RZ's of a segment are one phase per register index, from a
+// table per state; RY [[c, -s], [s, c]] is applied as c [[1, -t], [t, 1]]
+// (t = s / c; c and s swap roles where |c| < |s|), two multiply-adds per
+// component pair instead of four operations, and the product of the three
+// scales is folded into the phases.
+// Bound: shared memory (64 bytes per complex128 psi + lambda pair and segment,
+// 0.5 clk per SM) and FP64 (about 30 operations, 0.47 clk) together; 64 KiB
+// tiles, so three CTAs per SM overlap one's copies with the others' work.
+// Measured, 20 qubits, 8 layers, 256 vectors with gradients: 616 ms by
+// gate-by-gate passes with the CNOTs carried out (19 forward, 17 backward),
+// 134 ms by these (6 and 9); complex64 326 -> 116 ms.
+template <typename Real> struct HeaCfg;
+template <> struct HeaCfg<double> { static constexpr int FWD_BITS = 12, BACK_BITS = 11; };
+template <> struct HeaCfg<float> { static constexpr int FWD_BITS = 13, BACK_BITS = 12; };
+constexpr int kHeaThreads = 128, kHeaWarps = kHeaThreads / 32;
 
-// RY(angle) with c, s of the applied angle: [[c, -s], [s, c]].
-template <typename A, typename Real, int RT, bool DUAL>
-__device__ __forceinline__ void apply_ry(A (&v)[kG], A (&w)[kG], Real c, Real s) {
+// Per-state tables of a segment.
+template <typename Real>
+struct HeaTab {
+  typename Cplx<Real>::T ph[8];  // scale * exp(-+ i ...) per register index
+  Real t[3];                     // tangent, or cotangent where `flip`
+  uint32_t flip;                 // bit i: rotation i uses the cotangent form
+  double unscale;                // 1 / scale^2 (d/dRY is taken on scaled states)
+};
+
+// v[k], v[k1] <- RY (forward) or its inverse (BACK), up to the scale.
+template <typename A, typename Real, int RT, bool BACK>
+__device__ __forceinline__ void hea_ry(A (&v)[8], Real t, bool flip) {
 #pragma unroll
-  for (int k = 0; k < kG; k++) {
+  for (int k = 0; k < 8; k++) {
     if (k & (1 << RT)) continue;
-    const int k1 = k | (1 << RT);
-    A a0 = v[k], a1 = v[k1];
-    v[k] = {c * a0.x - s * a1.x, c * a0.y - s * a1.y};
-    v[k1] = {s * a0.x + c * a1.x, s * a0.y + c * a1.y};
-    if (DUAL) {
-      a0 = w[k]; a1 = w[k1];
-      w[k] = {c * a0.x - s * a1.x, c * a0.y - s * a1.y};
-      w[k1] = {s * a0.x + c * a1.x, s * a0.y + c * a1.y};
+    const A a = v[k], b = v[k | (1 << RT)];
+    const Real tt = BACK ? t : -t;
+    if (!flip) {
+      v[k] = {a.x + tt * b.x, a.y + tt * b.y};
+      v[k | (1 << RT)] = {b.x - tt * a.x, b.y - tt * a.y};
+    } else if (BACK) {
+      v[k] = {t * a.x + b.x, t * a.y + b.y};
+      v[k | (1 << RT)] = {t * b.x - a.x, t * b.y - a.y};
+    } else {
+      v[k] = {t * a.x - b.x, t * a.y - b.y};
+      v[k | (1 << RT)] = {t * b.x + a.x, t * b.y + a.y};
     }
   }
 }
 
-// Im<lambda|Y_q|psi> over the pairs of register bit RT:
-// (Y psi)_{q=0} = -i psi_{q=1},  (Y psi)_{q=1} = i psi_{q=0}.
+// Im<lambda|Y|psi> over the pairs of register bit RT:
+// (Y psi)_0 = -i psi_1, (Y psi)_1 = i psi_0.
 template <typename A, int RT>
-__device__ __forceinline__ double grad_y(const A (&v)[kG], const A (&w)[kG]) {
+__device__ __forceinline__ double hea_grad_y(const A (&v)[8], const A (&w)[8]) {
   double acc = 0.0;
 #pragma unroll
-  for (int k = 0; k < kG; k++) {
+  for (int k = 0; k < 8; k++) {
     if (k & (1 << RT)) continue;
-    const int k1 = k | (1 << RT);
-    const A p0 = v[k], p1 = v[k1], l0 = w[k], l1 = w[k1];
-    acc += -((double)l0.x * p1.x + (double)l0.y * p1.y) + ((double)l1.x * p0.x + (double)l1.y * p0.y);
+    const A p0 = v[k], p1 = v[k | (1 << RT)], l0 = w[k], l1 = w[k | (1 << RT)];
+    acc -= (double)l0.x * p1.x + (double)l0.y * p1.y;
+    acc += (double)l1.x * p0.x + (double)l1.y * p0.y;
   }
   return acc;
 }
 
-template <typename Real, bool DUAL, bool BACKWARD>
-__global__ void __launch_bounds__(AdjCfg<Real>::NT, 2)
-    k_adj_gates(typename Cplx<Real>::T* __restrict__ psi, typename Cplx<Real>::T* __restrict__ lam,
-                const AdjPass P, const AdjOp* __restrict__ ops, const double2* __restrict__ cs,
-                double* __restrict__ partials) {
-  using A = typename Cplx<Real>::T;
-  constexpr int NT = AdjCfg<Real>::NT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const uint32_t amps = 1u << (P.L + P.H);
-  A* sv = reinterpret_cast<A*>(smem_raw);
-  A* sw = sv + amps;
-  __shared__ uint64_t rowoff[1 << (AdjCfg<Real>::TB - 5)];
-  __shared__ AdjOp sops[kMaxAdjOps];
-  __shared__ double2 scs[kMaxAdjOps];
-  __shared__ uint8_t son[kMaxAdjOps];
-  __shared__ double red[NT / 32][kMaxAdjSlots];
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
 
-  for (uint32_t r = threadIdx.x; r < (1u << P.H); r += NT) {
-    uint64_t off = 0;
+template <typename Real, bool BACK>
+__global__ void __launch_bounds__(kHeaThreads, 3)
+    k_hea(const typename Cplx<Real>::T* src, typename Cplx<Real>::T* psi, typename Cplx<Real>::T* lam,
+          const __grid_constant__ HeaPass P, const HeaSeg* __restrict__ segs, const double2* __restrict__ cs,
+          double* __restrict__ partials, int part_stride) {
+  using A = typename Cplx<Real>::T;
+  constexpr int NT = kHeaThreads;
+  constexpr int UB = sizeof(A) == 16 ? 0 : 1;  // log2 of the amplitudes of a 16-byte unit
+  extern __shared__ __align__(128) unsigned char smem[];
+  const uint32_t tile_bytes = (uint32_t)sizeof(A) << P.m;
+  unsigned char* tables = smem + (BACK ? 2u : 1u) * tile_bytes;
+  HeaTab<Real>* tab = reinterpret_cast<HeaTab<Real>*>(tables);
+  double* red = reinterpret_cast<double*>(tab + P.num_segs);  // [warp][slot], backward only
+  __shared__ uint32_t joff[1 << (kMaxHeaBits - 7)];            // index offset of unit j * NT
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nslots = P.num_segs * kHeaSlots;
+  HeaSeg* sseg = reinterpret_cast<HeaSeg*>(red + (BACK ? kHeaWarps * nslots : 0));
+  const uint32_t units = 1u << (P.m - UB), groups = 1u << (P.m - 3);
+
+  for (uint32_t j = tid; j < (1u << (kMaxHeaBits - 7)); j += NT) {
+    uint32_t off = 0;
 #pragma unroll
-    for (int k = 0; k < kMaxHigh; k++)
-      if (k < P.H && (r >> k & 1u)) off |= 1ull << P.high[k];
-    rowoff[r] = off;
+    for (int b = 7; b < kMaxHeaBits - UB; b++)
+      if (b + UB < P.m && (j >> (b - 7) & 1u)) off ^= P.basis[b + UB];
+    joff[j] = off;
   }
-  for (int o = threadIdx.x; o < P.num_ops; o += NT) sops[o] = ops[o];
+  for (int i = tid; i < P.num_segs * (int)(sizeof(HeaSeg) / 4); i += NT)
+    reinterpret_cast<uint32_t*>(sseg)[i] = reinterpret_cast<const uint32_t*>(segs)[i];
+  uint32_t toff = 0;  // this thread's part of a unit's index
+#pragma unroll
+  for (int b = 0; b < 7; b++)
+    if (b + UB < P.m && (tid >> b & 1)) toff ^= P.basis[b + UB];
+  const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   __syncthreads();
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (uint64_t tile = blockIdx.x; tile < P.num_tiles; tile += gridDim.x) {
-    const uint64_t tb = tile_base_of(P, tile);
-    const uint64_t b = tile / P.tiles_per_state;
-    for (int o = threadIdx.x; o < P.num_ops; o += NT) {
-      const AdjOp& op = sops[o];
-      son[o] = (uint8_t)((tb & op.ocmask) == op.ocmask);
-      if (op.p >= 0) scs[o] = cs[b * P.num_params + op.p];
-    }
-    for (int i = threadIdx.x; i < (NT / 32) * kMaxAdjSlots; i += NT) (&red[0][0])[i] = 0.0;
-    load_tile<Real>(sv, psi, tb, rowoff, P.L, amps);
-    if (DUAL) load_tile<Real>(sw, lam, tb, rowoff, P.L, amps);
-    tile_loads_wait();
-    __syncthreads();
-
-    for (int s = 0; s < P.num_segments; s++) {
-      const AdjSeg& seg = P.segs[s];
-      uint32_t bm[kRB];
-#pragma unroll
-      for (int q = 0; q < kRB; q++) bm[q] = 1u << seg.bits[q];
-      const uint32_t groups = amps >> kRB;
-      // Every lane runs every iteration (the gradient partials use full-warp
-      // shuffles); lanes past the last group work on zeros and store nothing.
-      for (uint32_t g0 = 0; g0 < groups; g0 += NT) {
-        const uint32_t gi = g0 + threadIdx.x;
-        const bool active = gi < groups;
-        uint32_t gb = active ? gi : 0u;
-#pragma unroll
-        for (int q = 0; q < kRB; q++) {
-          const uint32_t p = seg.bits[q];
-          gb = ((gb >> p) << (p + 1)) | (gb & ((1u << p) - 1u));
+  for (uint64_t item = blockIdx.x; item < P.num_items; item += gridDim.x) {
+    const uint64_t b = item / P.items_per_state;
+    const uint32_t tile0 = (uint32_t)(item % P.items_per_state) * P.tiles_per_item;
+    const A* gs = src + (b << P.n);
+    A* gp = psi + (b << P.n);
+    A* gl = BACK ? lam + (b << P.n) : nullptr;
+    for (uint32_t ti = 0; ti < P.tiles_per_item; ti++) {
+      const uint32_t base = (uint32_t)pdep64(tile0 + ti, P.free_mask);
+      bool work = true;
+      if (!BACK && P.init) {
+        work = base == P.init_base;
+        for (uint32_t u = tid; u < units; u += NT) reinterpret_cast<double2*>(smem)[u] = make_double2(0.0, 0.0);
+        if (work) {
+          __syncthreads();
+          if (tid == 0)
+            *reinterpret_cast<A*>(smem + (UB ? tile_swz16(P.init_local >> 1) * 16u + (P.init_local & 1u) * 8u
+                                             : tile_swz16(P.init_local) * 16u)) = A{1, 0};
         }
-        A v[kG], w[kG];
-#pragma unroll
-        for (int k = 0; k < kG; k++) {
-          uint32_t loc = gb;
-#pragma unroll
-          for (int q = 0; q < kRB; q++)
-            if (k >> q & 1) loc |= bm[q];
-          v[k] = active ? sv[aswz<Real>(loc)] : A{0, 0};
-          if (DUAL) w[k] = active ? sw[aswz<Real>(loc)] : A{0, 0};
+      } else {
+        for (uint32_t u = tid, j = 0; u < units; u += NT, j++) {
+          const uint32_t off = base ^ toff ^ joff[j];
+          const uint32_t dst = sm0 + tile_swz16(u) * 16u;
+          cp_async16(dst, gs + off);
+          if (BACK) cp_async16(dst + tile_bytes, gl + off);
         }
-        for (int o = seg.op_begin; o < seg.op_end; o++) {
-          if (!son[o]) continue;
-          const AdjOp& op = sops[o];
-          const Real c = (Real)scs[o].x, sn = (Real)scs[o].y;
-          switch (op.kind * 4 + op.rt) {
-#define ADJ_X(r)                                                          \
-  case ADJ_KIND_X * 4 + r: apply_x<A, r, DUAL>(v, w, gb, bm, op.lcmask); break;
-            ADJ_X(0) ADJ_X(1) ADJ_X(2)
-#undef ADJ_X
-#define ADJ_RY(r)                                                                         \
-  case ADJ_KIND_RY * 4 + r:                                                               \
-    if (BACKWARD && op.slot >= 0) {                                                       \
-      const double t = warp_sum(grad_y<A, r>(v, w));                                      \
-      if (lane == 0) red[warp][op.slot] += t;                                             \
-    }                                                                                     \
-    apply_ry<A, Real, r, DUAL>(v, w, c, BACKWARD ? -sn : sn);                             \
-    break;
-            ADJ_RY(0) ADJ_RY(1) ADJ_RY(2)
-#undef ADJ_RY
-            default: {  // RZ (diagonal): phases (c -+ i s) keyed on the target bit
-              const uint32_t tkey = op.lt < 0 ? (uint32_t)((tb >> op.qt) & 1ull) : 0u;
-              double gz = 0.0;
+      }
+      if (ti == 0) {  // this state's tables, while the tile is on its way
+        for (int i = tid; i < P.num_segs * 8; i += NT) {
+          const HeaSeg& sg = sseg[i >> 3];
+          HeaTab<Real>& tb = tab[i >> 3];
+          const int k = i & 7;
+          double pr = 1.0, pi = 0.0, scale = 1.0;
+          uint32_t flips = 0;
 #pragma unroll
-              for (int k = 0; k < kG; k++) {
-                uint32_t loc = gb;
+          for (int g = 0; g < 3; g++) {
+            const int p = sg.param[g];
+            double2 y = make_double2(1.0, 0.0), z = make_double2(1.0, 0.0);
+            if (p >= 0) {
+              y = cs[b * P.num_params + p];
+              z = cs[b * P.num_params + p + 1];
+            }
+            // RZ: bit 0 -> c - i s, bit 1 -> c + i s; undone: the conjugate
+            const double zi = ((k >> g & 1) != 0) != BACK ? z.y : -z.y;
+            const double nr = pr * z.x - pi * zi, ni = pr * zi + pi * z.x;
+            pr = nr;
+            pi = ni;
+            // the scale belongs to the rounded t, so that |scale [[1, t], [-t, 1]]| is 1
+            const bool flip = fabs(y.x) < fabs(y.y);
+            const Real t = (Real)(flip ? y.x / y.y : y.y / y.x);
+            const double h = copysign(1.0 / sqrt(1.0 + (double)t * (double)t), flip ? y.y : y.x);
+            scale *= h;
+            if (flip) flips |= 1u << g;
+            if (k == g) tb.t[g] = t;
+          }
+          tb.ph[k] = A{(Real)(scale * pr), (Real)(scale * pi)};
+          if (k == 3) {
+            tb.flip = flips;
+            tb.unscale = 1.0 / (scale * scale);
+          }
+        }
+        if (BACK)
+          for (int i = tid; i < kHeaWarps * nslots; i += NT) red[i] = 0.0;
+      }
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+      __syncthreads();
+      for (int s = 0; s < (work ? P.num_segs : 0); s++) {
+        const HeaSeg& sg = sseg[s];
+        const HeaTab<Real>& tb = tab[s];
+        const uint32_t a0 = sg.alpha[0], a1 = sg.alpha[1], a2 = sg.alpha[2];
+        uint32_t off0 = 0;
+        if (__popc(sg.fun[0] & base) & 1) off0 ^= a0;
+        if (__popc(sg.fun[1] & base) & 1) off0 ^= a1;
+        if (__popc(sg.fun[2] & base) & 1) off0 ^= a2;
 #pragma unroll
-                for (int q = 0; q < kRB; q++)
-                  if (k >> q & 1) loc |= bm[q];
-                const uint32_t key = op.lt < 0 ? tkey : ((loc >> op.lt) & 1u);
-                if (BACKWARD && op.slot >= 0)
-                  gz += (key ? -1.0 : 1.0) * ((double)w[k].x * v[k].y - (double)w[k].y * v[k].x);
-                // forward RZ(theta): key 0 -> c - i s, key 1 -> c + i s; backward: conjugate
-                const Real si = ((key != 0) != BACKWARD) ? sn : -sn;
-                const A ph = {c, si};
+        for (int q = 0; q < 7; q++)
+          if (tid >> q & 1) off0 ^= sg.kappa[q];
+        const uint32_t flip = tb.flip;
+        const Real t0 = tb.t[0], t1 = tb.t[1], t2 = tb.t[2];
+        double acc[8];
+        if (BACK) {
+#pragma unroll
+          for (int i = 0; i < 8; i++) acc[i] = 0.0;
+        }
+        for (uint32_t g0 = 0; g0 < groups; g0 += NT) {
+          const bool active = g0 + tid < groups;
+          uint32_t off = off0;
+#pragma unroll
+          for (int q = 7; q < kMaxHeaBits - 3; q++)
+            if (g0 >> q & 1u) off ^= sg.kappa[q];
+          A v[8], w[8];
+          if (active) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              const unsigned char* at = smem + (off ^ (k & 1 ? a0 : 0u) ^ (k & 2 ? a1 : 0u) ^ (k & 4 ? a2 : 0u));
+              v[k] = *reinterpret_cast<const A*>(at);
+              if (BACK) w[k] = *reinterpret_cast<const A*>(at + tile_bytes);
+            }
+            if (BACK) {
+              // Im(conj(lambda) psi) per amplitude, summed with the sign of each target bit
+              double d[8];
+#pragma unroll
+              for (int k = 0; k < 8; k++) d[k] = (double)w[k].x * v[k].y - (double)w[k].y * v[k].x;
+              const double s0 = d[0] + d[1], s1 = d[2] + d[3], s2 = d[4] + d[5], s3 = d[6] + d[7];
+              acc[0] += ((d[0] - d[1]) + (d[2] - d[3])) + ((d[4] - d[5]) + (d[6] - d[7]));
+              acc[1] += (s0 - s1) + (s2 - s3);
+              acc[2] += (s0 + s1) - (s2 + s3);
+#pragma unroll
+              for (int k = 0; k < 8; k++) {
+                const A ph = tb.ph[k];
                 v[k] = cmul(ph, v[k]);
-                if (DUAL) w[k] = cmul(ph, w[k]);
+                w[k] = cmul(ph, w[k]);
               }
-              if (BACKWARD && op.slot >= 0) {
-                const double t = warp_sum(gz);
-                if (lane == 0) red[warp][op.slot] += t;
-              }
+              acc[3] += hea_grad_y<A, 0>(v, w);
+              acc[4] += hea_grad_y<A, 1>(v, w);
+              acc[5] += hea_grad_y<A, 2>(v, w);
+              hea_ry<A, Real, 0, true>(v, t0, flip & 1u);
+              hea_ry<A, Real, 0, true>(w, t0, flip & 1u);
+              hea_ry<A, Real, 1, true>(v, t1, flip & 2u);
+              hea_ry<A, Real, 1, true>(w, t1, flip & 2u);
+              hea_ry<A, Real, 2, true>(v, t2, flip & 4u);
+              hea_ry<A, Real, 2, true>(w, t2, flip & 4u);
+            } else {
+              hea_ry<A, Real, 0, false>(v, t0, flip & 1u);
+              hea_ry<A, Real, 1, false>(v, t1, flip & 2u);
+              hea_ry<A, Real, 2, false>(v, t2, flip & 4u);
+#pragma unroll
+              for (int k = 0; k < 8; k++) v[k] = cmul(tb.ph[k], v[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              unsigned char* at = smem + (off ^ (k & 1 ? a0 : 0u) ^ (k & 2 ? a1 : 0u) ^ (k & 4 ? a2 : 0u));
+              *reinterpret_cast<A*>(at) = v[k];
+              if (BACK) *reinterpret_cast<A*>(at + tile_bytes) = w[k];
             }
           }
         }
-        if (active) {
+        if (BACK) {
+          // 8 sums over 32 lanes: halve the values with each of the first
+          // three exchanges, then two full ones; lane 4 i ends with value i
+          double h4[4], h2[2], h1;
+          const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
 #pragma unroll
-          for (int k = 0; k < kG; k++) {
-            uint32_t loc = gb;
-#pragma unroll
-            for (int q = 0; q < kRB; q++)
-              if (k >> q & 1) loc |= bm[q];
-            sv[aswz<Real>(loc)] = v[k];
-            if (DUAL) sw[aswz<Real>(loc)] = w[k];
+          for (int i = 0; i < 4; i++) {
+            const double give = b4 ? acc[i] : acc[4 + i], keep = b4 ? acc[4 + i] : acc[i];
+            h4[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
           }
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const double give = b3 ? h4[i] : h4[2 + i], keep = b3 ? h4[2 + i] : h4[i];
+            h2[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+          }
+          const double give = b2 ? h2[0] : h2[1], keep = b2 ? h2[1] : h2[0];
+          h1 = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+          h1 += __shfl_xor_sync(0xffffffffu, h1, 2);
+          h1 += __shfl_xor_sync(0xffffffffu, h1, 1);
+          if ((lane & 3) == 0 && lane < 4 * kHeaSlots) red[warp * nslots + s * kHeaSlots + (lane >> 2)] += h1;
         }
+        __syncthreads();
+      }
+      for (uint32_t u = tid, j = 0; u < units; u += NT, j++) {
+        const uint32_t off = base ^ toff ^ joff[j];
+        const double2* at = reinterpret_cast<const double2*>(smem + tile_swz16(u) * 16u);
+        __stcs(reinterpret_cast<double2*>(gp + off), *at);
+        if (BACK) __stcs(reinterpret_cast<double2*>(gl + off), at[tile_bytes / 16]);
       }
       __syncthreads();
     }
-    store_tile<Real>(sv, psi, tb, rowoff, P.L, amps);
-    if (DUAL) store_tile<Real>(sw, lam, tb, rowoff, P.L, amps);
-    if (BACKWARD) {
-      for (int j = threadIdx.x; j < P.num_slots; j += NT) {
+    if (BACK) {
+      for (int j = tid; j < nslots; j += NT) {
         double t = 0.0;
-        for (int wp = 0; wp < NT / 32; wp++) t += red[wp][j];
-        partials[tile * P.num_slots + j] = t;
+        for (int wp = 0; wp < kHeaWarps; wp++) t += red[wp * nslots + j];
+        if (j % kHeaSlots >= 3) t *= tab[j / kHeaSlots].unscale;
+        partials[item * (uint64_t)part_stride + j] = t;
       }
+      __syncthreads();
     }
-    __syncthreads();
   }
 }
 
@@ -349,19 +437,75 @@ __global__ void __launch_bounds__(AdjCfg<Real>::NT, 1)
   }
 }
 
-// out[b * P + param_of_slot[j]] = sum over the tiles of batch element b of
-// partials[tile][j], in tile order.
-__global__ void k_adj_reduce(const double* __restrict__ partials, uint64_t tiles_per_state, int num_slots,
-                             uint64_t batch, const int* __restrict__ param_of_slot, int num_params,
-                             double* __restrict__ out) {
-  const uint64_t total = batch * (uint64_t)num_slots;
+// d_grads[b][p] = sum over state b's items, in order, of its parameter's slot.
+__global__ void __launch_bounds__(128) k_hea_reduce(const double* __restrict__ partials, uint32_t items,
+                                                    int part_stride, uint64_t batch,
+                                                    const int* __restrict__ slot_of_param, int num_params,
+                                                    double* __restrict__ grads) {
+  const uint64_t total = batch * (uint64_t)num_params;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t b = i / num_slots;
-    const int j = (int)(i % num_slots);
+    const uint64_t b = i / num_params;
+    const double* p = partials + b * items * (uint64_t)part_stride + slot_of_param[i % num_params];
     double s = 0.0;
-    const double* p = partials + b * tiles_per_state * num_slots + j;
-    for (uint64_t t = 0; t < tiles_per_state; t++) s += p[t * num_slots];
-    out[b * num_params + (param_of_slot ? param_of_slot[j] : 0)] = s;
+#pragma unroll 8
+    for (uint32_t t = 0; t < items; t++) s += p[t * (uint64_t)part_stride];
+    grads[i] = s;
+  }
+}
+
+// out[b] = sum over state b's tiles, in order.
+__global__ void k_adj_energy(const double* __restrict__ partials, uint64_t tiles_per_state, uint64_t batch,
+                             double* __restrict__ out) {
+  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < batch; b += (uint64_t)gridDim.x * blockDim.x) {
+    double s = 0.0;
+    for (uint64_t t = 0; t < tiles_per_state; t++) s += partials[b * tiles_per_state + t];
+    out[b] = s;
+  }
+}
+
+// dst[p] = src[C^-k p] on n-bit indices, C^-1 x = x ^ (x << 1): (1 + S)^k
+// over GF(2) is the product of 1 + S^(2^j) over the set bits j of k.
+__host__ __device__ inline uint32_t unladder_index(uint32_t x, int n, int k) {
+  for (int j = 0; (1 << j) < n; j++)
+    if (k >> j & 1) x ^= (x << (1 << j)) & (uint32_t)((1ull << n) - 1ull);
+  return x;
+}
+struct UnladderPass {
+  int32_t n, k, m;
+  uint32_t dst[kUnladderBits];       // dst index part of local bit b
+  uint32_t src[kUnladderBits];       // src index part of load bit b
+  uint32_t src_local[kUnladderBits]; // and its local index part
+  uint64_t free_mask, num_tiles, tiles_per_state;
+};
+// Tiles hold whole rows of both orders: 2^kUnladderLow contiguous amplitudes
+// of src on the way in, of dst on the way out.
+__global__ void __launch_bounds__(256) k_unladder(const float2* __restrict__ src, float2* __restrict__ dst,
+                                                  const __grid_constant__ UnladderPass P) {
+  __shared__ float2 sm[1 << kUnladderBits];
+  const uint32_t amps = 1u << P.m;
+  for (uint64_t tile = blockIdx.x; tile < P.num_tiles; tile += gridDim.x) {
+    const uint64_t b = tile / P.tiles_per_state;
+    const uint32_t base = (uint32_t)pdep64(tile % P.tiles_per_state, P.free_mask);
+    const uint32_t sbase = unladder_index(base, P.n, P.k);
+    for (uint32_t e = threadIdx.x; e < amps; e += 256) {
+      uint32_t off = sbase, t = 0;
+#pragma unroll
+      for (int q = 0; q < kUnladderBits; q++)
+        if (e >> q & 1u) {
+          off ^= P.src[q];
+          t ^= P.src_local[q];
+        }
+      sm[t ^ (t >> 4 & 15u)] = src[(b << P.n) + off];
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < amps; e += 256) {
+      uint32_t off = base;
+#pragma unroll
+      for (int q = 0; q < kUnladderBits; q++)
+        if (e >> q & 1u) off ^= P.dst[q];
+      dst[(b << P.n) + off] = sm[e ^ (e >> 4 & 15u)];
+    }
+    __syncthreads();
   }
 }
 
@@ -372,25 +516,21 @@ __global__ void k_adj_init(typename Cplx<Real>::T* __restrict__ psi, uint64_t di
     psi[i] = ((i % dim) == hf) ? A{1, 0} : A{0, 0};
 }
 
-template <typename Real>
-int launch_gates_t(void* psi, void* lam, const AdjPass& P, const AdjOp* d_ops, const double2* d_cs,
-                   double* d_partials, bool dual, bool backward, int num_sms, cudaStream_t stream) {
+template <typename Real, bool BACK>
+int launch_hea_t(const void* src, void* psi, void* lam, const HeaPass& P, const HeaSeg* d_segs, const double2* d_cs,
+                 double* d_partials, int part_stride, int num_sms, cudaStream_t stream) {
   using A = typename Cplx<Real>::T;
-  const size_t smem = sizeof(A) * ((size_t)(dual ? 2 : 1) << (P.L + P.H));
-  auto launch = [&](auto kern) {
-    // Every instantiation has the same pointer type, so the opt-in is set per
-    // launch (an idempotent attribute write) rather than once per type.
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(2 * sizeof(A) << AdjCfg<Real>::TB));
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, AdjCfg<Real>::NT, smem);
-    uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);
-    if (grid > P.num_tiles) grid = P.num_tiles;
-    kern<<<(unsigned)grid, AdjCfg<Real>::NT, smem, stream>>>((A*)psi, (A*)lam, P, d_ops, d_cs, d_partials);
-  };
-  if (!dual) launch(k_adj_gates<Real, false, false>);
-  else if (backward) launch(k_adj_gates<Real, true, true>);
-  else launch(k_adj_gates<Real, true, false>);
+  const size_t tile = sizeof(A) << P.m;
+  const size_t red = BACK ? sizeof(double) * kHeaWarps * kHeaSlots : 0;
+  const size_t smem = (BACK ? 2 : 1) * tile + P.num_segs * (sizeof(HeaTab<Real>) + red + sizeof(HeaSeg));
+  auto kern = k_hea<Real, BACK>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kHeaThreads, smem);
+  uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);
+  if (grid > P.num_items) grid = P.num_items;
+  kern<<<(unsigned)grid, kHeaThreads, smem, stream>>>((const A*)src, (A*)psi, (A*)lam, P, d_segs, d_cs, d_partials,
+                                                      part_stride);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }
@@ -418,9 +558,10 @@ int launch_pauli_t(const void* psi, void* lam, const AdjPass& P, const AdjTerm* 
 
 }  // namespace
 
-int adj_tile_bits(int dtype, bool dual) {
-  const int tb = dtype == MLB_C128 ? AdjCfg<double>::TB : AdjCfg<float>::TB;
-  return dual ? tb : tb;  // both arrays share the CTA's shared memory at this size
+int adj_tile_bits(int dtype) { return dtype == MLB_C128 ? AdjCfg<double>::TB : AdjCfg<float>::TB; }
+int hea_tile_bits(int dtype, bool backward) {
+  if (dtype == MLB_C128) return backward ? HeaCfg<double>::BACK_BITS : HeaCfg<double>::FWD_BITS;
+  return backward ? HeaCfg<float>::BACK_BITS : HeaCfg<float>::FWD_BITS;
 }
 
 int launch_adj_init(int dtype, void* psi, int n, uint64_t batch, uint64_t hf, cudaStream_t stream) {
@@ -433,13 +574,16 @@ int launch_adj_init(int dtype, void* psi, int n, uint64_t batch, uint64_t hf, cu
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }
 
-int launch_adj_gates(int dtype, void* psi, void* lam, const AdjPass& P, const AdjOp* d_ops, const double2* d_cs,
-                     double* d_partials, bool dual, bool backward, int num_sms, cudaStream_t stream) {
-  if (P.num_ops < 1 || P.num_ops > kMaxAdjOps || P.num_segments > kMaxAdjSegs || P.num_slots > kMaxAdjSlots)
+int launch_hea_pass(int dtype, const void* psi_src, void* psi, void* lam, const HeaPass& P, const HeaSeg* d_segs,
+                    const double2* d_cs, double* d_partials, int part_stride, bool backward, int num_sms,
+                    cudaStream_t stream) {
+  if (P.num_segs < 1 || P.num_segs > kMaxHeaSegs || P.m < 3 || P.m > hea_tile_bits(dtype, backward) || P.n > 30)
     return MLB_ERR_INVALID_ARG;
-  if (dtype == MLB_C128)
-    return launch_gates_t<double>(psi, lam, P, d_ops, d_cs, d_partials, dual, backward, num_sms, stream);
-  return launch_gates_t<float>(psi, lam, P, d_ops, d_cs, d_partials, dual, backward, num_sms, stream);
+  auto run = [&](auto f) {
+    return f(psi_src, psi, lam, P, d_segs, d_cs, d_partials, part_stride, num_sms, stream);
+  };
+  if (dtype == MLB_C128) return backward ? run(launch_hea_t<double, true>) : run(launch_hea_t<double, false>);
+  return backward ? run(launch_hea_t<float, true>) : run(launch_hea_t<float, false>);
 }
 
 int launch_adj_pauli(int dtype, const void* psi, void* lam, const AdjPass& P, const AdjTerm* d_terms,
@@ -450,14 +594,62 @@ int launch_adj_pauli(int dtype, const void* psi, void* lam, const AdjPass& P, co
   return launch_pauli_t<float>(psi, lam, P, d_terms, accumulate, energy, d_epart, num_sms, stream);
 }
 
-int launch_adj_reduce(const double* d_partials, uint64_t tiles_per_state, int num_slots, uint64_t batch,
-                      const int* d_param_of_slot, int num_params, double* d_out, cudaStream_t stream) {
-  const uint64_t total = batch * (uint64_t)num_slots;
+int launch_hea_reduce(const double* d_partials, uint32_t items, int part_stride, uint64_t batch,
+                      const int* d_slot_of_param, int num_params, double* d_grads, cudaStream_t stream) {
+  const uint64_t total = batch * (uint64_t)num_params;
   uint64_t grid = (total + 127) / 128;
   if (grid < 1) grid = 1;
   if (grid > 148ull * 16) grid = 148ull * 16;
-  k_adj_reduce<<<(unsigned)grid, 128, 0, stream>>>(d_partials, tiles_per_state, num_slots, batch, d_param_of_slot,
-                                                   num_params, d_out);
+  k_hea_reduce<<<(unsigned)grid, 128, 0, stream>>>(d_partials, items, part_stride, batch, d_slot_of_param, num_params,
+                                                   d_grads);
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
+}
+
+int launch_adj_energy(const double* d_partials, uint64_t tiles_per_state, uint64_t batch, double* d_out,
+                      cudaStream_t stream) {
+  uint64_t grid = (batch + 31) / 32;
+  if (grid > 148ull * 16) grid = 148ull * 16;
+  k_adj_energy<<<(unsigned)grid, 32, 0, stream>>>(d_partials, tiles_per_state, batch, d_out);
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
+}
+
+int launch_unladder(const void* src, void* dst, int n, int k, uint64_t batch, int num_sms, cudaStream_t stream) {
+  if (n < 3 || n > 30 || batch < 1 || k < 0) return MLB_ERR_INVALID_ARG;
+  UnladderPass P{};
+  P.n = n;
+  P.k = k;
+  P.m = n < kUnladderBits ? n : kUnladderBits;
+  // the tile: rows of dst (low unit vectors), rows of src (C^k e_i), then
+  // low unit vectors; load order: src's rows first
+  hea::Basis B, S;
+  std::vector<uint64_t> load;
+  const int low = P.m < 2 * kUnladderLow ? P.m / 2 : kUnladderLow;
+  for (int i = 0; i < low; i++) B.add(1ull << i);
+  for (int i = 0; i < low; i++) {
+    uint64_t v = 1ull << i;
+    for (int j = 0; j < k; j++) v = hea::ladder(v, n);
+    B.add(v);
+    S.add(v);
+    load.push_back(v);
+  }
+  for (int b = 0; b < n && (int)B.v.size() < P.m; b++) B.add(1ull << b);
+  for (uint64_t v : B.v)
+    if (S.add(v)) load.push_back(v);
+  uint64_t pivots = 0;
+  for (int b = 0; b < P.m; b++) {
+    P.dst[b] = (uint32_t)B.v[b];
+    P.src[b] = unladder_index((uint32_t)load[b], n, k);
+    P.src_local[b] = B.coords(load[b]);
+    pivots |= 1ull << B.piv[b];
+  }
+  P.free_mask = ((1ull << n) - 1ull) & ~pivots;
+  P.tiles_per_state = 1ull << (n - P.m);
+  P.num_tiles = P.tiles_per_state * batch;
+  uint64_t grid = (uint64_t)num_sms * 8;
+  if (grid > P.num_tiles) grid = P.num_tiles;
+  k_unladder<<<(unsigned)grid, 256, 0, stream>>>((const float2*)src, (float2*)dst, P);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }

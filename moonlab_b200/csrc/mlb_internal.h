@@ -114,26 +114,28 @@ __host__ __device__ inline uint32_t tile_swz16(uint32_t e) {
 // Adjoint-gradient passes (kernels_adjoint.cu).  A pass covers a batch of
 // states stored back to back, [B][2^n]; tiles never span two states.
 // ---------------------------------------------------------------------------
-constexpr int kMaxAdjOps = 160;
-constexpr int kMaxAdjSegs = 64;
-constexpr int kMaxAdjSlots = 96;   // parameter gradients accumulated per pass
+enum AdjKind : int32_t { ADJ_KIND_X = 0, ADJ_KIND_RY = 1, ADJ_KIND_RZ = 2 };  // ansatz gates (X: CNOT with a control)
 constexpr int kMaxAdjTerms = 128;  // Pauli terms per lambda pass
-enum AdjKind : int32_t { ADJ_KIND_X = 0, ADJ_KIND_RY = 1, ADJ_KIND_RZ = 2 };
-
-struct AdjOp {
-  int32_t kind;      // ADJ_KIND_*; X with a control mask is CNOT
-  int32_t rt;        // register bit of the target (X, RY)
-  int32_t lt;        // RZ: local bit of the target, -1 when outside the tile
-  int32_t qt;        // RZ: global target qubit (tile-constant key when outside)
-  int32_t p;         // parameter index (RY, RZ), -1 otherwise
-  int32_t slot;      // backward: gradient slot of this pass, -1 none
-  uint32_t lcmask;   // local control mask (CNOT control inside the tile)
-  uint32_t pad;
-  uint64_t ocmask;   // outside control mask (global bits)
+// Rotation passes over linear subspaces of the index space (hea_plan.h).
+constexpr int kMaxHeaSegs = 24;    // segments of a pass (their tables live in shared memory)
+constexpr int kMaxHeaBits = 13;    // bits of a tile
+constexpr int kHeaSlots = 6;       // gradients of a segment: d/dRZ of its three rotations, then d/dRY
+struct HeaSeg {        // up to three commuting rotations (RY, then RZ)
+  uint16_t alpha[3];   // byte offsets in the tile of their directions
+  uint16_t kappa[kMaxHeaBits - 3];  // byte offsets of the groups' basis
+  uint16_t pad;
+  uint32_t fun[3];     // the target bit of base + representative: parity(fun & base)
+  int32_t param[3];    // parameter of the RY (the RZ's is the next); -1: an idle place
 };
-struct AdjSeg {
-  int32_t op_begin, op_end;
-  int32_t bits[3];   // register bits (ascending local bit positions)
+struct HeaPass {
+  int32_t n, m, num_segs, num_params;
+  uint32_t basis[kMaxHeaBits];      // local bit k of an amplitude adds basis[k] to its index
+  int32_t init;                     // the state is |init_index>: nothing is read
+  uint32_t init_base, init_local;   // its tile's base and local index
+  uint64_t free_mask;               // bits that enumerate the tiles of a state
+  uint64_t tiles_per_state;
+  uint32_t items_per_state, tiles_per_item;  // a work item is a run of one state's tiles
+  uint64_t num_items;
 };
 struct AdjTerm {     // one Pauli string restricted to a tile
   uint32_t xl, zl;   // local X / Z masks
@@ -142,19 +144,31 @@ struct AdjTerm {     // one Pauli string restricted to a tile
 };
 struct AdjPass {
   int32_t n, L, H;
-  int32_t num_ops, num_segments, num_slots, num_params;
+  int32_t num_ops;
   int32_t high[kMaxHigh];
   uint64_t tiles_per_state, num_tiles, tile_free_mask;
-  AdjSeg segs[kMaxAdjSegs];
 };
-int adj_tile_bits(int dtype, bool dual);
+int hea_tile_bits(int dtype, bool backward);
+// Rotation pass: psi_src -> psi (the same buffer, or another of the batch's
+// size), and in the backward sweep lam in place and partials[(state *
+// items_per_state + item) * part_stride + slot] for the pass's slots.
+int launch_hea_pass(int dtype, const void* psi_src, void* psi, void* lam, const HeaPass& P, const HeaSeg* d_segs,
+                    const double2* d_cs, double* d_partials, int part_stride, bool backward, int num_sms,
+                    cudaStream_t stream);
+// d_grads[b * num_params + p] = sum over a state's items, in order, of the
+// partials of parameter p's slot.
+int launch_hea_reduce(const double* d_partials, uint32_t items, int part_stride, uint64_t batch,
+                      const int* d_slot_of_param, int num_params, double* d_grads, cudaStream_t stream);
+// d_out[b] = the sum of state b's tiles' energy partials, in order.
+int launch_adj_energy(const double* d_partials, uint64_t tiles_per_state, uint64_t batch, double* d_out,
+                      cudaStream_t stream);
+// complex64: dst[b][p] = src[b][C^-k p], C the CNOT ladder on n qubits
+// (hea_plan.h).
+int launch_unladder(const void* src, void* dst, int n, int k, uint64_t batch, int num_sms, cudaStream_t stream);
+int adj_tile_bits(int dtype);
 int launch_adj_init(int dtype, void* psi, int n, uint64_t batch, uint64_t hf, cudaStream_t stream);
-int launch_adj_gates(int dtype, void* psi, void* lam, const AdjPass& P, const AdjOp* d_ops, const double2* d_cs,
-                     double* d_partials, bool dual, bool backward, int num_sms, cudaStream_t stream);
 int launch_adj_pauli(int dtype, const void* psi, void* lam, const AdjPass& P, const AdjTerm* d_terms,
                      bool accumulate, bool energy, double* d_epart, int num_sms, cudaStream_t stream);
-int launch_adj_reduce(const double* d_partials, uint64_t tiles_per_state, int num_slots, uint64_t batch,
-                      const int* d_param_of_slot, int num_params, double* d_out, cudaStream_t stream);
 // d_norm[b] = |psi_b|^2 of a complex64 batch; then d_out ([B] energies,
 // [B][P] gradients) divided by it.
 int launch_batch_norm(const void* psi_c64, uint64_t dim, uint64_t batch, double* d_norm, cudaStream_t stream);

@@ -1,0 +1,187 @@
+// pauli_plan.h -- plans a sum of Pauli strings as tile passes over linear
+// subspaces of the index space (kernels_pauli.cu).  Host-only.
+//
+// P_k |i> = i^{ny} (-1)^{|i & z|} |i ^ x>: a string pairs i with i ^ x, so a
+// tile base ^ span(u_0 .. u_{m-1}) holds both amplitudes of every string
+// whose X mask lies in the span.  The first L basis vectors are the low unit
+// vectors (rows of 2^L contiguous amplitudes); the others are X masks, chosen
+// to cover as many of the remaining strings as possible, whatever qubits
+// they touch.  Inside a pass, a segment holds groups of 8 amplitudes in
+// registers along three directions and takes the strings whose mask is one
+// of their 8 combinations, so a tile is read once per ~3 masks.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+#include <map>
+#include <vector>
+
+#include "hea_plan.h"
+#include "mlb_internal.h"
+
+namespace mlb {
+namespace pauli {
+
+struct Pass {
+  PauliPass dev{};
+  std::vector<PauliSeg> segs;
+  std::vector<PauliTerm> terms;
+  size_t segs_off = 0, terms_off = 0;  // in the caller's device arrays
+};
+
+// Greedy: the independent masks that, added to V (up to `dims` vectors),
+// bring the most of `masks` (weighted) into its span.
+inline void grow(hea::Basis& V, const std::vector<uint64_t>& masks, const std::vector<int>& weight, int dims) {
+  while ((int)V.v.size() < dims) {
+    // a candidate's gain: the masks equal to it modulo the span
+    std::map<uint64_t, int> gain;
+    for (size_t i = 0; i < masks.size(); i++) {
+      const uint64_t r = V.reduce(masks[i]);
+      if (r) gain[r] += weight[i];
+    }
+    if (gain.empty()) break;
+    // first look one step ahead: with r in, masks a ^ b = r pairs come closer
+    uint64_t best = 0;
+    int most = -1;
+    for (auto& [r, g] : gain) {
+      int ahead = 0;
+      for (auto& [s, gs] : gain)
+        if (s != r && gain.count(s ^ r)) ahead += gs;
+      if (64 * g + ahead > most) {
+        most = 64 * g + ahead;
+        best = r;
+      }
+    }
+    V.add(best);
+  }
+}
+
+// `lambda`: the strings of a lambda pass (out[i ^ x] += c i^{ny} ... in[i]),
+// else of an expectation value.
+inline void plan(int n, int TB, int L, int dtype, size_t num, const uint64_t* xm, const uint64_t* zm,
+                 const double* coeff, bool lambda, std::vector<Pass>& out) {
+  const int m = std::min(n, TB);
+  L = std::min(L, m);
+  std::vector<size_t> rem(num);
+  for (size_t i = 0; i < num; i++) rem[i] = i;
+  std::stable_sort(rem.begin(), rem.end(), [&](size_t a, size_t b) { return xm[a] < xm[b]; });
+  while (!rem.empty()) {
+    std::vector<uint64_t> masks;
+    std::vector<int> weight;
+    for (size_t i : rem)
+      if (xm[i]) {
+        if (masks.empty() || masks.back() != xm[i]) {
+          masks.push_back(xm[i]);
+          weight.push_back(0);
+        }
+        weight.back()++;
+      }
+    hea::Basis V;
+    for (int b = 0; b < L; b++) V.add(1ull << b);
+    grow(V, masks, weight, m);
+    for (int b = 0; b < n && (int)V.v.size() < m; b++) V.add(1ull << b);
+    std::vector<size_t> take, left;
+    for (size_t i : rem) (take.size() < (size_t)kMaxPauliTerms && !V.reduce(xm[i]) ? take : left).push_back(i);
+    Pass P;
+    P.dev.n = n;
+    P.dev.m = m;
+    uint64_t pivots = 0;
+    for (int b = 0; b < m; b++) {
+      P.dev.basis[b] = V.v[b];
+      pivots |= 1ull << V.piv[b];
+    }
+    P.dev.free_mask = ((1ull << n) - 1ull) & ~pivots;
+    P.dev.tiles_per_state = 1ull << (n - m);
+    while (!take.empty()) {
+      // three directions of this segment, in the tile's local coordinates
+      std::vector<uint64_t> loc;
+      std::vector<int> w;
+      for (size_t i : take)
+        if (xm[i]) {
+          const uint64_t t = V.coords(xm[i]);
+          if (loc.empty() || loc.back() != t) {
+            loc.push_back(t);
+            w.push_back(0);
+          }
+          w.back()++;
+        }
+      hea::Basis R;
+      grow(R, loc, w, 3);
+      for (int b = m; b-- > 0 && (int)R.v.size() < 3;) R.add(1ull << b);
+      PauliSeg s{};
+      for (int i = 0; i < 3; i++) s.alpha[i] = (uint16_t)hea::slot_bytes((uint32_t)R.v[i], dtype);
+      // groups: a complement of the three directions, lanes on distinct banks first
+      std::vector<uint32_t> comp, order;
+      {
+        hea::Basis full = R;
+        for (int b = 0; b < m; b++)
+          if (full.add(1ull << b)) comp.push_back(1u << b);
+      }
+      hea::Basis banks, chosen;
+      const int want = dtype == MLB_C128 ? 3 : 4;
+      for (uint32_t mix = 1; mix < (1u << comp.size()) && (int)order.size() < want; mix++) {
+        if (__builtin_popcount(mix) > 3) continue;
+        uint32_t t = 0;
+        for (size_t i = 0; i < comp.size(); i++)
+          if (mix >> i & 1u) t ^= comp[i];
+        hea::Basis nb = banks, nc = chosen;
+        if (nb.add(hea::bank_of(t, dtype)) && nc.add(t)) {
+          banks = nb;
+          chosen = nc;
+          order.push_back(t);
+        }
+      }
+      for (uint32_t t : comp)
+        if (chosen.add(t)) order.push_back(t);
+      for (size_t i = 0; i < order.size(); i++) s.kappa[i] = (uint16_t)hea::slot_bytes(order[i], dtype);
+      auto global = [&](uint64_t t) {
+        uint64_t g = 0;
+        for (int b = 0; b < m; b++)
+          if (t >> b & 1ull) g ^= V.v[b];
+        return g;
+      };
+      s.term_begin = (int)P.terms.size();
+      std::vector<size_t> later;
+      for (size_t i : take) {
+        const uint64_t t = V.coords(xm[i]);
+        if (R.reduce(t)) {
+          later.push_back(i);
+          continue;
+        }
+        PauliTerm d{};
+        d.z = zm[i];
+        d.kap = (uint8_t)R.coords(t);
+        for (int k = 0; k < 8; k++) {
+          uint64_t g = 0;
+          for (int j = 0; j < 3; j++)
+            if (k >> j & 1) g ^= global(R.v[j]);
+          if (hea::parity(g & zm[i])) d.pat |= (uint8_t)(1u << k);
+        }
+        for (size_t j = 0; j < order.size(); j++)
+          if (hea::parity(global(order[j]) & zm[i])) d.zg |= (uint16_t)(1u << j);
+        const int ny = __builtin_popcountll(xm[i] & zm[i]) & 3;
+        const double c = coeff ? coeff[i] : 1.0;
+        d.odd = (uint8_t)(ny & 1);
+        if (lambda) {
+          // the source's sign, (-1)^{|i & z|}, seen from the target i ^ x: (-1)^{ny} times it;
+          // i^{ny}: 1, i, -1, -i
+          d.c = ny == 1 || ny == 2 ? -c : c;
+        } else {
+          // both members of a pair, i the one kept: 2 s(i) {re, -im, -re, im}
+          d.c = (xm[i] ? 2.0 : 1.0) * (ny == 1 || ny == 2 ? -c : c);
+        }
+        P.terms.push_back(d);
+      }
+      s.term_end = (int)P.terms.size();
+      P.segs.push_back(s);
+      take.swap(later);
+    }
+    P.dev.num_segs = (int)P.segs.size();
+    P.dev.num_terms = (int)P.terms.size();
+    out.push_back(std::move(P));
+    rem.swap(left);
+  }
+}
+
+}  // namespace pauli
+}  // namespace mlb
