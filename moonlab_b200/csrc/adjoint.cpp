@@ -34,6 +34,7 @@
 #include "fused.h"
 #include "hea_plan.h"
 #include "mlb_internal.h"
+#include "pauli_plan.h"
 #include "planner.h"
 
 using namespace mlb;
@@ -59,12 +60,6 @@ struct TapeOp {
   int p;
 };
 
-struct TermPass {
-  AdjPass P;
-  std::vector<AdjTerm> terms;
-  size_t terms_off = 0;
-};
-
 }  // namespace
 
 struct mlb_hea {
@@ -87,7 +82,7 @@ struct mlb_hea {
   size_t ckpt_cap = 0;       // bytes
   int last_ckpt = 0;
   size_t last_chunks = 0;
-  std::vector<TermPass> lam;
+  std::vector<pauli::Pass> lam;
   cudaStream_t stream = nullptr;
   // device buffers
   void* psi = nullptr;
@@ -100,7 +95,8 @@ struct mlb_hea {
   double* d_epart = nullptr;
   size_t epart_cap = 0;
   HeaSeg* d_segs = nullptr;
-  AdjTerm* d_terms = nullptr;
+  PauliTerm* d_terms = nullptr;
+  PauliSeg* d_psegs = nullptr;
   int* d_slots = nullptr;  // slot of each parameter
   double* d_out = nullptr;  // [B] energies then [B][P] grads
   size_t out_cap = 0;
@@ -203,67 +199,6 @@ HeaPass pass_for_batch(const hea::Pass& p, size_t B) {
   return P;
 }
 
-// Partition the Pauli terms into lambda passes: a term fits a pass when its
-// X-part lies inside the tile (Z-part may lie anywhere).  Terms commute in
-// the sum, so no ordering constraint applies.
-void plan_terms(mlb_hea* h) {
-  const int TB = adj_tile_bits(h->dtype);
-  const int n = (int)h->n;
-  const int L = n <= TB ? n : 5;
-  const int Hmax = n <= TB ? 0 : TB - L;
-  const uint64_t lowm = (1ull << L) - 1ull;
-  std::vector<int> rem(h->xm.size());
-  for (size_t i = 0; i < rem.size(); i++) rem[i] = (int)i;
-  while (!rem.empty()) {
-    uint64_t SH = 0;
-    std::vector<int> taken, left;
-    for (int t : rem) {
-      const uint64_t need = h->xm[t] & ~lowm & ~SH;
-      if ((int)taken.size() < kMaxAdjTerms && __builtin_popcountll(SH | need) <= Hmax) {
-        SH |= need;
-        taken.push_back(t);
-      } else {
-        left.push_back(t);
-      }
-    }
-    TermPass tp{};
-    AdjPass& P = tp.P;
-    P.n = n;
-    P.L = L;
-    int local_of[64];
-    for (int q = 0; q < 64; q++) local_of[q] = q < L ? q : -1;
-    int H = 0;
-    for (int q = L; q < n; q++)
-      if (SH >> q & 1ull) {
-        P.high[H] = q;
-        local_of[q] = L + H;
-        H++;
-      }
-    P.H = H;
-    const uint64_t allm = (1ull << n) - 1ull;
-    P.tile_free_mask = allm & ~(((1ull << L) - 1ull) | SH);
-    P.tiles_per_state = 1ull << (n - L - H);
-    for (int t : taken) {
-      AdjTerm a{};
-      for (int b = 0; b < n; b++) {
-        if (h->xm[t] >> b & 1ull) a.xl |= 1u << local_of[b];
-        if (h->zm[t] >> b & 1ull) {
-          if (local_of[b] >= 0) a.zl |= 1u << local_of[b];
-          else a.zo |= 1ull << b;
-        }
-      }
-      const int ny = __builtin_popcountll(h->xm[t] & h->zm[t]) & 3;
-      const double c = h->coeff[t];
-      a.cr = ny == 0 ? c : ny == 2 ? -c : 0.0;
-      a.ci = ny == 1 ? c : ny == 3 ? -c : 0.0;
-      tp.terms.push_back(a);
-    }
-    P.num_ops = (int)tp.terms.size();
-    h->lam.push_back(std::move(tp));
-    rem.swap(left);
-  }
-}
-
 // Fused plans of the forward sweep (complex64, N >= 13): each segment's gates
 // grouped into <= 5-qubit blocks and tile passes by the fused planner (on
 // stand-in ops: only their qubits matter), each block's gates recorded in
@@ -338,18 +273,23 @@ int upload_programs(mlb_hea* h) {
       h->num_slots += kHeaSlots;
     }
   }
-  std::vector<AdjTerm> all_terms;
-  for (auto& tp : h->lam) {
-    tp.terms_off = all_terms.size();
-    all_terms.insert(all_terms.end(), tp.terms.begin(), tp.terms.end());
+  std::vector<PauliTerm> all_terms;
+  std::vector<PauliSeg> all_psegs;
+  for (auto& p : h->lam) {
+    p.terms_off = all_terms.size();
+    p.segs_off = all_psegs.size();
+    all_terms.insert(all_terms.end(), p.terms.begin(), p.terms.end());
+    all_psegs.insert(all_psegs.end(), p.segs.begin(), p.segs.end());
   }
   cudaError_t e = cudaMalloc((void**)&h->d_segs, all_segs.size() * sizeof(HeaSeg));
   if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_slots, slot_of_param.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_terms, std::max<size_t>(1, all_terms.size()) * sizeof(AdjTerm));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_terms, all_terms.size() * sizeof(PauliTerm));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_psegs, all_psegs.size() * sizeof(PauliSeg));
   if (e != cudaSuccess) return cfail(e, "adjoint program upload");
   cudaMemcpy(h->d_segs, all_segs.data(), all_segs.size() * sizeof(HeaSeg), cudaMemcpyHostToDevice);
   cudaMemcpy(h->d_slots, slot_of_param.data(), slot_of_param.size() * sizeof(int), cudaMemcpyHostToDevice);
-  e = cudaMemcpy(h->d_terms, all_terms.data(), all_terms.size() * sizeof(AdjTerm), cudaMemcpyHostToDevice);
+  cudaMemcpy(h->d_terms, all_terms.data(), all_terms.size() * sizeof(PauliTerm), cudaMemcpyHostToDevice);
+  e = cudaMemcpy(h->d_psegs, all_psegs.data(), all_psegs.size() * sizeof(PauliSeg), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cfail(e, "adjoint program upload");
   if (h->fused_ok) {
     e = cudaMalloc((void**)&h->d_fblocks, h->fblocks.size() * sizeof(FusedBlockDev));
@@ -410,8 +350,7 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
       h->ckpt_cap = need;
     }
   }
-  size_t max_tiles = 1;
-  for (auto& tp : h->lam) max_tiles = std::max(max_tiles, tp.P.tiles_per_state * B);
+  const size_t max_tiles = h->lam[0].dev.tiles_per_state * B;  // every lambda pass's tile has the same size
   const uint32_t items = pass_for_batch(h->bwd[0], B).items_per_state;
   if (h_G && (rc = grow(h->d_part, h->part_cap, (size_t)items * B * h->num_slots))) return rc;
   if ((rc = grow(h->d_epart, h->epart_cap, max_tiles))) return rc;
@@ -476,11 +415,12 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
   }
   // 3. lambda = H psi and the energies
   for (size_t k = 0; k < h->lam.size(); k++) {
-    AdjPass P = h->lam[k].P;
+    PauliPass P = h->lam[k].dev;
     P.num_tiles = P.tiles_per_state * B;
     const bool last = k + 1 == h->lam.size();
-    if ((rc = launch_adj_pauli(h->dtype, h->psi, h->lamb, P, h->d_terms + h->lam[k].terms_off, k > 0, last,
-                               h->d_epart, h->num_sms, h->stream)))
+    if ((rc = launch_pauli_apply(h->dtype, h->psi, h->lamb, P, h->d_psegs + h->lam[k].segs_off,
+                                 h->d_terms + h->lam[k].terms_off, k > 0, last ? h->d_epart : nullptr, h->num_sms,
+                                 h->stream)))
       return hfail(rc, "lambda pass");
     if (last && (rc = launch_adj_energy(h->d_epart, P.tiles_per_state, B, h->d_out, h->stream)))
       return hfail(rc, "energy reduce");
@@ -691,7 +631,8 @@ int mlb_hea_create(uint32_t n, uint32_t layers, uint64_t hf, size_t num_terms, c
   }
   for (auto* vec : {&h->fwd, &h->bwd})
     for (auto& p : *vec) p.dev.num_params = (int)h->P;
-  plan_terms(h);
+  pauli::plan((int)h->n, pauli_tile_bits(dtype, true), dtype == MLB_C128 ? 2 : 3, dtype, h->xm.size(), h->xm.data(),
+              h->zm.data(), h->coeff.data(), true, h->lam);
   // the tensor-core forward sweep's plans (used by complex64 problems by default)
   if (dtype == MLB_C64 && h->n == n && n >= (uint32_t)fused::kTileBits) {
     h->fused_ok = plan_fused_forward(h, cut);
@@ -720,7 +661,7 @@ void mlb_hea_free(mlb_hea_t* h) {
   Guard g(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : {h->psi, h->lamb, h->ckpt, (void*)h->d_cs, (void*)h->d_part, (void*)h->d_epart,
-                  (void*)h->d_segs, (void*)h->d_terms, (void*)h->d_slots, (void*)h->d_out, (void*)h->d_gram,
+                  (void*)h->d_segs, (void*)h->d_terms, (void*)h->d_psegs, (void*)h->d_slots, (void*)h->d_out, (void*)h->d_gram,
                   (void*)h->d_fblocks, (void*)h->d_gblocks, (void*)h->d_gops, (void*)h->d_images,
                   (void*)h->d_ferr, (void*)h->d_norm})
     if (p) cudaFree(p);

@@ -25,6 +25,7 @@
 #include "dense.h"
 #include "fused.h"
 #include "mlb_internal.h"
+#include "pauli_plan.h"
 #include "planner.h"
 
 extern "C" {
@@ -1218,45 +1219,58 @@ int mlb_expect_pauli_sum(mlb_state_t* s, size_t num_terms, const uint64_t* xm, c
   DeviceGuard dg(s->device);
   int rc = flush_impl(s);
   if (rc) return rc;
-  // group terms by X mask (<= 16 per launch)
-  std::vector<size_t> order(num_terms);
-  for (size_t i = 0; i < num_terms; i++) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return xm[a] < xm[b]; });
-  const size_t need = sizeof(double) * ((size_t)s->num_sms * 8 * 16 + 64) + 64 * (sizeof(uint64_t) + sizeof(int)) + 256;
-  rc = ensure_scratch(s, need);
-  if (rc) return rc;
-  std::vector<double> vals(num_terms, 0.0);
-  double* d_terms = s->d_scratch;
-  uint64_t* d_z = reinterpret_cast<uint64_t*>(s->d_scratch + 16);
-  int* d_ny = reinterpret_cast<int*>(s->d_scratch + 32);
-  double* d_parts = s->d_scratch + 64;
-  size_t i = 0;
-  while (i < num_terms) {
-    const uint64_t x = xm[order[i]];
-    size_t j = i;
-    uint64_t hz[16];
-    int hny[16];
-    while (j < num_terms && xm[order[j]] == x && j - i < 16) {
-      hz[j - i] = zm[order[j]];
-      hny[j - i] = popc(xm[order[j]] & zm[order[j]]);
-      j++;
+  *out = 0.0;
+  if (num_terms == 0) return MLB_OK;
+  // one upload (through the plan buffers), the passes' kernels, one result
+  std::vector<pauli::Pass> passes;
+  std::vector<unsigned char> blob;
+  auto put = [&](const void* p, size_t bytes) {
+    const size_t at = (blob.size() + 15) & ~(size_t)15;
+    blob.resize(at + bytes);
+    std::memcpy(blob.data() + at, p, bytes);
+    return at;
+  };
+  size_t xoff = 0, zoff = 0, coff = 0;
+  if (s->n < 3) {
+    std::vector<double> ones;
+    if (!coeffs) ones.assign(num_terms, 1.0);
+    xoff = put(xm, num_terms * sizeof(uint64_t));
+    zoff = put(zm, num_terms * sizeof(uint64_t));
+    coff = put(coeffs ? coeffs : ones.data(), num_terms * sizeof(double));
+  } else {
+    pauli::plan((int)s->n, pauli_tile_bits(s->dtype, false), s->dtype == MLB_C128 ? 2 : 3, s->dtype, num_terms, xm, zm,
+                coeffs, false, passes);
+    for (auto& p : passes) {
+      p.terms_off = put(p.terms.data(), p.terms.size() * sizeof(PauliTerm));
+      p.segs_off = put(p.segs.data(), p.segs.size() * sizeof(PauliSeg));
     }
-    const int cnt = (int)(j - i);
-    cudaMemcpyAsync(d_z, hz, cnt * sizeof(uint64_t), cudaMemcpyHostToDevice, s->stream);
-    cudaMemcpyAsync(d_ny, hny, cnt * sizeof(int), cudaMemcpyHostToDevice, s->stream);
-    rc = launch_pauli_group(s->dtype, s->amp, (int)s->n, x, cnt, d_z, d_ny, d_terms, d_parts, s->num_sms, s->stream);
-    if (rc) return fail(rc, "pauli launch");
-    double hv[16];
-    cudaMemcpyAsync(hv, d_terms, cnt * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
-    rc = sync_stream(s);
-    if (rc) return rc;
-    for (int k = 0; k < cnt; k++) vals[order[i + k]] = hv[k];
-    i = j;
   }
-  double acc = 0.0;
-  for (size_t t = 0; t < num_terms; t++) acc += (coeffs ? coeffs[t] : 1.0) * vals[t];
-  *out = acc;
-  return MLB_OK;
+  const size_t per_pass = (size_t)s->num_sms * kPauliCtasPerSm;
+  rc = ensure_scratch(s, sizeof(double) * (1 + std::max<size_t>(1, passes.size()) * per_pass));
+  if (rc) return rc;
+  rc = upload_plan(s, blob.data(), blob.size());
+  if (rc) return rc;
+  const unsigned char* d = static_cast<const unsigned char*>(s->d_plan);
+  double* d_parts = s->d_scratch + 1;
+  int count = 0;
+  if (s->n < 3) {
+    rc = launch_pauli_tiny(s->dtype, s->amp, (int)s->n, (int)num_terms, reinterpret_cast<const uint64_t*>(d + xoff),
+                           reinterpret_cast<const uint64_t*>(d + zoff), reinterpret_cast<const double*>(d + coff),
+                           d_parts, s->stream);
+    count = 1;
+  }
+  for (size_t k = 0; !rc && k < passes.size(); k++) {
+    int parts = 0;
+    rc = launch_pauli_sum(s->dtype, s->amp, passes[k].dev, reinterpret_cast<const PauliSeg*>(d + passes[k].segs_off),
+                          reinterpret_cast<const PauliTerm*>(d + passes[k].terms_off), d_parts + count, s->num_sms,
+                          s->stream, &parts);
+    count += parts;
+  }
+  if (!rc) rc = launch_sum_partials(d_parts, count, s->d_scratch, s->stream);
+  if (rc) return fail(rc, "pauli launch");
+  cudaError_t e = cudaMemcpyAsync(out, s->d_scratch, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "pauli readback");
+  return sync_stream(s);
 }
 int mlb_expect_pauli(mlb_state_t* s, uint64_t xmask, uint64_t zmask, double* out) {
   const double one = 1.0;

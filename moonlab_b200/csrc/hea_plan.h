@@ -106,6 +106,27 @@ inline uint32_t bank_of(uint32_t t, int dtype) {
   return dtype == MLB_C128 ? (b >> 4) & 7u : (b >> 3) & 15u;
 }
 
+// A basis of span(vecs) whose first vectors (the lanes of one access phase)
+// reach distinct bank groups where the span allows.
+inline std::vector<uint32_t> bank_order(const std::vector<uint32_t>& vecs, int dtype) {
+  const int want = dtype == MLB_C128 ? 3 : 4;
+  std::vector<uint32_t> order;
+  Basis banks, chosen;
+  for (uint32_t mix = 1; mix < (1u << vecs.size()) && (int)order.size() < want; mix++) {
+    if (__builtin_popcount(mix) > 3) continue;
+    uint32_t t = 0;
+    for (size_t i = 0; i < vecs.size(); i++)
+      if (mix >> i & 1u) t ^= vecs[i];
+    if (!banks.reduce(bank_of(t, dtype)) || !chosen.reduce(t)) continue;
+    banks.add(bank_of(t, dtype));
+    chosen.add(t);
+    order.push_back(t);
+  }
+  for (uint32_t t : vecs)
+    if (chosen.add(t)) order.push_back(t);
+  return order;
+}
+
 // One segment: the rotations `rot` (at most 3, mutually commuting) in the
 // pass's local coordinates.
 inline HeaSeg lower_segment(const std::vector<const Rot*>& rot, const Basis& B, int m, int dtype) {
@@ -153,23 +174,7 @@ inline HeaSeg lower_segment(const std::vector<const Rot*>& rot, const Basis& B, 
       if (rho[i] >> b & 1u) t ^= al[i];
     if (kb.add(t)) ker.push_back(t);
   }
-  const int want = dtype == MLB_C128 ? 3 : 4;
-  std::vector<uint32_t> order;
-  Basis banks, chosen;
-  for (uint32_t mix = 1; mix < (1u << ker.size()) && (int)order.size() < want; mix++) {
-    if (__builtin_popcount(mix) > 3) continue;
-    uint32_t t = 0;
-    for (size_t i = 0; i < ker.size(); i++)
-      if (mix >> i & 1u) t ^= ker[i];
-    Basis nb = banks, nc = chosen;
-    if (nb.add(bank_of(t, dtype)) && nc.add(t)) {
-      banks = nb;
-      chosen = nc;
-      order.push_back(t);
-    }
-  }
-  for (uint32_t t : ker)
-    if (chosen.add(t)) order.push_back(t);
+  const std::vector<uint32_t> order = bank_order(ker, dtype);
   for (size_t i = 0; i < order.size(); i++) s.kappa[i] = (uint16_t)slot_bytes(order[i], dtype);
   return s;
 }

@@ -15,9 +15,8 @@
 // Kernels (all tile passes, one HBM read + write of each array per pass):
 //   k_hea       : rotations on psi (forward) or on psi and lambda together
 //                 with the per-parameter partial inner products (backward).
-//   k_adj_pauli : lambda (+)= sum_k c_k P_k psi for the Pauli terms whose
-//                 X-part lies inside the tile; the last pass also emits the
-//                 per-tile partial of Re<psi|lambda> (the energy).
+//   k_pauli_apply (kernels_pauli.cu): lambda = H psi and the per-tile
+//                 partials of the energy.
 //   k_hea_reduce, k_adj_energy: fixed-order sums of the partials
 //                 (deterministic, and the same for every batch size).
 //   k_unladder  : a complex64 batch from the index order of a layer boundary
@@ -34,50 +33,7 @@ namespace mlb {
 
 namespace {
 
-template <typename Real> struct AdjCfg;
-template <> struct AdjCfg<double> { static constexpr int TB = 11, NT = 256, SW_SHIFT = 3, SW_MASK = 7; };
-template <> struct AdjCfg<float> { static constexpr int TB = 12, NT = 256, SW_SHIFT = 4, SW_MASK = 15; };
-
 constexpr int kUnladderBits = 11, kUnladderLow = 4;  // tile of k_unladder, contiguous bits of its rows
-
-template <typename Real>
-__device__ __forceinline__ uint32_t aswz(uint32_t e) {
-  return e ^ ((e >> AdjCfg<Real>::SW_SHIFT) & AdjCfg<Real>::SW_MASK);
-}
-
-__device__ __forceinline__ uint64_t tile_base_of(const AdjPass& P, uint64_t tile) {
-  const uint64_t b = tile / P.tiles_per_state, t = tile % P.tiles_per_state;
-  return (b << P.n) | pdep64(t, P.tile_free_mask);
-}
-
-// HBM -> shared by asynchronous copies: every load of the tile is in flight
-// at once (a load-then-store loop would wait out each load's latency in
-// turn).  The caller completes them with tile_loads_wait() and a barrier.
-template <typename Real>
-__device__ __forceinline__ void load_tile(typename Cplx<Real>::T* __restrict__ sm,
-                                          const typename Cplx<Real>::T* __restrict__ g,
-                                          uint64_t tile_base, const uint64_t* rowoff, int L, uint32_t amps) {
-  using A = typename Cplx<Real>::T;
-  constexpr int NT = AdjCfg<Real>::NT;
-  const uint32_t lm = (1u << L) - 1u;
-  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
-#pragma unroll 1
-  for (uint32_t e = threadIdx.x; e < amps; e += NT) {
-    const A* src = &g[tile_base | rowoff[e >> L] | (e & lm)];
-    const uint32_t dst = base + aswz<Real>(e) * (uint32_t)sizeof(A);
-    if constexpr (sizeof(A) == 16)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-    else
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
-  }
-}
-__device__ __forceinline__ void tile_loads_wait() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // ---------------------------------------------------------------------------
 // rotation passes
@@ -367,76 +323,6 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
   }
 }
 
-// ---------------------------------------------------------------------------
-// lambda (+)= sum_k c_k P_k psi, P_k|i> = i^{ny} (-1)^{|i & z|} |i ^ x>
-// ---------------------------------------------------------------------------
-template <typename Real>
-__global__ void __launch_bounds__(AdjCfg<Real>::NT, 1)
-    k_adj_pauli(const typename Cplx<Real>::T* __restrict__ psi, typename Cplx<Real>::T* __restrict__ lam,
-                const AdjPass P, const AdjTerm* __restrict__ terms, int accumulate, int want_energy,
-                double* __restrict__ energy_partials) {
-  using A = typename Cplx<Real>::T;
-  constexpr int NT = AdjCfg<Real>::NT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const uint32_t amps = 1u << (P.L + P.H);
-  A* sv = reinterpret_cast<A*>(smem_raw);
-  __shared__ uint64_t rowoff[1 << (AdjCfg<Real>::TB - 5)];
-  __shared__ AdjTerm st[kMaxAdjTerms];
-  __shared__ double red[NT / 32];
-  for (uint32_t r = threadIdx.x; r < (1u << P.H); r += NT) {
-    uint64_t off = 0;
-#pragma unroll
-    for (int k = 0; k < kMaxHigh; k++)
-      if (k < P.H && (r >> k & 1u)) off |= 1ull << P.high[k];
-    rowoff[r] = off;
-  }
-  for (int t = threadIdx.x; t < P.num_ops; t += NT) st[t] = terms[t];
-  __syncthreads();
-  const uint32_t lm = (1u << P.L) - 1u;
-  for (uint64_t tile = blockIdx.x; tile < P.num_tiles; tile += gridDim.x) {
-    const uint64_t tb = tile_base_of(P, tile);
-    load_tile<Real>(sv, psi, tb, rowoff, P.L, amps);
-    tile_loads_wait();
-    __syncthreads();
-    double e_acc = 0.0;
-    for (uint32_t e = threadIdx.x; e < amps; e += NT) {
-      double ax = 0.0, ay = 0.0;
-      for (int t = 0; t < P.num_ops; t++) {
-        const AdjTerm& T = st[t];
-        const uint32_t src = e ^ T.xl;
-        const A a = sv[aswz<Real>(src)];
-        // sign from the source index: local part plus the tile-constant part
-        const int par = (__popc(src & T.zl) + (int)__popcll(tb & T.zo)) & 1;
-        const double cr = par ? -T.cr : T.cr, ci = par ? -T.ci : T.ci;
-        ax += cr * a.x - ci * a.y;
-        ay += cr * a.y + ci * a.x;
-      }
-      const uint64_t gidx = tb | rowoff[e >> P.L] | (e & lm);
-      if (accumulate) {
-        const A old = lam[gidx];
-        ax += old.x;
-        ay += old.y;
-      }
-      lam[gidx] = A{(Real)ax, (Real)ay};
-      if (want_energy) {
-        const A p = sv[aswz<Real>(e)];
-        e_acc += (double)p.x * (Real)ax + (double)p.y * (Real)ay;  // Re(conj(psi) lambda)
-      }
-    }
-    if (want_energy) {
-      const double t = warp_sum(e_acc);
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < NT / 32; w++) s += red[w];
-        energy_partials[tile] = s;
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // d_grads[b][p] = sum over state b's items, in order, of its parameter's slot.
 __global__ void __launch_bounds__(128) k_hea_reduce(const double* __restrict__ partials, uint32_t items,
                                                     int part_stride, uint64_t batch,
@@ -535,30 +421,8 @@ int launch_hea_t(const void* src, void* psi, void* lam, const HeaPass& P, const 
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }
 
-template <typename Real>
-int launch_pauli_t(const void* psi, void* lam, const AdjPass& P, const AdjTerm* d_terms, bool accumulate,
-                   bool energy, double* d_epart, int num_sms, cudaStream_t stream) {
-  using A = typename Cplx<Real>::T;
-  const size_t smem = sizeof(A) << (P.L + P.H);
-  static bool set = false;
-  if (!set) {
-    cudaFuncSetAttribute(k_adj_pauli<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(A) << AdjCfg<Real>::TB));
-    set = true;
-  }
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_pauli<Real>, AdjCfg<Real>::NT, smem);
-  uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);
-  if (grid > P.num_tiles) grid = P.num_tiles;
-  k_adj_pauli<Real><<<(unsigned)grid, AdjCfg<Real>::NT, smem, stream>>>((const A*)psi, (A*)lam, P, d_terms,
-                                                                       accumulate ? 1 : 0, energy ? 1 : 0, d_epart);
-  count_launch();
-  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
-}
-
 }  // namespace
 
-int adj_tile_bits(int dtype) { return dtype == MLB_C128 ? AdjCfg<double>::TB : AdjCfg<float>::TB; }
 int hea_tile_bits(int dtype, bool backward) {
   if (dtype == MLB_C128) return backward ? HeaCfg<double>::BACK_BITS : HeaCfg<double>::FWD_BITS;
   return backward ? HeaCfg<float>::BACK_BITS : HeaCfg<float>::FWD_BITS;
@@ -584,14 +448,6 @@ int launch_hea_pass(int dtype, const void* psi_src, void* psi, void* lam, const 
   };
   if (dtype == MLB_C128) return backward ? run(launch_hea_t<double, true>) : run(launch_hea_t<double, false>);
   return backward ? run(launch_hea_t<float, true>) : run(launch_hea_t<float, false>);
-}
-
-int launch_adj_pauli(int dtype, const void* psi, void* lam, const AdjPass& P, const AdjTerm* d_terms,
-                     bool accumulate, bool energy, double* d_epart, int num_sms, cudaStream_t stream) {
-  if (P.num_ops < 1 || P.num_ops > kMaxAdjTerms) return MLB_ERR_INVALID_ARG;
-  if (dtype == MLB_C128)
-    return launch_pauli_t<double>(psi, lam, P, d_terms, accumulate, energy, d_epart, num_sms, stream);
-  return launch_pauli_t<float>(psi, lam, P, d_terms, accumulate, energy, d_epart, num_sms, stream);
 }
 
 int launch_hea_reduce(const double* d_partials, uint32_t items, int part_stride, uint64_t batch,

@@ -1,0 +1,421 @@
+// kernels_pauli.cu -- sums of Pauli strings in tile passes over linear
+// subspaces of the index space (planned by pauli_plan.h).
+//
+//   k_pauli_sum   : partials of sum_k c_k <psi|P_k|psi>, one per CTA.
+//   k_pauli_apply : lambda (+)= sum_k c_k P_k psi for a batch of states; the
+//                   last pass also emits the per-tile partial of
+//                   Re<psi|lambda> (the energy).
+//
+// A tile holds both amplitudes of every pair of its strings, whatever qubits
+// they touch: its basis is the strings' X masks beside the low unit vectors.
+// The 16-byte units of a tile come by cp.async, all in flight at once.  A
+// thread keeps 8 amplitudes per segment in registers along three masks, so
+// one shared-memory read serves up to 7 masks, and the strings' signs are
+// one bit pattern over the register index, one functional of the group
+// index and one sign per tile (folded into the coefficient table).
+// Bound: HBM for few strings; the FP64 products (two or three multiply-adds
+// per pair and string) and their issue for many.  Three CTAs per SM overlap
+// one's copies with the others' sums.
+// Measured: norm, <Z>, 58 random one- and two-local strings and 4096 samples
+// of a 29-qubit complex128 state 68.1 -> 28.6 ms (one pass over the state per
+// distinct X mask before, three passes for all of them now); lambda = H psi
+// of 80 strings on 256 states of 20 qubits: the whole gradient 134 -> 107 ms.
+#include "kernels_common.cuh"
+#include "mlb_internal.h"
+
+namespace mlb {
+
+namespace {
+
+constexpr int kSumThreads = 128, kApplyThreads = 128;
+constexpr int kMaxUnitSteps = 64;  // units of a tile per thread
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ double flip_sign(double c, uint32_t bit) {  // bit in 0/1
+  return __hiloint2double(__double2hiint(c) ^ (int)(bit << 31), __double2loint(c));
+}
+
+// A tile's index offsets: unit tid + j NT adds toff ^ joff[j] to the base.
+template <int NT, int UB>
+struct UnitOffsets {
+  static_assert(NT == 128, "seven thread bits");
+  uint64_t toff;
+  __device__ __forceinline__ void init(const PauliPass& P, uint64_t* joff) {
+    constexpr int TB = 7;
+    for (uint32_t j = threadIdx.x; j < kMaxUnitSteps; j += NT) {
+      uint64_t off = 0;
+#pragma unroll
+      for (int b = TB; b < kMaxPauliBits - UB; b++)
+        if (b + UB < P.m && (j >> (b - TB) & 1u)) off ^= P.basis[b + UB];
+      joff[j] = off;
+    }
+    toff = 0;
+#pragma unroll
+    for (int b = 0; b < TB; b++)
+      if (b + UB < P.m && (threadIdx.x >> b & 1u)) toff ^= P.basis[b + UB];
+  }
+};
+
+// Byte offset of group gi in the tile: tid's bits here, the loop's by the caller.
+template <int TB>
+__device__ __forceinline__ uint32_t group_lane_offset(const PauliSeg& s) {
+  uint32_t off = 0;
+#pragma unroll
+  for (int q = 0; q < TB; q++)
+    if (threadIdx.x >> q & 1u) off ^= s.kappa[q];
+  return off;
+}
+template <int TB>
+__device__ __forceinline__ uint32_t group_step_offset(const PauliSeg& s, uint32_t g0) {
+  uint32_t off = 0;
+#pragma unroll
+  for (int q = TB; q < kMaxPauliBits - 3; q++)
+    if (g0 >> q & 1u) off ^= s.kappa[q];
+  return off;
+}
+
+// One string on 8 amplitudes: acc += sum over its pairs of +-c (re or im).
+template <typename A, int KAP>
+__device__ __forceinline__ double pairs(const A (&v)[8], double c, uint32_t pat, bool odd, double acc) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    if (k & (KAP & -KAP)) continue;  // the member without the lowest mask bit
+    const double ix = v[k].x, iy = v[k].y, px = v[k ^ KAP].x, py = v[k ^ KAP].y;
+    const double x = odd ? px * iy - py * ix : px * ix + py * iy;
+    acc = fma(flip_sign(c, pat >> k & 1u), x, acc);
+  }
+  return acc;
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(kSumThreads, 3)
+    k_pauli_sum(const typename Cplx<Real>::T* __restrict__ amp, const __grid_constant__ PauliPass P,
+                const PauliSeg* __restrict__ segs, const PauliTerm* __restrict__ terms,
+                double* __restrict__ partials) {
+  using A = typename Cplx<Real>::T;
+  constexpr int NT = kSumThreads, UB = sizeof(A) == 16 ? 0 : 1;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint64_t joff[kMaxUnitSteps];
+  __shared__ double red[NT / 32];
+  const uint32_t tile_bytes = (uint32_t)sizeof(A) << P.m;
+  double* coef = reinterpret_cast<double*>(smem + tile_bytes);       // [term] with the tile's sign
+  PauliTerm* st = reinterpret_cast<PauliTerm*>(coef + P.num_terms);
+  PauliSeg* ss = reinterpret_cast<PauliSeg*>(st + P.num_terms);
+  const int tid = threadIdx.x;
+  for (int i = tid; i < P.num_terms * (int)(sizeof(PauliTerm) / 4); i += NT)
+    reinterpret_cast<uint32_t*>(st)[i] = reinterpret_cast<const uint32_t*>(terms)[i];
+  for (int i = tid; i < P.num_segs * (int)(sizeof(PauliSeg) / 4); i += NT)
+    reinterpret_cast<uint32_t*>(ss)[i] = reinterpret_cast<const uint32_t*>(segs)[i];
+  UnitOffsets<NT, UB> uo;
+  uo.init(P, joff);
+  const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const uint32_t units = 1u << (P.m - UB), groups = 1u << (P.m - 3);
+  __syncthreads();
+  double acc = 0.0;
+  for (uint64_t tile = blockIdx.x; tile < P.tiles_per_state; tile += gridDim.x) {
+    const uint64_t base = pdep64(tile, P.free_mask);
+    for (uint32_t u = tid, j = 0; u < units; u += NT, j++)
+      cp_async16(sm0 + tile_swz16(u) * 16u, amp + (base ^ uo.toff ^ joff[j]));
+    for (int t = tid; t < P.num_terms; t += NT) coef[t] = flip_sign(st[t].c, __popcll(st[t].z & base) & 1);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    for (int s = 0; s < P.num_segs; s++) {
+      const PauliSeg& sg = ss[s];
+      const uint32_t a0 = sg.alpha[0], a1 = sg.alpha[1], a2 = sg.alpha[2];
+      const uint32_t lane_off = group_lane_offset<7>(sg);
+      for (uint32_t g0 = 0; g0 + tid < groups; g0 += NT) {
+        const uint32_t off = lane_off ^ group_step_offset<7>(sg, g0);
+        A v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          v[k] = *reinterpret_cast<const A*>(smem + (off ^ (k & 1 ? a0 : 0u) ^ (k & 2 ? a1 : 0u) ^ (k & 4 ? a2 : 0u)));
+        for (int t = sg.term_begin; t < sg.term_end; t++) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(&st[t].zg);  // zg, kap, pat
+          const double c = flip_sign(coef[t], __popc(w & 0xffffu & (g0 + tid)) & 1);
+          const uint32_t pat = w >> 24;
+          const bool odd = st[t].odd != 0;
+          switch (w >> 16 & 7u) {
+            case 0:
+#pragma unroll
+              for (int k = 0; k < 8; k++) {
+                const double x = v[k].x, y = v[k].y;
+                acc = fma(flip_sign(c, pat >> k & 1u), x * x + y * y, acc);
+              }
+              break;
+            case 1: acc = pairs<A, 1>(v, c, pat, odd, acc); break;
+            case 2: acc = pairs<A, 2>(v, c, pat, odd, acc); break;
+            case 3: acc = pairs<A, 3>(v, c, pat, odd, acc); break;
+            case 4: acc = pairs<A, 4>(v, c, pat, odd, acc); break;
+            case 5: acc = pairs<A, 5>(v, c, pat, odd, acc); break;
+            case 6: acc = pairs<A, 6>(v, c, pat, odd, acc); break;
+            default: acc = pairs<A, 7>(v, c, pat, odd, acc); break;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if ((tid & 31) == 0) red[tid >> 5] = acc;
+  __syncthreads();
+  if (tid == 0) {
+    double s = 0.0;
+    for (int w = 0; w < NT / 32; w++) s += red[w];
+    partials[blockIdx.x] = s;
+  }
+}
+
+// States of fewer than 8 amplitudes: one thread per string and amplitude in turn.
+template <typename Real>
+__global__ void k_pauli_tiny(const typename Cplx<Real>::T* __restrict__ amp, int n, int num_terms,
+                             const uint64_t* __restrict__ xm, const uint64_t* __restrict__ zm,
+                             const double* __restrict__ coeff, double* __restrict__ partials) {
+  double acc = 0.0;
+  for (int t = threadIdx.x; t < num_terms; t += 32) {
+    const int ny = __popcll(xm[t] & zm[t]) & 3;
+    double v = 0.0;
+    for (uint32_t i = 0; i < (1u << n); i++) {
+      const auto a = amp[i], b = amp[i ^ (uint32_t)xm[t]];
+      const double re = (double)b.x * a.x + (double)b.y * a.y, im = (double)b.x * a.y - (double)b.y * a.x;
+      const double x = ny == 0 ? re : ny == 1 ? -im : ny == 2 ? -re : im;  // Re(i^ny conj(b) a)
+      v += __popcll(i & zm[t]) & 1 ? -x : x;
+    }
+    acc += coeff[t] * v;
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (threadIdx.x == 0) partials[0] = acc;
+}
+
+__global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__ partials, int count,
+                                                      double* __restrict__ out) {
+  __shared__ double red[256];
+  double v = 0.0;
+  for (int i = threadIdx.x; i < count; i += 256) v += partials[i];
+  red[threadIdx.x] = v;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[0] = red[0];
+}
+
+// lambda[k] += +-c (1 or i) psi[k ^ KAP]; the sign is that of the source.
+template <typename A, int KAP>
+__device__ __forceinline__ void apply_string(const A (&v)[8], double2 (&l)[8], double c, uint32_t pat, bool odd) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const double cs = flip_sign(c, pat >> (k ^ KAP) & 1u);
+    const double x = v[k ^ KAP].x, y = v[k ^ KAP].y;
+    if (odd) {  // times i
+      l[k].x = fma(-cs, y, l[k].x);
+      l[k].y = fma(cs, x, l[k].y);
+    } else {
+      l[k].x = fma(cs, x, l[k].x);
+      l[k].y = fma(cs, y, l[k].y);
+    }
+  }
+}
+
+// The tile of lambda is held in FP64 for both types and rounded to the
+// state's type once, at its store.
+template <typename Real>
+__global__ void __launch_bounds__(kApplyThreads, sizeof(Real) == 8 ? 3 : 2)
+    k_pauli_apply(const typename Cplx<Real>::T* __restrict__ psi, typename Cplx<Real>::T* __restrict__ lam,
+                  const __grid_constant__ PauliPass P, const PauliSeg* __restrict__ segs,
+                  const PauliTerm* __restrict__ terms, int accumulate, double* __restrict__ energy_partials) {
+  using A = typename Cplx<Real>::T;
+  constexpr int NT = kApplyThreads, UB = sizeof(A) == 16 ? 0 : 1;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint64_t joff[kMaxUnitSteps];
+  __shared__ double red[NT / 32];
+  const uint32_t tile_bytes = (uint32_t)sizeof(A) << P.m;
+  unsigned char* ltile = smem + tile_bytes;  // [2^m] double2, at twice psi's offsets for complex64
+  double* coef = reinterpret_cast<double*>(ltile + (16u << P.m));
+  PauliTerm* st = reinterpret_cast<PauliTerm*>(coef + P.num_terms);
+  PauliSeg* ss = reinterpret_cast<PauliSeg*>(st + P.num_terms);
+  const int tid = threadIdx.x;
+  for (int i = tid; i < P.num_terms * (int)(sizeof(PauliTerm) / 4); i += NT)
+    reinterpret_cast<uint32_t*>(st)[i] = reinterpret_cast<const uint32_t*>(terms)[i];
+  for (int i = tid; i < P.num_segs * (int)(sizeof(PauliSeg) / 4); i += NT)
+    reinterpret_cast<uint32_t*>(ss)[i] = reinterpret_cast<const uint32_t*>(segs)[i];
+  UnitOffsets<NT, UB> uo;
+  uo.init(P, joff);
+  const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const uint32_t units = 1u << (P.m - UB), groups = 1u << (P.m - 3);
+  __syncthreads();
+  for (uint64_t tile = blockIdx.x; tile < P.num_tiles; tile += gridDim.x) {
+    const uint64_t b = tile / P.tiles_per_state;
+    const uint64_t base = pdep64(tile % P.tiles_per_state, P.free_mask);
+    const A* gs = psi + (b << P.n);
+    A* gl = lam + (b << P.n);
+    for (uint32_t u = tid, j = 0; u < units; u += NT, j++) {
+      const uint64_t off = base ^ uo.toff ^ joff[j];
+      const uint32_t dst = tile_swz16(u) * 16u;
+      cp_async16(sm0 + dst, gs + off);
+      if constexpr (UB == 0) {
+        if (accumulate) cp_async16(sm0 + tile_bytes + dst, gl + off);
+        else *reinterpret_cast<double2*>(ltile + dst) = make_double2(0.0, 0.0);
+      } else {
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (accumulate) o = *reinterpret_cast<const float4*>(gl + off);
+        *reinterpret_cast<double2*>(ltile + 2 * dst) = make_double2(o.x, o.y);
+        *reinterpret_cast<double2*>(ltile + 2 * dst + 16) = make_double2(o.z, o.w);
+      }
+    }
+    for (int t = tid; t < P.num_terms; t += NT) coef[t] = flip_sign(st[t].c, __popcll(st[t].z & base) & 1);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    for (int s = 0; s < P.num_segs; s++) {
+      const PauliSeg& sg = ss[s];
+      const uint32_t a0 = sg.alpha[0], a1 = sg.alpha[1], a2 = sg.alpha[2];
+      const uint32_t lane_off = group_lane_offset<7>(sg);
+      for (uint32_t g0 = 0; g0 + tid < groups; g0 += NT) {
+        const uint32_t off = lane_off ^ group_step_offset<7>(sg, g0);
+        A v[8];
+        double2 l[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const uint32_t at = off ^ (k & 1 ? a0 : 0u) ^ (k & 2 ? a1 : 0u) ^ (k & 4 ? a2 : 0u);
+          v[k] = *reinterpret_cast<const A*>(smem + at);
+          l[k] = *reinterpret_cast<const double2*>(ltile + (at << UB));
+        }
+        for (int t = sg.term_begin; t < sg.term_end; t++) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(&st[t].zg);  // zg, kap, pat
+          const double c = flip_sign(coef[t], __popc(w & 0xffffu & (g0 + tid)) & 1);
+          const uint32_t pat = w >> 24;
+          const bool odd = st[t].odd != 0;
+          switch (w >> 16 & 7u) {
+            case 0: apply_string<A, 0>(v, l, c, pat, odd); break;
+            case 1: apply_string<A, 1>(v, l, c, pat, odd); break;
+            case 2: apply_string<A, 2>(v, l, c, pat, odd); break;
+            case 3: apply_string<A, 3>(v, l, c, pat, odd); break;
+            case 4: apply_string<A, 4>(v, l, c, pat, odd); break;
+            case 5: apply_string<A, 5>(v, l, c, pat, odd); break;
+            case 6: apply_string<A, 6>(v, l, c, pat, odd); break;
+            default: apply_string<A, 7>(v, l, c, pat, odd); break;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          *reinterpret_cast<double2*>(ltile + ((off ^ (k & 1 ? a0 : 0u) ^ (k & 2 ? a1 : 0u) ^ (k & 4 ? a2 : 0u)) << UB)) = l[k];
+      }
+      __syncthreads();
+    }
+    double e_acc = 0.0;
+    for (uint32_t u = tid, j = 0; u < units; u += NT, j++) {
+      const uint64_t off = base ^ uo.toff ^ joff[j];
+      const uint32_t at = tile_swz16(u) * 16u;
+      if constexpr (UB == 0) {
+        const double2 x = *reinterpret_cast<const double2*>(ltile + at);
+        const double2 p = *reinterpret_cast<const double2*>(smem + at);
+        gl[off] = x;
+        e_acc += p.x * x.x + p.y * x.y;  // Re(conj(psi) lambda)
+      } else {
+        const double2 x = *reinterpret_cast<const double2*>(ltile + 2 * at);
+        const double2 y = *reinterpret_cast<const double2*>(ltile + 2 * at + 16);
+        const float4 p = *reinterpret_cast<const float4*>(smem + at);
+        const float4 o = make_float4((float)x.x, (float)x.y, (float)y.x, (float)y.y);
+        *reinterpret_cast<float4*>(gl + off) = o;
+        e_acc += (double)p.x * o.x + (double)p.y * o.y;
+        e_acc += (double)p.z * o.z + (double)p.w * o.w;
+      }
+    }
+    if (energy_partials) {
+      for (int o = 16; o > 0; o >>= 1) e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
+      if ((tid & 31) == 0) red[tid >> 5] = e_acc;
+      __syncthreads();
+      if (tid == 0) {
+        double s = 0.0;
+        for (int w = 0; w < NT / 32; w++) s += red[w];
+        energy_partials[tile] = s;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+size_t tables_bytes(const PauliPass& P) {
+  return P.num_terms * (sizeof(double) + sizeof(PauliTerm)) + P.num_segs * sizeof(PauliSeg);
+}
+
+template <typename Real>
+int launch_sum_t(const void* amp, const PauliPass& P, const PauliSeg* d_segs, const PauliTerm* d_terms,
+                 double* d_partials, int num_sms, cudaStream_t stream, int* parts) {
+  using A = typename Cplx<Real>::T;
+  const size_t smem = (sizeof(A) << P.m) + tables_bytes(P);
+  auto kern = k_pauli_sum<Real>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSumThreads, smem);
+  uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm > kPauliCtasPerSm ? kPauliCtasPerSm : per_sm);
+  if (grid > P.tiles_per_state) grid = P.tiles_per_state;
+  kern<<<(unsigned)grid, kSumThreads, smem, stream>>>((const A*)amp, P, d_segs, d_terms, d_partials);
+  count_launch();
+  *parts = (int)grid;
+  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
+}
+
+template <typename Real>
+int launch_apply_t(const void* psi, void* lam, const PauliPass& P, const PauliSeg* d_segs, const PauliTerm* d_terms,
+                   bool accumulate, double* d_epart, int num_sms, cudaStream_t stream) {
+  using A = typename Cplx<Real>::T;
+  const size_t smem = ((sizeof(A) + 16) << P.m) + tables_bytes(P);
+  auto kern = k_pauli_apply<Real>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kApplyThreads, smem);
+  uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);
+  if (grid > P.num_tiles) grid = P.num_tiles;
+  kern<<<(unsigned)grid, kApplyThreads, smem, stream>>>((const A*)psi, (A*)lam, P, d_segs, d_terms,
+                                                        accumulate ? 1 : 0, d_epart);
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
+}
+
+}  // namespace
+
+int pauli_tile_bits(int dtype, bool apply) {
+  if (dtype == MLB_C128) return apply ? 11 : 12;
+  return apply ? 12 : 13;
+}
+
+int launch_pauli_sum(int dtype, const void* amp, const PauliPass& P, const PauliSeg* d_segs,
+                     const PauliTerm* d_terms, double* d_partials, int num_sms, cudaStream_t stream, int* parts) {
+  if (P.m < 3 || P.m > pauli_tile_bits(dtype, false) || P.num_terms < 1 || P.num_terms > kMaxPauliTerms)
+    return MLB_ERR_INVALID_ARG;
+  return dtype == MLB_C128 ? launch_sum_t<double>(amp, P, d_segs, d_terms, d_partials, num_sms, stream, parts)
+                           : launch_sum_t<float>(amp, P, d_segs, d_terms, d_partials, num_sms, stream, parts);
+}
+
+int launch_pauli_tiny(int dtype, const void* amp, int n, int num_terms, const uint64_t* d_xm, const uint64_t* d_zm,
+                      const double* d_coeff, double* d_partials, cudaStream_t stream) {
+  if (n > 2) return MLB_ERR_INVALID_ARG;
+  if (dtype == MLB_C128)
+    k_pauli_tiny<double><<<1, 32, 0, stream>>>((const double2*)amp, n, num_terms, d_xm, d_zm, d_coeff, d_partials);
+  else
+    k_pauli_tiny<float><<<1, 32, 0, stream>>>((const float2*)amp, n, num_terms, d_xm, d_zm, d_coeff, d_partials);
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
+}
+
+int launch_sum_partials(const double* d_partials, int count, double* d_out, cudaStream_t stream) {
+  k_sum_partials<<<1, 256, 0, stream>>>(d_partials, count, d_out);
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
+}
+
+int launch_pauli_apply(int dtype, const void* psi, void* lam, const PauliPass& P, const PauliSeg* d_segs,
+                       const PauliTerm* d_terms, bool accumulate, double* d_epart, int num_sms,
+                       cudaStream_t stream) {
+  if (P.m < 3 || P.m > pauli_tile_bits(dtype, true) || P.num_terms < 1 || P.num_terms > kMaxPauliTerms)
+    return MLB_ERR_INVALID_ARG;
+  return dtype == MLB_C128
+             ? launch_apply_t<double>(psi, lam, P, d_segs, d_terms, accumulate, d_epart, num_sms, stream)
+             : launch_apply_t<float>(psi, lam, P, d_segs, d_terms, accumulate, d_epart, num_sms, stream);
+}
+
+}  // namespace mlb

@@ -122,77 +122,6 @@ __global__ void __launch_bounds__(kRT) k_probs_z_pass2(const double* __restrict_
   }
 }
 
-// <psi|P|psi> for Pauli strings sharing one X mask: P|i> = i^{ny}
-// (-1)^{|i & z|} |i ^ x>.  Each pair (i, i^x) is read once; x = 0 gives the
-// diagonal (Z-only) strings.  out[t] gets coeff_t * Re(...), summed later.
-template <typename Real>
-__global__ void __launch_bounds__(kRT) k_pauli(const typename Cplx<Real>::T* __restrict__ amp,
-                                               int n, uint64_t xmask, int num_terms,
-                                               const uint64_t* __restrict__ zmasks,
-                                               const int* __restrict__ nys,
-                                               double* __restrict__ partials) {
-  __shared__ double red[kRT / 32];
-  constexpr int kMaxT = 16;
-  double acc[kMaxT];
-#pragma unroll
-  for (int t = 0; t < kMaxT; t++) acc[t] = 0.0;
-  const uint64_t dim = 1ull << n;
-  const int hb = xmask ? 63 - __clzll(xmask) : -1;
-  const uint64_t items = xmask ? dim >> 1 : dim;
-  const uint64_t stride = (uint64_t)gridDim.x * kRT;
-  for (uint64_t j = (uint64_t)blockIdx.x * kRT + threadIdx.x; j < items; j += stride) {
-    if (xmask) {
-      const uint64_t lo = j & ((1ull << hb) - 1ull);
-      const uint64_t i = ((j >> hb) << (hb + 1)) | lo;  // bit hb = 0
-      const uint64_t k = i ^ xmask;
-      const auto ai = amp[i], ak = amp[k];
-      // conj(a_k) a_i and conj(a_i) a_k = conj of the former
-      const double re = (double)ak.x * ai.x + (double)ak.y * ai.y;
-      const double im = (double)ak.x * ai.y - (double)ak.y * ai.x;
-#pragma unroll
-      for (int t = 0; t < kMaxT; t++) {
-        if (t >= num_terms) break;
-        const uint64_t z = zmasks[t];
-        const int ny = nys[t] & 3;
-        const double si = parity64(i & z) ? -1.0 : 1.0;
-        const double sk = parity64(k & z) ? -1.0 : 1.0;
-        // term_i = i^ny si conj(a_k) a_i ; term_k = i^ny sk conj(a_i) a_k
-        double tr_i, tr_k;
-        switch (ny) {
-          case 0: tr_i = re; tr_k = re; break;
-          case 1: tr_i = -im; tr_k = im; break;
-          case 2: tr_i = -re; tr_k = -re; break;
-          default: tr_i = im; tr_k = -im; break;
-        }
-        acc[t] += si * tr_i + sk * tr_k;
-      }
-    } else {
-      const auto a = amp[j];
-      const double p = norm2(a);
-#pragma unroll
-      for (int t = 0; t < kMaxT; t++) {
-        if (t >= num_terms) break;
-        acc[t] += parity64(j & zmasks[t]) ? -p : p;
-      }
-    }
-  }
-  for (int t = 0; t < num_terms && t < kMaxT; t++) {
-    const double v = block_sum(acc[t], red);
-    if (threadIdx.x == 0) partials[(size_t)blockIdx.x * kMaxT + t] = v;
-  }
-}
-
-__global__ void k_fold_partials(const double* __restrict__ partials, int num_parts, int stride,
-                                int count, double* __restrict__ out) {
-  __shared__ double red[kRT / 32];
-  for (int j = 0; j < count; j++) {
-    double v = 0.0;
-    for (int i = threadIdx.x; i < num_parts; i += kRT) v += partials[(size_t)i * stride + j];
-    v = block_sum(v, red);
-    if (threadIdx.x == 0) out[j] = v;
-  }
-}
-
 template <typename Real>
 __global__ void k_probabilities(const typename Cplx<Real>::T* __restrict__ amp, uint64_t dim,
                                 int rule, double* __restrict__ out) {
@@ -260,23 +189,6 @@ int launch_reduce_probs_z(int dtype, const void* amp, int n, double* d_out, doub
     k_probs_z_pass1<float><<<grid, kRT, 0, stream>>>((const float2*)amp, num_chunks, chunk_amps,
                                                      chunk_tot, parts);
   k_probs_z_pass2<<<1, kRT, 0, stream>>>(chunk_tot, num_chunks, parts, grid, n, d_out);
-  count_launch(2);
-  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
-}
-
-// Grouped Pauli expectation (called by the host with one X-mask group).
-int launch_pauli_group(int dtype, const void* amp, int n, uint64_t xmask, int num_terms,
-                       const uint64_t* d_zmasks, const int* d_nys, double* d_out_terms,
-                       double* d_partials, int num_sms, cudaStream_t stream) {
-  const uint64_t items = xmask ? (1ull << n) >> 1 : (1ull << n);
-  const int grid = rgrid(items, num_sms);
-  if (dtype == MLB_C128)
-    k_pauli<double><<<grid, kRT, 0, stream>>>((const double2*)amp, n, xmask, num_terms, d_zmasks,
-                                              d_nys, d_partials);
-  else
-    k_pauli<float><<<grid, kRT, 0, stream>>>((const float2*)amp, n, xmask, num_terms, d_zmasks,
-                                             d_nys, d_partials);
-  k_fold_partials<<<1, kRT, 0, stream>>>(d_partials, grid, 16, num_terms, d_out_terms);
   count_launch(2);
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }

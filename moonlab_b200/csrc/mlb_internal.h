@@ -115,7 +115,6 @@ __host__ __device__ inline uint32_t tile_swz16(uint32_t e) {
 // states stored back to back, [B][2^n]; tiles never span two states.
 // ---------------------------------------------------------------------------
 enum AdjKind : int32_t { ADJ_KIND_X = 0, ADJ_KIND_RY = 1, ADJ_KIND_RZ = 2 };  // ansatz gates (X: CNOT with a control)
-constexpr int kMaxAdjTerms = 128;  // Pauli terms per lambda pass
 // Rotation passes over linear subspaces of the index space (hea_plan.h).
 constexpr int kMaxHeaSegs = 24;    // segments of a pass (their tables live in shared memory)
 constexpr int kMaxHeaBits = 13;    // bits of a tile
@@ -137,17 +136,6 @@ struct HeaPass {
   uint32_t items_per_state, tiles_per_item;  // a work item is a run of one state's tiles
   uint64_t num_items;
 };
-struct AdjTerm {     // one Pauli string restricted to a tile
-  uint32_t xl, zl;   // local X / Z masks
-  uint64_t zo;       // Z mask outside the tile (global bits)
-  double cr, ci;     // c_k * i^{#Y}
-};
-struct AdjPass {
-  int32_t n, L, H;
-  int32_t num_ops;
-  int32_t high[kMaxHigh];
-  uint64_t tiles_per_state, num_tiles, tile_free_mask;
-};
 int hea_tile_bits(int dtype, bool backward);
 // Rotation pass: psi_src -> psi (the same buffer, or another of the batch's
 // size), and in the backward sweep lam in place and partials[(state *
@@ -165,15 +153,52 @@ int launch_adj_energy(const double* d_partials, uint64_t tiles_per_state, uint64
 // complex64: dst[b][p] = src[b][C^-k p], C the CNOT ladder on n qubits
 // (hea_plan.h).
 int launch_unladder(const void* src, void* dst, int n, int k, uint64_t batch, int num_sms, cudaStream_t stream);
-int adj_tile_bits(int dtype);
 int launch_adj_init(int dtype, void* psi, int n, uint64_t batch, uint64_t hf, cudaStream_t stream);
-int launch_adj_pauli(int dtype, const void* psi, void* lam, const AdjPass& P, const AdjTerm* d_terms,
-                     bool accumulate, bool energy, double* d_epart, int num_sms, cudaStream_t stream);
 // d_norm[b] = |psi_b|^2 of a complex64 batch; then d_out ([B] energies,
 // [B][P] gradients) divided by it.
 int launch_batch_norm(const void* psi_c64, uint64_t dim, uint64_t batch, double* d_norm, cudaStream_t stream);
 int launch_divide_by_norm(double* d_out, uint64_t batch, int num_params, const double* d_norm,
                           cudaStream_t stream);
+
+// ---- sums of Pauli strings (pauli_plan.h, kernels_pauli.cu) ----
+constexpr int kMaxPauliBits = 13;    // bits of a tile
+constexpr int kMaxPauliTerms = 256;  // strings of a pass (their table lives in shared memory)
+constexpr int kPauliCtasPerSm = 4;   // bounds the partials of a pass
+struct PauliTerm {
+  double c;          // coefficient with the string's constant signs
+  uint64_t z;        // Z mask; the tile's sign is parity(z & base)
+  uint16_t zg;       // the group's: parity(zg & group index)
+  uint8_t kap;       // its X mask among the segment's directions
+  uint8_t pat;       // bit k: the sign of register index k
+  uint8_t odd;       // an odd number of Y's: the imaginary part
+  uint8_t pad[3];
+};
+struct PauliSeg {
+  uint16_t alpha[3];                 // byte offsets in the tile of its directions
+  uint16_t kappa[kMaxPauliBits - 3]; // and of the groups' basis
+  uint16_t pad;
+  int32_t term_begin, term_end;
+};
+struct PauliPass {
+  int32_t n, m, num_segs, num_terms;
+  uint64_t basis[kMaxPauliBits];     // local bit k of an amplitude adds basis[k] to its index
+  uint64_t free_mask;                // bits that enumerate the tiles of a state
+  uint64_t tiles_per_state, num_tiles;
+};
+int pauli_tile_bits(int dtype, bool apply);
+// One pass of an expectation value: *parts partials (at most num_sms *
+// kPauliCtasPerSm) whose sum is the pass's strings'.
+int launch_pauli_sum(int dtype, const void* amp, const PauliPass& P, const PauliSeg* d_segs,
+                     const PauliTerm* d_terms, double* d_partials, int num_sms, cudaStream_t stream, int* parts);
+// The whole sum for a state of one or two qubits (one partial).
+int launch_pauli_tiny(int dtype, const void* amp, int n, int num_terms, const uint64_t* d_xm, const uint64_t* d_zm,
+                      const double* d_coeff, double* d_partials, cudaStream_t stream);
+int launch_sum_partials(const double* d_partials, int count, double* d_out, cudaStream_t stream);
+// lambda (+)= the pass's strings on psi, for P.num_tiles tiles of a batch;
+// d_epart (or null): per-tile Re<psi|lambda>.
+int launch_pauli_apply(int dtype, const void* psi, void* lam, const PauliPass& P, const PauliSeg* d_segs,
+                       const PauliTerm* d_terms, bool accumulate, double* d_epart, int num_sms,
+                       cudaStream_t stream);
 
 // Gram matrix of B complex128 states stored back to back ([B][dim]):
 // d_G[a * B + b] = sum_x conj(S_a[x]) S_b[x] for a <= b (the rest of d_G is
@@ -205,10 +230,6 @@ int launch_convert(int dst_dtype, void* dst, int src_dtype, const void* src, uin
 // Reductions: results written into a device FP64 scratch block, then copied.
 int launch_reduce_probs_z(int dtype, const void* amp, int n, double* d_out /* n+1 */,
                           double* d_partials, int num_sms, cudaStream_t stream);
-// Pauli strings sharing one X mask (<= 16 per call); out_terms[t] = Re<P_t>.
-int launch_pauli_group(int dtype, const void* amp, int n, uint64_t xmask, int num_terms,
-                       const uint64_t* d_zmasks, const int* d_nys, double* d_out_terms,
-                       double* d_partials, int num_sms, cudaStream_t stream);
 int launch_probabilities(int dtype, const void* amp, int n, int rule, double* d_out,
                          cudaStream_t stream);
 int launch_scale(int dtype, void* amp, int n, double factor, uint64_t zero_mask,

@@ -13,7 +13,7 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <map>
+#include <utility>
 #include <vector>
 
 #include "hea_plan.h"
@@ -29,28 +29,33 @@ struct Pass {
   size_t segs_off = 0, terms_off = 0;  // in the caller's device arrays
 };
 
-// Greedy: the independent masks that, added to V (up to `dims` vectors),
-// bring the most of `masks` (weighted) into its span.
+// Greedy: masks added to V (up to `dims` vectors), each the one that brings
+// the most strings into the span with it; among equals, the one whose qubits
+// the most masks touch.  masks: sorted, with their numbers of strings.
 inline void grow(hea::Basis& V, const std::vector<uint64_t>& masks, const std::vector<int>& weight, int dims) {
+  int degree[64] = {};
+  for (uint64_t x : masks)
+    for (uint64_t y = x; y; y &= y - 1) degree[__builtin_ctzll(y)]++;
+  std::vector<std::pair<uint64_t, int>> res;
   while ((int)V.v.size() < dims) {
-    // a candidate's gain: the masks equal to it modulo the span
-    std::map<uint64_t, int> gain;
-    for (size_t i = 0; i < masks.size(); i++) {
-      const uint64_t r = V.reduce(masks[i]);
-      if (r) gain[r] += weight[i];
-    }
-    if (gain.empty()) break;
-    // first look one step ahead: with r in, masks a ^ b = r pairs come closer
+    res.clear();  // the masks modulo the span: equal residues come in together
+    for (size_t i = 0; i < masks.size(); i++)
+      if (const uint64_t r = V.reduce(masks[i])) res.push_back({r, weight[i]});
+    if (res.empty()) break;
+    std::sort(res.begin(), res.end());
     uint64_t best = 0;
-    int most = -1;
-    for (auto& [r, g] : gain) {
-      int ahead = 0;
-      for (auto& [s, gs] : gain)
-        if (s != r && gain.count(s ^ r)) ahead += gs;
-      if (64 * g + ahead > most) {
-        most = 64 * g + ahead;
-        best = r;
+    long most = -1;
+    for (size_t i = 0; i < res.size();) {
+      long gain = 0, touch = 0;
+      size_t j = i;
+      for (; j < res.size() && res[j].first == res[i].first; j++) gain += res[j].second;
+      for (uint64_t y = res[i].first; y; y &= y - 1) touch += degree[__builtin_ctzll(y)];
+      const long score = (gain << 32) + (touch << 8) / __builtin_popcountll(res[i].first);
+      if (score > most) {
+        most = score;
+        best = res[i].first;
       }
+      i = j;
     }
     V.add(best);
   }
@@ -78,7 +83,7 @@ inline void plan(int n, int TB, int L, int dtype, size_t num, const uint64_t* xm
       }
     hea::Basis V;
     for (int b = 0; b < L; b++) V.add(1ull << b);
-    grow(V, masks, weight, m);
+    if (n > m) grow(V, masks, weight, m);
     for (int b = 0; b < n && (int)V.v.size() < m; b++) V.add(1ull << b);
     std::vector<size_t> take, left;
     for (size_t i : rem) (take.size() < (size_t)kMaxPauliTerms && !V.reduce(xm[i]) ? take : left).push_back(i);
@@ -111,28 +116,13 @@ inline void plan(int n, int TB, int L, int dtype, size_t num, const uint64_t* xm
       PauliSeg s{};
       for (int i = 0; i < 3; i++) s.alpha[i] = (uint16_t)hea::slot_bytes((uint32_t)R.v[i], dtype);
       // groups: a complement of the three directions, lanes on distinct banks first
-      std::vector<uint32_t> comp, order;
+      std::vector<uint32_t> comp;
       {
         hea::Basis full = R;
         for (int b = 0; b < m; b++)
           if (full.add(1ull << b)) comp.push_back(1u << b);
       }
-      hea::Basis banks, chosen;
-      const int want = dtype == MLB_C128 ? 3 : 4;
-      for (uint32_t mix = 1; mix < (1u << comp.size()) && (int)order.size() < want; mix++) {
-        if (__builtin_popcount(mix) > 3) continue;
-        uint32_t t = 0;
-        for (size_t i = 0; i < comp.size(); i++)
-          if (mix >> i & 1u) t ^= comp[i];
-        hea::Basis nb = banks, nc = chosen;
-        if (nb.add(hea::bank_of(t, dtype)) && nc.add(t)) {
-          banks = nb;
-          chosen = nc;
-          order.push_back(t);
-        }
-      }
-      for (uint32_t t : comp)
-        if (chosen.add(t)) order.push_back(t);
+      const std::vector<uint32_t> order = hea::bank_order(comp, dtype);
       for (size_t i = 0; i < order.size(); i++) s.kappa[i] = (uint16_t)hea::slot_bytes(order[i], dtype);
       auto global = [&](uint64_t t) {
         uint64_t g = 0;
@@ -163,9 +153,7 @@ inline void plan(int n, int TB, int L, int dtype, size_t num, const uint64_t* xm
         const double c = coeff ? coeff[i] : 1.0;
         d.odd = (uint8_t)(ny & 1);
         if (lambda) {
-          // the source's sign, (-1)^{|i & z|}, seen from the target i ^ x: (-1)^{ny} times it;
-          // i^{ny}: 1, i, -1, -i
-          d.c = ny == 1 || ny == 2 ? -c : c;
+          d.c = ny >= 2 ? -c : c;  // i^{ny}: 1, i, -1, -i
         } else {
           // both members of a pair, i the one kept: 2 s(i) {re, -im, -re, im}
           d.c = (xm[i] ? 2.0 : 1.0) * (ny == 1 || ny == 2 ? -c : c);
