@@ -18,7 +18,8 @@
 // one's copies with the others' sums.
 // Measured: norm, <Z>, 58 random one- and two-local strings and 4096 samples
 // of a 29-qubit complex128 state 68.1 -> 28.6 ms (one pass over the state per
-// distinct X mask before, three passes for all of them now); lambda = H psi
+// distinct X mask before, three passes for all of them now), 22.1 ms with two
+// groups per thread and a routine per kind of string; lambda = H psi
 // of 80 strings on 256 states of 20 qubits: the whole gradient 134 -> 107 ms.
 #include "kernels_common.cuh"
 #include "mlb_internal.h"
@@ -77,17 +78,32 @@ __device__ __forceinline__ uint32_t group_step_offset(const PauliSeg& s, uint32_
   return off;
 }
 
-// One string on 8 amplitudes: acc += sum over its pairs of +-c (re or im).
-template <typename A, int KAP>
-__device__ __forceinline__ double pairs(const A (&v)[8], double c, uint32_t pat, bool odd, double acc) {
+// Keeps products of the amplitudes inside the loop over strings: they are the
+// same for every string of a mask, and hoisted ones would spill.
+__device__ __forceinline__ void opaque(double2 (&v)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) asm volatile("" : "+d"(v[k].x), "+d"(v[k].y));
+}
+__device__ __forceinline__ void opaque(float2 (&v)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) asm volatile("" : "+f"(v[k].x), "+f"(v[k].y));
+}
+
+// One string on two groups of 8 amplitudes: acc += sum over its pairs of
+// +-c times the real (ODD: imaginary) part.  KAP: its X mask among the
+// segment's directions, 0: its diagonal.
+template <typename A, int KAP, bool ODD>
+__device__ __forceinline__ void pairs(const A (&v)[2][8], const double (&c)[2], uint32_t pat, double (&acc)[2]) {
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     if (k & (KAP & -KAP)) continue;  // the member without the lowest mask bit
-    const double ix = v[k].x, iy = v[k].y, px = v[k ^ KAP].x, py = v[k ^ KAP].y;
-    const double x = odd ? px * iy - py * ix : px * ix + py * iy;
-    acc = fma(flip_sign(c, pat >> k & 1u), x, acc);
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+      const double ix = v[g][k].x, iy = v[g][k].y, px = v[g][k ^ KAP].x, py = v[g][k ^ KAP].y;
+      const double x = ODD ? px * iy - py * ix : px * ix + py * iy;
+      acc[g] = fma(flip_sign(c[g], pat >> k & 1u), x, acc[g]);
+    }
   }
-  return acc;
 }
 
 template <typename Real>
@@ -114,7 +130,7 @@ __global__ void __launch_bounds__(kSumThreads, 3)
   const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   const uint32_t units = 1u << (P.m - UB), groups = 1u << (P.m - 3);
   __syncthreads();
-  double acc = 0.0;
+  double acc[2] = {0.0, 0.0};
   for (uint64_t tile = blockIdx.x; tile < P.tiles_per_state; tile += gridDim.x) {
     const uint64_t base = pdep64(tile, P.free_mask);
     for (uint32_t u = tid, j = 0; u < units; u += NT, j++)
@@ -126,40 +142,44 @@ __global__ void __launch_bounds__(kSumThreads, 3)
       const PauliSeg& sg = ss[s];
       const uint32_t a0 = sg.alpha[0], a1 = sg.alpha[1], a2 = sg.alpha[2];
       const uint32_t lane_off = group_lane_offset<7>(sg);
-      for (uint32_t g0 = 0; g0 + tid < groups; g0 += NT) {
+      for (uint32_t g0 = 0; g0 + tid < groups; g0 += 2 * NT) {
+        const bool two = g0 + NT + tid < groups;
         const uint32_t off = lane_off ^ group_step_offset<7>(sg, g0);
-        A v[8];
+        const uint32_t off1 = two ? lane_off ^ group_step_offset<7>(sg, g0 + NT) : off;
+        A v[2][8];
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-          v[k] = *reinterpret_cast<const A*>(smem + (off ^ (k & 1 ? a0 : 0u) ^ (k & 2 ? a1 : 0u) ^ (k & 4 ? a2 : 0u)));
+        for (int k = 0; k < 8; k++) {
+          const uint32_t ak = (k & 1 ? a0 : 0u) ^ (k & 2 ? a1 : 0u) ^ (k & 4 ? a2 : 0u);
+          v[0][k] = *reinterpret_cast<const A*>(smem + (off ^ ak));
+          v[1][k] = *reinterpret_cast<const A*>(smem + (off1 ^ ak));
+        }
+        uint32_t wn = *reinterpret_cast<const uint32_t*>(&st[sg.term_begin].zg);  // zg, kap, pat
+        double cn = coef[sg.term_begin];
         for (int t = sg.term_begin; t < sg.term_end; t++) {
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(&st[t].zg);  // zg, kap, pat
-          const double c = flip_sign(coef[t], __popc(w & 0xffffu & (g0 + tid)) & 1);
-          const uint32_t pat = w >> 24;
-          const bool odd = st[t].odd != 0;
-          switch (w >> 16 & 7u) {
-            case 0:
-#pragma unroll
-              for (int k = 0; k < 8; k++) {
-                const double x = v[k].x, y = v[k].y;
-                acc = fma(flip_sign(c, pat >> k & 1u), x * x + y * y, acc);
-              }
-              break;
-            case 1: acc = pairs<A, 1>(v, c, pat, odd, acc); break;
-            case 2: acc = pairs<A, 2>(v, c, pat, odd, acc); break;
-            case 3: acc = pairs<A, 3>(v, c, pat, odd, acc); break;
-            case 4: acc = pairs<A, 4>(v, c, pat, odd, acc); break;
-            case 5: acc = pairs<A, 5>(v, c, pat, odd, acc); break;
-            case 6: acc = pairs<A, 6>(v, c, pat, odd, acc); break;
-            default: acc = pairs<A, 7>(v, c, pat, odd, acc); break;
+          const uint32_t w = wn, pat = w >> 24;
+          const double ct = cn;
+          const int tn = t + 1 < sg.term_end ? t + 1 : t;  // the next string's, while this one is summed
+          wn = *reinterpret_cast<const uint32_t*>(&st[tn].zg);
+          cn = coef[tn];
+          const double c[2] = {flip_sign(ct, __popc(w & 0xffffu & (g0 + tid)) & 1),
+                               two ? flip_sign(ct, __popc(w & 0xffffu & (g0 + NT + tid)) & 1) : 0.0};
+          opaque(v[0]);
+          opaque(v[1]);
+          switch (w >> 16 & 15u) {
+#define MLB_P(k) \
+  case k: pairs<A, k & 7, (k > 7)>(v, c, pat, acc); break;
+            MLB_P(0) MLB_P(1) MLB_P(2) MLB_P(3) MLB_P(4) MLB_P(5) MLB_P(6) MLB_P(7)
+            MLB_P(9) MLB_P(10) MLB_P(11) MLB_P(12) MLB_P(13) MLB_P(14) MLB_P(15)
+#undef MLB_P
           }
         }
       }
     }
     __syncthreads();
   }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if ((tid & 31) == 0) red[tid >> 5] = acc;
+  double sum = acc[0] + acc[1];
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+  if ((tid & 31) == 0) red[tid >> 5] = sum;
   __syncthreads();
   if (tid == 0) {
     double s = 0.0;
@@ -203,20 +223,15 @@ __global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__
   if (threadIdx.x == 0) out[0] = red[0];
 }
 
-// lambda[k] += +-c (1 or i) psi[k ^ KAP]; the sign is that of the source.
-template <typename A, int KAP>
-__device__ __forceinline__ void apply_string(const A (&v)[8], double2 (&l)[8], double c, uint32_t pat, bool odd) {
+// lambda[k] += +-c (ODD: times i) psi[k ^ KAP]; the sign is that of the source.
+template <typename A, int KAP, bool ODD>
+__device__ __forceinline__ void apply_string(const A (&v)[8], double2 (&l)[8], double c, uint32_t pat) {
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     const double cs = flip_sign(c, pat >> (k ^ KAP) & 1u);
     const double x = v[k ^ KAP].x, y = v[k ^ KAP].y;
-    if (odd) {  // times i
-      l[k].x = fma(-cs, y, l[k].x);
-      l[k].y = fma(cs, x, l[k].y);
-    } else {
-      l[k].x = fma(cs, x, l[k].x);
-      l[k].y = fma(cs, y, l[k].y);
-    }
+    l[k].x = ODD ? fma(-cs, y, l[k].x) : fma(cs, x, l[k].x);
+    l[k].y = ODD ? fma(cs, x, l[k].y) : fma(cs, y, l[k].y);
   }
 }
 
@@ -283,20 +298,20 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(Real) == 8 ? 3 : 2)
           v[k] = *reinterpret_cast<const A*>(smem + at);
           l[k] = *reinterpret_cast<const double2*>(ltile + (at << UB));
         }
+        uint32_t wn = *reinterpret_cast<const uint32_t*>(&st[sg.term_begin].zg);  // zg, kap, pat
+        double cn = coef[sg.term_begin];
         for (int t = sg.term_begin; t < sg.term_end; t++) {
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(&st[t].zg);  // zg, kap, pat
-          const double c = flip_sign(coef[t], __popc(w & 0xffffu & (g0 + tid)) & 1);
-          const uint32_t pat = w >> 24;
-          const bool odd = st[t].odd != 0;
-          switch (w >> 16 & 7u) {
-            case 0: apply_string<A, 0>(v, l, c, pat, odd); break;
-            case 1: apply_string<A, 1>(v, l, c, pat, odd); break;
-            case 2: apply_string<A, 2>(v, l, c, pat, odd); break;
-            case 3: apply_string<A, 3>(v, l, c, pat, odd); break;
-            case 4: apply_string<A, 4>(v, l, c, pat, odd); break;
-            case 5: apply_string<A, 5>(v, l, c, pat, odd); break;
-            case 6: apply_string<A, 6>(v, l, c, pat, odd); break;
-            default: apply_string<A, 7>(v, l, c, pat, odd); break;
+          const uint32_t w = wn, pat = w >> 24;
+          const double c = flip_sign(cn, __popc(w & 0xffffu & (g0 + tid)) & 1);
+          const int tn = t + 1 < sg.term_end ? t + 1 : t;
+          wn = *reinterpret_cast<const uint32_t*>(&st[tn].zg);
+          cn = coef[tn];
+          switch (w >> 16 & 15u) {
+#define MLB_A(k) \
+  case k: apply_string<A, k & 7, (k > 7)>(v, l, c, pat); break;
+            MLB_A(0) MLB_A(1) MLB_A(2) MLB_A(3) MLB_A(4) MLB_A(5) MLB_A(6) MLB_A(7)
+            MLB_A(9) MLB_A(10) MLB_A(11) MLB_A(12) MLB_A(13) MLB_A(14) MLB_A(15)
+#undef MLB_A
           }
         }
 #pragma unroll

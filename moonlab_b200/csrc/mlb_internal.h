@@ -168,10 +168,9 @@ struct PauliTerm {
   double c;          // coefficient with the string's constant signs
   uint64_t z;        // Z mask; the tile's sign is parity(z & base)
   uint16_t zg;       // the group's: parity(zg & group index)
-  uint8_t kap;       // its X mask among the segment's directions
+  uint8_t kap;       // its X mask among the segment's directions; + 8: an odd number of Y's
   uint8_t pat;       // bit k: the sign of register index k
-  uint8_t odd;       // an odd number of Y's: the imaginary part
-  uint8_t pad[3];
+  uint32_t pad;
 };
 struct PauliSeg {
   uint16_t alpha[3];                 // byte offsets in the tile of its directions

@@ -151,7 +151,7 @@ inline void plan(int n, int TB, int L, int dtype, size_t num, const uint64_t* xm
           if (hea::parity(global(order[j]) & zm[i])) d.zg |= (uint16_t)(1u << j);
         const int ny = __builtin_popcountll(xm[i] & zm[i]) & 3;
         const double c = coeff ? coeff[i] : 1.0;
-        d.odd = (uint8_t)(ny & 1);
+        if (ny & 1) d.kap |= 8;
         if (lambda) {
           d.c = ny >= 2 ? -c : c;  // i^{ny}: 1, i, -1, -i
         } else {
