@@ -54,7 +54,8 @@ constexpr int kUnladderBits = 11, kUnladderLow = 4;  // tile of k_unladder, cont
 // tiles, so three CTAs per SM overlap one's copies with the others' work.
 // Measured, 20 qubits, 8 layers, 256 vectors with gradients: 616 ms by
 // gate-by-gate passes with the CNOTs carried out (19 forward, 17 backward),
-// 134 ms by these (6 and 9); complex64 326 -> 116 ms.
+// 134 ms by these (6 and 9); complex64 326 -> 116 ms, and of 100 ms after
+// lambda's passes 90 ms with values converted to FP64 once a segment.
 template <typename Real> struct HeaCfg;
 template <> struct HeaCfg<double> { static constexpr int FWD_BITS = 12, BACK_BITS = 11; };
 template <> struct HeaCfg<float> { static constexpr int FWD_BITS = 13, BACK_BITS = 12; };
@@ -63,10 +64,10 @@ constexpr int kHeaThreads = 128, kHeaWarps = kHeaThreads / 32;
 // Per-state tables of a segment.
 template <typename Real>
 struct HeaTab {
-  typename Cplx<Real>::T ph[8];  // scale * exp(-+ i ...) per register index
+  typename Cplx<Real>::T ph[4];  // scale * exp(-+ i ...) for register indexes 0 .. 3; 7 - k has the conjugate of k's
   Real t[3];                     // tangent, or cotangent where `flip`
   uint32_t flip;                 // bit i: rotation i uses the cotangent form
-  double unscale;                // 1 / scale^2 (d/dRY is taken on scaled states)
+  double unscale;                // 1 / scale^2 (the gradients are taken on scaled states)
 };
 
 // v[k], v[k1] <- RY (forward) or its inverse (BACK), up to the scale.
@@ -90,19 +91,25 @@ __device__ __forceinline__ void hea_ry(A (&v)[8], Real t, bool flip) {
   }
 }
 
-// Im<lambda|Y|psi> over the pairs of register bit RT:
-// (Y psi)_0 = -i psi_1, (Y psi)_1 = i psi_0.
-template <typename A, int RT>
-__device__ __forceinline__ double hea_grad_y(const A (&v)[8], const A (&w)[8]) {
+// Im<lambda|Y|psi> over the pairs of register bit RT.
+template <int RT>
+__device__ __forceinline__ double hea_grad_y(const double2 (&v)[8], const double2 (&w)[8]) {
   double acc = 0.0;
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     if (k & (1 << RT)) continue;
-    const A p0 = v[k], p1 = v[k | (1 << RT)], l0 = w[k], l1 = w[k | (1 << RT)];
-    acc -= (double)l0.x * p1.x + (double)l0.y * p1.y;
-    acc += (double)l1.x * p0.x + (double)l1.y * p0.y;
+    const double2 p0 = v[k], p1 = v[k | (1 << RT)], l0 = w[k], l1 = w[k | (1 << RT)];
+    acc -= l0.x * p1.x + l0.y * p1.y;
+    acc += l1.x * p0.x + l1.y * p0.y;
   }
   return acc;
+}
+
+// x times the phase of register index k (a constant): conj(ph[7 - k]) from 4 on.
+template <typename A>
+__device__ __forceinline__ A turn(const A (&ph)[4], int k, A x) {
+  const A p = k < 4 ? ph[k] : ph[7 - k];
+  return k < 4 ? A{p.x * x.x - p.y * x.y, p.x * x.y + p.y * x.x} : A{p.x * x.x + p.y * x.y, p.x * x.y - p.y * x.x};
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -171,10 +178,10 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
         }
       }
       if (ti == 0) {  // this state's tables, while the tile is on its way
-        for (int i = tid; i < P.num_segs * 8; i += NT) {
-          const HeaSeg& sg = sseg[i >> 3];
-          HeaTab<Real>& tb = tab[i >> 3];
-          const int k = i & 7;
+        for (int i = tid; i < P.num_segs * 4; i += NT) {
+          const HeaSeg& sg = sseg[i >> 2];
+          HeaTab<Real>& tb = tab[i >> 2];
+          const int k = i & 3;
           double pr = 1.0, pi = 0.0, scale = 1.0;
           uint32_t flips = 0;
 #pragma unroll
@@ -222,6 +229,9 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
           if (tid >> q & 1) off0 ^= sg.kappa[q];
         const uint32_t flip = tb.flip;
         const Real t0 = tb.t[0], t1 = tb.t[1], t2 = tb.t[2];
+        A ph[4];  // read once: a broadcast 16-byte load takes four wavefronts
+#pragma unroll
+        for (int k = 0; k < 4; k++) ph[k] = tb.ph[k];
         double acc[8];
         if (BACK) {
 #pragma unroll
@@ -242,23 +252,32 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
               if (BACK) w[k] = *reinterpret_cast<const A*>(at + tile_bytes);
             }
             if (BACK) {
-              // Im(conj(lambda) psi) per amplitude, summed with the sign of each target bit
+#pragma unroll
+              for (int k = 0; k < 8; k++) {
+                v[k] = turn(ph, k, v[k]);
+                w[k] = turn(ph, k, w[k]);
+              }
+              // On the scaled states (the phases cancel): Im(conj(lambda) psi)
+              // per amplitude, summed with the sign of each target bit, and
+              // Im<lambda|Y|psi> of each: (Y psi)_0 = -i psi_1, (Y psi)_1 = i psi_0.
+              // complex64 values are converted once: conversions run at a
+              // quarter of the FP64 rate.
+              double2 V[8], L[8];
+#pragma unroll
+              for (int k = 0; k < 8; k++) {
+                V[k] = make_double2(v[k].x, v[k].y);
+                L[k] = make_double2(w[k].x, w[k].y);
+              }
               double d[8];
 #pragma unroll
-              for (int k = 0; k < 8; k++) d[k] = (double)w[k].x * v[k].y - (double)w[k].y * v[k].x;
+              for (int k = 0; k < 8; k++) d[k] = L[k].x * V[k].y - L[k].y * V[k].x;
               const double s0 = d[0] + d[1], s1 = d[2] + d[3], s2 = d[4] + d[5], s3 = d[6] + d[7];
               acc[0] += ((d[0] - d[1]) + (d[2] - d[3])) + ((d[4] - d[5]) + (d[6] - d[7]));
               acc[1] += (s0 - s1) + (s2 - s3);
               acc[2] += (s0 + s1) - (s2 + s3);
-#pragma unroll
-              for (int k = 0; k < 8; k++) {
-                const A ph = tb.ph[k];
-                v[k] = cmul(ph, v[k]);
-                w[k] = cmul(ph, w[k]);
-              }
-              acc[3] += hea_grad_y<A, 0>(v, w);
-              acc[4] += hea_grad_y<A, 1>(v, w);
-              acc[5] += hea_grad_y<A, 2>(v, w);
+              acc[3] += hea_grad_y<0>(V, L);
+              acc[4] += hea_grad_y<1>(V, L);
+              acc[5] += hea_grad_y<2>(V, L);
               hea_ry<A, Real, 0, true>(v, t0, flip & 1u);
               hea_ry<A, Real, 0, true>(w, t0, flip & 1u);
               hea_ry<A, Real, 1, true>(v, t1, flip & 2u);
@@ -270,7 +289,7 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
               hea_ry<A, Real, 1, false>(v, t1, flip & 2u);
               hea_ry<A, Real, 2, false>(v, t2, flip & 4u);
 #pragma unroll
-              for (int k = 0; k < 8; k++) v[k] = cmul(tb.ph[k], v[k]);
+              for (int k = 0; k < 8; k++) v[k] = turn(ph, k, v[k]);
             }
 #pragma unroll
             for (int k = 0; k < 8; k++) {
@@ -315,8 +334,7 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
       for (int j = tid; j < nslots; j += NT) {
         double t = 0.0;
         for (int wp = 0; wp < kHeaWarps; wp++) t += red[wp * nslots + j];
-        if (j % kHeaSlots >= 3) t *= tab[j / kHeaSlots].unscale;
-        partials[item * (uint64_t)part_stride + j] = t;
+        partials[item * (uint64_t)part_stride + j] = t * tab[j / kHeaSlots].unscale;
       }
       __syncthreads();
     }
