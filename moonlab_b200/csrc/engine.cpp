@@ -1154,9 +1154,7 @@ static int probs_z(mlb_state_t* s, std::vector<double>& out) {
   DeviceGuard dg(s->device);
   int rc = flush_impl(s);
   if (rc) return rc;
-  const uint64_t dim = 1ull << s->n;
-  const uint64_t chunks = s->n >= 13 ? dim >> 13 : 1;
-  const size_t need = sizeof(double) * ((size_t)s->num_sms * 4 * 14 + chunks + 64 + 64);
+  const size_t need = sizeof(double) * ((size_t)s->num_sms * 4 * 35 + 64);  // results, then every CTA's 35 sums
   rc = ensure_scratch(s, need);
   if (rc) return rc;
   double* d_out = s->d_scratch;

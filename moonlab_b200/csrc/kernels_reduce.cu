@@ -6,8 +6,9 @@
 // reads amplitudes t + 256 k (k < 32), so the low 8 index bits are the
 // thread's own (constant), bits 8..12 are the loop counter (compile-time
 // after unrolling) and bits >= 13 are the chunk index (constant per chunk).
-// Per amplitude that costs one |a|^2 and ~2.5 FP64 adds; the chunk totals go
-// to a small buffer that a second kernel folds into the high-bit sums.
+// Per amplitude that costs one |a|^2 and ~2.5 FP64 adds; lane b of a CTA's
+// first warp adds a chunk's total to the sum of bit 13 + b.  A second kernel
+// folds the CTAs' sums.
 // All reductions use a fixed order, so results are identical run to run.
 #include <algorithm>
 #include <atomic>
@@ -24,6 +25,7 @@ namespace {
 constexpr int kRT = 256;        // threads per CTA
 constexpr int kRK = 32;         // amplitudes per thread per chunk
 constexpr int kChunkBits = 13;  // 2^13 amplitudes per chunk
+constexpr int kSums = 1 + 34;    // a CTA's sums: the total, then every bit's
 
 template <typename A> __device__ __forceinline__ double norm2(const A& a) {
   const double x = (double)a.x, y = (double)a.y;
@@ -42,15 +44,15 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return r;  // valid in thread 0
 }
 
-// Pass 1: per-CTA sums for bits 0..12 (+ total) and per-chunk totals.
+// Pass 1: every CTA's total and its sum for every bit.
 template <typename Real>
 __global__ void __launch_bounds__(kRT) k_probs_z_pass1(const typename Cplx<Real>::T* __restrict__ amp,
                                                        uint64_t num_chunks, uint32_t chunk_amps,
-                                                       double* __restrict__ chunk_tot,
                                                        double* __restrict__ partials) {
   __shared__ double red[kRT / 32];
   double low_tot = 0.0;                 // this thread's total (its low bits are fixed)
   double mid[kChunkBits - 8] = {0, 0, 0, 0, 0};
+  double high = 0.0;                    // first warp: the sum of bit 13 + lane
   for (uint64_t c = blockIdx.x; c < num_chunks; c += gridDim.x) {
     const uint64_t base = c << kChunkBits;
     double ctot = 0.0;
@@ -76,11 +78,15 @@ __global__ void __launch_bounds__(kRT) k_probs_z_pass1(const typename Cplx<Real>
       }
     }
     low_tot += ctot;
-    const double t = block_sum(ctot, red);
-    if (threadIdx.x == 0) chunk_tot[c] = t;
+    double t = ctot;
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x < 32 && (c >> threadIdx.x & 1ull))
+      for (int w = 0; w < kRT / 32; w++) high += red[w];
   }
-  // Per-CTA partials: [0] total, [1+b] bit b for b < 13.
-  double* out = partials + (size_t)blockIdx.x * (1 + kChunkBits);
+  double* out = partials + (size_t)blockIdx.x * kSums;
   double v = block_sum(low_tot, red);
   if (threadIdx.x == 0) out[0] = v;
   for (int b = 0; b < 8; b++) {
@@ -91,34 +97,17 @@ __global__ void __launch_bounds__(kRT) k_probs_z_pass1(const typename Cplx<Real>
     v = block_sum(mid[b], red);
     if (threadIdx.x == 0) out[1 + 8 + b] = v;
   }
+  if (threadIdx.x < kSums - 1 - kChunkBits) out[1 + kChunkBits + threadIdx.x] = high;
 }
 
-// Pass 2 (one CTA): fold CTA partials and chunk totals into out[0..n) = P1,
-// out[n] = norm.
-__global__ void __launch_bounds__(kRT) k_probs_z_pass2(const double* __restrict__ chunk_tot,
-                                                       uint64_t num_chunks,
-                                                       const double* __restrict__ partials,
-                                                       int num_parts, int n,
+// Pass 2 (one CTA, a warp per sum): out[0..n) = P1, out[n] = norm.
+__global__ void __launch_bounds__(kRT) k_probs_z_pass2(const double* __restrict__ partials, int num_parts, int n,
                                                        double* __restrict__ out) {
-  __shared__ double red[kRT / 32];
-  // low bits and total from the CTA partials (fixed order)
-  for (int j = 0; j < 1 + kChunkBits; j++) {
+  for (int j = threadIdx.x >> 5; j <= n; j += kRT / 32) {
     double v = 0.0;
-    for (int i = threadIdx.x; i < num_parts; i += kRT) v += partials[(size_t)i * (1 + kChunkBits) + j];
-    v = block_sum(v, red);
-    if (threadIdx.x == 0) {
-      if (j == 0) out[n] = v;
-      else if (j - 1 < n) out[j - 1] = v;
-    }
-  }
-  // high bits from the chunk totals
-  for (int b = kChunkBits; b < n; b++) {
-    const int cb = b - kChunkBits;
-    double v = 0.0;
-    for (uint64_t c = threadIdx.x; c < num_chunks; c += kRT)
-      if (c >> cb & 1ull) v += chunk_tot[c];
-    v = block_sum(v, red);
-    if (threadIdx.x == 0) out[b] = v;
+    for (int i = threadIdx.x & 31; i < num_parts; i += 32) v += partials[(size_t)i * kSums + j];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) out[j == 0 ? n : j - 1] = v;
   }
 }
 
@@ -179,16 +168,11 @@ int launch_reduce_probs_z(int dtype, const void* amp, int n, double* d_out, doub
   const uint64_t num_chunks = n >= kChunkBits ? dim >> kChunkBits : 1;
   const uint32_t chunk_amps = n >= kChunkBits ? (1u << kChunkBits) : (uint32_t)dim;
   int grid = (int)std::min<uint64_t>(num_chunks, (uint64_t)num_sms * 4);
-  // partials layout: [grid x 14] then chunk totals
-  double* parts = d_partials;
-  double* chunk_tot = d_partials + (size_t)grid * (1 + kChunkBits);
   if (dtype == MLB_C128)
-    k_probs_z_pass1<double><<<grid, kRT, 0, stream>>>((const double2*)amp, num_chunks, chunk_amps,
-                                                      chunk_tot, parts);
+    k_probs_z_pass1<double><<<grid, kRT, 0, stream>>>((const double2*)amp, num_chunks, chunk_amps, d_partials);
   else
-    k_probs_z_pass1<float><<<grid, kRT, 0, stream>>>((const float2*)amp, num_chunks, chunk_amps,
-                                                     chunk_tot, parts);
-  k_probs_z_pass2<<<1, kRT, 0, stream>>>(chunk_tot, num_chunks, parts, grid, n, d_out);
+    k_probs_z_pass1<float><<<grid, kRT, 0, stream>>>((const float2*)amp, num_chunks, chunk_amps, d_partials);
+  k_probs_z_pass2<<<1, kRT, 0, stream>>>(d_partials, grid, n, d_out);
   count_launch(2);
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }
@@ -222,16 +206,14 @@ int launch_scale(int dtype, void* amp, int n, double factor, uint64_t keep_mask,
 // ---- probs_z without device allocation -------------------------------------
 // mlb_prob_one_all_noalloc runs the probs_z reduction above on caller-owned
 // buffers, with its scratch in one fixed array per device instead of a
-// cudaMalloc'd buffer.  Scratch use: pass-1 partials ([grid x 14] doubles,
-// grid <= kNoAllocMaxParts) followed by one total per 2^13-amplitude chunk
-// (2^(n-13) doubles, at most 2^17 for n = 30).  Pass 1 writes every entry
-// pass 2 reads, so nothing is cleared between calls.
+// cudaMalloc'd buffer.  Scratch use: pass-1 partials ([grid x 35] doubles,
+// grid <= kNoAllocMaxParts).  Pass 1 writes every entry pass 2 reads, so
+// nothing is cleared between calls.
 namespace {
 
 constexpr uint32_t kNoAllocMaxQubits = 30;
 constexpr int kNoAllocMaxParts = 1024;  // pass-1 CTAs; the grid is min(chunks, 4 * SMs)
-constexpr size_t kNoAllocScratchDoubles =
-    (size_t)kNoAllocMaxParts * (1 + 13) + (size_t(1) << (kNoAllocMaxQubits - 13));  // 145,408
+constexpr size_t kNoAllocScratchDoubles = (size_t)kNoAllocMaxParts * mlb::kSums;  // 35,840
 constexpr int kNoAllocMaxDevices = 64;
 
 static __device__ __align__(256) double g_probs_z_scratch[kNoAllocScratchDoubles];

@@ -48,8 +48,9 @@ constexpr int kCB = 12;             // chunk = 2^12 elements (33 KiB of p in sha
 constexpr int kCT = 256;            // threads per CTA
 constexpr int kPer = (1 << kCB) / kCT;  // 32 contiguous elements per thread
 constexpr long long kTwo53 = 1ll << 53;
-constexpr int kDPer = 8;                // phase D: chunks per thread in one scan
-constexpr int kDBatch = kCT * kDPer;     // phase D: 2048 chunks per scan
+constexpr int kDT = 512;                 // phase D: threads of its one CTA
+constexpr int kDPer = 8;                 // phase D: chunks per thread in one scan
+constexpr int kDBatch = kDT * kDPer;     // phase D: 4096 chunks per scan
 constexpr int kNoBinade = -0x40000000;   // matches no candidate binade
 constexpr int kZeroChunk = 0x7fffffff;   // Xfer::e[0] of a chunk that adds 0 for every s
 
@@ -66,6 +67,7 @@ struct SeqScratch {
   Xfer* xfer;          // [nc]
   double* s_in;        // [nc + 1] exact running value before chunk c; s_in[nc] = total
   long long* lastnz;   // [1] largest index with p > 0 (within the filter), -1 if none
+  uint32_t* slow;      // [1 + nc] chunks left to the ordered phase C: their number, then they
   double* uni;         // [num] uniforms (sampling)
   unsigned long long* outc;  // [num] outcomes (sampling)
 };
@@ -115,7 +117,7 @@ template <typename Real, bool FUSED>
 __device__ __forceinline__ void load_chunk_p(const typename Cplx<Real>::T* __restrict__ amp,
                                              uint64_t base, uint32_t len, uint64_t fmask,
                                              uint64_t fval, double* sp) {
-  for (uint32_t j = threadIdx.x; j < len; j += kCT)
+  for (uint32_t j = threadIdx.x; j < len; j += blockDim.x)
     sp[j + (j >> 5)] = elem_val<Real, FUSED>(amp, base + j, fmask, fval);
 }
 
@@ -276,29 +278,92 @@ __device__ __forceinline__ Fn elem_fn(double v, double inv_g) {
   return f;
 }
 
-// Phase C: transfer tables for the two candidate binades of each chunk.
+// The candidate binades of the running value at a chunk's start: the prefix
+// estimate S +- a bound on both its error and the reference's.
+__device__ __forceinline__ void candidates(double S, uint64_t base, int (&ecand)[2]) {
+  ecand[0] = ecand[1] = INT32_MIN;
+  if (!(S > 0.0)) return;
+  const double rel = ((double)base * 4.0 + 1.0e6) * 0x1p-53;
+  const int elo = binade_of(S * (1.0 - rel)), ehi = binade_of(S * (1.0 + rel));
+  if (ehi - elo > 1) return;  // too uncertain
+  ecand[0] = elo;
+  if (ehi != elo) ecand[1] = ehi;
+}
+
+// Phase C, the common chunks: one candidate binade and every element's
+// x^2 + y^2 where it rounds as its contribution does (elem_p_on_grids), no
+// tie among them.  The increments are then the same for both parities and
+// add up in any order, so a warp takes a chunk with coalesced loads and no
+// staging: HBM-bound (30 qubits: 5.8 ms by ordered tables for every chunk,
+// 2.9 ms by these).  Other chunks go to k_seq_c's list.
+template <typename Real, bool FUSED>
+__global__ void __launch_bounds__(kCT) k_seq_c_sums(const typename Cplx<Real>::T* __restrict__ amp, uint64_t nc,
+                                                    uint32_t clen, uint64_t fmask, uint64_t fval,
+                                                    const double* __restrict__ ctot, const double* __restrict__ pre,
+                                                    Xfer* __restrict__ xfer, uint32_t* __restrict__ slow) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t nwarps = (uint64_t)gridDim.x * (kCT / 32);
+  for (uint64_t c = (uint64_t)blockIdx.x * (kCT / 32) + (threadIdx.x >> 5); c < nc; c += nwarps) {
+    const uint64_t base = c * clen;
+    int ecand[2];
+    candidates(pre[c], base, ecand);
+    bool ordered = ecand[1] != INT32_MIN;
+    long long sum = 0;
+    if (ecand[0] != INT32_MIN && !ordered && ctot[c] != 0.0) {
+      const double ig = 1.0 / grid_of(ecand[0]);
+      bool unsafe = false;
+      for (uint32_t j0 = lane; j0 < clen; j0 += 32 * 8) {
+        typename Cplx<Real>::T a[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {  // eight loads in flight
+          const uint32_t j = j0 + 32 * k;
+          a[k].x = a[k].y = 0;
+          if (j < clen && ((base + j) & fmask) == fval) a[k] = amp[base + j];
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const double x = (double)a[k].x, y = (double)a[k].y;
+          const double pa = fma(x, x, y * y), q = pa * ig;
+          const bool zero = x == 0.0 && y == 0.0, ok = pa >= 0x1p-1000 && grid_safe(pa, ig);
+          unsafe = unsafe || !(ok || zero);
+          // q < 2^52: q + 2^52 rounds q to an integer, ties aside as the sum does
+          sum += ok ? __double_as_longlong(q + 0x1p52) - 0x4330000000000000ll : 0ll;
+        }
+      }
+      sum = sum > kTwo53 ? kTwo53 : sum;
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      ordered = __any_sync(0xffffffffu, unsafe);
+    }
+    if (lane != 0) continue;
+    if (ordered) {
+      slow[1 + atomicAdd(&slow[0], 1u)] = (uint32_t)c;
+      continue;
+    }
+    Xfer x;
+    x.e[0] = ctot[c] == 0.0 ? kZeroChunk : ecand[0];
+    x.e[1] = INT32_MIN;
+    x.K[0][0] = x.K[0][1] = sum > kTwo53 ? kTwo53 : sum;
+    x.K[1][0] = x.K[1][1] = 0;
+    x.P = (int)(x.K[0][0] & 1) | (int)((x.K[0][0] + 1) & 1) << 1 | 2 << 2;
+    x.pad = 0;
+    xfer[c] = x;
+  }
+}
+
+// Phase C, the listed chunks: transfer tables for both candidate binades.
 template <typename Real, bool FUSED>
 __global__ void __launch_bounds__(kCT) k_seq_c(const typename Cplx<Real>::T* __restrict__ amp,
-                                               uint64_t nc, uint32_t clen, uint64_t fmask,
+                                               uint32_t clen, uint64_t fmask,
                                                uint64_t fval, const double* __restrict__ ctot,
                                                const double* __restrict__ pre,
-                                               Xfer* __restrict__ xfer) {
+                                               Xfer* __restrict__ xfer, const uint32_t* __restrict__ slow) {
   __shared__ double sp[(1 << kCB) + (1 << kCB) / 32];
   __shared__ Fn red[kCT / 32][2];
-  const double u = 0x1p-53;
-  for (uint64_t c = blockIdx.x; c < nc; c += gridDim.x) {
-    const uint64_t base = c * clen;
-    // candidate binades of the running value at the chunk start: the
-    // prefix estimate +- a bound on both its error and the reference's.
-    const double S = pre[c];
-    int ecand[2] = {INT32_MIN, INT32_MIN};
-    if (S > 0.0) {
-      const double rel = ((double)base * 4.0 + 1.0e6) * u;
-      const int elo = binade_of(S * (1.0 - rel)), ehi = binade_of(S * (1.0 + rel));
-      ecand[0] = elo;
-      ecand[1] = (ehi == elo) ? INT32_MIN : ehi;
-      if (ehi - elo > 1) { ecand[0] = INT32_MIN; ecand[1] = INT32_MIN; }  // too uncertain
-    }
+  const uint32_t listed = slow[0];
+  for (uint32_t l = blockIdx.x; l < listed; l += gridDim.x) {
+    const uint64_t c = slow[1 + l], base = c * clen;
+    int ecand[2];
+    candidates(pre[c], base, ecand);
     const double ig0 = ecand[0] != INT32_MIN ? 1.0 / grid_of(ecand[0]) : 0.0;  // exact: powers of two
     const double ig1 = ecand[1] != INT32_MIN ? 1.0 / grid_of(ecand[1]) : 0.0;
     for (uint32_t j = threadIdx.x; j < clen; j += kCT)
@@ -382,12 +447,12 @@ __device__ __forceinline__ Fn shfl_up_fn(const Fn& f, int o) {
 }
 
 template <typename Real, bool FUSED>
-__global__ void __launch_bounds__(kCT) k_seq_d(const typename Cplx<Real>::T* __restrict__ amp,
+__global__ void __launch_bounds__(kDT) k_seq_d(const typename Cplx<Real>::T* __restrict__ amp,
                                                uint64_t nc, uint32_t clen, uint64_t fmask,
                                                uint64_t fval, const Xfer* __restrict__ xfer,
                                                double* __restrict__ s_in) {
   __shared__ double sp[(1 << kCB) + (1 << kCB) / 32];
-  __shared__ Fn wtot[kCT / 32];
+  __shared__ Fn wtot[kDT / 32];
   __shared__ unsigned int s_fail;
   __shared__ double s_run;
   const Fn ident = {0, 0, 0, 1};
@@ -450,7 +515,7 @@ __global__ void __launch_bounds__(kCT) k_seq_d(const typename Cplx<Real>::T* __r
     const unsigned int fail = s_fail;
     if (fail == 0xffffffffu) {
       Fn tot = ident;
-      for (int w = 0; w < kCT / 32; w++) tot = compose(tot, wtot[w]);
+      for (int w = 0; w < kDT / 32; w++) tot = compose(tot, wtot[w]);
       b += (unsigned long long)(pb ? tot.K1 : tot.K0);
       c = min(nc, c0 + (uint64_t)kDBatch);
       __syncthreads();  // wtot is rewritten by the next batch
@@ -533,7 +598,8 @@ thread_local Cache g_cache;
 
 SeqScratch get_scratch(uint64_t nc, size_t num, cudaStream_t stream) {
   const size_t need = sizeof(double) * nc * 2 + sizeof(Xfer) * nc + sizeof(double) * (nc + 1) +
-                      sizeof(long long) + sizeof(double) * num + sizeof(uint64_t) * num + 256 * 7;
+                      sizeof(long long) + sizeof(uint32_t) * (nc + 1) + sizeof(double) * num + sizeof(uint64_t) * num +
+                      256 * 8;
   int dev = 0;
   cudaGetDevice(&dev);
   if (g_cache.mem == nullptr || g_cache.bytes < need || g_cache.device != dev) {
@@ -557,6 +623,7 @@ SeqScratch get_scratch(uint64_t nc, size_t num, cudaStream_t stream) {
   s.xfer = (Xfer*)take(sizeof(Xfer) * nc);
   s.s_in = (double*)take(sizeof(double) * (nc + 1));
   s.lastnz = (long long*)take(sizeof(long long));
+  s.slow = (uint32_t*)take(sizeof(uint32_t) * (nc + 1));
   s.uni = (double*)take(sizeof(double) * num);
   s.outc = (unsigned long long*)take(sizeof(uint64_t) * num);
   return s;
@@ -575,16 +642,18 @@ int seq_prepare(const void* amp_v, int n, uint64_t fmask, uint64_t fval, size_t 
   if (!sc.chunk_tot) return MLB_ERR_OUT_OF_MEMORY;
   const long long neg1 = -1;
   cudaMemcpyAsync(sc.lastnz, &neg1, sizeof(neg1), cudaMemcpyHostToDevice, stream);
+  cudaMemsetAsync(sc.slow, 0, sizeof(uint32_t), stream);
   // phase A: one warp per chunk, 5 CTAs per SM (its 48 registers allow 5);
   // phase C: one CTA per chunk, 6 CTAs per SM (its shared memory allows 6)
   const int grid_a = (int)std::min<uint64_t>((nc + kCT / 32 - 1) / (kCT / 32), (uint64_t)num_sms * 5);
   const int grid = (int)std::min<uint64_t>(nc, (uint64_t)num_sms * 6);
   k_seq_a<Real, FUSED><<<grid_a, kCT, 0, stream>>>(amp, nc, clen, fmask, fval, sc.chunk_tot, sc.lastnz);
   k_seq_b<<<1, 1024, 0, stream>>>(sc.chunk_tot, nc, sc.chunk_pre);
-  k_seq_c<Real, FUSED><<<grid, kCT, 0, stream>>>(amp, nc, clen, fmask, fval, sc.chunk_tot,
-                                                 sc.chunk_pre, sc.xfer);
-  k_seq_d<Real, FUSED><<<1, kCT, 0, stream>>>(amp, nc, clen, fmask, fval, sc.xfer, sc.s_in);
-  count_launch(4);
+  k_seq_c_sums<Real, FUSED><<<grid_a, kCT, 0, stream>>>(amp, nc, clen, fmask, fval, sc.chunk_tot, sc.chunk_pre,
+                                                        sc.xfer, sc.slow);
+  k_seq_c<Real, FUSED><<<grid, kCT, 0, stream>>>(amp, clen, fmask, fval, sc.chunk_tot, sc.chunk_pre, sc.xfer, sc.slow);
+  k_seq_d<Real, FUSED><<<1, kDT, 0, stream>>>(amp, nc, clen, fmask, fval, sc.xfer, sc.s_in);
+  count_launch(5);
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }
 
