@@ -398,16 +398,17 @@ void mlb_control_destroy(mlb_control_t *c);
 typedef struct {
     uint64_t passes;
     uint64_t ops;
-    uint64_t dense_blocks;   /* fused complex64 blocks, or complex128 segments run as dense
-                                matrices on the FP64 tensor cores */
+    uint64_t dense_blocks;   /* fused complex64 blocks, or complex128 segments run as products of
+                                their gates: 16x16 matrices on the FP64 tensor cores, or rotation
+                                programs */
     uint64_t bytes_moved;    /* HBM bytes of the tiles the launched passes ran over (2 x state
                                 bytes per pass, less the tiles skipped as all-zero) */
     uint64_t kernel_launches;
     uint64_t segments;       /* shared-memory register-group round trips over all passes */
     double   gpu_ms;         /* device time of the flush's kernels (timing enabled), else 0 */
     uint64_t plan_cache_hit; /* 1 when the plan came from the state's plan cache */
-    uint64_t dense_amps;     /* complex128: amplitudes times dense segments applied to them
-                                (FP64 tensor-core work = 96 flops each) */
+    uint64_t dense_amps;     /* complex128: amplitudes times tensor-core segments applied to them
+                                (96 flops each) */
 } mlb_flush_stats_t;
 int  mlb_last_flush_stats(mlb_state_t *s, mlb_flush_stats_t *out);
 /* Plan cache for repeated circuit shapes (tiled mode): up to `entries` plans
@@ -455,8 +456,10 @@ int  mlb_plan_ops(const mlb_op_t *ops, size_t num_ops, uint32_t num_qubits, int 
  * among its register bits (tile bits bits[0..nbits-1]).  mode: 0 gate by
  * gate, 1 one generic 4x4 op in shared memory, 2 a dense 16x16 complex128
  * matrix on the FP64 tensor cores (dtype MLB_C128 with dense segments on,
- * as a state flushes by default).  Segments index the ops [op_begin,
- * op_end) of the execution order.  Call with NULL buffers to learn the
+ * as a state flushes by default).  A pass of one-qubit unitaries, CNOTs,
+ * SWAPs and diagonals may run its ops as one rotation program instead of
+ * these segments (complex128 from 13 qubits, complex64 from 21).  Segments
+ * index the ops [op_begin, op_end) of the execution order.  Call with NULL buffers to learn the
  * sizes; a buffer too small gives MLB_ERR_INVALID_ARG. */
 typedef struct {
     uint8_t  high[16];

@@ -27,6 +27,7 @@
 #include "mlb_internal.h"
 #include "pauli_plan.h"
 #include "planner.h"
+#include "rotate_plan.h"
 
 extern "C" {
 void mlb_mat_rx(double theta, double m[8]);
@@ -536,9 +537,37 @@ int flush_fused(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   return MLB_OK;
 }
 
+// Where tile passes run as rotation programs (rotate_plan.h), measured on
+// brickwork circuits (depth 20, ZZ every 4 layers; wall ms, programs against
+// the segments that ran before):
+//   complex128, dense 16x16 segments: 13 qubits 1.05 / 1.48, 20: 1.48 / 3.12,
+//     24: 5.4 / 6.6, 25: 9.9 / 10.3, 26: 19.0 / 18.6, 28: 75.9 / 69.4 (QAOA,
+//     3 layers, 28: 36.1 / 37.4).  Up to 25 qubits the matrices' host time
+//     counts as much as the passes, above each pass takes the cheaper form.
+//   complex64, gate by gate: 18 qubits 1.48 / 1.15, 20: 1.54 / 1.42, 22: 1.95 /
+//     2.64, 24: 4.1 / 8.2, 28: 52 / 138 (QAOA: 20: 0.56 / 0.48, 22: 0.83 /
+//     1.81, 28: 20 / 82).
+constexpr uint32_t kRotMinC128 = 13, kRotAllC128 = 25, kRotMinC64 = 21;
+
+// A program's cost beside a dense segment's, from their times per pass of a
+// 30-qubit complex128 state (ms).
+double rot_cost(const rot::Program& p) {
+  double c = 1.03 * (double)p.segs.size();
+  for (const RotOp& o : p.ops) c += (o.flags & kRotTable ? 0.39 : 0.0) + (o.flags & kRotTurn ? 0.58 : 0.0);
+  return c;
+}
+constexpr double kDenseSegmentCost = 3.0;
+
 // Tile passes for ops (tiled mode, and the parts of a fused flush that need
 // them), the plan taken from the state's plan cache when the shape repeats.
-int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_t& st) {
+int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& given, mlb_flush_stats_t& st) {
+  const bool rot_on = s->dtype == MLB_C64 ? s->n >= kRotMinC64 : s->dense_c128 && s->n >= kRotMinC128;
+  std::vector<mlb_op_t> pushed;
+  if (rot_on && std::all_of(given.begin(), given.end(), rot::covers)) {
+    pushed = given;
+    rot::push_forward(pushed, s->n);
+  }
+  const std::vector<mlb_op_t>& ops = pushed.empty() ? given : pushed;
   const uint64_t dim = 1ull << s->n;
   const uint64_t ab = s->dtype == MLB_C128 ? 16 : 8;
   // the plan: from the cache when this shape ran before, else planned now
@@ -581,19 +610,62 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
     s->plan_hits++;
   }
   E->last_use = ++s->plan_clock;
-  // complex128: register segments that fit run as dense 16x16 matrices on
-  // the FP64 tensor cores (mode 2), built from this circuit's matrices every
-  // flush; which segments fit depends only on the plan's shape, so the upload
-  // layout (and a captured graph's pointers) repeat with the shape
+  // Passes of one-qubit unitaries, CNOTs, SWAPs and diagonals run as rotation
+  // programs (rotate_plan.h), built from this circuit's matrices every flush.
+  // In the others, complex128 register segments that fit run as dense 16x16
+  // matrices on the FP64 tensor cores (mode 2); which segments fit depends
+  // only on the plan's shape, so the upload layout (and a captured graph's
+  // pointers) repeat with the shape.
+  const size_t np = E->passes.size();
+  auto pass_ops = [&](size_t k) {
+    const auto& pp = E->passes[k];
+    return std::make_pair(E->segs[pp.seg_begin].op_begin, E->segs[pp.seg_end - 1].op_end);
+  };
+  std::vector<char> is_rot(np, 0);
+  if (rot_on)
+    for (size_t k = 0; k < np; k++) {
+      const auto [b, e] = pass_ops(k);
+      is_rot[k] = 1;
+      for (int i = b; i < e && is_rot[k]; i++) is_rot[k] = rot::covers(ops[E->src[i]]);
+    }
+  std::vector<rot::Program> progs(np);
+  std::vector<DevPass> rot_pass(np);
+  auto in_threads = [](size_t threads, size_t count, auto&& one) {
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+      for (size_t k; (k = next.fetch_add(1)) < count;) one(k);
+    };
+    const size_t nth = std::min<size_t>({(size_t)std::max(1u, std::thread::hardware_concurrency()), (size_t)16, threads});
+    std::vector<std::thread> pool;
+    for (size_t t = 1; t < nth; t++) pool.emplace_back(work);
+    work();
+    for (auto& t : pool) t.join();
+  };
+  size_t nrot = 0;
+  for (char r : is_rot) nrot += r;
+  in_threads(1 + nrot / 4, np, [&](size_t k) {
+    if (!is_rot[k]) return;
+    std::vector<const mlb_op_t*> po;
+    const auto [b, e] = pass_ops(k);
+    for (int i = b; i < e; i++) po.push_back(&ops[E->src[i]]);
+    rot_pass[k] = rot::filled(E->passes[k].pass, s->dtype == MLB_C128 ? kTileBitsC128 : 13);
+    is_rot[k] = rot::Lower::lower(rot_pass[k], s->dtype, po, progs[k]);
+    if (s->dtype == MLB_C128 && s->n > kRotAllC128 &&
+        rot_cost(progs[k]) > kDenseSegmentCost * E->passes[k].pass.num_segments)
+      is_rot[k] = 0;
+  });
+  nrot = 0;
+  for (char r : is_rot) nrot += r;
   std::vector<DevSegment> dev_segs(E->segs);
   std::vector<DenseSegDev> dsegs;
   std::vector<dense::SegPlan> dplans;
   std::vector<int> dsrc;  // segment of each dense segment
   size_t nfrag = 0;
   if (s->dtype == MLB_C128 && s->dense_c128) {
-    for (const auto& pp : E->passes)
-      for (int k = 0; k < pp.pass.num_segments; k++) {
-        const int si = pp.seg_begin + k;
+    for (size_t k = 0; k < np; k++) {
+      if (is_rot[k]) continue;
+      const auto& pp = E->passes[k];
+      for (int si = pp.seg_begin; si < pp.seg_end; si++) {
         DenseSegDev D;
         dense::SegPlan S;
         if (dense::plan_segment(pp.pass, E->segs[si], E->dops.data(), D, S)) {
@@ -606,38 +678,65 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
           dsrc.push_back(si);
         }
       }
+    }
   }
-  // one upload: ops, segments, dense segments, dense fragments
-  const size_t ob = E->dops.size() * sizeof(DevOp);
-  const size_t sb = dev_segs.size() * sizeof(DevSegment);
-  const size_t soff = (ob + 15) & ~(size_t)15;
-  const size_t doff = (soff + sb + 15) & ~(size_t)15;
-  const size_t foff = (doff + dsegs.size() * sizeof(DenseSegDev) + 15) & ~(size_t)15;
-  const size_t total = foff + nfrag * sizeof(double);
+  // the segment matrices, in parallel over segments (~1 ms of host time each
+  // for 64 variants)
+  std::unique_ptr<double[]> frags(new double[nfrag]);
+  in_threads(1 + nfrag / (256 * 1024), dsegs.size(), [&](size_t d) {
+    dense::fill_fragments(E->segs[dsrc[d]], E->dops.data(), dsegs[d], dplans[d], frags.get() + dsegs[d].frag_off);
+  });
+  // one upload: ops, segments, dense segments, dense fragments, rotation programs
+  size_t total = 0;
+  auto room = [&](size_t bytes) {
+    const size_t at = total;
+    total = (total + bytes + 15) & ~(size_t)15;
+    return at;
+  };
+  const bool any_old = nrot < np;
+  const size_t ob = any_old ? E->dops.size() * sizeof(DevOp) : 0;
+  const size_t sb = any_old ? dev_segs.size() * sizeof(DevSegment) : 0;
+  const size_t ooff = room(ob), soff = room(sb), doff = room(dsegs.size() * sizeof(DenseSegDev));
+  const size_t foff = room(nfrag * sizeof(double));
+  struct RotAt {
+    size_t segs, ops, table;
+  };
+  std::vector<RotAt> at(np);
+  size_t rot_segs = 0, old_segs = 0;
+  for (size_t k = 0; k < np; k++) {
+    if (!is_rot[k]) {
+      old_segs += (size_t)E->passes[k].pass.num_segments;
+      continue;
+    }
+    const rot::Program& pr = progs[k];
+    rot_segs += pr.segs.size();
+    at[k] = {room(pr.segs.size() * sizeof(RotSeg)), room(pr.ops.size() * sizeof(RotOp)), room(pr.table.size() * ab)};
+  }
   std::unique_ptr<unsigned char[]> blob(new unsigned char[total]);
-  std::memset(blob.get(), 0, foff);
-  std::memcpy(blob.get(), E->dops.data(), ob);
-  std::memcpy(blob.get() + soff, dev_segs.data(), sb);
+  if (ob) std::memcpy(blob.get() + ooff, E->dops.data(), ob);
+  if (sb) std::memcpy(blob.get() + soff, dev_segs.data(), sb);
   if (!dsegs.empty()) {
     std::memcpy(blob.get() + doff, dsegs.data(), dsegs.size() * sizeof(DenseSegDev));
-    // the segment matrices, in parallel over segments (~1 ms of host time each
-    // for 64 variants)
-    double* fr = reinterpret_cast<double*>(blob.get() + foff);
-    std::atomic<size_t> next{0};
-    auto work = [&]() {
-      for (size_t k; (k = next.fetch_add(1)) < dsegs.size();)
-        dense::fill_fragments(E->segs[dsrc[k]], E->dops.data(), dsegs[k], dplans[k], fr + dsegs[k].frag_off);
-    };
-    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t nth = std::min<size_t>({hw, (size_t)16, 1 + nfrag / (256 * 1024)});
-    std::vector<std::thread> pool;
-    for (size_t t = 1; t < nth; t++) pool.emplace_back(work);
-    work();
-    for (auto& t : pool) t.join();
+    std::memcpy(blob.get() + foff, frags.get(), nfrag * sizeof(double));
+  }
+  for (size_t k = 0; k < np; k++) {
+    if (!is_rot[k]) continue;
+    const rot::Program& pr = progs[k];
+    std::memcpy(blob.get() + at[k].segs, pr.segs.data(), pr.segs.size() * sizeof(RotSeg));
+    std::memcpy(blob.get() + at[k].ops, pr.ops.data(), pr.ops.size() * sizeof(RotOp));
+    if (s->dtype == MLB_C128) {
+      std::memcpy(blob.get() + at[k].table, pr.table.data(), pr.table.size() * ab);
+    } else {
+      float* t = reinterpret_cast<float*>(blob.get() + at[k].table);
+      for (const rot::cd& x : pr.table) {
+        *t++ = (float)x.real();
+        *t++ = (float)x.imag();
+      }
+    }
   }
   int rc = upload_plan(s, blob.get(), total);
   if (rc) return rc;
-  const DevOp* d_ops = reinterpret_cast<const DevOp*>(s->d_plan);
+  const DevOp* d_ops = reinterpret_cast<const DevOp*>((unsigned char*)s->d_plan + ooff);
   const DevSegment* d_segs = reinterpret_cast<const DevSegment*>((unsigned char*)s->d_plan + soff);
   const DenseSegDev* d_dsegs = reinterpret_cast<const DenseSegDev*>((unsigned char*)s->d_plan + doff);
   const double* d_frags = reinterpret_cast<const double*>((unsigned char*)s->d_plan + foff);
@@ -655,14 +754,16 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   auto launch_passes = [&](bool restrict) -> int {
     uint64_t sup = sup0;
     moved = dense_amps = 0;
-    for (const auto& pp : E->passes) {
+    for (size_t pi = 0; pi < np; pi++) {
+      const auto& pp = E->passes[pi];
       bool all_dense = pp.pass.num_segments > 0;
       int ndense = 0;
       for (int k = 0; k < pp.pass.num_segments; k++) {
         all_dense = all_dense && dev_segs[pp.seg_begin + k].mode == 2;
         ndense += dev_segs[pp.seg_begin + k].mode == 2;
       }
-      DevPass pass = pp.pass;
+      if (is_rot[pi]) ndense = 0;
+      DevPass pass = is_rot[pi] ? rot_pass[pi] : pp.pass;
       if (restrict) {
         pass.tile_free_mask &= sup;
         pass.num_tiles = 1ull << popc(pass.tile_free_mask);
@@ -671,6 +772,17 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
       const uint64_t amps = pass.num_tiles << (pass.L + pass.H);
       moved += 2 * ab * amps;
       dense_amps += (uint64_t)ndense * amps;
+      if (is_rot[pi]) {
+        RotPass rp = progs[pi].dev;
+        rp.free_mask = pass.tile_free_mask;
+        rp.num_tiles = pass.num_tiles;
+        const unsigned char* d = static_cast<const unsigned char*>(s->d_plan);
+        const int r = launch_rot_pass(s->dtype, s->amp, rp, reinterpret_cast<const RotSeg*>(d + at[pi].segs),
+                                      reinterpret_cast<const RotOp*>(d + at[pi].ops), d + at[pi].table, s->num_sms,
+                                      s->stream);
+        if (r) return r;
+        continue;
+      }
       const int r = launch_tile_pass(s->dtype, s->amp, pass, d_segs + pp.seg_begin, d_ops, d_dsegs, d_frags,
                                      s->num_sms, s->stream, all_dense);
       if (r) return r;
@@ -679,8 +791,10 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   };
   if (sparse) {
     if ((rc = launch_passes(true))) return fail(rc, "tile pass launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-  } else if (s->plan_cache_cap && E != &local) {
-    // replay the captured launches (capture once per plan buffer)
+  } else if (s->plan_cache_cap && E != &local && !nrot) {
+    // replay the captured launches (capture once per plan buffer; a rotation
+    // program's sizes can change with its matrices, so passes with one are
+    // launched)
     if (E->exec && E->graph_dplan != s->d_plan) {
       cudaGraphExecDestroy(E->exec);
       E->exec = nullptr;
@@ -721,8 +835,8 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   st.bytes_moved += moved;
   st.dense_amps += dense_amps;
   st.ops += ops.size();
-  st.segments += E->segs.size();
-  st.dense_blocks += dsegs.size();
+  st.segments += old_segs + rot_segs;
+  st.dense_blocks += dsegs.size() + (s->dtype == MLB_C128 ? rot_segs : 0);
   st.plan_cache_hit = hit ? 1 : 0;
   return MLB_OK;
 }

@@ -160,6 +160,46 @@ int launch_batch_norm(const void* psi_c64, uint64_t dim, uint64_t batch, double*
 int launch_divide_by_norm(double* d_out, uint64_t batch, int num_params, const double* d_norm,
                           cudaStream_t stream);
 
+// ---- rotation programs of tile passes (rotate_plan.h, kernels_rotate.cu) ----
+constexpr int kRotBits = 13;     // bits of a tile
+constexpr int kRotMaxVar = 4;    // functionals that choose a table's variant
+constexpr int kRotTable = 1, kRotTurn = 2;
+struct RotOp {         // a round: register permutation, table, rotations
+  double t[4];         // tangent at each register bit, with its constant sign
+  uint64_t tout[4];    // its sign's outside functional
+  uint64_t vout[kRotMaxVar];  // the table variant's
+  uint16_t tzg[4];     // and the group index's
+  uint16_t vzg[kRotMaxVar];
+  uint32_t table;      // first entry (a multiple of 16)
+  uint32_t perm;       // steps of 4 bits, 4 i + j: register index bit j ^= bit i; 0: the end
+  uint8_t nv;          // variant functionals
+  uint8_t flags;
+  uint8_t pad[6];
+};
+struct RotSeg {
+  uint16_t alpha[4];               // byte offsets in the tile of its directions
+  uint16_t alpha_out[4];           // and of the register bits' at its end
+  uint16_t kappa[kRotBits - 4];    // and of the groups' basis
+  uint16_t pad;
+  int32_t op_begin, op_end;
+};
+struct RotPass {
+  int32_t n, m, num_segs, num_ops;
+  uint64_t basis[kRotBits];        // local bit k of an index adds basis[k]
+  uint64_t label_out[kRotBits];    // logical bit i at the end: its outside functional
+  uint16_t dir_slot[kRotBits];     // byte offset of the direction that flips it
+  uint16_t pad;
+  uint32_t label_const;            // and its constant
+  uint32_t entries;                // of its tables
+  uint64_t free_mask, num_tiles;   // the tiles: those of free_mask's bits
+};
+constexpr size_t kRotMaxShared = 40 * 1024;  // of a program's ops and tables (two CTAs per SM beside their tiles)
+size_t rot_shared_bytes(int dtype, size_t num_ops, size_t entries);
+// d_segs, d_ops, d_table: the program on the device (table entries in the
+// state's type).
+int launch_rot_pass(int dtype, void* amp, const RotPass& pass, const RotSeg* d_segs, const RotOp* d_ops,
+                    const void* d_table, int num_sms, cudaStream_t stream);
+
 // ---- sums of Pauli strings (pauli_plan.h, kernels_pauli.cu) ----
 constexpr int kMaxPauliBits = 13;    // bits of a tile
 constexpr int kMaxPauliTerms = 256;  // strings of a pass (their table lives in shared memory)

@@ -1,0 +1,704 @@
+// rotate_plan.h -- lowers the ops of one tile pass into a program of plane
+// rotations and diagonal tables (run by kernels_rotate.cu).  Host-only.
+//
+// The ops of most circuits are one-qubit unitaries, CNOTs, SWAPs and
+// diagonals.  Inside a tile:
+//   * X, CNOT and SWAP are not carried out.  They relabel: logical bit i of
+//     an amplitude at local index t is an affine functional of t and of the
+//     tile's outside bits, and flipping logical bit i moves along a direction
+//     (an XOR mask of t).  The store at the end of the pass writes every
+//     amplitude to the index its labels spell, a permutation of the tile.
+//   * A one-qubit unitary is diag(u1, u2) s [[1, -t], [t, 1]] diag(1, w),
+//     0 <= t <= 1 (the columns swapped first, an X, where |U00| < |U10|).  The
+//     rotation costs two multiply-adds per component pair; s is folded into
+//     the next table.
+//   * Diagonals (those factors, RZ, phases, ZZ, controlled phases) are
+//     products over the functionals they read.  All that are due are merged
+//     into one table of a complex factor per register index, in up to 8
+//     variants for the parities of functionals that the registers do not hold.
+// A segment keeps 16 amplitudes of a group in registers along four
+// directions and runs every rotation whose direction lies in their span, in
+// rounds: a permutation of the registers, a table and up to four commuting
+// rotations, each along one register bit that it alone reads.  Program order
+// is kept between rotations and diagonals that do not commute (a functional
+// of one that changes along the other's direction).
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+#include <complex>
+#include <cstdint>
+#include <vector>
+
+#include "hea_plan.h"
+#include "mlb_internal.h"
+#include "planner.h"
+
+namespace mlb {
+namespace rot {
+
+using cd = std::complex<double>;
+
+struct Fun {  // parity(row & t) ^ parity(out & tile base) ^ c
+  uint32_t row = 0;
+  uint64_t out = 0;
+  bool c = false;
+  void add(const Fun& o) { row ^= o.row; out ^= o.out; c ^= o.c; }
+  bool same(const Fun& o) const { return row == o.row && out == o.out; }
+};
+
+constexpr int kMaxItems = 512, kWords = kMaxItems / 64;  // a pass's ops give at most three items each
+static_assert(3 * kMaxPassOps <= kMaxItems, "items of a pass");
+
+struct Set {
+  uint64_t w[kWords] = {};
+  void add(int i) { w[i >> 6] |= 1ull << (i & 63); }
+  bool has(int i) const { return w[i >> 6] >> (i & 63) & 1ull; }
+};
+
+struct Item {
+  bool rotation = false;
+  // rotation: direction, its target bit and its tangent; scale owed
+  uint32_t dir = 0;
+  Fun fun;
+  double t = 0, s = 1;
+  // diagonal: where every condition holds, d[0] or d[1] by the key (no key: d[1])
+  Fun cond[3];
+  int nc = 0;
+  bool keyed = false;
+  Fun key;
+  cd d[2] = {1.0, 1.0};
+  Set pred, succ;
+  int height = 0;
+};
+
+inline cd mul(cd a, cd b) {
+  return {a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()};
+}
+
+struct Program {
+  RotPass dev{};
+  std::vector<RotSeg> segs;
+  std::vector<RotOp> ops;
+  std::vector<cd> table;  // 16 << nv entries a table op: [variant][register index]
+};
+
+// Whether the rotation program covers an op (matrix values aside from
+// unitarity included): what it does not cover runs as before.
+inline bool covers(const mlb_op_t& o) {
+  switch (o.kind) {
+    case MLB_OP_1Q: {
+      if (o.cmask) return false;
+      const cd a(o.m[0], o.m[1]), b(o.m[2], o.m[3]), c(o.m[4], o.m[5]), d(o.m[6], o.m[7]);
+      // columns of length one and orthogonal, to rounding
+      return std::abs(std::norm(a) + std::norm(c) - 1.0) < 2e-14 && std::abs(std::norm(b) + std::norm(d) - 1.0) < 2e-14 &&
+             std::abs(std::conj(a) * b + std::conj(c) * d) < 2e-14;
+    }
+    case MLB_OP_X: return plan::popc(o.cmask) <= 1;
+    case MLB_OP_SWAP: return o.cmask == 0;
+    case MLB_OP_DIAG1: return plan::popc(o.cmask) <= 2;
+    case MLB_OP_ZZ: return true;
+    case MLB_OP_PHASE: return plan::popc(o.cmask) <= 3;
+    default: return false;
+  }
+}
+
+// Moves what a one-qubit unitary ends with past the ops that it commutes with
+// and into the next unitary of its qubit, so that most need no diagonal after
+// their rotation: a phase past controls and diagonals, an X rotation past
+// CNOTs that have the qubit as target (U = RX(alpha) V with V's first column
+// real up to a phase).
+inline void push_forward(std::vector<mlb_op_t>& ops, uint32_t n) {
+  struct Open {
+    int op = -1;      // the qubit's last one-qubit unitary
+    int between = 0;  // ops since: 1 diagonal on it, 2 X on it, 3 neither way
+  };
+  std::vector<Open> open(n);
+  auto at = [](const mlb_op_t& o, int k) { return cd(o.m[2 * k], o.m[2 * k + 1]); };
+  auto set = [](mlb_op_t& o, int k, cd x) {
+    o.m[2 * k] = x.real();
+    o.m[2 * k + 1] = x.imag();
+  };
+  for (size_t i = 0; i < ops.size(); i++) {
+    mlb_op_t& o = ops[i];
+    const uint64_t T = plan::op_targets(o);
+    for (uint64_t b = plan::op_qubits(o) & ~T; b; b &= b - 1) open[__builtin_ctzll(b)].between |= 1;
+    if (o.kind == MLB_OP_X) {
+      open[o.target].between |= 2;
+      continue;
+    }
+    if (o.kind != MLB_OP_1Q || o.cmask) {
+      for (uint64_t b = T; b; b &= b - 1) open[__builtin_ctzll(b)].op = -1;
+      continue;
+    }
+    Open& e = open[o.target];
+    if (e.op >= 0 && (e.between == 1 || e.between == 2)) {
+      mlb_op_t& p = ops[e.op];
+      const cd a = at(p, 0), b = at(p, 1), c = at(p, 2), d = at(p, 3);
+      cd f[4] = {1.0, 0.0, 0.0, 1.0};  // p = f V
+      if (e.between == 1) {
+        // the second row's phase beside the first's, of the larger column
+        const bool first = std::norm(a) >= std::norm(c);
+        const cd x = first ? mul(c, std::conj(a)) : mul(d, std::conj(b));
+        if (std::abs(x) > 0) f[3] = x / std::abs(x);
+      } else {
+        const cd x = mul(std::conj(a), c);
+        const double y = 2 * x.imag(), z = std::norm(a) - std::norm(c), alpha = std::atan2(-y, z);
+        f[0] = f[3] = std::cos(alpha / 2);
+        f[1] = f[2] = cd(0.0, -std::sin(alpha / 2));
+      }
+      // V = f^-1 p; o takes f first
+      const cd g[4] = {std::conj(f[0]), std::conj(f[2]), std::conj(f[1]), std::conj(f[3])};
+      set(p, 0, mul(g[0], a) + mul(g[1], c));
+      set(p, 1, mul(g[0], b) + mul(g[1], d));
+      set(p, 2, mul(g[2], a) + mul(g[3], c));
+      set(p, 3, mul(g[2], b) + mul(g[3], d));
+      const cd A = at(o, 0), B = at(o, 1), C = at(o, 2), D = at(o, 3);
+      set(o, 0, mul(A, f[0]) + mul(B, f[2]));
+      set(o, 1, mul(A, f[1]) + mul(B, f[3]));
+      set(o, 2, mul(C, f[0]) + mul(D, f[2]));
+      set(o, 3, mul(C, f[1]) + mul(D, f[3]));
+    }
+    e.op = (int)i;
+    e.between = 0;
+  }
+}
+
+// The pass with its tile filled to `bits` by the lowest qubits outside it.
+inline DevPass filled(DevPass p, int bits) {
+  for (int q = 0; q < p.n && p.L + p.H < bits; q++)
+    if (p.tile_free_mask >> q & 1ull) {
+      p.high[p.H++] = q;
+      p.tile_free_mask &= ~(1ull << q);
+      p.num_tiles >>= 1;
+    }
+  return p;
+}
+
+struct Lower {
+  const DevPass& P;
+  int dtype, m;
+  int local_of[64];
+  std::vector<Item> items;
+  Fun label[kRotBits];
+  uint32_t dir[kRotBits];
+
+  Lower(const DevPass& pass, int dt) : P(pass), dtype(dt), m(pass.L + pass.H) {
+    for (int& x : local_of) x = -1;
+    for (int q = 0; q < P.L; q++) local_of[q] = q;
+    for (int h = 0; h < P.H; h++) local_of[P.high[h]] = P.L + h;
+    for (int i = 0; i < m; i++) {
+      label[i].row = 1u << i;
+      dir[i] = 1u << i;
+    }
+  }
+
+  Fun fun(int q) const {
+    if (local_of[q] >= 0) return label[local_of[q]];
+    Fun f;
+    f.out = 1ull << q;
+    return f;
+  }
+
+  void diag(const std::vector<Fun>& cond, bool keyed, const Fun& key, cd d0, cd d1) {
+    if (keyed && cond.empty())  // one on the same functional, with no rotation between that changes it: merged
+      for (int i = (int)items.size(); i-- > 0;) {
+        Item& it = items[i];
+        if (it.rotation) {
+          if (hea::parity(key.row & it.dir)) break;
+        } else if (it.keyed && it.nc == 0 && it.key.same(key)) {
+          const bool x = it.key.c != key.c;
+          it.d[0] = mul(it.d[0], x ? d1 : d0);
+          it.d[1] = mul(it.d[1], x ? d0 : d1);
+          return;
+        }
+      }
+    Item it;
+    for (const Fun& f : cond) it.cond[it.nc++] = f;
+    it.keyed = keyed;
+    it.key = key;
+    it.d[0] = d0;
+    it.d[1] = d1;
+    items.push_back(it);
+  }
+
+  void add(const mlb_op_t& o) {
+    std::vector<Fun> cond;
+    for (uint64_t c = o.cmask; c; c &= c - 1) cond.push_back(fun(__builtin_ctzll(c)));
+    switch (o.kind) {
+      case MLB_OP_X: {
+        Fun& f = label[local_of[o.target]];
+        if (cond.empty()) {
+          f.c = !f.c;
+        } else {
+          const int c = __builtin_ctzll(o.cmask);
+          f.add(cond[0]);
+          if (local_of[c] >= 0) dir[local_of[c]] ^= dir[local_of[o.target]];
+        }
+        return;
+      }
+      case MLB_OP_SWAP: {
+        const int a = local_of[o.target], b = local_of[o.target2];
+        std::swap(label[a], label[b]);
+        std::swap(dir[a], dir[b]);
+        return;
+      }
+      case MLB_OP_DIAG1: diag(cond, true, fun(o.target), cd(o.m[0], o.m[1]), cd(o.m[2], o.m[3])); return;
+      case MLB_OP_PHASE: diag(cond, false, Fun(), 1.0, cd(o.m[0], o.m[1])); return;
+      case MLB_OP_ZZ: {
+        Fun f = fun(o.target);
+        f.add(fun(o.target2));
+        diag({}, true, f, cd(o.m[0], o.m[1]), cd(o.m[2], o.m[3]));
+        return;
+      }
+      default: break;
+    }
+    const int q = local_of[o.target];
+    cd a(o.m[0], o.m[1]), b(o.m[2], o.m[3]), c(o.m[4], o.m[5]), d(o.m[6], o.m[7]);
+    if (std::norm(a) < std::norm(c)) {  // the columns swapped: an X first
+      label[q].c = !label[q].c;
+      std::swap(a, b);
+      std::swap(c, d);
+    }
+    // a = s u, c = s u t v, d = s u w v: diag(1, v) s [[1, -t], [t, 1]] diag(u, u w).
+    // A real c / a needs no diag(1, v) (t takes the sign).
+    const double s = std::abs(a);
+    const cd u = a / s, r = mul(c, std::conj(u)) / s;  // t v
+    double t = std::abs(r);
+    cd v = 1.0;
+    if (std::abs(r.imag()) <= 4e-16) t = r.real();
+    else v = r / t;
+    const cd w = mul(mul(d, std::conj(u)), std::conj(v)) / std::abs(d);
+    diag({}, true, label[q], u, mul(u, w));
+    Item it;
+    it.rotation = true;
+    it.dir = dir[q];
+    it.fun = label[q];
+    it.t = t;
+    it.s = s;
+    items.push_back(it);
+    if (v != 1.0) diag({}, true, label[q], 1.0, v);
+  }
+
+  // The pass's program, with fewer variants a table where its tables would
+  // outgrow shared memory.  False: it does not fit.
+  static bool lower(const DevPass& pass, int dtype, const std::vector<const mlb_op_t*>& ops, Program& out) {
+    for (int max_var = kRotMaxVar; max_var >= 1; max_var--) {
+      Program p;
+      double scale = 1.0;
+      Lower(pass, dtype).build(ops, scale, true, p, max_var);
+      if (rot_shared_bytes(dtype, p.ops.size(), p.table.size()) > kRotMaxShared) continue;
+      p.dev.entries = (uint32_t)p.table.size();
+      out = std::move(p);
+      return true;
+    }
+    return false;
+  }
+
+  static bool moves(const Item& d, uint32_t dir) {  // a functional of diagonal d changes along dir
+    bool m = d.keyed && hea::parity(d.key.row & dir);
+    for (int i = 0; i < d.nc; i++) m = m || hea::parity(d.cond[i].row & dir);
+    return m;
+  }
+
+  void order() {
+    const int N = (int)items.size();
+    std::vector<int> rots, diags;
+    auto edge = [&](int i, int j) {
+      items[i].succ.add(j);
+      items[j].pred.add(i);
+    };
+    for (int j = 0; j < N; j++) {
+      Item& y = items[j];
+      if (y.rotation) {
+        for (int i : rots)
+          if (hea::parity(items[i].fun.row & y.dir) || hea::parity(y.fun.row & items[i].dir)) edge(i, j);
+        for (int i : diags)
+          if (moves(items[i], y.dir)) edge(i, j);
+        rots.push_back(j);
+      } else {
+        for (int i : rots)
+          if (moves(y, items[i].dir)) edge(i, j);
+        diags.push_back(j);
+      }
+    }
+    for (int i = N; i-- > 0;)
+      for (int k = 0; k < kWords; k++)
+        for (uint64_t b = items[i].succ.w[k]; b; b &= b - 1) {
+          const Item& y = items[64 * k + __builtin_ctzll(b)];
+          items[i].height = std::max(items[i].height, y.height + (y.rotation ? 1 : 0));
+        }
+  }
+
+  // A functional in a segment's coordinates: its value over the register
+  // index, and what is left (group index and tile).
+  struct Split {
+    uint32_t reg = 0, zg = 0;
+    uint64_t out = 0;
+    bool c = false;
+    bool rest() const { return zg || out; }
+  };
+
+  using Rest = std::pair<uint32_t, uint64_t>;  // (group functional, outside functional)
+
+  // The program of `ops`.  `scale`: the factor owed by rotations so far, left
+  // for a later pass's table unless `settle`.  A table has up to 2^max_var variants.
+  void build(const std::vector<const mlb_op_t*>& ops, double& scale, bool settle, Program& out, int max_var) {
+    for (const mlb_op_t* o : ops) add(*o);
+    order();
+    const int N = (int)items.size(), words = (N + 63) / 64;
+    int left = 0;
+    for (const Item& it : items) left += it.rotation;
+    int diags = N - left;
+    RotPass& D = out.dev;
+    D.n = P.n;
+    D.m = m;
+    for (int i = 0; i < m; i++) D.basis[i] = i < P.L ? 1ull << i : 1ull << P.high[i - P.L];
+    Set done;
+    auto after = [&](const Item& it, const Set& before) {  // its predecessors lie in `before`
+      for (int k = 0; k < words; k++)
+        if (it.pred.w[k] & ~before.w[k]) return false;
+      return true;
+    };
+    while (left || diags || (settle && scale != 1.0) || out.segs.empty()) {
+      // 1. the segment's directions and its rounds; a round's diagonals are
+      // those its rotations wait for, `free` the others that could join
+      hea::Basis W;
+      std::vector<uint32_t> al, rows;
+      struct Round {
+        std::vector<int> diag, rot, free;
+      };
+      std::vector<Round> rounds;
+      Set marked;
+      while (left) {
+        std::vector<int> cand;
+        Round r;
+        Set open = done;  // and the diagonals that can run now
+        for (int i = 0; i < N; i++)
+          if (!items[i].rotation && !done.has(i) && after(items[i], done)) {
+            open.add(i);
+            r.free.push_back(i);
+          }
+        for (int i = 0; i < N; i++)
+          if (items[i].rotation && !done.has(i) && after(items[i], open)) cand.push_back(i);
+        // a new direction: the rotation that shares the most later ones with
+        // the directions so far, then the one that the longest chain waits for
+        while ((int)al.size() < 4) {
+          int best = -1;
+          long most = -1;
+          for (int i : cand) {
+            if (!W.reduce(items[i].dir)) continue;
+            long common = 0;
+            for (int k = 0; k < words; k++) common += __builtin_popcountll(items[i].succ.w[k] & marked.w[k]);
+            const long score = common * 4096 + items[i].height;
+            if (score > most) {
+              most = score;
+              best = i;
+            }
+          }
+          if (best < 0) break;
+          W.add(items[best].dir);
+          al.push_back(items[best].dir);
+          rows.push_back(items[best].fun.row);
+          for (int k = 0; k < words; k++) marked.w[k] |= items[best].succ.w[k];
+        }
+        for (int i : cand)
+          if (!W.reduce(items[i].dir)) r.rot.push_back(i);
+        if (r.rot.empty()) break;
+        for (int i : r.free)
+          for (int j : r.rot)
+            if (items[j].pred.has(i)) {
+              done.add(i);
+              diags--;
+              r.diag.push_back(i);
+              break;
+            }
+        for (int i : r.rot) {
+          done.add(i);
+          left--;
+        }
+        rounds.push_back(std::move(r));
+      }
+      for (int b = 0; b < m && (int)al.size() < 4; b++)
+        if (W.add(1u << b)) al.push_back(1u << b);
+      // 2. the groups: the common kernel of four functionals that are
+      // independent on the directions, the rotations' own first
+      uint32_t fn[4], mat[4], comb[16];
+      int nf = 0;
+      {
+        hea::Basis rank;
+        auto take = [&](uint32_t f) {
+          uint32_t v = 0;
+          for (int i = 0; i < 4; i++) v |= (uint32_t)hea::parity(f & al[i]) << i;
+          if (nf < 4 && rank.add(v)) {
+            fn[nf] = f;
+            mat[nf++] = v;
+          }
+        };
+        for (uint32_t f : rows) take(f);
+        for (int b = 0; b < m; b++) take(1u << b);
+      }
+      for (uint32_t k = 0; k < 16; k++) {  // combinations of the directions
+        comb[k] = 0;
+        for (int i = 0; i < 4; i++)
+          if (k >> i & 1) comb[k] ^= al[i];
+      }
+      hea::Basis span;
+      std::vector<uint32_t> ker;
+      for (int b = 0; b < m; b++)
+        for (uint32_t k = 0; k < 16; k++) {  // the unit vector, corrected along the directions
+          const uint32_t t = (1u << b) ^ comb[k];
+          bool in = true;
+          for (int i = 0; i < 4; i++) in = in && !hea::parity(fn[i] & t);
+          if (in && span.add(t)) ker.push_back(t);
+        }
+      // lanes (the first five group bits) where the tables' variants do not
+      // depend on them, so that a warp reads one variant: the common kernel of
+      // the rounds' functionals, the commonest first, while it has five dimensions
+      std::vector<uint32_t> lanes = ker;
+      {
+        std::vector<std::pair<int, uint32_t>> seen;
+        auto see = [&](const Fun& f) {
+          bool rest = false;
+          for (uint32_t t : ker) rest = rest || hea::parity(f.row & t);
+          if (!rest) return;
+          for (auto& x : seen)
+            if (x.second == f.row) {
+              x.first--;
+              return;
+            }
+          seen.push_back({-1, f.row});
+        };
+        for (const Round& r : rounds)
+          for (int i : r.diag) {
+            if (items[i].keyed) see(items[i].key);
+            for (int c = 0; c < items[i].nc; c++) see(items[i].cond[c]);
+          }
+        std::stable_sort(seen.begin(), seen.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+        for (auto& x : seen) {
+          std::vector<uint32_t> in;
+          uint32_t odd = 0;
+          for (uint32_t t : lanes)
+            if (!hea::parity(x.second & t)) in.push_back(t);
+            else if (!odd) odd = t;
+            else in.push_back(t ^ odd);
+          if (in.size() >= 5) lanes = in;
+        }
+      }
+      std::vector<uint32_t> kap = hea::bank_order(lanes, dtype);
+      {
+        hea::Basis have;
+        for (uint32_t t : kap) have.add(t);
+        for (uint32_t t : ker)
+          if (have.add(t)) kap.push_back(t);
+      }
+      RotSeg sg{};
+      for (int i = 0; i < 4; i++) sg.alpha[i] = (uint16_t)hea::slot_bytes(al[i], dtype);
+      for (size_t i = 0; i < kap.size(); i++) sg.kappa[i] = (uint16_t)hea::slot_bytes(kap[i], dtype);
+      sg.op_begin = (int)out.ops.size();
+      // the directions of the register index bits; a round first adds
+      // directions to one another (a permutation of the registers) until its
+      // rotations move along single bits and read them alone
+      uint32_t cur[4] = {al[0], al[1], al[2], al[3]};
+      std::vector<uint32_t> steps;  // 4 i + j: direction i += direction j
+      auto step = [&](int i, int j) {
+        cur[i] ^= cur[j];
+        steps.push_back((uint32_t)(4 * i + j));
+      };
+      auto emit = [&](RotOp op) {  // with the steps before it, up to 8 an op
+        while (steps.size() > 8) {
+          RotOp more{};
+          for (int k = 0; k < 8; k++) more.perm |= steps[k] << (4 * k);
+          steps.erase(steps.begin(), steps.begin() + 8);
+          out.ops.push_back(more);
+        }
+        for (size_t k = 0; k < steps.size(); k++) op.perm |= steps[k] << (4 * k);
+        steps.clear();
+        out.ops.push_back(op);
+      };
+      auto split = [&](const Fun& f) {
+        Split s;
+        for (int i = 0; i < 4; i++) s.reg |= (uint32_t)hea::parity(f.row & cur[i]) << i;
+        for (size_t j = 0; j < kap.size(); j++) s.zg |= (uint32_t)hea::parity(f.row & kap[j]) << j;
+        s.out = f.out;
+        s.c = f.c;
+        return s;
+      };
+      // 3. emit: tables of the diagonals, and the rotations
+      hea::Basis held;  // functionals that the registers hold alone
+      for (int i = 0; i < 4; i++) held.add(fn[i]);
+      std::vector<Rest> var;  // the open table's variant functionals
+      std::vector<int> open;
+      auto combo = [&](const Rest& r) {  // r as a sum of variant functionals, -1: none
+        for (uint32_t v = 0; v < (1u << var.size()); v++) {
+          Rest x{0, 0};
+          for (size_t j = 0; j < var.size(); j++)
+            if (v >> j & 1u) {
+              x.first ^= var[j].first;
+              x.second ^= var[j].second;
+            }
+          if (x == r) return (int)v;
+        }
+        return -1;
+      };
+      auto plain = [&](const Item& d) {
+        if (d.keyed && (d.key.out || held.reduce(d.key.row))) return false;
+        for (int i = 0; i < d.nc; i++)
+          if (d.cond[i].out || held.reduce(d.cond[i].row)) return false;
+        return true;
+      };
+      auto known = [&](const Item& d) {  // read by the registers and the open table's variants
+        auto in = [&](const Fun& f) {
+          const Split s = split(f);
+          return combo({s.zg, s.out}) >= 0;
+        };
+        bool k = !d.keyed || in(d.key);
+        for (int i = 0; i < d.nc && k; i++) k = in(d.cond[i]);
+        return k;
+      };
+      auto put = [&](int i) {  // false: no room for its functionals
+        const size_t before = var.size();
+        auto need = [&](const Fun& f) {
+          const Split s = split(f);
+          if (combo({s.zg, s.out}) < 0) var.push_back({s.zg, s.out});
+        };
+        if (items[i].keyed) need(items[i].key);
+        for (int c = 0; c < items[i].nc; c++) need(items[i].cond[c]);
+        if (var.size() > (size_t)max_var && !open.empty()) {
+          var.resize(before);
+          return false;
+        }
+        open.push_back(i);
+        return true;
+      };
+      auto close = [&](RotOp op) {  // emits op with the open table
+        const uint32_t nv = (uint32_t)var.size();
+        const size_t at = out.table.size();
+        out.table.resize(at + ((size_t)16 << nv), cd(scale, 0.0));
+        scale = 1.0;
+        struct Bit {
+          uint32_t reg, v, c;  // patterns over the register index and the variant
+          uint32_t at(uint32_t k, uint32_t x) const { return ((reg >> k) ^ (v >> x) ^ c) & 1u; }
+        };
+        auto pattern = [](uint32_t f) {
+          uint32_t p = 0;
+          for (uint32_t k = 0; k < 16; k++) p |= (uint32_t)hea::parity(f & k) << k;
+          return p;
+        };
+        for (int i : open) {
+          const Item& d = items[i];
+          auto bit = [&](const Fun& f) {
+            const Split s = split(f);
+            return Bit{pattern(s.reg), pattern((uint32_t)combo({s.zg, s.out})), s.c ? 1u : 0u};
+          };
+          Bit cond[3];
+          for (int c = 0; c < d.nc; c++) cond[c] = bit(d.cond[c]);
+          const Bit key = d.keyed ? bit(d.key) : Bit{0, 0, 1};
+          for (uint32_t k = 0; k < 16; k++)
+            for (uint32_t x = 0; x < (1u << nv); x++) {
+              bool on = true;
+              for (int c = 0; c < d.nc; c++) on = on && cond[c].at(k, x);
+              cd& e = out.table[at + 16 * x + k];
+              if (on) e = mul(e, d.d[key.at(k, x)]);
+            }
+        }
+        op.table = (uint32_t)at;
+        op.nv = (uint8_t)nv;
+        op.flags |= kRotTable;
+        for (uint32_t j = 0; j < nv; j++) {
+          op.vzg[j] = (uint16_t)var[j].first;
+          op.vout[j] = var[j].second;
+        }
+        emit(op);
+        var.clear();
+        open.clear();
+      };
+      // a diagonal on the very functional of a later rotation joins that one's table
+      auto later_same = [&](const Item& d) {
+        if (d.keyed && d.nc == 0)
+          for (int k = 0; k < words; k++)
+            for (uint64_t b = d.succ.w[k] & ~done.w[k]; b; b &= b - 1)
+              if (items[64 * k + __builtin_ctzll(b)].fun.same(d.key)) return true;
+        return false;
+      };
+      auto join = [&](int i) {
+        if (put(i)) {
+          done.add(i);
+          diags--;
+        }
+      };
+      for (const Round& r : rounds) {
+        RotOp op{};
+        int place[4] = {-1, -1, -1, -1};  // rotation at each register bit
+        for (int i : r.rot)
+          for (int b = 0; b < 4; b++)
+            if (place[b] < 0 && cur[b] == items[i].dir) {
+              place[b] = i;
+              break;
+            }
+        for (int i : r.rot) {
+          if (place[0] == i || place[1] == i || place[2] == i || place[3] == i) continue;
+          uint32_t x = 0;  // its direction in the current ones
+          for (uint32_t k = 1; k < 16; k++) {
+            uint32_t v = 0;
+            for (int b = 0; b < 4; b++)
+              if (k >> b & 1u) v ^= cur[b];
+            if (v == items[i].dir) x = k;
+          }
+          int b = 0;
+          while (place[b] >= 0 || !(x >> b & 1u)) b++;
+          for (int j = 0; j < 4; j++)
+            if (j != b && (x >> j & 1u)) step(b, j);
+          place[b] = i;
+        }
+        for (int b = 0; b < 4; b++)
+          for (int j = 0; j < 4; j++)
+            if (place[b] < 0 && place[j] >= 0 && hea::parity(items[place[j]].fun.row & cur[b])) step(b, j);
+        for (int b = 0; b < 4; b++)
+          if (place[b] >= 0) {
+            const Item& it = items[place[b]];
+            const Split sp = split(it.fun);
+            op.t[b] = sp.c ? -it.t : it.t;
+            op.tzg[b] = (uint16_t)sp.zg;
+            op.tout[b] = sp.out;
+            op.flags |= kRotTurn;
+          }
+        for (int i : r.diag)
+          if (!put(i)) {
+            close(RotOp{});
+            put(i);
+          }
+        for (int i : r.rot) scale *= items[i].s;
+        if (!open.empty())  // the table is paid for: others that may run now, with no variant more
+          for (int i : r.free)
+            if (!done.has(i) && !later_same(items[i]) && known(items[i])) join(i);
+        if (!open.empty() || scale < 0x1p-10 || (settle && scale != 1.0)) close(op);
+        else emit(op);
+      }
+      // what the registers hold now goes here; with no rotation left, all of it
+      do {
+        std::vector<int> now;
+        for (int i = 0; i < N && diags; i++)
+          if (!items[i].rotation && !done.has(i) && after(items[i], done) && !later_same(items[i])) now.push_back(i);
+        for (int form = 0; form < 2; form++)
+          for (int i : now)
+            if (!done.has(i) && plain(items[i]) == (form == 0) && (form == 0 || left == 0 || (!open.empty() && known(items[i]))))
+              join(i);
+        if (!open.empty() || (settle && !left && !diags && scale != 1.0)) close(RotOp{});
+      } while (!left && diags);
+      for (int i = 0; i < 4; i++) sg.alpha_out[i] = (uint16_t)hea::slot_bytes(cur[i], dtype);
+      sg.op_end = (int)out.ops.size();
+      out.segs.push_back(sg);
+    }
+    D.num_ops = (int)out.ops.size();
+    D.num_segs = (int)out.segs.size();
+    for (int i = 0; i < m; i++) {
+      D.dir_slot[i] = (uint16_t)hea::slot_bytes(dir[i], dtype);
+      D.label_out[i] = label[i].out;
+      if (label[i].c) D.label_const |= 1u << i;
+    }
+  }
+};
+
+}  // namespace rot
+}  // namespace mlb

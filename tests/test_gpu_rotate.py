@@ -1,0 +1,87 @@
+"""Rotation programs of tile passes (kernels_rotate.cu) against gate-by-gate
+execution and the CPU oracle: every kind of op they take (one-qubit
+unitaries, X, CNOT, SWAP, diagonals on one to three qubits) on arbitrary
+qubits, at the smallest register each type runs them on, where tiles have
+free qubits and where the form is chosen pass by pass; ops they do not take
+(controlled rotations, two controls, matrices that are not unitary) between
+them; registers that are mostly zero after a reset.  complex128 1e-12 per
+amplitude (the tolerance of the other paths), complex64 2e-5."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from moonlab_b200 import StateVector
+from moonlab_b200.circuits import GATE_DTYPE, brickwork
+from oracle import bindings as B
+
+pytestmark = pytest.mark.gpu
+TAKEN = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 20, 21, 22, 23, 27]  # gate record types
+
+
+def circuit(n, count, seed, types=TAKEN):
+    rng = np.random.default_rng(seed)
+    g = np.zeros(count, dtype=GATE_DTYPE)
+    for i in range(count):
+        t = int(rng.choice(types))
+        a, b = rng.choice(n, 2, replace=False)
+        two = t in (10, 11, 12, 13) or t >= 23
+        # a fifth of the angles at multiples of pi / 2, where a sine or cosine vanishes
+        th = rng.integers(-4, 5) * np.pi / 2 if rng.random() < 0.2 else rng.uniform(-np.pi, np.pi)
+        g[i] = (t, int(a), int(b) if two else -1, 0, float(th))
+    return g
+
+
+@pytest.mark.parametrize("n,count,seed", [(13, 1, 1), (13, 300, 2), (14, 500, 3), (16, 400, 4), (18, 300, 5)])
+def test_matches_the_oracle(gpu, n, count, seed):
+    g = circuit(n, count, seed)
+    with StateVector(n) as sv:
+        sv.run(g)
+        got = sv.amplitudes()
+        assert sv.flush_stats()["dense_blocks"] > 0
+    assert np.abs(got - B.port_run(n, g)).max() < 1e-12
+
+
+@pytest.mark.parametrize("n", [21, 22])
+def test_complex64_against_complex128(gpu, n):
+    g = np.concatenate([circuit(n, 200, n), brickwork(n, 4, n, zz_every=2)])
+    with StateVector(n) as a, StateVector(n, "c64") as b:
+        a.set_dense(False)
+        a.run(g)
+        b.set_exec_mode("tiled")
+        b.run(g)
+        want, got = a.amplitudes(), b.amplitudes()
+    assert np.abs(got - want).max() < 2e-5
+
+
+@pytest.mark.parametrize("form", ["brickwork", "random"])
+def test_pass_by_pass_choice(gpu, form):
+    """26 qubits: each pass runs in its cheaper form."""
+    n = 26
+    g = brickwork(n, 5, 77, zz_every=2) if form == "brickwork" else circuit(n, 250, 78)
+    with StateVector(n) as a, StateVector(n) as b:
+        a.run(g)
+        b.set_dense(False)
+        b.run(g)
+        x, y = a.amplitudes(), b.amplitudes()
+    assert np.abs(x - y).max() < 1e-12
+
+
+def test_ops_of_both_kinds(gpu):
+    """Ops that a program does not take, between ops that it takes."""
+    n = 15
+    rng = np.random.default_rng(9)
+    parts = [circuit(n, 60, 20 + k, TAKEN + [24, 25, 26]) for k in range(4)]
+    m = rng.standard_normal((2, 2)) + 1j * rng.standard_normal((2, 2))  # not unitary
+    with StateVector(n) as a, StateVector(n) as b:
+        b.set_dense(False)
+        for sv in (a, b):
+            for k, g in enumerate(parts):
+                sv.run(g)
+                sv.mcz([1, 5, 9])
+                sv.mcx([0, 7], 3 + k)
+                sv.mcz([2, 4, 6, 8])
+                if k == 2:
+                    sv.apply_1q(4, m / np.linalg.norm(m))
+        x, y = a.amplitudes(), b.amplitudes()
+    assert np.abs(x - y).max() < 1e-12
