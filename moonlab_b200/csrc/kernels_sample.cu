@@ -51,6 +51,9 @@ constexpr long long kTwo53 = 1ll << 53;
 constexpr int kDT = 512;                 // phase D: threads of its one CTA
 constexpr int kDPer = 8;                 // phase D: chunks per thread in one scan
 constexpr int kDBatch = kDT * kDPer;     // phase D: 4096 chunks per scan
+constexpr uint32_t kDSerial = 64;        // phase D: elements added in order where a binade ends
+static_assert(kDSerial * kDT >= (1 << kCB), "a thread's elements are among those it adds in order");
+constexpr int kDRounds = 24;             // phase D: scans of one chunk's elements before it is added in order
 constexpr int kNoBinade = -0x40000000;   // matches no candidate binade
 constexpr int kZeroChunk = 0x7fffffff;   // Xfer::e[0] of a chunk that adds 0 for every s
 
@@ -446,6 +449,27 @@ __device__ __forceinline__ Fn shfl_up_fn(const Fn& f, int o) {
   return r;
 }
 
+// The grid of a running value with bit pattern b (s >= 0).  s = N g in its
+// binade; (N + K) g has the bit pattern b + K while N + K < 2^53, i.e. while
+// b + K stays below `limit` (for a subnormal s the grid 2^-1074 also covers
+// the lowest normal binade).
+struct Grid {
+  int e;
+  unsigned long long limit;
+};
+__device__ __forceinline__ Grid grid_at(unsigned long long b) {
+  const int ex = (int)(b >> 52);
+  if (b == 0ull) return {kNoBinade, 1};     // only zero contributions pass
+  if (ex == 0x7ff) return {kNoBinade, 0};   // inf / nan: replayed
+  return {ex ? ex - 1023 : -1023, ex ? ((unsigned long long)(ex + 1) << 52) : (2ull << 52)};
+}
+// An element's map on that grid: without a binade, only a zero is the identity.
+template <bool FUSED>
+__device__ __forceinline__ Fn elem_on(double v, int e, double inv_g) {
+  if (e != kNoBinade) return elem_fn<FUSED>(v, inv_g);
+  return v == 0.0 ? Fn{0, 0, 0, 1} : Fn{kTwo53, kTwo53, 0, 1};
+}
+
 template <typename Real, bool FUSED>
 __global__ void __launch_bounds__(kDT) k_seq_d(const typename Cplx<Real>::T* __restrict__ amp,
                                                uint64_t nc, uint32_t clen, uint64_t fmask,
@@ -461,18 +485,9 @@ __global__ void __launch_bounds__(kDT) k_seq_d(const typename Cplx<Real>::T* __r
   uint64_t c = 0;
   unsigned long long b = 0;  // bit pattern of the exact running value (s >= 0)
   while (c < nc) {
-    // s = N g in its binade; (N + K) g has the bit pattern b + K while
-    // N + K < 2^53, i.e. while b + K stays below `limit` (for a subnormal s
-    // the grid 2^-1074 also covers the lowest normal binade).
-    const int ex = (int)(b >> 52);
-    int e;
-    unsigned long long limit;
-    if (b == 0ull) { e = kNoBinade; limit = 1; }                // only all-zero chunks pass
-    else if (ex == 0x7ff) { e = kNoBinade; limit = 0; }         // inf / nan: replayed
-    else {
-      e = ex ? ex - 1023 : -1023;
-      limit = ex ? ((unsigned long long)(ex + 1) << 52) : (2ull << 52);
-    }
+    const Grid gr = grid_at(b);
+    const int e = gr.e;
+    const unsigned long long limit = gr.limit;
     const int pb = (int)(b & 1ull);
     const uint64_t c0 = c;
     const uint64_t lo = c0 + (uint64_t)threadIdx.x * kDPer;
@@ -521,14 +536,57 @@ __global__ void __launch_bounds__(kDT) k_seq_d(const typename Cplx<Real>::T* __r
       __syncthreads();  // wtot is rewritten by the next batch
       continue;
     }
-    // element-by-element replay of the first failing chunk from its exact start
+    // the first failing chunk from its exact start: the same scan over its
+    // elements, a few per thread; the thread in which the value leaves the
+    // binade adds the next 64 elements one by one, and the scan goes on after
+    // them in the new binade.  (A replay of all 4096 adds by one thread takes
+    // 25 us; about 18 chunks of a spread-out state cross a binade.  1024
+    // samples of 20 qubits: 816 -> 432 us with phase E's scans.)
     c = c0 + fail;
     load_chunk_p<Real, FUSED>(amp, c * clen, clen, fmask, fval, sp);
+    b = s_bits[c];
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = __longlong_as_double((long long)s_bits[c]);
-#pragma unroll 8
-      for (uint32_t j = 0; j < clen; j++) s = elem_add<FUSED>(s, sp[j + (j >> 5)]);
+    const uint32_t per = (clen + kDT - 1) / kDT;
+    uint32_t pos = 0;
+    for (int round = 0; round < kDRounds && pos < clen; round++) {
+      const Grid eg = grid_at(b);
+      const double inv_g = eg.e == kNoBinade ? 0.0 : 1.0 / grid_of(eg.e);
+      const int pbe = (int)(b & 1ull);
+      const uint32_t j0 = threadIdx.x * per, j1 = min(clen, j0 + per);
+      Fn acc = ident;
+      for (uint32_t j = max(j0, pos); j < j1; j++) acc = compose(acc, elem_on<FUSED>(sp[j + (j >> 5)], eg.e, inv_g));
+      for (int o = 1; o < 32; o <<= 1) {
+        const Fn other = shfl_up_fn(acc, o);
+        if (lane >= o) acc = compose(other, acc);
+      }
+      if (lane == 31) wtot[warp] = acc;
+      if (threadIdx.x == 0) s_fail = 0xffffffffu;
+      __syncthreads();
+      Fn before = ident;
+      for (int w = 0; w < warp; w++) before = compose(before, wtot[w]);
+      const Fn end = compose(before, acc), lane_ex = shfl_up_fn(acc, 1);
+      if (lane > 0) before = compose(before, lane_ex);
+      if (b + (unsigned long long)(pbe ? end.K1 : end.K0) >= eg.limit) atomicMin(&s_fail, threadIdx.x);
+      __syncthreads();
+      const unsigned int ft = s_fail;
+      if (ft == 0xffffffffu) {
+        if (threadIdx.x == kDT - 1) s_run = __longlong_as_double((long long)(b + (unsigned long long)(pbe ? end.K1 : end.K0)));
+        pos = clen;
+      } else {
+        if (threadIdx.x == ft) {
+          double s = __longlong_as_double((long long)(b + (unsigned long long)(pbe ? before.K1 : before.K0)));
+          const uint32_t from = max(j0, pos), to = min(clen, from + kDSerial);
+          for (uint32_t j = from; j < to; j++) s = elem_add<FUSED>(s, sp[j + (j >> 5)]);
+          s_run = s;
+        }
+        pos = min(clen, max(ft * per, pos) + kDSerial);
+      }
+      __syncthreads();
+      b = (unsigned long long)__double_as_longlong(s_run);
+    }
+    if (pos < clen && threadIdx.x == 0) {  // many crossings (inf, nan): the rest in order
+      double s = __longlong_as_double((long long)b);
+      for (uint32_t j = pos; j < clen; j++) s = elem_add<FUSED>(s, sp[j + (j >> 5)]);
       s_run = s;
     }
     __syncthreads();
@@ -566,22 +624,51 @@ __global__ void __launch_bounds__(kCT) k_seq_e(const typename Cplx<Real>::T* __r
     }
     return;
   }
+  // 32 elements at a time: the running value after each is the start's plus a
+  // scan of the elements' increments while it stays in the binade (as in
+  // phase D); otherwise lane 0 adds them in order.
   const uint64_t c = lo, base = c * clen;
-  double s = s_in[c];
+  unsigned long long b = (unsigned long long)__double_as_longlong(s_in[c]);
   unsigned long long found = ~0ull;
   for (uint32_t j0 = 0; j0 < clen && found == ~0ull; j0 += 32) {
     const uint32_t j = j0 + lane;
     const double p = j < clen ? elem_p<Real>(amp, base + j, 0, 0) : 0.0;
-    // lane 0 replays the 32 adds in order
-    for (int l = 0; l < 32; l++) {
-      const double pl = __shfl_sync(0xffffffffu, p, l);
-      if (lane == 0 && found == ~0ull && j0 + l < clen) {
-        s = __dadd_rn(s, pl);
-        const bool hit = rule == 0 ? (s >= u) : (u < s);
-        if (hit) found = base + j0 + l;
+    const Grid gr = grid_at(b);
+    Fn f = elem_on<false>(p, gr.e, gr.e == kNoBinade ? 0.0 : 1.0 / grid_of(gr.e));
+    long long K;
+    if (!__any_sync(0xffffffffu, f.K0 != f.K1)) {  // no tie: plain sums (at most 32 x 2^53)
+      K = f.K0;
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long other = __shfl_up_sync(0xffffffffu, K, o);
+        if (lane >= o) K += other;
       }
+    } else {
+      for (int o = 1; o < 32; o <<= 1) {
+        const Fn other = shfl_up_fn(f, o);
+        if (lane >= o) f = compose(other, f);
+      }
+      K = (b & 1ull) ? f.K1 : f.K0;
     }
-    found = __shfl_sync(0xffffffffu, found, 0);
+    const unsigned long long after = b + (unsigned long long)K;
+    const bool in = after < gr.limit;
+    const double sv = __longlong_as_double((long long)after);
+    const bool hit = in && j < clen && (rule == 0 ? (sv >= u) : (u < sv));
+    const unsigned hits = __ballot_sync(0xffffffffu, hit), outs = __ballot_sync(0xffffffffu, !in);
+    if (hits && (!outs || __ffs(hits) < __ffs(outs))) {
+      found = base + j0 + (uint32_t)(__ffs(hits) - 1);
+    } else if (!outs) {
+      b = __shfl_sync(0xffffffffu, after, 31);
+    } else {
+      double s = __longlong_as_double((long long)b);
+      for (int l = 0; l < 32; l++) {
+        const double pl = __shfl_sync(0xffffffffu, p, l);
+        if (found == ~0ull && j0 + l < clen) {  // every lane alike
+          s = __dadd_rn(s, pl);
+          if (rule == 0 ? (s >= u) : (u < s)) found = base + j0 + l;
+        }
+      }
+      b = (unsigned long long)__double_as_longlong(s);
+    }
   }
   if (lane == 0) {
     // The chunk end passes u, so the replay must hit inside it.
