@@ -14,8 +14,8 @@
 // one bit pattern over the register index, one functional of the group
 // index and one sign per tile (folded into the coefficient table).
 // Bound: HBM for few strings; the FP64 products (two or three multiply-adds
-// per pair and string) and their issue for many.  Three CTAs per SM overlap
-// one's copies with the others' sums.
+// per pair and string) and their issue for many.  Two CTAs per SM overlap
+// one's copies with the other's sums.
 // Measured: norm, <Z>, 58 random one- and two-local strings and 4096 samples
 // of a 29-qubit complex128 state 68.1 -> 28.6 ms (one pass over the state per
 // distinct X mask before, three passes for all of them now), 22.1 ms with two
@@ -28,7 +28,7 @@ namespace mlb {
 
 namespace {
 
-constexpr int kSumThreads = 128, kApplyThreads = 128;
+constexpr int kThreads = 256;       // two CTAs per SM: 16 warps at 128 registers
 constexpr int kMaxUnitSteps = 64;  // units of a tile per thread
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -42,10 +42,10 @@ __device__ __forceinline__ double flip_sign(double c, uint32_t bit) {  // bit in
 // A tile's index offsets: unit tid + j NT adds toff ^ joff[j] to the base.
 template <int NT, int UB>
 struct UnitOffsets {
-  static_assert(NT == 128, "seven thread bits");
+  static_assert(NT == 256, "eight thread bits");
   uint64_t toff;
   __device__ __forceinline__ void init(const PauliPass& P, uint64_t* joff) {
-    constexpr int TB = 7;
+    constexpr int TB = 8;
     for (uint32_t j = threadIdx.x; j < kMaxUnitSteps; j += NT) {
       uint64_t off = 0;
 #pragma unroll
@@ -107,12 +107,12 @@ __device__ __forceinline__ void pairs(const A (&v)[2][8], const double (&c)[2], 
 }
 
 template <typename Real>
-__global__ void __launch_bounds__(kSumThreads, 3)
+__global__ void __launch_bounds__(kThreads, 2)
     k_pauli_sum(const typename Cplx<Real>::T* __restrict__ amp, const __grid_constant__ PauliPass P,
                 const PauliSeg* __restrict__ segs, const PauliTerm* __restrict__ terms,
                 double* __restrict__ partials) {
   using A = typename Cplx<Real>::T;
-  constexpr int NT = kSumThreads, UB = sizeof(A) == 16 ? 0 : 1;
+  constexpr int NT = kThreads, UB = sizeof(A) == 16 ? 0 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t joff[kMaxUnitSteps];
   __shared__ double red[NT / 32];
@@ -141,11 +141,11 @@ __global__ void __launch_bounds__(kSumThreads, 3)
     for (int s = 0; s < P.num_segs; s++) {
       const PauliSeg& sg = ss[s];
       const uint32_t a0 = sg.alpha[0], a1 = sg.alpha[1], a2 = sg.alpha[2];
-      const uint32_t lane_off = group_lane_offset<7>(sg);
+      const uint32_t lane_off = group_lane_offset<8>(sg);
       for (uint32_t g0 = 0; g0 + tid < groups; g0 += 2 * NT) {
         const bool two = g0 + NT + tid < groups;
-        const uint32_t off = lane_off ^ group_step_offset<7>(sg, g0);
-        const uint32_t off1 = two ? lane_off ^ group_step_offset<7>(sg, g0 + NT) : off;
+        const uint32_t off = lane_off ^ group_step_offset<8>(sg, g0);
+        const uint32_t off1 = two ? lane_off ^ group_step_offset<8>(sg, g0 + NT) : off;
         A v[2][8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
@@ -238,12 +238,12 @@ __device__ __forceinline__ void apply_string(const A (&v)[8], double2 (&l)[8], d
 // The tile of lambda is held in FP64 for both types and rounded to the
 // state's type once, at its store.
 template <typename Real>
-__global__ void __launch_bounds__(kApplyThreads, sizeof(Real) == 8 ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, 2)
     k_pauli_apply(const typename Cplx<Real>::T* __restrict__ psi, typename Cplx<Real>::T* __restrict__ lam,
                   const __grid_constant__ PauliPass P, const PauliSeg* __restrict__ segs,
                   const PauliTerm* __restrict__ terms, int accumulate, double* __restrict__ energy_partials) {
   using A = typename Cplx<Real>::T;
-  constexpr int NT = kApplyThreads, UB = sizeof(A) == 16 ? 0 : 1;
+  constexpr int NT = kThreads, UB = sizeof(A) == 16 ? 0 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t joff[kMaxUnitSteps];
   __shared__ double red[NT / 32];
@@ -287,9 +287,9 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(Real) == 8 ? 3 : 2)
     for (int s = 0; s < P.num_segs; s++) {
       const PauliSeg& sg = ss[s];
       const uint32_t a0 = sg.alpha[0], a1 = sg.alpha[1], a2 = sg.alpha[2];
-      const uint32_t lane_off = group_lane_offset<7>(sg);
+      const uint32_t lane_off = group_lane_offset<8>(sg);
       for (uint32_t g0 = 0; g0 + tid < groups; g0 += NT) {
-        const uint32_t off = lane_off ^ group_step_offset<7>(sg, g0);
+        const uint32_t off = lane_off ^ group_step_offset<8>(sg, g0);
         A v[8];
         double2 l[8];
 #pragma unroll
@@ -365,10 +365,10 @@ int launch_sum_t(const void* amp, const PauliPass& P, const PauliSeg* d_segs, co
   auto kern = k_pauli_sum<Real>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSumThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
   uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm > kPauliCtasPerSm ? kPauliCtasPerSm : per_sm);
   if (grid > P.tiles_per_state) grid = P.tiles_per_state;
-  kern<<<(unsigned)grid, kSumThreads, smem, stream>>>((const A*)amp, P, d_segs, d_terms, d_partials);
+  kern<<<(unsigned)grid, kThreads, smem, stream>>>((const A*)amp, P, d_segs, d_terms, d_partials);
   count_launch();
   *parts = (int)grid;
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
@@ -382,10 +382,10 @@ int launch_apply_t(const void* psi, void* lam, const PauliPass& P, const PauliSe
   auto kern = k_pauli_apply<Real>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kApplyThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
   uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);
   if (grid > P.num_tiles) grid = P.num_tiles;
-  kern<<<(unsigned)grid, kApplyThreads, smem, stream>>>((const A*)psi, (A*)lam, P, d_segs, d_terms,
+  kern<<<(unsigned)grid, kThreads, smem, stream>>>((const A*)psi, (A*)lam, P, d_segs, d_terms,
                                                         accumulate ? 1 : 0, d_epart);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
