@@ -39,7 +39,7 @@ constexpr int kUnladderBits = 11, kUnladderLow = 4;  // tile of k_unladder, cont
 // rotation passes
 // ---------------------------------------------------------------------------
 // One tile per step and CTA: 2^m amplitudes base ^ span(basis), whose local
-// index bits 0.. are contiguous amplitudes.  Four warps; the 16-byte units of
+// index bits 0.. are contiguous amplitudes.  The 16-byte units of
 // a tile (one complex128 or two complex64 amplitudes) come by cp.async, all
 // in flight at once.  A segment's thread holds groups of 8 amplitudes whose
 // register index is the segment's three target bits, so every rotation is
@@ -56,10 +56,13 @@ constexpr int kUnladderBits = 11, kUnladderLow = 4;  // tile of k_unladder, cont
 // gate-by-gate passes with the CNOTs carried out (19 forward, 17 backward),
 // 134 ms by these (6 and 9); complex64 326 -> 116 ms, and of 100 ms after
 // lambda's passes 90 ms with values converted to FP64 once a segment.
-template <typename Real> struct HeaCfg;
-template <> struct HeaCfg<double> { static constexpr int FWD_BITS = 12, BACK_BITS = 11; };
-template <> struct HeaCfg<float> { static constexpr int FWD_BITS = 13, BACK_BITS = 12; };
-constexpr int kHeaThreads = 128, kHeaWarps = kHeaThreads / 32;
+template <typename Real, bool BACK> struct HeaCfg;
+// Three CTAs of four warps, at 168 registers.  Two of eight warps at 128
+// registers measured 8 % slower forward and 20 % slower backward in complex64.
+template <> struct HeaCfg<double, false> { static constexpr int BITS = 12, NT = 128, CTAS = 3; };
+template <> struct HeaCfg<double, true> { static constexpr int BITS = 11, NT = 128, CTAS = 3; };
+template <> struct HeaCfg<float, false> { static constexpr int BITS = 13, NT = 128, CTAS = 3; };
+template <> struct HeaCfg<float, true> { static constexpr int BITS = 12, NT = 128, CTAS = 3; };
 
 // Per-state tables of a segment.
 template <typename Real>
@@ -117,36 +120,36 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 }
 
 template <typename Real, bool BACK>
-__global__ void __launch_bounds__(kHeaThreads, 3)
+__global__ void __launch_bounds__(HeaCfg<Real, BACK>::NT, HeaCfg<Real, BACK>::CTAS)
     k_hea(const typename Cplx<Real>::T* src, typename Cplx<Real>::T* psi, typename Cplx<Real>::T* lam,
           const __grid_constant__ HeaPass P, const HeaSeg* __restrict__ segs, const double2* __restrict__ cs,
           double* __restrict__ partials, int part_stride) {
   using A = typename Cplx<Real>::T;
-  constexpr int NT = kHeaThreads;
+  constexpr int NT = HeaCfg<Real, BACK>::NT, TB = NT == 256 ? 8 : 7, kWarps = NT / 32;
   constexpr int UB = sizeof(A) == 16 ? 0 : 1;  // log2 of the amplitudes of a 16-byte unit
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t tile_bytes = (uint32_t)sizeof(A) << P.m;
   unsigned char* tables = smem + (BACK ? 2u : 1u) * tile_bytes;
   HeaTab<Real>* tab = reinterpret_cast<HeaTab<Real>*>(tables);
   double* red = reinterpret_cast<double*>(tab + P.num_segs);  // [warp][slot], backward only
-  __shared__ uint32_t joff[1 << (kMaxHeaBits - 7)];            // index offset of unit j * NT
+  __shared__ uint32_t joff[1 << (kMaxHeaBits - TB)];            // index offset of unit j * NT
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nslots = P.num_segs * kHeaSlots;
-  HeaSeg* sseg = reinterpret_cast<HeaSeg*>(red + (BACK ? kHeaWarps * nslots : 0));
+  HeaSeg* sseg = reinterpret_cast<HeaSeg*>(red + (BACK ? kWarps * nslots : 0));
   const uint32_t units = 1u << (P.m - UB), groups = 1u << (P.m - 3);
 
-  for (uint32_t j = tid; j < (1u << (kMaxHeaBits - 7)); j += NT) {
+  for (uint32_t j = tid; j < (1u << (kMaxHeaBits - TB)); j += NT) {
     uint32_t off = 0;
 #pragma unroll
-    for (int b = 7; b < kMaxHeaBits - UB; b++)
-      if (b + UB < P.m && (j >> (b - 7) & 1u)) off ^= P.basis[b + UB];
+    for (int b = TB; b < kMaxHeaBits - UB; b++)
+      if (b + UB < P.m && (j >> (b - TB) & 1u)) off ^= P.basis[b + UB];
     joff[j] = off;
   }
   for (int i = tid; i < P.num_segs * (int)(sizeof(HeaSeg) / 4); i += NT)
     reinterpret_cast<uint32_t*>(sseg)[i] = reinterpret_cast<const uint32_t*>(segs)[i];
   uint32_t toff = 0;  // this thread's part of a unit's index
 #pragma unroll
-  for (int b = 0; b < 7; b++)
+  for (int b = 0; b < TB; b++)
     if (b + UB < P.m && (tid >> b & 1)) toff ^= P.basis[b + UB];
   const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   __syncthreads();
@@ -212,7 +215,7 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
           }
         }
         if (BACK)
-          for (int i = tid; i < kHeaWarps * nslots; i += NT) red[i] = 0.0;
+          for (int i = tid; i < kWarps * nslots; i += NT) red[i] = 0.0;
       }
       asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
       __syncthreads();
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
         if (__popc(sg.fun[1] & base) & 1) off0 ^= a1;
         if (__popc(sg.fun[2] & base) & 1) off0 ^= a2;
 #pragma unroll
-        for (int q = 0; q < 7; q++)
+        for (int q = 0; q < TB; q++)
           if (tid >> q & 1) off0 ^= sg.kappa[q];
         const uint32_t flip = tb.flip;
         const Real t0 = tb.t[0], t1 = tb.t[1], t2 = tb.t[2];
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
           const bool active = g0 + tid < groups;
           uint32_t off = off0;
 #pragma unroll
-          for (int q = 7; q < kMaxHeaBits - 3; q++)
+          for (int q = TB; q < kMaxHeaBits - 3; q++)
             if (g0 >> q & 1u) off ^= sg.kappa[q];
           A v[8], w[8];
           if (active) {
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(kHeaThreads, 3)
     if (BACK) {
       for (int j = tid; j < nslots; j += NT) {
         double t = 0.0;
-        for (int wp = 0; wp < kHeaWarps; wp++) t += red[wp * nslots + j];
+        for (int wp = 0; wp < kWarps; wp++) t += red[wp * nslots + j];
         partials[item * (uint64_t)part_stride + j] = t * tab[j / kHeaSlots].unscale;
       }
       __syncthreads();
@@ -425,15 +428,15 @@ int launch_hea_t(const void* src, void* psi, void* lam, const HeaPass& P, const 
                  double* d_partials, int part_stride, int num_sms, cudaStream_t stream) {
   using A = typename Cplx<Real>::T;
   const size_t tile = sizeof(A) << P.m;
-  const size_t red = BACK ? sizeof(double) * kHeaWarps * kHeaSlots : 0;
+  const size_t red = BACK ? sizeof(double) * (HeaCfg<Real, BACK>::NT / 32) * kHeaSlots : 0;
   const size_t smem = (BACK ? 2 : 1) * tile + P.num_segs * (sizeof(HeaTab<Real>) + red + sizeof(HeaSeg));
   auto kern = k_hea<Real, BACK>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kHeaThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, HeaCfg<Real, BACK>::NT, smem);
   uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);
   if (grid > P.num_items) grid = P.num_items;
-  kern<<<(unsigned)grid, kHeaThreads, smem, stream>>>((const A*)src, (A*)psi, (A*)lam, P, d_segs, d_cs, d_partials,
+  kern<<<(unsigned)grid, HeaCfg<Real, BACK>::NT, smem, stream>>>((const A*)src, (A*)psi, (A*)lam, P, d_segs, d_cs, d_partials,
                                                       part_stride);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
@@ -442,8 +445,8 @@ int launch_hea_t(const void* src, void* psi, void* lam, const HeaPass& P, const 
 }  // namespace
 
 int hea_tile_bits(int dtype, bool backward) {
-  if (dtype == MLB_C128) return backward ? HeaCfg<double>::BACK_BITS : HeaCfg<double>::FWD_BITS;
-  return backward ? HeaCfg<float>::BACK_BITS : HeaCfg<float>::FWD_BITS;
+  if (dtype == MLB_C128) return backward ? HeaCfg<double, true>::BITS : HeaCfg<double, false>::BITS;
+  return backward ? HeaCfg<float, true>::BITS : HeaCfg<float, false>::BITS;
 }
 
 int launch_adj_init(int dtype, void* psi, int n, uint64_t batch, uint64_t hf, cudaStream_t stream) {
