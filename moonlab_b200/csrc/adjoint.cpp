@@ -375,7 +375,7 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
       return hfail(rc, "operand image build");
     cudaMemsetAsync(h->d_ferr, 0, sizeof(int), h->stream);
     // |0...0>: the tape itself starts with X on the hf_reference bits (vqe.c:1953-1959)
-    if ((rc = launch_adj_init(h->dtype, h->psi, (int)h->n, B, 0, h->stream))) return hfail(rc, "init kernel");
+    if ((rc = launch_adj_init(h->psi, (int)h->n, B, h->stream))) return hfail(rc, "init kernel");
   }
   for (size_t k = 0; k < nseg; k++) {
     if (fused) {

@@ -416,11 +416,10 @@ __global__ void __launch_bounds__(256) k_unladder(const float2* __restrict__ src
   }
 }
 
-template <typename Real>
-__global__ void k_adj_init(typename Cplx<Real>::T* __restrict__ psi, uint64_t dim, uint64_t total, uint64_t hf) {
-  using A = typename Cplx<Real>::T;
+// |0...0> in every state, for the tensor-core forward sweep (complex64).
+__global__ void k_adj_init(float2* __restrict__ psi, uint64_t dim, uint64_t total) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x)
-    psi[i] = ((i % dim) == hf) ? A{1, 0} : A{0, 0};
+    psi[i] = (i & (dim - 1)) == 0 ? make_float2(1.f, 0.f) : make_float2(0.f, 0.f);
 }
 
 template <typename Real, bool BACK>
@@ -449,12 +448,11 @@ int hea_tile_bits(int dtype, bool backward) {
   return backward ? HeaCfg<float, true>::BITS : HeaCfg<float, false>::BITS;
 }
 
-int launch_adj_init(int dtype, void* psi, int n, uint64_t batch, uint64_t hf, cudaStream_t stream) {
+int launch_adj_init(void* psi, int n, uint64_t batch, cudaStream_t stream) {
   const uint64_t dim = 1ull << n, total = dim * batch;
   uint64_t grid = (total + 255) / 256;
   if (grid > 148ull * 32) grid = 148ull * 32;
-  if (dtype == MLB_C128) k_adj_init<double><<<(unsigned)grid, 256, 0, stream>>>((double2*)psi, dim, total, hf);
-  else k_adj_init<float><<<(unsigned)grid, 256, 0, stream>>>((float2*)psi, dim, total, hf);
+  k_adj_init<<<(unsigned)grid, 256, 0, stream>>>((float2*)psi, dim, total);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }

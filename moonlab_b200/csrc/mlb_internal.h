@@ -153,7 +153,7 @@ int launch_adj_energy(const double* d_partials, uint64_t tiles_per_state, uint64
 // complex64: dst[b][p] = src[b][C^-k p], C the CNOT ladder on n qubits
 // (hea_plan.h).
 int launch_unladder(const void* src, void* dst, int n, int k, uint64_t batch, int num_sms, cudaStream_t stream);
-int launch_adj_init(int dtype, void* psi, int n, uint64_t batch, uint64_t hf, cudaStream_t stream);
+int launch_adj_init(void* psi, int n, uint64_t batch, cudaStream_t stream);
 // d_norm[b] = |psi_b|^2 of a complex64 batch; then d_out ([B] energies,
 // [B][P] gradients) divided by it.
 int launch_batch_norm(const void* psi_c64, uint64_t dim, uint64_t batch, double* d_norm, cudaStream_t stream);
