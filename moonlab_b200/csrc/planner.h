@@ -1,12 +1,12 @@
 // planner.h -- groups a gate-op sequence into tile passes and, inside a
-// pass, into register-group segments (used by the state engine and by the
-// adjoint-gradient engine).  Host-only.
+// pass, into register-group segments, for the state engine.  Host-only.
 #pragma once
 
 #include <algorithm>
-#include <iterator>
 #include <cstdint>
 #include <cstring>
+#include <functional>
+#include <iterator>
 #include <vector>
 
 #include "mlb_internal.h"
@@ -52,7 +52,6 @@ struct Planner {
   uint32_t n;
   int dtype;
   Geo g;
-  int max_ops = kMaxPassOps;  // ops per pass (the op program lives in shared memory)
   // complex128 with dense segments: a register segment is closed before an
   // op that would take its conditioning qubits (controls and diagonal keys
   // outside its four register bits) past what one dense 16x16 segment holds,
@@ -68,6 +67,7 @@ struct Planner {
   std::vector<DevSegment> segs;
   std::vector<DevOp> dops;
   std::vector<int> dop_src;  // index into the planned ops of every entry of dops
+  std::function<void(const PlannedPass&)> on_pass;  // called with each pass once it is final
 
   // Choose the ops of one pass from `rem` (indices into ops), program order.
   // Returns taken indices; fills high mask.
@@ -85,7 +85,7 @@ struct Planner {
         const uint64_t Q = op_qubits(o), T = op_targets(o);
         if (Q & blocked) { blocked |= Q; if (blocked == allm) break; continue; }
         const uint64_t need = T & ~lowm & ~SH;
-        if (cnt >= max_ops) break;
+        if (cnt >= kMaxPassOps) break;  // the op program lives in shared memory
         if (need == 0 || (grow && popc(SH | need) <= Hmax)) {
           SH |= need;
           cnt++;
@@ -159,22 +159,35 @@ struct Planner {
     };
     cut.assign(N, 0);
     std::vector<int> blockers(N, 0);
-    std::vector<std::vector<int>> after(N);
-    for (size_t i = 0; i < N; i++)
-      for (size_t j = 0; j < i; j++) {
-        const bool commute = (T[i] & (T[j] | D[j])) == 0 && (T[j] & (T[i] | D[i])) == 0;
-        if (!commute) {
+    const size_t W = (N + 63) / 64;
+    std::vector<uint64_t> after(N * W, 0), ready(W, 0);  // bits: the ops waiting for op j; those with no blocker left
+    for (size_t i = 0; i < N; i++) {
+      const uint32_t t = T[i], td = T[i] | D[i];
+      for (size_t j = 0; j < i; j++)
+        if ((t & (T[j] | D[j])) | (T[j] & td)) {  // the two do not commute
           blockers[i]++;
-          after[j].push_back((int)i);
+          after[j * W + (i >> 6)] |= 1ull << (i & 63);
         }
-      }
-    std::vector<bool> done(N, false);
+      if (!blockers[i]) ready[i >> 6] |= 1ull << (i & 63);
+    }
     std::vector<int> out;
     out.reserve(N);
     auto take = [&](size_t i) {
-      done[i] = true;
+      ready[i >> 6] &= ~(1ull << (i & 63));
       out.push_back(taken[i]);
-      for (int k : after[i]) blockers[k]--;
+      for (size_t w = 0; w < W; w++)
+        for (uint64_t b = after[i * W + w]; b; b &= b - 1) {
+          const size_t k = 64 * w + (size_t)__builtin_ctzll(b);
+          if (--blockers[k] == 0) ready[w] |= 1ull << (k & 63);
+        }
+    };
+    // the first op at or after i that may run (taking one only frees later ones)
+    auto next_ready = [&](size_t i) {
+      for (size_t w = i >> 6; w < W; w++) {
+        const uint64_t b = w == i >> 6 ? ready[w] & (~0ull << (i & 63)) : ready[w];
+        if (b) return 64 * w + (size_t)__builtin_ctzll(b);
+      }
+      return N;
     };
     while (out.size() < N) {
       cut[out.size()] = 1;
@@ -184,8 +197,7 @@ struct Planner {
       bool progress = true;
       while (progress) {
         progress = false;
-        for (size_t i = 0; i < N; i++) {
-          if (done[i] || blockers[i] != 0) continue;
+        for (size_t i = next_ready(0); i < N; i = next_ready(i + 1)) {
           if (wide[i]) {  // a generic 4x4 op forms its own segment
             if (!any) {
               take(i);
@@ -208,13 +220,6 @@ struct Planner {
       }
     }
     return out;
-  }
-
-  template <typename LocalMask>
-  std::vector<int> schedule_segments(const std::vector<mlb_op_t>& ops, const std::vector<int>& taken,
-                                     LocalMask&& local_mask, int RB) {
-    std::vector<char> cut;
-    return schedule_segments(ops, taken, local_mask, RB, cut);
   }
 
   void lower_pass(const std::vector<mlb_op_t>& ops, const std::vector<int>& taken, int L, uint64_t SH) {
@@ -423,6 +428,7 @@ struct Planner {
           taken.swap(kept);
         }
       }
+      if (on_pass) on_pass(passes.back());
       // remove taken (both lists ascending)
       std::vector<int> next;
       next.reserve(rem.size() - taken.size());

@@ -295,31 +295,40 @@ struct Lower {
     return false;
   }
 
-  static bool moves(const Item& d, uint32_t dir) {  // a functional of diagonal d changes along dir
-    bool m = d.keyed && hea::parity(d.key.row & dir);
-    for (int i = 0; i < d.nc; i++) m = m || hea::parity(d.cond[i].row & dir);
-    return m;
-  }
-
   void order() {
     const int N = (int)items.size();
-    std::vector<int> rots, diags;
+    struct Turn {
+      uint32_t dir, row;
+      int i;
+    };
+    struct Read {  // a functional that diagonal i reads
+      uint32_t row;
+      int i;
+    };
+    std::vector<Turn> turns;
+    std::vector<Read> reads;
+    turns.reserve(N);
+    reads.reserve(2 * N);
     auto edge = [&](int i, int j) {
       items[i].succ.add(j);
       items[j].pred.add(i);
     };
     for (int j = 0; j < N; j++) {
-      Item& y = items[j];
+      const Item& y = items[j];
       if (y.rotation) {
-        for (int i : rots)
-          if (hea::parity(items[i].fun.row & y.dir) || hea::parity(y.fun.row & items[i].dir)) edge(i, j);
-        for (int i : diags)
-          if (moves(items[i], y.dir)) edge(i, j);
-        rots.push_back(j);
+        const uint32_t dir = y.dir, row = y.fun.row;
+        for (const Turn& x : turns)
+          if (hea::parity(x.row & dir) || hea::parity(row & x.dir)) edge(x.i, j);
+        for (const Read& x : reads)
+          if (hea::parity(x.row & dir)) edge(x.i, j);
+        turns.push_back({dir, row, j});
       } else {
-        for (int i : rots)
-          if (moves(y, items[i].dir)) edge(i, j);
-        diags.push_back(j);
+        const size_t first = reads.size();
+        if (y.keyed) reads.push_back({y.key.row, j});
+        for (int c = 0; c < y.nc; c++) reads.push_back({y.cond[c].row, j});
+        for (const Turn& x : turns)
+          for (size_t k = first; k < reads.size(); k++)
+            if (hea::parity(reads[k].row & x.dir)) edge(x.i, j);
       }
     }
     for (int i = N; i-- > 0;)
@@ -344,6 +353,7 @@ struct Lower {
   // The program of `ops`.  `scale`: the factor owed by rotations so far, left
   // for a later pass's table unless `settle`.  A table has up to 2^max_var variants.
   void build(const std::vector<const mlb_op_t*>& ops, double& scale, bool settle, Program& out, int max_var) {
+    items.reserve(3 * ops.size());
     for (const mlb_op_t* o : ops) add(*o);
     order();
     const int N = (int)items.size(), words = (N + 63) / 64;
@@ -354,7 +364,12 @@ struct Lower {
     D.n = P.n;
     D.m = m;
     for (int i = 0; i < m; i++) D.basis[i] = i < P.L ? 1ull << i : 1ull << P.high[i - P.L];
-    Set done;
+    Set done, turns, reads;  // the rotations and the diagonals
+    for (int i = 0; i < N; i++) (items[i].rotation ? turns : reads).add(i);
+    auto each_left = [&](const Set& of, auto&& f) {  // in program order
+      for (int k = 0; k < words; k++)
+        for (uint64_t b = of.w[k] & ~done.w[k]; b; b &= b - 1) f(64 * k + __builtin_ctzll(b));
+    };
     auto after = [&](const Item& it, const Set& before) {  // its predecessors lie in `before`
       for (int k = 0; k < words; k++)
         if (it.pred.w[k] & ~before.w[k]) return false;
@@ -374,13 +389,14 @@ struct Lower {
         std::vector<int> cand;
         Round r;
         Set open = done;  // and the diagonals that can run now
-        for (int i = 0; i < N; i++)
-          if (!items[i].rotation && !done.has(i) && after(items[i], done)) {
-            open.add(i);
-            r.free.push_back(i);
-          }
-        for (int i = 0; i < N; i++)
-          if (items[i].rotation && !done.has(i) && after(items[i], open)) cand.push_back(i);
+        each_left(reads, [&](int i) {
+          if (!after(items[i], done)) return;
+          open.add(i);
+          r.free.push_back(i);
+        });
+        each_left(turns, [&](int i) {
+          if (after(items[i], open)) cand.push_back(i);
+        });
         // a new direction: the rotation that shares the most later ones with
         // the directions so far, then the one that the longest chain waits for
         while ((int)al.size() < 4) {
@@ -450,7 +466,9 @@ struct Lower {
           const uint32_t t = (1u << b) ^ comb[k];
           bool in = true;
           for (int i = 0; i < 4; i++) in = in && !hea::parity(fn[i] & t);
-          if (in && span.add(t)) ker.push_back(t);
+          if (!in) continue;  // one combination of the directions corrects it
+          if (span.add(t)) ker.push_back(t);
+          break;
         }
       // lanes (the first five group bits) where the tables' variants do not
       // depend on them, so that a warp reads one variant: the common kernel of
@@ -678,8 +696,9 @@ struct Lower {
       // what the registers hold now goes here; with no rotation left, all of it
       do {
         std::vector<int> now;
-        for (int i = 0; i < N && diags; i++)
-          if (!items[i].rotation && !done.has(i) && after(items[i], done) && !later_same(items[i])) now.push_back(i);
+        each_left(reads, [&](int i) {
+          if (after(items[i], done) && !later_same(items[i])) now.push_back(i);
+        });
         for (int form = 0; form < 2; form++)
           for (int i : now)
             if (!done.has(i) && plain(items[i]) == (form == 0) && (form == 0 || left == 0 || (!open.empty() && known(items[i]))))
