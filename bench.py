@@ -643,17 +643,20 @@ def vqe_leg(local, with_cpu: bool):
         t = statistics.median(times)
         grads[dt] = G
         # algorithmic bytes of one batch (per vector, S = one state's bytes):
-        # forward passes read + write psi (2 S each), the first lambda pass
-        # reads psi and writes lambda (2 S), later ones also read lambda (3 S),
-        # backward passes read + write psi and lambda (4 S each), and each
-        # checkpoint is saved and restored once (2 S + 2 S)
+        # forward passes read + write psi (2 S each; the first, from |0...0>,
+        # only writes), the first lambda pass reads psi and writes lambda
+        # (2 S), later ones also read lambda (3 S), backward passes read +
+        # write psi and lambda (4 S each).  Checkpoints are passes' own
+        # inputs and outputs, except with the tensor-core forward sweep: that
+        # one starts from a written state, saves and restores each checkpoint
+        # by a copy (2 S + 2 S) and reads the final state's norm.
         ps, ev = p.plan_stats(), p.last_eval_stats()
         S = (16 if dt == "c128" else 8) << 20
         ck = 0
         if ev["checkpoints"]:
             ck = -(-8 // ev["segment_layers"]) - 1  # segments - 1
-        fwd = ev["fused_forward_passes"] if ev["fused_forward"] else ps["forward_passes"]
-        per_vec = S * (2 * fwd + 2 + 3 * (ps["lambda_passes"] - 1) + 4 * ps["backward_passes"] + 4 * ck)
+        fwd = 2 * ev["fused_forward_passes"] + 2 + 4 * ck if ev["fused_forward"] else 2 * ps["forward_passes"] - 1
+        per_vec = S * (fwd + 2 + 3 * (ps["lambda_passes"] - 1) + 4 * ps["backward_passes"])
         achieved = per_vec * len(prob.params) / t / 1e9
         path = ("complex128 adjoint tile passes on the CUDA cores" if dt == "c128" else
                 "complex64: forward sweep on the tensor cores (fused <= 5-qubit blocks, per-vector operand "
@@ -666,7 +669,7 @@ def vqe_leg(local, with_cpu: bool):
                    "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                                 "frac": achieved / peak, "peak_source": peak_kind,
                                 "algorithmic_bytes_per_vector": per_vec,
-                                "kernel": "k_adj_gates / k_adj_pauli (whole evaluation)"}}
+                                "kernel": "k_hea / k_pauli_apply (whole evaluation)"}}
         p.close()
     res["c64_max_rel_grad_err"] = float(np.abs(grads["c64"] - grads["c128"]).max() /
                                         max(1e-300, np.abs(grads["c128"]).max()))

@@ -152,7 +152,7 @@ int  mlb_expect_pauli_sum(mlb_state_t *s, size_t num_terms, const uint64_t *xmas
  * reserved all of HBM up front under a fixed budget (a serving process, or a
  * host framework whose own allocator owns the device), and latency-critical
  * loops where cudaMalloc / cudaFree would stall on device synchronisation.
- * Its scratch is one fixed array per device inside this library, 1,163,264
+ * Its scratch is one fixed array per device inside this library, 286,720
  * bytes, which sets the limit: num_qubits 1..30, else MLB_ERR_NUM_QUBITS.
  * All calls on a device share that array: two calls whose kernels overlap on
  * the GPU (different streams, or different host threads) race and return
