@@ -12,9 +12,12 @@
 //     0 <= t <= 1 (the columns swapped first, an X, where |U00| < |U10|).  The
 //     rotation costs two multiply-adds per component pair; s is folded into
 //     the next table.
+//     Factors and their products are long double until a table's entry is
+//     rounded: 20 qubits, depth 16: the norm drifts 5e-16, with doubles
+//     4.8e-15, as 16x16 matrices 2.8e-15.
 //   * Diagonals (those factors, RZ, phases, ZZ, controlled phases) are
 //     products over the functionals they read.  All that are due are merged
-//     into one table of a complex factor per register index, in up to 8
+//     into one table of a complex factor per register index, in up to 16
 //     variants for the parities of functionals that the registers do not hold.
 // A segment keeps 16 amplitudes of a group in registers along four
 // directions and runs every rotation whose direction lies in their span, in
@@ -38,6 +41,7 @@ namespace mlb {
 namespace rot {
 
 using cd = std::complex<double>;
+using cl = std::complex<long double>;  // products of many factors, rounded once
 
 struct Fun {  // parity(row & t) ^ parity(out & tile base) ^ c
   uint32_t row = 0;
@@ -61,17 +65,22 @@ struct Item {
   // rotation: direction, its target bit and its tangent; scale owed
   uint32_t dir = 0;
   Fun fun;
-  double t = 0, s = 1;
+  double t = 0;
+  long double s = 1;
   // diagonal: where every condition holds, d[0] or d[1] by the key (no key: d[1])
   Fun cond[3];
   int nc = 0;
   bool keyed = false;
   Fun key;
-  cd d[2] = {1.0, 1.0};
+  cl d[2] = {1.0L, 1.0L};
   Set pred, succ;
   int height = 0;
 };
 
+inline cl mul(cl a, cl b) {
+  const long double br = b.real(), bi = b.imag();
+  return {a.real() * br - a.imag() * bi, a.real() * bi + a.imag() * br};
+}
 inline cd mul(cd a, cd b) {
   return {a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()};
 }
@@ -200,7 +209,7 @@ struct Lower {
     return f;
   }
 
-  void diag(const std::vector<Fun>& cond, bool keyed, const Fun& key, cd d0, cd d1) {
+  void diag(const std::vector<Fun>& cond, bool keyed, const Fun& key, cl d0, cl d1) {
     if (keyed && cond.empty())  // one on the same functional, with no rotation between that changes it: merged
       for (int i = (int)items.size(); i-- > 0;) {
         Item& it = items[i];
@@ -262,22 +271,24 @@ struct Lower {
     }
     // a = s u, c = s u t v, d = s u w v: diag(1, v) s [[1, -t], [t, 1]] diag(u, u w).
     // A real c / a needs no diag(1, v) (t takes the sign).
-    const double s = std::abs(a);
-    const cd u = a / s, r = mul(c, std::conj(u)) / s;  // t v
-    double t = std::abs(r);
-    cd v = 1.0;
-    if (std::abs(r.imag()) <= 4e-16) t = r.real();
-    else v = r / t;
-    const cd w = mul(mul(d, std::conj(u)), std::conj(v)) / std::abs(d);
+    auto wide = [](cd x) { return cl(x.real(), x.imag()); };
+    auto size = [](cl x) { return std::sqrt(x.real() * x.real() + x.imag() * x.imag()); };
+    const long double s = size(wide(a));
+    const cl u = wide(a) / s, r = mul(wide(c), std::conj(u)) / s;  // t v
+    double t = (double)size(r);
+    cl v = 1.0L;
+    if (std::abs(r.imag()) <= 4e-16L) t = (double)r.real();
+    else v = r / size(r);
+    const cl w = mul(mul(wide(d), std::conj(u)), std::conj(v)) / size(wide(d));
     diag({}, true, label[q], u, mul(u, w));
     Item it;
     it.rotation = true;
     it.dir = dir[q];
     it.fun = label[q];
-    it.t = t;
-    it.s = s;
+    it.t = dtype == MLB_C128 ? t : (double)(float)t;  // as the kernel holds it
+    it.s = 1.0L / std::sqrt(1.0L + (long double)it.t * it.t);  // of the rounded t: the rotation keeps norms
     items.push_back(it);
-    if (v != 1.0) diag({}, true, label[q], 1.0, v);
+    if (v != cl(1.0L)) diag({}, true, label[q], 1.0L, v);
   }
 
   // The pass's program, with fewer variants a table where its tables would
@@ -285,7 +296,7 @@ struct Lower {
   static bool lower(const DevPass& pass, int dtype, const std::vector<const mlb_op_t*>& ops, Program& out) {
     for (int max_var = kRotMaxVar; max_var >= 1; max_var--) {
       Program p;
-      double scale = 1.0;
+      long double scale = 1.0;
       Lower(pass, dtype).build(ops, scale, true, p, max_var);
       if (rot_shared_bytes(dtype, p.ops.size(), p.table.size()) > kRotMaxShared) continue;
       p.dev.entries = (uint32_t)p.table.size();
@@ -352,7 +363,7 @@ struct Lower {
 
   // The program of `ops`.  `scale`: the factor owed by rotations so far, left
   // for a later pass's table unless `settle`.  A table has up to 2^max_var variants.
-  void build(const std::vector<const mlb_op_t*>& ops, double& scale, bool settle, Program& out, int max_var) {
+  void build(const std::vector<const mlb_op_t*>& ops, long double& scale, bool settle, Program& out, int max_var) {
     items.reserve(3 * ops.size());
     for (const mlb_op_t* o : ops) add(*o);
     order();
@@ -592,7 +603,8 @@ struct Lower {
       auto close = [&](RotOp op) {  // emits op with the open table
         const uint32_t nv = (uint32_t)var.size();
         const size_t at = out.table.size();
-        out.table.resize(at + ((size_t)16 << nv), cd(scale, 0.0));
+        out.table.resize(at + ((size_t)16 << nv));
+        std::vector<cl> wide((size_t)16 << nv, cl(scale, 0.0L));
         scale = 1.0;
         struct Bit {
           uint32_t reg, v, c;  // patterns over the register index and the variant
@@ -616,10 +628,11 @@ struct Lower {
             for (uint32_t x = 0; x < (1u << nv); x++) {
               bool on = true;
               for (int c = 0; c < d.nc; c++) on = on && cond[c].at(k, x);
-              cd& e = out.table[at + 16 * x + k];
+              cl& e = wide[16 * x + k];
               if (on) e = mul(e, d.d[key.at(k, x)]);
             }
         }
+        for (size_t k = 0; k < wide.size(); k++) out.table[at + k] = cd((double)wide[k].real(), (double)wide[k].imag());
         op.table = (uint32_t)at;
         op.nv = (uint8_t)nv;
         op.flags |= kRotTable;
