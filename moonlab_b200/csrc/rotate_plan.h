@@ -106,7 +106,7 @@ inline bool covers(const mlb_op_t& o) {
     case MLB_OP_X: return plan::popc(o.cmask) <= 1;
     case MLB_OP_SWAP: return o.cmask == 0;
     case MLB_OP_DIAG1: return plan::popc(o.cmask) <= 2;
-    case MLB_OP_ZZ: return true;
+    case MLB_OP_ZZ: return plan::popc(o.cmask) <= 3;
     case MLB_OP_PHASE: return plan::popc(o.cmask) <= 3;
     default: return false;
   }
@@ -257,7 +257,7 @@ struct Lower {
       case MLB_OP_ZZ: {
         Fun f = fun(o.target);
         f.add(fun(o.target2));
-        diag({}, true, f, cd(o.m[0], o.m[1]), cd(o.m[2], o.m[3]));
+        diag(cond, true, f, cd(o.m[0], o.m[1]), cd(o.m[2], o.m[3]));
         return;
       }
       default: break;

@@ -1,0 +1,110 @@
+"""Rotation programs (rotate_plan.h) on the host: lowered as a state lowers
+them, run as the kernel runs them (rotate_plan_host.cpp), against the ops
+themselves in numpy.  Every form that a program takes: controls and targets
+inside and outside the tile, on as many qubits as it accepts.  Tolerance
+1e-12 per amplitude of a normalised state, as for the kernels."""
+from __future__ import annotations
+
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from moonlab_b200 import _lib
+from tests.test_tile_plan import OP_1Q, OP_DIAG1, OP_PHASE, OP_SWAP, OP_X, OP_ZZ, apply_op
+
+ROOT = Path(__file__).resolve().parent.parent
+TILE = 0b1011010111  # 7 of 10 qubits
+LIMIT = {OP_1Q: 0, OP_X: 1, OP_SWAP: 0, OP_DIAG1: 2, OP_ZZ: 3, OP_PHASE: 3}  # controls that a program takes
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    out = tmp_path_factory.mktemp("rot") / "rotate_plan_host.so"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I/usr/local/cuda/include",
+                    f"-I{ROOT}/include", f"-I{ROOT}/moonlab_b200/csrc", "-o", str(out),
+                    str(ROOT / "tests" / "rotate_plan_host.cpp")], check=True)
+    lib = C.CDLL(str(out))
+    lib.host_run.argtypes = [C.c_void_p, C.c_size_t, C.c_int, C.c_uint64, C.c_int, C.c_void_p]
+    lib.host_push_forward.argtypes = [C.c_void_p, C.c_size_t, C.c_uint32]
+    lib.host_covers.argtypes = [C.c_void_p]
+    return lib
+
+
+def unitary(rng):
+    q, r = np.linalg.qr(rng.standard_normal((2, 2)) + 1j * rng.standard_normal((2, 2)))
+    return (q * (np.diag(r) / np.abs(np.diag(r)))).reshape(-1)
+
+
+def make(kind, target, target2=-1, controls=(), m=()):
+    o = _lib.MlbOp()
+    o.kind, o.target, o.target2 = kind, target, target2
+    o.cmask = sum(1 << int(c) for c in controls)
+    for i, x in enumerate(m):
+        o.m[2 * i], o.m[2 * i + 1] = x.real, x.imag
+    return o
+
+
+def random_op(rng, n, tile, kind, controls):
+    inside = [q for q in range(n) if tile >> q & 1]
+    moved = kind in (OP_1Q, OP_X, OP_SWAP)
+    t = int(rng.choice(inside if moved else range(n)))
+    rest = [q for q in (inside if kind == OP_SWAP else range(n)) if q != t]
+    pick = [int(q) for q in rng.permutation(rest)[:1 + controls]]
+    phases = np.exp(1j * rng.uniform(-np.pi, np.pi, 2))
+    if kind in (OP_SWAP, OP_ZZ):
+        return make(kind, t, pick[0], pick[1:], () if kind == OP_SWAP else phases)
+    if kind == OP_PHASE:
+        return make(kind, t, -1, [t] + pick[1:controls], phases[:1])
+    return make(kind, t, -1, pick[1:], unitary(rng) if kind == OP_1Q else () if kind == OP_X else phases)
+
+
+def run_both(host, n, tile, ops, dtype, seed):
+    rng = np.random.default_rng(seed)
+    a = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    a /= np.linalg.norm(a)
+    want, got = a.copy(), a.copy()
+    arr = (_lib.MlbOp * len(ops))(*ops)
+    for o in ops:
+        apply_op(want, n, o)
+    assert host.host_run(arr, len(ops), n, tile, dtype, got.ctypes.data) == 0
+    return want, got
+
+
+@pytest.mark.parametrize("dtype", [_lib.MLB_C128, _lib.MLB_C64])
+@pytest.mark.parametrize("kind,controls", [(k, c) for k, most in LIMIT.items() for c in range(most + 1)
+                                           if not (k == OP_PHASE and c == 0)])
+def test_each_form(host, kind, controls, dtype):
+    rng = np.random.default_rng(17 * kind + controls)
+    for trial in range(6):  # the form between rotations, so that nothing merges it away
+        ops = []
+        for _ in range(8):
+            ops += [random_op(rng, 10, TILE, OP_1Q, 0) for _ in range(3)]
+            ops += [random_op(rng, 10, TILE, kind, controls) for _ in range(2)]
+        assert host.host_covers(C.byref(ops[-1]))
+        want, got = run_both(host, 10, TILE, ops, dtype, trial)
+        # complex64 programs hold their tangents in 32 bits
+        assert np.abs(got - want).max() < (1e-12 if dtype == _lib.MLB_C128 else 2e-6)
+
+
+@pytest.mark.parametrize("kind", list(LIMIT))
+def test_more_controls_are_left_to_the_other_path(host, kind):
+    rng = np.random.default_rng(kind)
+    for controls in range(LIMIT[kind] + 1, 6):
+        o = random_op(rng, 12, (1 << 12) - 1, kind, controls)
+        assert not host.host_covers(C.byref(o))
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_mixed_ops(host, seed):
+    rng = np.random.default_rng(900 + seed)
+    n = int(rng.integers(6, 12))
+    tile = 3 | sum(1 << int(q) for q in rng.choice(np.arange(2, n), min(n - 2, 4), replace=False))
+    ops = []
+    for _ in range(int(rng.integers(1, 50))):
+        kind = int(rng.choice(list(LIMIT)))
+        ops.append(random_op(rng, n, tile, kind, int(rng.integers(kind == OP_PHASE, LIMIT[kind] + 1))))
+    want, got = run_both(host, n, tile, ops, _lib.MLB_C128, seed)
+    assert np.abs(got - want).max() < 1e-12
