@@ -426,11 +426,14 @@ template <typename Real, bool BACK>
 int launch_hea_t(const void* src, void* psi, void* lam, const HeaPass& P, const HeaSeg* d_segs, const double2* d_cs,
                  double* d_partials, int part_stride, int num_sms, cudaStream_t stream) {
   using A = typename Cplx<Real>::T;
-  const size_t tile = sizeof(A) << P.m;
-  const size_t red = BACK ? sizeof(double) * (HeaCfg<Real, BACK>::NT / 32) * kHeaSlots : 0;
-  const size_t smem = (BACK ? 2 : 1) * tile + P.num_segs * (sizeof(HeaTab<Real>) + red + sizeof(HeaSeg));
+  auto shared = [](int bits, int segs) {
+    const size_t red = BACK ? sizeof(double) * (HeaCfg<Real, BACK>::NT / 32) * kHeaSlots : 0;
+    return ((BACK ? 2 : 1) * sizeof(A) << bits) + segs * (sizeof(HeaTab<Real>) + red + sizeof(HeaSeg));
+  };
+  const size_t smem = shared(P.m, P.num_segs);
   auto kern = k_hea<Real, BACK>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> allowed{0};
+  allow_shared(allowed, kern, shared(HeaCfg<Real, BACK>::BITS, kMaxHeaSegs));
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, HeaCfg<Real, BACK>::NT, smem);
   uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);

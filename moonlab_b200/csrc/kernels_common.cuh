@@ -4,6 +4,8 @@
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <atomic>
 #include <cstdint>
 
 namespace mlb {
@@ -53,5 +55,19 @@ __device__ __forceinline__ uint64_t pdep64(uint64_t j, uint64_t mask) {
 }
 
 __device__ __forceinline__ int parity64(uint64_t x) { return __popcll(x) & 1; }
+
+// A kernel's dynamic shared-memory limit, raised once per device to the most
+// that any launch of it takes.  The limit belongs to the function and not to
+// a launch: set to one launch's own size, it would refuse a larger launch of
+// another thread in between.
+template <typename Kernel>
+void allow_shared(std::atomic<uint64_t>& done, Kernel* kernel, size_t most) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess)
+    done.fetch_or(bit, std::memory_order_release);
+}
 
 }  // namespace mlb

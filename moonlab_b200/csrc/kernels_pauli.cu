@@ -353,17 +353,25 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
 }
 
-size_t tables_bytes(const PauliPass& P) {
-  return P.num_terms * (sizeof(double) + sizeof(PauliTerm)) + P.num_segs * sizeof(PauliSeg);
+template <typename Real>
+constexpr int tile_bits(bool apply) {
+  return (sizeof(Real) == 8 ? 12 : 13) - (apply ? 1 : 0);
 }
+
+constexpr size_t tables_bytes(size_t terms, size_t segs) {
+  return terms * (sizeof(double) + sizeof(PauliTerm)) + segs * sizeof(PauliSeg);
+}
+// every segment takes a string at least
+constexpr size_t kMaxTables = tables_bytes(kMaxPauliTerms, kMaxPauliTerms);
 
 template <typename Real>
 int launch_sum_t(const void* amp, const PauliPass& P, const PauliSeg* d_segs, const PauliTerm* d_terms,
                  double* d_partials, int num_sms, cudaStream_t stream, int* parts) {
   using A = typename Cplx<Real>::T;
-  const size_t smem = (sizeof(A) << P.m) + tables_bytes(P);
+  const size_t smem = (sizeof(A) << P.m) + tables_bytes(P.num_terms, P.num_segs);
   auto kern = k_pauli_sum<Real>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> allowed{0};
+  allow_shared(allowed, kern, (sizeof(A) << tile_bits<Real>(false)) + kMaxTables);
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
   uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm > kPauliCtasPerSm ? kPauliCtasPerSm : per_sm);
@@ -378,9 +386,10 @@ template <typename Real>
 int launch_apply_t(const void* psi, void* lam, const PauliPass& P, const PauliSeg* d_segs, const PauliTerm* d_terms,
                    bool accumulate, double* d_epart, int num_sms, cudaStream_t stream) {
   using A = typename Cplx<Real>::T;
-  const size_t smem = ((sizeof(A) + 16) << P.m) + tables_bytes(P);
+  const size_t smem = ((sizeof(A) + 16) << P.m) + tables_bytes(P.num_terms, P.num_segs);
   auto kern = k_pauli_apply<Real>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> allowed{0};
+  allow_shared(allowed, kern, ((sizeof(A) + 16) << tile_bits<Real>(true)) + kMaxTables);
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
   uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm);
@@ -394,13 +403,13 @@ int launch_apply_t(const void* psi, void* lam, const PauliPass& P, const PauliSe
 }  // namespace
 
 int pauli_tile_bits(int dtype, bool apply) {
-  if (dtype == MLB_C128) return apply ? 11 : 12;
-  return apply ? 12 : 13;
+  return dtype == MLB_C128 ? tile_bits<double>(apply) : tile_bits<float>(apply);
 }
 
 int launch_pauli_sum(int dtype, const void* amp, const PauliPass& P, const PauliSeg* d_segs,
                      const PauliTerm* d_terms, double* d_partials, int num_sms, cudaStream_t stream, int* parts) {
-  if (P.m < 3 || P.m > pauli_tile_bits(dtype, false) || P.num_terms < 1 || P.num_terms > kMaxPauliTerms)
+  if (P.m < 3 || P.m > pauli_tile_bits(dtype, false) || P.num_terms < 1 || P.num_terms > kMaxPauliTerms ||
+      P.num_segs > P.num_terms)
     return MLB_ERR_INVALID_ARG;
   return dtype == MLB_C128 ? launch_sum_t<double>(amp, P, d_segs, d_terms, d_partials, num_sms, stream, parts)
                            : launch_sum_t<float>(amp, P, d_segs, d_terms, d_partials, num_sms, stream, parts);
@@ -426,7 +435,8 @@ int launch_sum_partials(const double* d_partials, int count, double* d_out, cuda
 int launch_pauli_apply(int dtype, const void* psi, void* lam, const PauliPass& P, const PauliSeg* d_segs,
                        const PauliTerm* d_terms, bool accumulate, double* d_epart, int num_sms,
                        cudaStream_t stream) {
-  if (P.m < 3 || P.m > pauli_tile_bits(dtype, true) || P.num_terms < 1 || P.num_terms > kMaxPauliTerms)
+  if (P.m < 3 || P.m > pauli_tile_bits(dtype, true) || P.num_terms < 1 || P.num_terms > kMaxPauliTerms ||
+      P.num_segs > P.num_terms)
     return MLB_ERR_INVALID_ARG;
   return dtype == MLB_C128
              ? launch_apply_t<double>(psi, lam, P, d_segs, d_terms, accumulate, d_epart, num_sms, stream)

@@ -22,8 +22,6 @@
 // 192 ms the rotations (FP64), and about 190 ms the part of the memory phases
 // that other CTAs' work does not cover; the same circuit in complex64 takes
 // 457 ms (1197 ms gate by gate).  engine.cpp states where each form runs.
-#include <atomic>
-
 #include "kernels_common.cuh"
 #include "mlb_internal.h"
 
@@ -234,24 +232,13 @@ __global__ void __launch_bounds__(RotCfg<Real>::NT, RotCfg<Real>::CTAS)
 }
 
 template <typename Real>
-void prepare_rot_t() {
-  static std::atomic<uint64_t> set{0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const uint64_t bit = 1ull << (dev & 63);
-  if (set.load(std::memory_order_acquire) & bit) return;
-  cudaFuncSetAttribute(k_rotate<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)((sizeof(typename Cplx<Real>::T) << RotCfg<Real>::BITS) + kRotMaxShared));
-  set.fetch_or(bit, std::memory_order_release);
-}
-
-template <typename Real>
 int launch_rot_t(void* amp, const RotPass& P, const RotSeg* d_segs, const RotOp* d_ops, const void* d_table,
                  int num_sms, cudaStream_t stream) {
   using A = typename Cplx<Real>::T;
   const size_t prog = P.num_ops * sizeof(TileOp<Real>) + P.entries * sizeof(A);
   if (P.m != RotCfg<Real>::BITS || prog > kRotMaxShared) return MLB_ERR_INVALID_ARG;  // whole tiles: every lane has a group
-  prepare_rot_t<Real>();
+  static std::atomic<uint64_t> allowed{0};
+  allow_shared(allowed, k_rotate<Real>, (sizeof(A) << RotCfg<Real>::BITS) + kRotMaxShared);
   const size_t smem = (sizeof(A) << P.m) + prog;
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rotate<Real>, RotCfg<Real>::NT, smem);
