@@ -72,7 +72,14 @@ struct mlb_hea {
   std::vector<TapeOp> tape;
   std::vector<hea::Pass> fwd, bwd;
   std::vector<uint32_t> bound;  // layers before segment k; the last entry is all layers
-  int num_slots = 0;            // gradient slots of all backward passes
+  // backward passes in groups whose gradients are summed together
+  struct GradGroup {
+    size_t end;        // backward passes before this one
+    size_t slots_off;  // the group's first entry of d_slots
+    int slots;
+  };
+  std::vector<GradGroup> groups;
+  int group_slots = 0;  // of the largest group
   // segments: fwd passes [fwd_seg[k], fwd_seg[k+1]) run segment k; bwd
   // passes [bwd_seg[j], bwd_seg[j+1]) run segment C-1-j backwards
   std::vector<size_t> fwd_seg, bwd_seg;
@@ -97,7 +104,7 @@ struct mlb_hea {
   HeaSeg* d_segs = nullptr;
   PauliTerm* d_terms = nullptr;
   PauliSeg* d_psegs = nullptr;
-  int* d_slots = nullptr;  // slot of each parameter
+  int* d_slots = nullptr;  // parameter of each gradient slot, group by group
   double* d_out = nullptr;  // [B] energies then [B][P] grads
   size_t out_cap = 0;
   unsigned char* d_gram = nullptr;  // geometry: Gram matrix, then the Gram kernel's scratch
@@ -199,6 +206,13 @@ HeaPass pass_for_batch(const hea::Pass& p, size_t B) {
   return P;
 }
 
+// Gradient slots of a group of backward passes.  They bound the partials of a
+// vector whatever the depth: with 2^11 complex128 or 2^12 complex64 amplitudes
+// a tile, 512 doubles an item are 1/16 of psi and lambda (18 qubits, 200
+// layers, complex128: 0.5 MB of 8.4; all passes' at once were 7.4 MB).
+constexpr int kGroupSlots = 512;
+static_assert(kMaxHeaSegs * kHeaSlots <= kGroupSlots, "a group holds a pass at least");
+
 // Fused plans of the forward sweep (complex64, N >= 13): each segment's gates
 // grouped into <= 5-qubit blocks and tile passes by the fused planner (on
 // stand-in ops: only their qubits matter), each block's gates recorded in
@@ -260,18 +274,22 @@ int upload_programs(mlb_hea* h) {
       p.segs_off = all_segs.size();
       all_segs.insert(all_segs.end(), p.segs.begin(), p.segs.end());
     }
-  std::vector<int> slot_of_param(h->P, 0);
-  h->num_slots = 0;
-  for (auto& p : h->bwd) {
-    p.slots_off = (size_t)h->num_slots;
-    for (const HeaSeg& sg : p.segs) {
-      for (int i = 0; i < 3; i++)
-        if (sg.param[i] >= 0) {
-          slot_of_param[sg.param[i] + 1] = h->num_slots + i;  // RZ
-          slot_of_param[sg.param[i]] = h->num_slots + 3 + i;  // RY
-        }
-      h->num_slots += kHeaSlots;
-    }
+  std::vector<int> param_of_slot;
+  for (size_t i = 0; i < h->bwd.size(); i++) {
+    hea::Pass& p = h->bwd[i];
+    const int slots = (int)p.segs.size() * kHeaSlots;
+    if (h->groups.empty() || h->groups.back().slots + slots > kGroupSlots)
+      h->groups.push_back({i, param_of_slot.size(), 0});
+    mlb_hea::GradGroup& g = h->groups.back();
+    p.slots_off = (size_t)g.slots;
+    g.end = i + 1;
+    g.slots += slots;
+    h->group_slots = std::max(h->group_slots, g.slots);
+    for (const HeaSeg& sg : p.segs)
+      for (int k = 0; k < kHeaSlots; k++) {  // d/dRZ of its rotations, then d/dRY
+        const int param = sg.param[k % 3];
+        param_of_slot.push_back(param < 0 ? -1 : k < 3 ? param + 1 : param);
+      }
   }
   std::vector<PauliTerm> all_terms;
   std::vector<PauliSeg> all_psegs;
@@ -282,12 +300,12 @@ int upload_programs(mlb_hea* h) {
     all_psegs.insert(all_psegs.end(), p.segs.begin(), p.segs.end());
   }
   cudaError_t e = cudaMalloc((void**)&h->d_segs, all_segs.size() * sizeof(HeaSeg));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_slots, slot_of_param.size() * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_slots, param_of_slot.size() * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_terms, all_terms.size() * sizeof(PauliTerm));
   if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_psegs, all_psegs.size() * sizeof(PauliSeg));
   if (e != cudaSuccess) return cfail(e, "adjoint program upload");
   cudaMemcpy(h->d_segs, all_segs.data(), all_segs.size() * sizeof(HeaSeg), cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_slots, slot_of_param.data(), slot_of_param.size() * sizeof(int), cudaMemcpyHostToDevice);
+  cudaMemcpy(h->d_slots, param_of_slot.data(), param_of_slot.size() * sizeof(int), cudaMemcpyHostToDevice);
   cudaMemcpy(h->d_terms, all_terms.data(), all_terms.size() * sizeof(PauliTerm), cudaMemcpyHostToDevice);
   e = cudaMemcpy(h->d_psegs, all_psegs.data(), all_psegs.size() * sizeof(PauliSeg), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cfail(e, "adjoint program upload");
@@ -352,7 +370,7 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
   }
   const size_t max_tiles = h->lam[0].dev.tiles_per_state * B;  // every lambda pass's tile has the same size
   const uint32_t items = pass_for_batch(h->bwd[0], B).items_per_state;
-  if (h_G && (rc = grow(h->d_part, h->part_cap, (size_t)items * B * h->num_slots))) return rc;
+  if (h_G && (rc = grow(h->d_part, h->part_cap, (size_t)items * B * h->group_slots))) return rc;
   if ((rc = grow(h->d_epart, h->epart_cap, max_tiles))) return rc;
   if ((rc = grow(h->d_out, h->out_cap, B + B * h->P))) return rc;
   // 2. forward
@@ -427,6 +445,7 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
   }
   // 4. backward
   if (h_G) {
+    size_t g = 0;
     for (size_t j = 0; j < nseg; j++) {
       const size_t k = nseg - 1 - j;  // segment swept backwards
       const void* src = h->psi;
@@ -441,14 +460,18 @@ int evaluate_chunk(mlb_hea* h, size_t B, const double* h_params, double* h_E, do
       }
       for (size_t i = h->bwd_seg[j]; i < h->bwd_seg[j + 1]; i++) {
         const hea::Pass& p = h->bwd[i];
+        const mlb_hea::GradGroup& grp = h->groups[g];
         if ((rc = launch_hea_pass(h->dtype, src, h->psi, h->lamb, pass_for_batch(p, B), h->d_segs + p.segs_off,
-                                  h->d_cs, h->d_part + p.slots_off, h->num_slots, true, h->num_sms, h->stream)))
+                                  h->d_cs, h->d_part + p.slots_off, grp.slots, true, h->num_sms, h->stream)))
           return hfail(rc, "backward pass");
         src = h->psi;
+        if (i + 1 < grp.end) continue;
+        if ((rc = launch_hea_reduce(h->d_part, items, grp.slots, B, h->d_slots + grp.slots_off, (int)h->P, h->d_out + B,
+                                    h->stream)))
+          return hfail(rc, "gradient reduce");
+        g++;
       }
     }
-    if ((rc = launch_hea_reduce(h->d_part, items, h->num_slots, B, h->d_slots, (int)h->P, h->d_out + B, h->stream)))
-      return hfail(rc, "gradient reduce");
   }
   if (fused && (rc = launch_divide_by_norm(h->d_out, B, (int)h->P, h->d_norm, h->stream)))
     return hfail(rc, "norm correction");

@@ -91,7 +91,7 @@ struct Pass {
   std::vector<HeaSeg> segs;
   Basis basis;
   size_t segs_off = 0;  // in the problem's device array
-  size_t slots_off = 0; // backward: first gradient slot of the pass
+  size_t slots_off = 0; // backward: first gradient slot of the pass in its group
 };
 
 // Byte offset in the tile's shared memory of local index t: 16-byte units

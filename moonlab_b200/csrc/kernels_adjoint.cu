@@ -344,19 +344,21 @@ __global__ void __launch_bounds__(HeaCfg<Real, BACK>::NT, HeaCfg<Real, BACK>::CT
   }
 }
 
-// d_grads[b][p] = sum over state b's items, in order, of its parameter's slot.
-__global__ void __launch_bounds__(128) k_hea_reduce(const double* __restrict__ partials, uint32_t items,
-                                                    int part_stride, uint64_t batch,
-                                                    const int* __restrict__ slot_of_param, int num_params,
-                                                    double* __restrict__ grads) {
-  const uint64_t total = batch * (uint64_t)num_params;
+// grads[b][p] = sum over state b's items, in order, for the parameter p of
+// each of `slots` slots (-1: none).
+__global__ void __launch_bounds__(128) k_hea_reduce(const double* __restrict__ partials, uint32_t items, int slots,
+                                                    uint64_t batch, const int* __restrict__ param_of_slot,
+                                                    int num_params, double* __restrict__ grads) {
+  const uint64_t total = batch * (uint64_t)slots;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t b = i / num_params;
-    const double* p = partials + b * items * (uint64_t)part_stride + slot_of_param[i % num_params];
-    double s = 0.0;
+    const uint64_t b = i / slots, s = i % slots;
+    const int param = param_of_slot[s];
+    if (param < 0) continue;
+    const double* p = partials + b * items * (uint64_t)slots + s;
+    double sum = 0.0;
 #pragma unroll 8
-    for (uint32_t t = 0; t < items; t++) s += p[t * (uint64_t)part_stride];
-    grads[i] = s;
+    for (uint32_t t = 0; t < items; t++) sum += p[t * (uint64_t)slots];
+    grads[b * (uint64_t)num_params + param] = sum;
   }
 }
 
@@ -472,13 +474,13 @@ int launch_hea_pass(int dtype, const void* psi_src, void* psi, void* lam, const 
   return backward ? run(launch_hea_t<float, true>) : run(launch_hea_t<float, false>);
 }
 
-int launch_hea_reduce(const double* d_partials, uint32_t items, int part_stride, uint64_t batch,
-                      const int* d_slot_of_param, int num_params, double* d_grads, cudaStream_t stream) {
-  const uint64_t total = batch * (uint64_t)num_params;
+int launch_hea_reduce(const double* d_partials, uint32_t items, int slots, uint64_t batch, const int* d_param_of_slot,
+                      int num_params, double* d_grads, cudaStream_t stream) {
+  const uint64_t total = batch * (uint64_t)slots;
   uint64_t grid = (total + 127) / 128;
   if (grid < 1) grid = 1;
   if (grid > 148ull * 16) grid = 148ull * 16;
-  k_hea_reduce<<<(unsigned)grid, 128, 0, stream>>>(d_partials, items, part_stride, batch, d_slot_of_param, num_params,
+  k_hea_reduce<<<(unsigned)grid, 128, 0, stream>>>(d_partials, items, slots, batch, d_param_of_slot, num_params,
                                                    d_grads);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;

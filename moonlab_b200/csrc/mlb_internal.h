@@ -144,9 +144,9 @@ int launch_hea_pass(int dtype, const void* psi_src, void* psi, void* lam, const 
                     const double2* d_cs, double* d_partials, int part_stride, bool backward, int num_sms,
                     cudaStream_t stream);
 // d_grads[b * num_params + p] = sum over a state's items, in order, of the
-// partials of parameter p's slot.
-int launch_hea_reduce(const double* d_partials, uint32_t items, int part_stride, uint64_t batch,
-                      const int* d_slot_of_param, int num_params, double* d_grads, cudaStream_t stream);
+// partials of each slot, p its parameter (-1: none).
+int launch_hea_reduce(const double* d_partials, uint32_t items, int slots, uint64_t batch, const int* d_param_of_slot,
+                      int num_params, double* d_grads, cudaStream_t stream);
 // d_out[b] = the sum of state b's tiles' energy partials, in order.
 int launch_adj_energy(const double* d_partials, uint64_t tiles_per_state, uint64_t batch, double* d_out,
                       cudaStream_t stream);
