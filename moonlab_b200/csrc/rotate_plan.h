@@ -147,9 +147,11 @@ inline void push_forward(std::vector<mlb_op_t>& ops, uint32_t n) {
       cd f[4] = {1.0, 0.0, 0.0, 1.0};  // p = f V
       if (e.between == 1) {
         // the second row's phase beside the first's, of the larger column
+        // (entries of rounding's size or less have none that matters, and a
+        // subnormal one is no unit phase over its rounded size)
         const bool first = std::norm(a) >= std::norm(c);
         const cd x = first ? mul(c, std::conj(a)) : mul(d, std::conj(b));
-        if (std::abs(x) > 0) f[3] = x / std::abs(x);
+        if (std::abs(x) > 1e-150) f[3] = x / std::abs(x);
       } else {
         const cd x = mul(std::conj(a), c);
         const double y = 2 * x.imag(), z = std::norm(a) - std::norm(c), alpha = std::atan2(-y, z);

@@ -108,3 +108,28 @@ def test_mixed_ops(host, seed):
         ops.append(random_op(rng, n, tile, kind, int(rng.integers(kind == OP_PHASE, LIMIT[kind] + 1))))
     want, got = run_both(host, n, tile, ops, _lib.MLB_C128, seed)
     assert np.abs(got - want).max() < 1e-12
+
+
+@pytest.mark.parametrize("e", [5e-324, 1e-323, 1e-320, 1e-300, 1e-160, 1e-100, 1e-17, 0.0])
+def test_push_forward_keeps_tiny_entries_unitary(host, e):
+    """A unitary whose off-diagonal is almost nothing, a controlled phase, then
+    a Hadamard: the pushed matrices stay unitary and the product the same, to
+    eight roundings of 2^-53."""
+    h = np.sqrt(0.5)
+    ops = [make(OP_1Q, 0, -1, (), [1, complex(-e, e), complex(e, e), 1]),
+           make(OP_PHASE, 0, -1, (0, 1), [np.exp(0.7j)]), make(OP_1Q, 0, -1, (), [h, h, h, -h])]
+    want = run_ops(ops)
+    arr = (_lib.MlbOp * 3)(*ops)
+    host.host_push_forward(arr, 3, 2)
+    for o in (arr[0], arr[2]):
+        u = (np.ctypeslib.as_array(o.m)[0:8:2] + 1j * np.ctypeslib.as_array(o.m)[1:8:2]).reshape(2, 2)
+        assert np.abs(u.conj().T @ u - np.eye(2)).max() < 1e-15
+    assert np.abs(run_ops(arr) - want).max() < 1e-15
+
+
+def run_ops(ops, n=2):
+    out = np.eye(1 << n, dtype=complex)
+    for col in out:
+        for o in ops:
+            apply_op(col, n, o)
+    return out
