@@ -98,16 +98,21 @@ extern "C" {
 
 int host_covers(const mlb_op_t* op) { return rot::covers(*op); }
 
+// The pushed matrices, rounded, in place.
 void host_push_forward(mlb_op_t* ops, size_t num, uint32_t n) {
-  std::vector<mlb_op_t> v(ops, ops + num);
-  rot::push_forward(v, n);
-  std::copy(v.begin(), v.end(), ops);
+  const std::vector<rot::Unitary> u = rot::push_forward(std::vector<mlb_op_t>(ops, ops + num), n);
+  for (size_t i = 0; i < num; i++)
+    for (int k = 0; k < 4 && ops[i].kind == MLB_OP_1Q; k++) {
+      ops[i].m[2 * k] = (double)u[i].m[k].real();
+      ops[i].m[2 * k + 1] = (double)u[i].m[k].imag();
+    }
 }
 
 // The ops on n qubits as one pass whose tile holds the qubits of `tile`
-// (qubits 0 and 1 among them), on amp in place.  1: an op is not covered,
-// 2: the program does not fit, 3: an amplitude is written twice.
-int host_run(const mlb_op_t* ops, size_t num, int n, uint64_t tile, int dtype, double* amp) {
+// (qubits 0 and 1 among them), on amp in place, pushed forward first if
+// `push`.  1: an op is not covered, 2: the program does not fit, 3: an
+// amplitude is written twice.
+int host_run(const mlb_op_t* ops, size_t num, int n, uint64_t tile, int dtype, int push, double* amp) {
   DevPass P{};
   P.n = n;
   P.L = 2;
@@ -115,10 +120,12 @@ int host_run(const mlb_op_t* ops, size_t num, int n, uint64_t tile, int dtype, d
     if (tile >> q & 1) P.high[P.H++] = q;
   P.tile_free_mask = ((1ull << n) - 1) & ~tile;
   P.num_tiles = 1ull << (n - P.L - P.H);
-  std::vector<const mlb_op_t*> list;
+  std::vector<rot::Unitary> units;
+  if (push) units = rot::push_forward(std::vector<mlb_op_t>(ops, ops + num), n);
+  std::vector<rot::Gate> list;
   for (size_t i = 0; i < num; i++) {
     if (!rot::covers(ops[i])) return 1;
-    list.push_back(ops + i);
+    list.push_back({ops + i, push ? &units[i] : nullptr});
   }
   rot::Program pr;
   if (!rot::Lower::lower(P, dtype, list, pr)) return 2;
