@@ -344,22 +344,33 @@ __global__ void __launch_bounds__(HeaCfg<Real, BACK>::NT, HeaCfg<Real, BACK>::CT
   }
 }
 
-// grads[b][p] = sum over state b's items, in order, for the parameter p of
-// each of `slots` slots (-1: none).
-__global__ void __launch_bounds__(128) k_hea_reduce(const double* __restrict__ partials, uint32_t items, int slots,
-                                                    uint64_t batch, const int* __restrict__ param_of_slot,
-                                                    int num_params, double* __restrict__ grads) {
-  const uint64_t total = batch * (uint64_t)slots;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t b = i / slots, s = i % slots;
-    const int param = param_of_slot[s];
-    if (param < 0) continue;
-    const double* p = partials + b * items * (uint64_t)slots + s;
-    double sum = 0.0;
-#pragma unroll 8
-    for (uint32_t t = 0; t < items; t++) sum += p[t * (uint64_t)slots];
-    grads[b * (uint64_t)num_params + param] = sum;
+// grads[b][p] = sum over state b's items for the parameter p of each of
+// `slots` slots (-1: none).  A CTA takes 32 slots of one state, its warps an
+// eighth of the items each, in order; then the eight sums in order.  (One
+// thread a slot took 25 us for 256 items of two states, by the loads' latency.)
+constexpr int kReduceWarps = 8;
+__global__ void __launch_bounds__(32 * kReduceWarps) k_hea_reduce(const double* __restrict__ partials, uint32_t items,
+                                                                  int slots, const int* __restrict__ param_of_slot,
+                                                                  int num_params, double* __restrict__ grads) {
+  __shared__ double sums[kReduceWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slot = blockIdx.x * 32 + lane;
+  const uint64_t b = blockIdx.y;
+  const double* p = partials + b * items * (uint64_t)slots + slot;
+  const uint32_t each = (items + kReduceWarps - 1) / kReduceWarps, t0 = warp * each;
+  const uint32_t t1 = t0 + each < items ? t0 + each : items;
+  double sum = 0.0;
+  if (slot < slots) {
+#pragma unroll 32
+    for (uint32_t t = t0; t < t1; t++) sum += p[t * (uint64_t)slots];
   }
+  sums[warp][lane] = sum;
+  __syncthreads();
+  if (warp > 0 || slot >= slots) return;
+  const int param = param_of_slot[slot];
+  if (param < 0) return;
+  for (int w = 1; w < kReduceWarps; w++) sum += sums[w][lane];
+  grads[b * (uint64_t)num_params + param] = sum;
 }
 
 // out[b] = sum over state b's tiles, in order.
@@ -476,13 +487,14 @@ int launch_hea_pass(int dtype, const void* psi_src, void* psi, void* lam, const 
 
 int launch_hea_reduce(const double* d_partials, uint32_t items, int slots, uint64_t batch, const int* d_param_of_slot,
                       int num_params, double* d_grads, cudaStream_t stream) {
-  const uint64_t total = batch * (uint64_t)slots;
-  uint64_t grid = (total + 127) / 128;
-  if (grid < 1) grid = 1;
-  if (grid > 148ull * 16) grid = 148ull * 16;
-  k_hea_reduce<<<(unsigned)grid, 128, 0, stream>>>(d_partials, items, slots, batch, d_param_of_slot, num_params,
-                                                   d_grads);
-  count_launch();
+  if (slots < 1) return MLB_ERR_INVALID_ARG;
+  for (uint64_t b0 = 0; b0 < batch; b0 += 65535) {  // grid.y's limit
+    const uint64_t nb = batch - b0 < 65535 ? batch - b0 : 65535;
+    k_hea_reduce<<<dim3((unsigned)((slots + 31) / 32), (unsigned)nb), 32 * kReduceWarps, 0, stream>>>(
+        d_partials + b0 * items * (uint64_t)slots, items, slots, d_param_of_slot, num_params,
+        d_grads + b0 * (uint64_t)num_params);
+    count_launch();
+  }
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }
 

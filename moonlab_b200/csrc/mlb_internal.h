@@ -143,8 +143,8 @@ int hea_tile_bits(int dtype, bool backward);
 int launch_hea_pass(int dtype, const void* psi_src, void* psi, void* lam, const HeaPass& P, const HeaSeg* d_segs,
                     const double2* d_cs, double* d_partials, int part_stride, bool backward, int num_sms,
                     cudaStream_t stream);
-// d_grads[b * num_params + p] = sum over a state's items, in order, of the
-// partials of each slot, p its parameter (-1: none).
+// d_grads[b * num_params + p] = sum over a state's items, in a fixed order, of
+// the partials of each slot, p its parameter (-1: none).
 int launch_hea_reduce(const double* d_partials, uint32_t items, int slots, uint64_t batch, const int* d_param_of_slot,
                       int num_params, double* d_grads, cudaStream_t stream);
 // d_out[b] = the sum of state b's tiles' energy partials, in order.
