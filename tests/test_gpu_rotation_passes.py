@@ -79,3 +79,15 @@ def test_memory_of_a_deep_narrow_problem(gpu):
     prob.evaluate(params)
     pair = 2 * 16 * batch << n
     assert free - torch.cuda.mem_get_info()[0] < pair * (1 + 1 / 16) + (8 << 20)
+
+
+def test_norms_do_not_drift(gpu):
+    """|psi|^2 (the energy of the identity) after 8 layers on 12 qubits.  An
+    entry of a segment's table is rounded once and multiplies an eighth of the
+    amplitudes: about 40 roundings of up to 2^-53 a component, at random
+    2 sqrt(40) 2^-53 / sqrt(3) = 8.1e-16 rms; half as much again is allowed.
+    Entries multiplied up in double gave 1.7e-15."""
+    n, layers = 12, 8
+    params = np.random.default_rng(1).uniform(-np.pi, np.pi, (64, 2 * n * layers))
+    E = HEAProblem(n, layers, [1.0], xmasks=[0], zmasks=[0]).evaluate(params)[0]
+    assert np.sqrt(np.mean((E - 1) ** 2)) < 1.2e-15
