@@ -411,12 +411,17 @@ typedef struct {
                                 (96 flops each) */
 } mlb_flush_stats_t;
 int  mlb_last_flush_stats(mlb_state_t *s, mlb_flush_stats_t *out);
+/* Of its passes, those that ran as rotation programs instead of the segments
+ * of their plan. */
+int  mlb_last_flush_rotation_passes(const mlb_state_t *s, uint64_t *out);
 /* Plan cache for repeated circuit shapes (tiled mode): up to `entries` plans
  * are kept per state, keyed by the shape of the flushed ops (kinds, qubits,
  * controls, real or complex 1-qubit matrices -- not the angles).  A flush
  * whose shape was seen before skips planning: it patches this circuit's
  * matrices into the cached op program and replays the passes' launches as
- * one CUDA graph (captured at the shape's first replay).  Results are
+ * one CUDA graph (captured at the shape's first replay), or launches them one
+ * by one where some run as rotation programs (lowered again from this
+ * circuit's matrices, which their sizes depend on).  Results are
  * identical with and without the cache.  0 entries (default) = off. */
 int  mlb_state_set_plan_cache(mlb_state_t *s, size_t entries);
 /* complex128 tiled mode: run each register segment that fits (4 register

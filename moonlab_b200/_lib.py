@@ -134,6 +134,7 @@ _SIGS = {
                                    C.POINTER(C.c_size_t)]),
     "mlb_run_gates": (C.c_int, [C.c_void_p, C.POINTER(MlbGate), C.c_size_t]),
     "mlb_last_flush_stats": (C.c_int, [C.c_void_p, C.POINTER(MlbFlushStats)]),
+    "mlb_last_flush_rotation_passes": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint64)]),
     "mlb_state_set_timing": (C.c_int, [C.c_void_p, C.c_int]),
     "mlb_test_fused_skip_copy": (C.c_int, [C.c_void_p]),
     "mlb_state_set_plan_cache": (C.c_int, [C.c_void_p, C.c_size_t]),

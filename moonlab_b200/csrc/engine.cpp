@@ -20,8 +20,8 @@
 #include <deque>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -114,6 +114,7 @@ struct mlb_state {
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   bool timed_pending = false;
   mlb_flush_stats_t stats{};
+  uint64_t rotation_passes = 0;  // of the last flush
   // fused path: device error word of the tensor-core kernel and its host copy
   int* d_ferr = nullptr;
   int* h_ferr = nullptr;
@@ -540,26 +541,65 @@ int flush_fused(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   return MLB_OK;
 }
 
-// Where tile passes run as rotation programs (rotate_plan.h), measured on
-// brickwork circuits (depth 20, ZZ every 4 layers; wall ms, programs against
-// the segments that ran before):
-//   complex128, dense 16x16 segments: 13 qubits 1.05 / 1.48, 20: 1.48 / 3.12,
-//     24: 5.4 / 6.6, 25: 9.9 / 10.3, 26: 19.0 / 18.6, 28: 75.9 / 69.4 (QAOA,
-//     3 layers, 28: 36.1 / 37.4).  Up to 25 qubits the matrices' host time
-//     counts as much as the passes, above each pass takes the cheaper form.
-//   complex64, gate by gate: 18 qubits 1.48 / 1.15, 20: 1.54 / 1.42, 22: 1.95 /
-//     2.64, 24: 4.1 / 8.2, 28: 52 / 138 (QAOA: 20: 0.56 / 0.48, 22: 0.83 /
-//     1.81, 28: 20 / 82).
-constexpr uint32_t kRotMinC128 = 13, kRotAllC128 = 25, kRotMinC64 = 21;
-
-// A program's cost beside a dense segment's, from their times per pass of a
-// 30-qubit complex128 state (ms).
-double rot_cost(const rot::Program& p) {
-  double c = 1.03 * (double)p.segs.size();
-  for (const RotOp& o : p.ops) c += (o.flags & kRotTable ? 0.39 : 0.0) + (o.flags & kRotTurn ? 0.58 : 0.0);
-  return c;
+// Asked once: the question is a system call.
+size_t host_cores() {
+  static const size_t n = std::max(1u, std::thread::hardware_concurrency());
+  return n;
 }
-constexpr double kDenseSegmentCost = 3.0;
+
+// Tile passes may run as rotation programs (rotate_plan.h) in registers of at
+// least so many qubits.
+constexpr uint32_t kRotMinC128 = 13, kRotMinC64 = 21;
+// Up to here complex128 flushes count host time beside the passes' (the
+// matrices of the dense segments, the programs' lowering); above, each pass
+// takes the form that the GPU runs faster.
+constexpr uint32_t kRotWholeC128 = 25;
+
+// What a pass costs in each form, in us, from counts that its plan has: least-
+// squares fits to 2000 passes of brickwork (depth 1 to 20, without and with
+// ZZ), QAOA, GHZ and RY circuits of 13 to 27 qubits (complex64: 18 to 24), each
+// run in both forms (a pass is 10 % off, rms).  `unit`: the pass's waves of
+// CTAs beside a 27-qubit state's.  Wall us of a flush on a full register, as
+// segments / as programs: complex128, 16 qubits, 2 layers 90 / 123, 20 layers
+// 1175 / 703; 20 qubits, 4 layers 189 / 303, 20 layers 1910 / 957, QAOA of 2
+// layers 1532 / 529; 25 qubits, 4 layers 1892 / 2647, with ZZ 4570 / 3498;
+// complex64, 21 qubits, QAOA of 1 layer 248 / 333, 20 layers 1183 / 1017; 24
+// qubits, 20 layers 7650 / 3927.  The cheaper form is taken in all but a few ties.
+struct FormCost {
+  double segments, program;  // with the host's part of the segments
+  double lowering;           // the host's part of the program, one thread
+};
+FormCost form_cost(const mlb_state* s, const DevPass& pass, uint64_t tiles, const DevSegment* segs, int num_segs,
+                   const DevOp* dops) {
+  int rotations = 0, diagonals = 0, moves = 0;
+  double fills = 0;  // ops times variants of the dense segments' matrices
+  for (int k = 0; k < num_segs; k++) {
+    const DevSegment& sg = segs[k];
+    uint32_t cl = 0;
+    uint64_t co = 0;
+    if (s->dtype == MLB_C128 && dense::conditioning(sg, dops, cl, co))
+      fills += (double)(sg.op_end - sg.op_begin) * (double)(1ull << (popc(cl) + popc(co)));
+    for (int o = sg.op_begin; o < sg.op_end; o++)
+      switch (dops[o].kind) {
+        case DOP_1Q_GEN:
+        case DOP_1Q_REAL: rotations++; break;
+        case DOP_X:
+        case DOP_SWAP: moves++; break;
+        default: diagonals++;
+      }
+  }
+  const bool c128 = s->dtype == MLB_C128;
+  const int bits = c128 ? kTileBitsC128 : 13, local = pass.L + pass.H;
+  const uint64_t full = std::max<uint64_t>(1, tiles >> (bits - local)), wave = (uint64_t)s->num_sms * (c128 ? 3 : 2);
+  const double unit = (double)((full + wave - 1) / wave * wave << bits) / (double)(1 << 27);
+  const double S = num_segs, K = rotations, D = diagonals, X = moves;
+  if (c128)
+    return {9 + unit * (415 + 430 * S) + 2.3 * S + 0.188 * fills,
+            8.5 + unit * (470 + 125 * S + 42 * K + 17 * D + 13 * X), 1.3 * K + 1.5 * D + 0.35 * X + 1.6 * S};
+  // unfilled tiles (complex64, a last pass of few ops): 12.5 ns each
+  return {10 + unit * (220 + 170 * S + 54 * K + 103 * D + 55 * X) + 0.0125 * (double)(tiles - full),
+          10 + unit * (260 + 60 * S + 34 * K + 8 * D), 1.55 * K + 1.6 * D + 0.2 * X + 1.5 * S};
+}
 
 // The passes' rotation programs, lowered by threads of their own while the
 // planner goes on (a pass takes 90 us, the planner 45).  With the planner's
@@ -569,42 +609,64 @@ constexpr double kDenseSegmentCost = 3.0;
 class Lowering {
  public:
   struct Pass {
-    bool rot = false;  // runs as a rotation program
+    bool fits = false;
     DevPass pass{};
     rot::Program prog;
   };
-  Lowering(const mlb_state* s, size_t num_ops) : n_(s->n), dtype_(s->dtype) {
-    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
-    const size_t count = std::min<size_t>({cores - 1, (size_t)15, num_ops / 200});
-    try {
-      for (size_t t = 0; t < count; t++) pool_.emplace_back([this]() { work(); });
-    } catch (const std::system_error&) {  // no more threads to be had: those there are, and the caller, do it
-    }
-  }
-  ~Lowering() { finish(); }
-  void put(const DevPass& pass, std::vector<rot::Gate> ops) {  // the next pass
+  // units: the ops' matrices where they differ (empty: nowhere), unchanged
+  // from start() or finish() on
+  Lowering(int dtype, const std::vector<mlb_op_t>& ops, const std::vector<rot::Unitary>& units)
+      : dtype_(dtype),
+        threads_(std::min<size_t>({host_cores() - 1, (size_t)15, ops.size() / 200})),
+        ops_(ops),
+        units_(units) {}
+  ~Lowering() { drop(); }
+  // the part of one thread's time that lowering takes beside the planner
+  double share() const { return threads_ == 0 ? 1.0 : 1.6 / (double)(threads_ + 1); }
+  int put(const DevPass& pass, std::vector<int> src) {  // the next pass; its number
     std::lock_guard<std::mutex> lock(mu_);
-    tasks_.push_back({Pass{}, pass, std::move(ops)});
+    tasks_.push_back({Pass{}, pass, std::move(src)});
     if (!pool_.empty()) cv_.notify_one();
+    return (int)tasks_.size() - 1;
+  }
+  bool started() const { return started_; }
+  void start() {
+    started_ = true;
+    try {
+      for (size_t t = 0; t < threads_; t++) pool_.emplace_back([this]() { work(); });
+    } catch (const std::exception&) {  // no more threads to be had: those there are, and the caller, do it
+    }
   }
   void finish() {  // every pass put so far is lowered, by the caller too
-    {
-      std::lock_guard<std::mutex> lock(mu_);
-      closed_ = true;
-    }
-    cv_.notify_all();
+    close(false);
     work();
-    for (auto& t : pool_) t.join();
-    pool_.clear();
+    join();
   }
+  void drop() {  // no pass that is not under way already
+    close(true);
+    join();
+  }
+  void forget() { close(true); }  // as drop(), the threads joined at the end
   Pass& operator[](size_t k) { return tasks_[k].out; }  // after finish()
 
  private:
   struct Task {
     Pass out;
     DevPass planned;
-    std::vector<rot::Gate> ops;
+    std::vector<int> src;
   };
+  void close(bool skip) {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      closed_ = true;
+      if (skip) next_ = tasks_.size();
+    }
+    cv_.notify_all();
+  }
+  void join() {
+    for (auto& t : pool_) t.join();
+    pool_.clear();
+  }
   void work() {
     for (;;) {
       Task* t;
@@ -618,34 +680,32 @@ class Lowering {
     }
   }
   void lower(Task& t) {
-    for (const rot::Gate& g : t.ops)
-      if (!rot::covers(*g.op)) return;
     Pass& out = t.out;
-    out.pass = rot::filled(t.planned, dtype_ == MLB_C128 ? kTileBitsC128 : 13);
-    out.rot = rot::Lower::lower(out.pass, dtype_, t.ops, out.prog);
-    if (dtype_ == MLB_C128 && n_ > kRotAllC128 && rot_cost(out.prog) > kDenseSegmentCost * t.planned.num_segments)
-      out.rot = false;
+    try {
+      std::vector<rot::Gate> gates;
+      gates.reserve(t.src.size());
+      for (int i : t.src) gates.push_back({&ops_[i], units_.empty() ? nullptr : &units_[i]});
+      out.pass = rot::filled(t.planned, dtype_ == MLB_C128 ? kTileBitsC128 : 13);
+      out.fits = rot::Lower::lower(out.pass, dtype_, gates, out.prog);
+    } catch (const std::bad_alloc&) {  // it runs in another form
+      out.fits = false;
+    }
   }
-  const uint32_t n_;
   const int dtype_;
+  const size_t threads_;
+  const std::vector<mlb_op_t>& ops_;
+  const std::vector<rot::Unitary>& units_;
   std::mutex mu_;
   std::condition_variable cv_;
   std::deque<Task> tasks_;
   size_t next_ = 0;
-  bool closed_ = false;
+  bool closed_ = false, started_ = false;
   std::vector<std::thread> pool_;
 };
 
 // Tile passes for ops (tiled mode, and the parts of a fused flush that need
 // them), the plan taken from the state's plan cache when the shape repeats.
 int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_t& st) {
-  const bool rot_on = s->dtype == MLB_C64 ? s->n >= kRotMinC64 : s->dense_c128 && s->n >= kRotMinC128;
-  // matrices that hand a part of one op to another, where every pass runs as
-  // a program: they are never rounded to doubles (as doubles, for the other
-  // forms, they cost accuracy: 30 qubits, depth 40: <Z> 7.4e-13 off, not 3.7e-13)
-  std::vector<rot::Unitary> units;
-  if (rot_on && (s->dtype == MLB_C64 || s->n <= kRotAllC128) && std::all_of(ops.begin(), ops.end(), rot::covers))
-    units = rot::push_forward(ops, s->n);
   const uint64_t dim = 1ull << s->n;
   const uint64_t ab = s->dtype == MLB_C128 ? 16 : 8;
   // the plan: from the cache when this shape ran before, else planned now
@@ -662,19 +722,47 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
         break;
       }
   }
-  // Passes of one-qubit unitaries, CNOTs, SWAPs and diagonals run as rotation
-  // programs (rotate_plan.h), built from this circuit's matrices every flush.
-  Lowering low(s, rot_on ? ops.size() : 0);
-  auto lower = [&](const PlannedPass& pp, const std::vector<DevSegment>& segs, const std::vector<int>& src) {
-    std::vector<rot::Gate> po;
-    for (int i = segs[pp.seg_begin].op_begin; i < segs[pp.seg_end - 1].op_end; i++)
-      po.push_back({&ops[src[i]], units.empty() ? nullptr : &units[src[i]]});
-    low.put(pp.pass, std::move(po));
+  // Passes of one-qubit unitaries, CNOTs, SWAPs and diagonals may run as
+  // rotation programs (rotate_plan.h), built from this circuit's matrices
+  // every flush.  Where all can, the flush takes the form that costs less in
+  // all, and programs take matrices that hand a part of one op to another,
+  // never rounded to doubles.  Otherwise each pass takes the cheaper form, of
+  // the ops' own matrices (pushed ones, rounded for the other forms, cost
+  // accuracy: 30 qubits, depth 40: <Z> 7.4e-13 off, not 3.7e-13).
+  const bool rot_on = s->dtype == MLB_C64 ? s->n >= kRotMinC64 : s->dense_c128 && s->n >= kRotMinC128;
+  const bool whole = rot_on && (s->dtype == MLB_C64 || s->n <= kRotWholeC128) &&
+                     std::all_of(ops.begin(), ops.end(), rot::covers);
+  const uint64_t allq = s->n >= 64 ? ~0ull : ((1ull << s->n) - 1ull);
+  std::vector<rot::Unitary> units;
+  Lowering low(s->dtype, ops, units);
+  std::vector<int> program;  // of each pass, -1: none
+  double cost_segments = 0, cost_programs = 0;
+  uint64_t reach = s->exposed ? allq : s->support & allq;  // of the amplitudes that may be nonzero
+  auto consider = [&](const PlannedPass& pp, const std::vector<DevSegment>& segs, const std::vector<DevOp>& dops,
+                      const std::vector<int>& src) {
+    program.push_back(-1);
+    if (!rot_on) return;
+    const uint64_t tiles = 1ull << popc(pp.pass.tile_free_mask & reach);
+    reach |= allq & ~pp.pass.tile_free_mask;
+    const int begin = segs[pp.seg_begin].op_begin, end = segs[pp.seg_end - 1].op_end;
+    if (!whole && !std::all_of(src.begin() + begin, src.begin() + end, [&](int i) { return rot::covers(ops[i]); }))
+      return;
+    const FormCost c =
+        form_cost(s, pp.pass, tiles, segs.data() + pp.seg_begin, pp.seg_end - pp.seg_begin, dops.data());
+    const double mine = c.program + low.share() * c.lowering;
+    if (!whole && mine >= c.segments) return;
+    cost_segments += c.segments;
+    cost_programs += mine;
+    program.back() = low.put(pp.pass, std::vector<int>(src.begin() + begin, src.begin() + end));
+    if (!low.started() && cost_programs < cost_segments) {
+      if (whole) units = rot::push_forward(ops, s->n);
+      low.start();
+    }
   };
   if (!hit) {
     Planner pl{s->n, s->dtype, geo(s->dtype)};
     pl.dense_limits = s->dtype == MLB_C128 && s->dense_c128;
-    if (rot_on) pl.on_pass = [&](const PlannedPass& pp) { lower(pp, pl.segs, pl.dop_src); };
+    pl.on_pass = [&](const PlannedPass& pp) { consider(pp, pl.segs, pl.dops, pl.dop_src); };
     pl.plan(ops);
     local.dops = std::move(pl.dops);
     local.src = std::move(pl.dop_src);
@@ -703,13 +791,18 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   // (mode 2); which segments fit depends only on the plan's shape, so the
   // upload layout (and a captured graph's pointers) repeat with the shape.
   const size_t np = E->passes.size();
-  if (rot_on && hit)
-    for (const auto& pp : E->passes) lower(pp, E->segs, E->src);
-  low.finish();
+  if (hit)
+    for (const auto& pp : E->passes) consider(pp, E->segs, E->dops, E->src);
+  if (whole && cost_programs >= cost_segments) {
+    low.forget();
+    std::fill(program.begin(), program.end(), -1);
+  } else {
+    low.finish();
+  }
   std::vector<char> is_rot(np, 0);
-  for (size_t k = 0; rot_on && k < np; k++) is_rot[k] = low[k].rot;
+  for (size_t k = 0; k < np; k++) is_rot[k] = program[k] >= 0 && low[program[k]].fits;
   if (!units.empty() && !std::all_of(is_rot.begin(), is_rot.end(), [](char r) { return r; }))
-    std::fill(is_rot.begin(), is_rot.end(), 0);  // a program did not fit
+    std::fill(is_rot.begin(), is_rot.end(), 0);  // the other forms' matrices are the ops' own
   size_t nrot = 0;
   for (char r : is_rot) nrot += r;
   std::vector<DevSegment> dev_segs(E->segs);
@@ -745,8 +838,7 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
       for (size_t d; (d = next.fetch_add(1)) < dsegs.size();)
         dense::fill_fragments(E->segs[dsrc[d]], E->dops.data(), dsegs[d], dplans[d], frags.get() + dsegs[d].frag_off);
     };
-    const size_t nth =
-        std::min<size_t>({(size_t)std::max(1u, std::thread::hardware_concurrency()), (size_t)16, 1 + nfrag / (256 * 1024)});
+    const size_t nth = std::min<size_t>({host_cores(), (size_t)16, 1 + nfrag / (256 * 1024)});
     std::vector<std::thread> pool;
     for (size_t t = 1; t < nth; t++) pool.emplace_back(work);
     work();
@@ -774,7 +866,7 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
       old_segs += (size_t)E->passes[k].pass.num_segments;
       continue;
     }
-    const rot::Program& pr = low[k].prog;
+    const rot::Program& pr = low[program[k]].prog;
     rot_segs += pr.segs.size();
     at[k] = {room(pr.segs.size() * sizeof(RotSeg)), room(pr.ops.size() * sizeof(RotOp)), room(pr.table.size() * ab)};
   }
@@ -787,7 +879,7 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   }
   for (size_t k = 0; k < np; k++) {
     if (!is_rot[k]) continue;
-    const rot::Program& pr = low[k].prog;
+    const rot::Program& pr = low[program[k]].prog;
     std::memcpy(blob.get() + at[k].segs, pr.segs.data(), pr.segs.size() * sizeof(RotSeg));
     std::memcpy(blob.get() + at[k].ops, pr.ops.data(), pr.ops.size() * sizeof(RotOp));
     if (s->dtype == MLB_C128) {
@@ -810,7 +902,6 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   // some qubit has not been touched since a reset, a pass runs only over the
   // tiles whose outside bits are touched ones.  Such launches depend on the
   // state's history, so they are never captured into a cached graph.
-  const uint64_t allq = s->n >= 64 ? ~0ull : ((1ull << s->n) - 1ull);
   const bool sparse = !s->exposed && (s->support & allq) != allq;
   // until every launch went out, nothing is assumed about the state's zeros
   const uint64_t sup0 = s->support;
@@ -829,7 +920,7 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
         ndense += dev_segs[pp.seg_begin + k].mode == 2;
       }
       if (is_rot[pi]) ndense = 0;
-      DevPass pass = is_rot[pi] ? low[pi].pass : pp.pass;
+      DevPass pass = is_rot[pi] ? low[program[pi]].pass : pp.pass;
       if (restrict) {
         pass.tile_free_mask &= sup;
         pass.num_tiles = 1ull << popc(pass.tile_free_mask);
@@ -839,7 +930,7 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
       moved += 2 * ab * amps;
       dense_amps += (uint64_t)ndense * amps;
       if (is_rot[pi]) {
-        RotPass rp = low[pi].prog.dev;
+        RotPass rp = low[program[pi]].prog.dev;
         rp.free_mask = pass.tile_free_mask;
         rp.num_tiles = pass.num_tiles;
         const unsigned char* d = static_cast<const unsigned char*>(s->d_plan);
@@ -896,6 +987,7 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
     moved = E->passes.size() * 2 * ab * dim;
     dense_amps = dsegs.size() << s->n;
   }
+  s->rotation_passes += nrot;
   st.passes += E->passes.size();
   st.kernel_launches += E->passes.size();
   st.bytes_moved += moved;
@@ -911,6 +1003,7 @@ int flush_impl(mlb_state* s) {
   if (s->queue.empty()) return MLB_OK;
   DeviceGuard dg(s->device);
   mlb_flush_stats_t st{};
+  s->rotation_passes = 0;
   const uint64_t dim = 1ull << s->n;
   const uint64_t ab = s->dtype == MLB_C128 ? 16 : 8;
   if (s->mode == MLB_EXEC_EAGER) {
@@ -1857,6 +1950,11 @@ int mlb_last_flush_stats(mlb_state_t* s, mlb_flush_stats_t* out) {
     s->timed_pending = false;
   }
   *out = s->stats;
+  return MLB_OK;
+}
+int mlb_last_flush_rotation_passes(const mlb_state_t* s, uint64_t* out) {
+  if (!s || !out) return fail(MLB_ERR_INVALID_ARG, "null argument");
+  *out = s->rotation_passes;
   return MLB_OK;
 }
 int mlb_state_set_timing(mlb_state_t* s, int enable) {

@@ -94,10 +94,13 @@ inline bool covers(const mlb_op_t& o) {
   switch (o.kind) {
     case MLB_OP_1Q: {
       if (o.cmask) return false;
-      const cd a(o.m[0], o.m[1]), b(o.m[2], o.m[3]), c(o.m[4], o.m[5]), d(o.m[6], o.m[7]);
       // columns of length one and orthogonal, to rounding
-      return std::abs(std::norm(a) + std::norm(c) - 1.0) < 2e-14 && std::abs(std::norm(b) + std::norm(d) - 1.0) < 2e-14 &&
-             std::abs(std::conj(a) * b + std::conj(c) * d) < 2e-14;
+      const double* m = o.m;
+      const double p = m[0] * m[0] + m[1] * m[1] + m[4] * m[4] + m[5] * m[5] - 1.0;
+      const double q = m[2] * m[2] + m[3] * m[3] + m[6] * m[6] + m[7] * m[7] - 1.0;
+      const double x = m[0] * m[2] + m[1] * m[3] + m[4] * m[6] + m[5] * m[7];  // conj(a) b + conj(c) d
+      const double y = m[0] * m[3] - m[1] * m[2] + m[4] * m[7] - m[5] * m[6];
+      return std::abs(p) < 2e-14 && std::abs(q) < 2e-14 && x * x + y * y < 4e-28;
     }
     case MLB_OP_X: return plan::popc(o.cmask) <= 1;
     case MLB_OP_SWAP: return o.cmask == 0;
@@ -117,12 +120,6 @@ inline Unitary unitary(const mlb_op_t& o) {
   Unitary u;
   for (int k = 0; k < 4; k++) u.m[k] = cl(o.m[2 * k], o.m[2 * k + 1]);
   return u;
-}
-inline Unitary mul(const Unitary& x, const Unitary& y) {
-  Unitary r;
-  for (int i = 0; i < 2; i++)
-    for (int j = 0; j < 2; j++) r.m[2 * i + j] = mul(x.m[2 * i], y.m[j]) + mul(x.m[2 * i + 1], y.m[2 + j]);
-  return r;
 }
 inline cl conj(cl a) { return {a.real(), -a.imag()}; }
 inline long double norm(cl a) { return a.real() * a.real() + a.imag() * a.imag(); }
@@ -157,25 +154,43 @@ inline std::vector<Unitary> push_forward(const std::vector<mlb_op_t>& ops, uint3
     out[i] = unitary(o);
     Open& e = open[o.target];
     if (e.op >= 0 && (e.between == 1 || e.between == 2)) {
-      Unitary& p = out[e.op];
-      const cl a = p.m[0], b = p.m[1], c = p.m[2], d = p.m[3];
-      Unitary f;  // p = f V
-      f.m[0] = f.m[3] = 1.0L;
+      cl* p = out[e.op].m;  // = f V: V stays, f goes to o
+      cl* q = out[i].m;
       if (e.between == 1) {
-        // the second row's phase beside the first's, of the larger column
-        // (an entry of rounding's size or less has none that matters)
-        const cl x = norm(a) >= norm(c) ? mul(c, conj(a)) : mul(d, conj(b));
-        if (size(x) > 1e-150L) f.m[3] = x / size(x);
+        // f = diag(1, x / |x|), the second row's phase beside the first's, of
+        // the larger column (an entry of rounding's size or less has none
+        // that matters)
+        const cl x = norm(p[0]) >= norm(p[2]) ? mul(p[2], conj(p[0])) : mul(p[3], conj(p[1]));
+        const long double r = size(x);
+        if (r > 1e-150L) {
+          const cl f = x / r;
+          p[2] = mul(p[2], conj(f));
+          p[3] = mul(p[3], conj(f));
+          q[1] = mul(q[1], f);
+          q[3] = mul(q[3], f);
+        }
       } else {
-        const cl x = mul(conj(a), c);
-        const long double alpha = std::atan2(-2 * x.imag(), norm(a) - norm(c));
-        f.m[0] = f.m[3] = std::cos(alpha / 2);
-        f.m[1] = f.m[2] = cl(0.0L, -std::sin(alpha / 2));
+        // f = [[co, -i si], [-i si, co]], half the angle of (z, y)
+        const long double y = -2 * mul(conj(p[0]), p[2]).imag(), z = norm(p[0]) - norm(p[2]),
+                          r = std::sqrt(y * y + z * z);
+        long double co = 1.0L, si = 0.0L;
+        if (z >= 0 && r > 0) {
+          co = std::sqrt((r + z) / (2 * r));
+          si = y / (2 * r * co);
+        } else if (r > 0) {
+          si = std::copysign(std::sqrt((r - z) / (2 * r)), y);
+          co = y / (2 * r * si);
+        }
+        auto turn = [&](cl& u, cl& v, long double t) {  // u, v <- co u + i t v, i t u + co v
+          const cl a = u, b = v;
+          u = {co * a.real() - t * b.imag(), co * a.imag() + t * b.real()};
+          v = {co * b.real() - t * a.imag(), co * b.imag() + t * a.real()};
+        };
+        turn(p[0], p[2], si);
+        turn(p[1], p[3], si);
+        turn(q[0], q[1], -si);
+        turn(q[2], q[3], -si);
       }
-      // V = f^-1 p; o takes f first
-      const Unitary back{{conj(f.m[0]), conj(f.m[2]), conj(f.m[1]), conj(f.m[3])}};
-      p = mul(back, p);
-      out[i] = mul(out[i], f);
     }
     e.op = (int)i;
     e.between = 0;

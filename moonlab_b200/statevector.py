@@ -102,7 +102,9 @@ class StateVector:
     def flush_stats(self) -> dict:
         st = _lib.MlbFlushStats()
         check(self._lib.mlb_last_flush_stats(self._h, C.byref(st)), "mlb_last_flush_stats")
-        return {f: getattr(st, f) for f, _ in st._fields_}
+        rot = C.c_uint64()
+        check(self._lib.mlb_last_flush_rotation_passes(self._h, C.byref(rot)), "mlb_last_flush_rotation_passes")
+        return {f: getattr(st, f) for f, _ in st._fields_} | {"rotation_passes": rot.value}
 
     def set_plan_cache(self, entries: int) -> None:
         check(self._lib.mlb_state_set_plan_cache(self._h, entries), "mlb_state_set_plan_cache")

@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from moonlab_b200 import StateVector, _lib
-from moonlab_b200.circuits import GATE_DTYPE, brickwork
+from moonlab_b200.circuits import GATE_DTYPE, brickwork, qaoa_circuit
 from oracle import bindings as B
 
 pytestmark = pytest.mark.gpu
@@ -110,3 +110,38 @@ def test_controlled_zz(gpu, n, dtype, mode):
         x, y = a.amplitudes(), b.amplitudes()
     # the whole state's error: a fidelity of 1 - 1e-6 is 1.4e-3 on the fused path
     assert np.linalg.norm(x - y) < {"c128": 1e-12, "c64": 2e-3 if mode == "fused" else 2e-5}[dtype]
+
+
+@pytest.mark.parametrize("n,dtype,gates,programs", [
+    # a few layers: the dense segments' matrices are cheaper than lowering
+    (16, "c128", "brickwork 2", 0), (20, "c128", "brickwork 4", 0), (24, "c128", "brickwork 4", 0),
+    # many, ZZ layers, QAOA: the matrices cost more
+    (20, "c128", "brickwork 20", 1), (20, "c128", "zz 6", 1), (24, "c128", "qaoa 2", 1), (25, "c128", "zz 4", 1),
+    # pass by pass: some of either form
+    (26, "c128", "brickwork 6", None), (26, "c128", "brickwork 14", None),
+    # registers below the programs' reach
+    (12, "c128", "brickwork 20", 0), (20, "c64", "brickwork 20", 0),
+    # complex64: a short circuit and a long one, and one whose last tile would hold few qubits
+    (21, "c64", "qaoa 1", 0), (21, "c64", "brickwork 20", 1), (22, "c64", "brickwork 1", 1)])
+def test_form_that_costs_less(gpu, n, dtype, gates, programs):
+    """Which form a flush takes, and its state against that of the other
+    forms' kernels (one per gate)."""
+    kind, depth = gates.split()
+    depth = int(depth)
+    g = qaoa_circuit(n, depth, 3) if kind == "qaoa" else brickwork(n, depth, 3, zz_every=int(kind == "zz"))
+    if programs == 0 and n >= 13:  # the ops' own matrices, whatever was pushed forward on the way
+        g = np.concatenate([g, circuit(n, 6, n, [4, 7])])
+    with StateVector(n, dtype) as a, StateVector(n) as b:
+        a.set_exec_mode("tiled")
+        b.set_exec_mode("eager")
+        for sv in (a, b):
+            sv.run(brickwork(n, 1, 1))
+            sv.flush()
+            sv.run(g)
+        x, y = a.amplitudes(), b.amplitudes()
+        st = a.flush_stats()
+    if programs is None:
+        assert 0 < st["rotation_passes"] < st["passes"]
+    else:
+        assert st["rotation_passes"] == programs * st["passes"]
+    assert np.abs(x - y).max() < (1e-12 if dtype == "c128" else 2e-5)
