@@ -13,7 +13,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <utility>
 #include <vector>
 
 #include "hea_plan.h"
@@ -36,28 +35,58 @@ inline void grow(hea::Basis& V, const std::vector<uint64_t>& masks, const std::v
   int degree[64] = {};
   for (uint64_t x : masks)
     for (uint64_t y = x; y; y &= y - 1) degree[__builtin_ctzll(y)]++;
-  std::vector<std::pair<uint64_t, int>> res;
-  while ((int)V.v.size() < dims) {
-    res.clear();  // the masks modulo the span: equal residues come in together
-    for (size_t i = 0; i < masks.size(); i++)
-      if (const uint64_t r = V.reduce(masks[i])) res.push_back({r, weight[i]});
-    if (res.empty()) break;
-    std::sort(res.begin(), res.end());
-    uint64_t best = 0;
-    long most = -1;
-    for (size_t i = 0; i < res.size();) {
-      long gain = 0, touch = 0;
-      size_t j = i;
-      for (; j < res.size() && res[j].first == res[i].first; j++) gain += res[j].second;
-      for (uint64_t y = res[i].first; y; y &= y - 1) touch += degree[__builtin_ctzll(y)];
-      const long score = (gain << 32) + (touch << 8) / __builtin_popcountll(res[i].first);
-      if (score > most) {
-        most = score;
-        best = res[i].first;
+  // the masks modulo the span: equal residues come in together
+  std::vector<uint64_t> res;
+  std::vector<int> strings;
+  for (size_t i = 0; i < masks.size(); i++)
+    if (const uint64_t r = V.reduce(masks[i])) {
+      res.push_back(r);
+      strings.push_back(weight[i]);
+    }
+  struct Class {
+    uint64_t r;
+    long gain;
+  };
+  std::vector<Class> classes;
+  int log = 4;
+  while ((size_t)1 << log < 2 * res.size()) log++;
+  std::vector<uint32_t> slot((size_t)1 << log);  // hash table: 1 + index of a class
+  while ((int)V.v.size() < dims && !res.empty()) {
+    classes.clear();
+    std::fill(slot.begin(), slot.end(), 0u);
+    for (size_t i = 0; i < res.size(); i++) {
+      size_t h = (res[i] * 0x9E3779B97F4A7C15ull) >> (64 - log);
+      while (slot[h] && classes[slot[h] - 1].r != res[i]) h = (h + 1) & (slot.size() - 1);
+      if (!slot[h]) {
+        classes.push_back({res[i], 0});
+        slot[h] = (uint32_t)classes.size();
       }
-      i = j;
+      classes[slot[h] - 1].gain += strings[i];
+    }
+    uint64_t best = 0;
+    long most = 0, score = -1;
+    for (const Class& c : classes) {
+      if (c.gain < most) continue;
+      long touch = 0;
+      for (uint64_t y = c.r; y; y &= y - 1) touch += degree[__builtin_ctzll(y)];
+      const long t = (touch << 8) / __builtin_popcountll(c.r);
+      if (c.gain > most || t > score || (t == score && c.r < best)) {
+        most = c.gain;
+        score = t;
+        best = c.r;
+      }
     }
     V.add(best);
+    const int pivot = __builtin_ctzll(best);
+    size_t left = 0;
+    for (size_t i = 0; i < res.size(); i++) {
+      const uint64_t r = res[i] >> pivot & 1ull ? res[i] ^ best : res[i];
+      if (!r) continue;
+      res[left] = r;
+      strings[left++] = strings[i];
+    }
+    res.resize(left);
+    strings.resize(left);
   }
 }
 
