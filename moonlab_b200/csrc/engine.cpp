@@ -1490,8 +1490,10 @@ int mlb_expect_pauli_sum(mlb_state_t* s, size_t num_terms, const uint64_t* xm, c
   DeviceGuard dg(s->device);
   int rc = flush_impl(s);
   if (rc) return rc;
-  *out = 0.0;
-  if (num_terms == 0) return MLB_OK;
+  if (num_terms == 0) {
+    *out = 0.0;
+    return MLB_OK;
+  }
   // one upload (through the plan buffers), the passes' kernels, one result
   std::vector<pauli::Pass> passes;
   std::vector<unsigned char> blob;
@@ -1501,6 +1503,8 @@ int mlb_expect_pauli_sum(mlb_state_t* s, size_t num_terms, const uint64_t* xm, c
     std::memcpy(blob.data() + at, p, bytes);
     return at;
   };
+  const unsigned zero = 0;
+  put(&zero, sizeof zero);  // the last pass's count of CTAs, at offset 0
   size_t xoff = 0, zoff = 0, coff = 0;
   if (s->n < 3) {
     std::vector<double> ones;
@@ -1521,23 +1525,17 @@ int mlb_expect_pauli_sum(mlb_state_t* s, size_t num_terms, const uint64_t* xm, c
   if (rc) return rc;
   rc = upload_plan(s, blob.data(), blob.size());
   if (rc) return rc;
-  const unsigned char* d = static_cast<const unsigned char*>(s->d_plan);
-  double* d_parts = s->d_scratch + 1;
-  int count = 0;
-  if (s->n < 3) {
+  unsigned char* d = static_cast<unsigned char*>(s->d_plan);
+  if (s->n < 3)
     rc = launch_pauli_tiny(s->dtype, s->amp, (int)s->n, (int)num_terms, reinterpret_cast<const uint64_t*>(d + xoff),
                            reinterpret_cast<const uint64_t*>(d + zoff), reinterpret_cast<const double*>(d + coff),
-                           d_parts, s->stream);
-    count = 1;
-  }
-  for (size_t k = 0; !rc && k < passes.size(); k++) {
-    int parts = 0;
+                           s->d_scratch, s->stream);
+  int parts = 0;
+  for (size_t k = 0; !rc && k < passes.size(); k++)
     rc = launch_pauli_sum(s->dtype, s->amp, passes[k].dev, reinterpret_cast<const PauliSeg*>(d + passes[k].segs_off),
-                          reinterpret_cast<const PauliTerm*>(d + passes[k].terms_off), d_parts + count, s->num_sms,
-                          s->stream, &parts);
-    count += parts;
-  }
-  if (!rc) rc = launch_sum_partials(d_parts, count, s->d_scratch, s->stream);
+                          reinterpret_cast<const PauliTerm*>(d + passes[k].terms_off), s->d_scratch + 1, &parts,
+                          reinterpret_cast<unsigned*>(d), k + 1 == passes.size() ? s->d_scratch : nullptr, s->num_sms,
+                          s->stream);
   if (rc) return fail(rc, "pauli launch");
   cudaError_t e = cudaMemcpyAsync(out, s->d_scratch, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
   if (e != cudaSuccess) return cuda_fail(e, "pauli readback");

@@ -1,7 +1,8 @@
 // kernels_pauli.cu -- sums of Pauli strings in tile passes over linear
 // subspaces of the index space (planned by pauli_plan.h).
 //
-//   k_pauli_sum   : partials of sum_k c_k <psi|P_k|psi>, one per CTA.
+//   k_pauli_sum   : partials of sum_k c_k <psi|P_k|psi>, one per CTA; the last
+//                   CTA of the last pass adds them up.
 //   k_pauli_apply : lambda (+)= sum_k c_k P_k psi for a batch of states; the
 //                   last pass also emits the per-tile partial of
 //                   Re<psi|lambda> (the energy).
@@ -110,12 +111,13 @@ template <typename Real>
 __global__ void __launch_bounds__(kThreads, 2)
     k_pauli_sum(const typename Cplx<Real>::T* __restrict__ amp, const __grid_constant__ PauliPass P,
                 const PauliSeg* __restrict__ segs, const PauliTerm* __restrict__ terms,
-                double* __restrict__ partials) {
+                double* partials, int before, unsigned* done, double* __restrict__ out) {
   using A = typename Cplx<Real>::T;
   constexpr int NT = kThreads, UB = sizeof(A) == 16 ? 0 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t joff[kMaxUnitSteps];
   __shared__ double red[NT / 32];
+  __shared__ bool last;
   const uint32_t tile_bytes = (uint32_t)sizeof(A) << P.m;
   double* coef = reinterpret_cast<double*>(smem + tile_bytes);       // [term] with the tile's sign
   PauliTerm* st = reinterpret_cast<PauliTerm*>(coef + P.num_terms);
@@ -184,15 +186,31 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (tid == 0) {
     double s = 0.0;
     for (int w = 0; w < NT / 32; w++) s += red[w];
-    partials[blockIdx.x] = s;
+    partials[before + blockIdx.x] = s;
+    __threadfence();
+    last = out && atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  if (!out) return;
+  __syncthreads();
+  if (!last) return;
+  // the last pass's last CTA: all passes' partials, in a fixed order
+  double v = 0.0;
+  for (int i = tid; i < before + (int)gridDim.x; i += NT) v += __ldcg(partials + i);
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((tid & 31) == 0) red[tid >> 5] = v;
+  __syncthreads();
+  if (tid == 0) {
+    double s = 0.0;
+    for (int w = 0; w < NT / 32; w++) s += red[w];
+    *out = s;
   }
 }
 
-// States of fewer than 8 amplitudes: one thread per string and amplitude in turn.
+// States of fewer than 8 amplitudes: a thread for every 32nd string, over the amplitudes in turn.
 template <typename Real>
 __global__ void k_pauli_tiny(const typename Cplx<Real>::T* __restrict__ amp, int n, int num_terms,
                              const uint64_t* __restrict__ xm, const uint64_t* __restrict__ zm,
-                             const double* __restrict__ coeff, double* __restrict__ partials) {
+                             const double* __restrict__ coeff, double* __restrict__ out) {
   double acc = 0.0;
   for (int t = threadIdx.x; t < num_terms; t += 32) {
     const int ny = __popcll(xm[t] & zm[t]) & 3;
@@ -206,21 +224,7 @@ __global__ void k_pauli_tiny(const typename Cplx<Real>::T* __restrict__ amp, int
     acc += coeff[t] * v;
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (threadIdx.x == 0) partials[0] = acc;
-}
-
-__global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__ partials, int count,
-                                                      double* __restrict__ out) {
-  __shared__ double red[256];
-  double v = 0.0;
-  for (int i = threadIdx.x; i < count; i += 256) v += partials[i];
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = red[0];
+  if (threadIdx.x == 0) *out = acc;
 }
 
 // lambda[k] += +-c (ODD: times i) psi[k ^ KAP]; the sign is that of the source.
@@ -366,7 +370,8 @@ constexpr size_t kMaxTables = tables_bytes(kMaxPauliTerms, kMaxPauliTerms);
 
 template <typename Real>
 int launch_sum_t(const void* amp, const PauliPass& P, const PauliSeg* d_segs, const PauliTerm* d_terms,
-                 double* d_partials, int num_sms, cudaStream_t stream, int* parts) {
+                 double* d_partials, int* parts, unsigned* d_done, double* d_out, int num_sms,
+                 cudaStream_t stream) {
   using A = typename Cplx<Real>::T;
   const size_t smem = (sizeof(A) << P.m) + tables_bytes(P.num_terms, P.num_segs);
   auto kern = k_pauli_sum<Real>;
@@ -376,9 +381,9 @@ int launch_sum_t(const void* amp, const PauliPass& P, const PauliSeg* d_segs, co
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
   uint64_t grid = (uint64_t)num_sms * (per_sm < 1 ? 1 : per_sm > kPauliCtasPerSm ? kPauliCtasPerSm : per_sm);
   if (grid > P.tiles_per_state) grid = P.tiles_per_state;
-  kern<<<(unsigned)grid, kThreads, smem, stream>>>((const A*)amp, P, d_segs, d_terms, d_partials);
+  kern<<<(unsigned)grid, kThreads, smem, stream>>>((const A*)amp, P, d_segs, d_terms, d_partials, *parts, d_done, d_out);
   count_launch();
-  *parts = (int)grid;
+  *parts += (int)grid;
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }
 
@@ -407,27 +412,22 @@ int pauli_tile_bits(int dtype, bool apply) {
 }
 
 int launch_pauli_sum(int dtype, const void* amp, const PauliPass& P, const PauliSeg* d_segs,
-                     const PauliTerm* d_terms, double* d_partials, int num_sms, cudaStream_t stream, int* parts) {
+                     const PauliTerm* d_terms, double* d_partials, int* parts, unsigned* d_done, double* d_out,
+                     int num_sms, cudaStream_t stream) {
   if (P.m < 3 || P.m > pauli_tile_bits(dtype, false) || P.num_terms < 1 || P.num_terms > kMaxPauliTerms ||
       P.num_segs > P.num_terms)
     return MLB_ERR_INVALID_ARG;
-  return dtype == MLB_C128 ? launch_sum_t<double>(amp, P, d_segs, d_terms, d_partials, num_sms, stream, parts)
-                           : launch_sum_t<float>(amp, P, d_segs, d_terms, d_partials, num_sms, stream, parts);
+  return dtype == MLB_C128 ? launch_sum_t<double>(amp, P, d_segs, d_terms, d_partials, parts, d_done, d_out, num_sms, stream)
+                           : launch_sum_t<float>(amp, P, d_segs, d_terms, d_partials, parts, d_done, d_out, num_sms, stream);
 }
 
 int launch_pauli_tiny(int dtype, const void* amp, int n, int num_terms, const uint64_t* d_xm, const uint64_t* d_zm,
-                      const double* d_coeff, double* d_partials, cudaStream_t stream) {
+                      const double* d_coeff, double* d_out, cudaStream_t stream) {
   if (n > 2) return MLB_ERR_INVALID_ARG;
   if (dtype == MLB_C128)
-    k_pauli_tiny<double><<<1, 32, 0, stream>>>((const double2*)amp, n, num_terms, d_xm, d_zm, d_coeff, d_partials);
+    k_pauli_tiny<double><<<1, 32, 0, stream>>>((const double2*)amp, n, num_terms, d_xm, d_zm, d_coeff, d_out);
   else
-    k_pauli_tiny<float><<<1, 32, 0, stream>>>((const float2*)amp, n, num_terms, d_xm, d_zm, d_coeff, d_partials);
-  count_launch();
-  return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
-}
-
-int launch_sum_partials(const double* d_partials, int count, double* d_out, cudaStream_t stream) {
-  k_sum_partials<<<1, 256, 0, stream>>>(d_partials, count, d_out);
+    k_pauli_tiny<float><<<1, 32, 0, stream>>>((const float2*)amp, n, num_terms, d_xm, d_zm, d_coeff, d_out);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? MLB_OK : MLB_ERR_DRIVER;
 }

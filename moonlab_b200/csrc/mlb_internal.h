@@ -225,14 +225,15 @@ struct PauliPass {
   uint64_t tiles_per_state, num_tiles;
 };
 int pauli_tile_bits(int dtype, bool apply);
-// One pass of an expectation value: *parts partials (at most num_sms *
-// kPauliCtasPerSm) whose sum is the pass's strings'.
+// One pass of an expectation value: partials (at most num_sms *
+// kPauliCtasPerSm) at d_partials + *parts, *parts raised by their number; with
+// d_out (the last pass) the sum of all of them there, by way of a zero at d_done.
 int launch_pauli_sum(int dtype, const void* amp, const PauliPass& P, const PauliSeg* d_segs,
-                     const PauliTerm* d_terms, double* d_partials, int num_sms, cudaStream_t stream, int* parts);
-// The whole sum for a state of one or two qubits (one partial).
+                     const PauliTerm* d_terms, double* d_partials, int* parts, unsigned* d_done, double* d_out,
+                     int num_sms, cudaStream_t stream);
+// The whole sum for a state of one or two qubits.
 int launch_pauli_tiny(int dtype, const void* amp, int n, int num_terms, const uint64_t* d_xm, const uint64_t* d_zm,
-                      const double* d_coeff, double* d_partials, cudaStream_t stream);
-int launch_sum_partials(const double* d_partials, int count, double* d_out, cudaStream_t stream);
+                      const double* d_coeff, double* d_out, cudaStream_t stream);
 // lambda (+)= the pass's strings on psi, for P.num_tiles tiles of a batch;
 // d_epart (or null): per-tile Re<psi|lambda>.
 int launch_pauli_apply(int dtype, const void* psi, void* lam, const PauliPass& P, const PauliSeg* d_segs,

@@ -1,7 +1,7 @@
 """mlb_expect_pauli_sum (kernels_pauli.cu) against numpy: registers below
 three qubits (their own kernel), of exactly a tile and one qubit either side
-of it, strings as wide as the register, repeated and empty X masks, and more
-strings than a pass holds.  Tolerance: a sum of T 2^n products in another
+of it, strings as wide as the register, repeated and empty X masks, more
+strings than a pass holds, and few strings on small states (smaller tiles).  Tolerance: a sum of T 2^n products in another
 order, 1e-15 T relative to the sum of |c_k| for a normalised state, plus
 complex64's own products (exact in FP64)."""
 from __future__ import annotations
@@ -22,7 +22,8 @@ def parity(v):
 
 
 @pytest.mark.parametrize("dtype", ["c128", "c64"])
-@pytest.mark.parametrize("n,terms", [(1, 6), (2, 9), (3, 20), (5, 700), (11, 40), (12, 300), (13, 33), (14, 50), (17, 30)])
+@pytest.mark.parametrize("n,terms", [(1, 6), (2, 9), (3, 20), (5, 700), (11, 40), (12, 300), (13, 33), (14, 50), (17, 30),
+                                     (7, 1), (10, 2), (13, 2), (16, 3), (18, 1), (19, 4)])
 def test_pauli_sum_matches_numpy(gpu, n, terms, dtype):
     rng = np.random.default_rng(100 * n + terms)
     a = rng.standard_normal(2 << n).view(np.complex128)
