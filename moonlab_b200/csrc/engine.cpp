@@ -1494,6 +1494,21 @@ int mlb_expect_pauli_sum(mlb_state_t* s, size_t num_terms, const uint64_t* xm, c
     *out = 0.0;
     return MLB_OK;
   }
+  // Coefficients are folded into the strings' signs and multiply every
+  // product: where that could overflow, underflow or meet infinities of both
+  // signs, they multiply the strings' values instead.
+  if (coeffs && !std::all_of(coeffs, coeffs + num_terms, [](double c) {
+        return c == 0.0 || (std::abs(c) >= 0x1p-900 && std::abs(c) <= 0x1p900);
+      })) {
+    double sum = 0.0;
+    for (size_t t = 0; t < num_terms; t++) {
+      double v = 0.0;
+      if ((rc = mlb_expect_pauli(s, xm[t], zm[t], &v))) return rc;
+      sum += coeffs[t] * v;
+    }
+    *out = sum;
+    return MLB_OK;
+  }
   // one upload (through the plan buffers), the passes' kernels, one result
   std::vector<pauli::Pass> passes;
   std::vector<unsigned char> blob;

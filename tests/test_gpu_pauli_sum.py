@@ -47,3 +47,23 @@ def test_pauli_sum_matches_numpy(gpu, n, terms, dtype):
     got = sv.expectation_pauli_sum(x, z, c)
     assert abs(got - want) < 1e-15 * terms * np.abs(c).sum() + 1e-14
     assert sv.expectation_pauli_sum([], [], []) == 0.0
+
+
+@pytest.mark.parametrize("c", [1e308, np.inf, -np.inf, 1e-310, np.nan])
+def test_extreme_coefficients(gpu, c):
+    """A coefficient multiplies its string's value, whatever its size: no
+    partial sum of it overflows, underflows or meets an infinity of the other
+    sign."""
+    n = 5
+    rng = np.random.default_rng(3)
+    a = rng.standard_normal(2 << n).view(np.complex128)
+    a /= np.linalg.norm(a)
+    with StateVector(n) as sv:
+        sv.set_amplitudes(a)
+        x, z = [0, 9, 21], [6, 2, 21]
+        v = [sv.expectation_pauli(p, q) for p, q in zip(x, z)]
+        got = sv.expectation_pauli_sum(x, z, [0.5, c, -2.0])
+        want = 0.5 * v[0] + c * v[1] + -2.0 * v[2]
+        tol = 16 * 2.0**-52 * (0.5 * abs(v[0]) + abs(c) * abs(v[1]) + 2 * abs(v[2]))  # sums of 32 products
+        assert got == want or (np.isnan(want) and np.isnan(got)) or abs(got - want) <= tol
+        assert sv.expectation_pauli_sum(x[1:2], z[1:2], [c]) == c * v[1] or np.isnan(c)
