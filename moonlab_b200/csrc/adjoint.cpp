@@ -101,10 +101,11 @@ struct mlb_hea {
   size_t part_cap = 0;
   double* d_epart = nullptr;
   size_t epart_cap = 0;
-  HeaSeg* d_segs = nullptr;
-  PauliTerm* d_terms = nullptr;
-  PauliSeg* d_psegs = nullptr;
-  int* d_slots = nullptr;  // parameter of each gradient slot, group by group
+  unsigned char* d_programs = nullptr;  // holds the next four
+  const HeaSeg* d_segs = nullptr;
+  const PauliTerm* d_terms = nullptr;
+  const PauliSeg* d_psegs = nullptr;
+  const int* d_slots = nullptr;  // parameter of each gradient slot, group by group
   double* d_out = nullptr;  // [B] energies then [B][P] grads
   size_t out_cap = 0;
   unsigned char* d_gram = nullptr;  // geometry: Gram matrix, then the Gram kernel's scratch
@@ -178,19 +179,26 @@ mlb_op_t proxy(const TapeOp& t) {
   return o;
 }
 
+// All rotations in program order, in the coordinates after the last layer.
+std::vector<hea::Rot> rotations(const mlb_hea* h) {
+  const uint32_t n = h->nr;
+  std::vector<hea::Rot> all((size_t)h->layers * n);
+  std::vector<uint64_t> dir(n), fun(n);
+  for (uint32_t q = 0; q < n; q++) dir[q] = fun[q] = 1ull << q;
+  for (uint32_t l = h->layers; l-- > 0;)  // one more ladder follows
+    for (uint32_t q = 0; q < n; q++) {
+      dir[q] = hea::ladder(dir[q], (int)n);
+      fun[q] = hea::unladder_functional(fun[q], (int)n);
+      all[(size_t)l * n + q] = {(int)l, (int)q, (int)(2 * (l * n + q)), dir[q], fun[q]};
+    }
+  return all;
+}
+
 // Plans one segment of layers [l0, l1) as rotation passes; the backward
 // sweep runs its rotations in reverse.
-void plan_rotations(mlb_hea* h, uint32_t l0, uint32_t l1, bool backward, std::vector<hea::Pass>& out) {
-  std::vector<hea::Rot> rots;
-  for (uint32_t l = l0; l < l1; l++)
-    for (uint32_t q = 0; q < h->nr; q++) {
-      hea::Rot r{(int)l, (int)q, (int)(2 * (l * h->nr + q)), 1ull << q, 1ull << q};
-      for (uint32_t k = l; k < h->layers; k++) {  // to the coordinates after the last layer
-        r.dir = hea::ladder(r.dir, (int)h->nr);
-        r.fun = hea::unladder_functional(r.fun, (int)h->nr);
-      }
-      rots.push_back(r);
-    }
+void plan_rotations(mlb_hea* h, const std::vector<hea::Rot>& all, uint32_t l0, uint32_t l1, bool backward,
+                    std::vector<hea::Pass>& out) {
+  std::vector<hea::Rot> rots(all.begin() + (size_t)l0 * h->nr, all.begin() + (size_t)l1 * h->nr);
   if (backward) std::reverse(rots.begin(), rots.end());
   // rows of 64 bytes
   hea::plan(rots, (int)h->n, hea_tile_bits(h->dtype, backward), h->dtype == MLB_C128 ? 2 : 3, h->dtype, out);
@@ -299,16 +307,23 @@ int upload_programs(mlb_hea* h) {
     all_terms.insert(all_terms.end(), p.terms.begin(), p.terms.end());
     all_psegs.insert(all_psegs.end(), p.segs.begin(), p.segs.end());
   }
-  cudaError_t e = cudaMalloc((void**)&h->d_segs, all_segs.size() * sizeof(HeaSeg));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_slots, param_of_slot.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_terms, all_terms.size() * sizeof(PauliTerm));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_psegs, all_psegs.size() * sizeof(PauliSeg));
+  // one allocation, one copy
+  std::vector<unsigned char> blob;
+  auto put = [&](const auto& v) {
+    const size_t at = (blob.size() + 15) & ~(size_t)15, bytes = v.size() * sizeof(v[0]);
+    blob.resize(at + bytes);
+    std::memcpy(blob.data() + at, v.data(), bytes);
+    return at;
+  };
+  const size_t segs_at = put(all_segs), slots_at = put(param_of_slot), terms_at = put(all_terms),
+               psegs_at = put(all_psegs);
+  cudaError_t e = cudaMalloc((void**)&h->d_programs, blob.size());
+  if (e == cudaSuccess) e = cudaMemcpy(h->d_programs, blob.data(), blob.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cfail(e, "adjoint program upload");
-  cudaMemcpy(h->d_segs, all_segs.data(), all_segs.size() * sizeof(HeaSeg), cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_slots, param_of_slot.data(), param_of_slot.size() * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_terms, all_terms.data(), all_terms.size() * sizeof(PauliTerm), cudaMemcpyHostToDevice);
-  e = cudaMemcpy(h->d_psegs, all_psegs.data(), all_psegs.size() * sizeof(PauliSeg), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) return cfail(e, "adjoint program upload");
+  h->d_segs = reinterpret_cast<const HeaSeg*>(h->d_programs + segs_at);
+  h->d_slots = reinterpret_cast<const int*>(h->d_programs + slots_at);
+  h->d_terms = reinterpret_cast<const PauliTerm*>(h->d_programs + terms_at);
+  h->d_psegs = reinterpret_cast<const PauliSeg*>(h->d_programs + psegs_at);
   if (h->fused_ok) {
     e = cudaMalloc((void**)&h->d_fblocks, h->fblocks.size() * sizeof(FusedBlockDev));
     if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_gblocks, h->gblocks.size() * sizeof(FusedGenBlock));
@@ -634,14 +649,15 @@ int mlb_hea_create(uint32_t n, uint32_t layers, uint64_t hf, size_t num_terms, c
   cut.push_back(h->tape.size());
   for (uint32_t l = 0; l < layers; l += h->seg_layers) h->bound.push_back(l);
   h->bound.push_back(layers);
+  const std::vector<hea::Rot> all = rotations(h);
   h->fwd_seg.push_back(0);
   for (size_t k = 0; k + 1 < h->bound.size(); k++) {
-    plan_rotations(h, h->bound[k], h->bound[k + 1], false, h->fwd);
+    plan_rotations(h, all, h->bound[k], h->bound[k + 1], false, h->fwd);
     h->fwd_seg.push_back(h->fwd.size());
   }
   h->bwd_seg.push_back(0);
   for (size_t k = h->bound.size() - 1; k-- > 0;) {
-    plan_rotations(h, h->bound[k], h->bound[k + 1], true, h->bwd);
+    plan_rotations(h, all, h->bound[k], h->bound[k + 1], true, h->bwd);
     h->bwd_seg.push_back(h->bwd.size());
   }
   {  // the first pass starts from |hf>
@@ -684,7 +700,7 @@ void mlb_hea_free(mlb_hea_t* h) {
   Guard g(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : {h->psi, h->lamb, h->ckpt, (void*)h->d_cs, (void*)h->d_part, (void*)h->d_epart,
-                  (void*)h->d_segs, (void*)h->d_terms, (void*)h->d_psegs, (void*)h->d_slots, (void*)h->d_out, (void*)h->d_gram,
+                  (void*)h->d_programs, (void*)h->d_out, (void*)h->d_gram,
                   (void*)h->d_fblocks, (void*)h->d_gblocks, (void*)h->d_gops, (void*)h->d_images,
                   (void*)h->d_ferr, (void*)h->d_norm})
     if (p) cudaFree(p);

@@ -58,11 +58,26 @@ struct Rot {
 
 inline bool conflict(const Rot& x, const Rot& y) { return parity(x.fun & y.dir) || parity(y.fun & x.dir); }
 
+// A list of at most 64 entries in place.
+template <typename T>
+struct Few {
+  T at[64];
+  size_t count = 0;
+  size_t size() const { return count; }
+  void push_back(T x) { at[count++] = x; }
+  T& operator[](size_t i) { return at[i]; }
+  const T& operator[](size_t i) const { return at[i]; }
+  T* begin() { return at; }
+  T* end() { return at + count; }
+  const T* begin() const { return at; }
+  const T* end() const { return at + count; }
+};
+
 // Reduced basis of a subspace: basis[i] has pivot bit piv[i] and zeros at
 // every other pivot.
 struct Basis {
-  std::vector<uint64_t> v;
-  std::vector<int> piv;
+  Few<uint64_t> v;
+  Few<int> piv;
   uint64_t reduce(uint64_t x) const {
     for (size_t i = 0; i < v.size(); i++)
       if (x >> piv[i] & 1ull) x ^= v[i];
@@ -109,19 +124,28 @@ inline uint32_t bank_of(uint32_t t, int dtype) {
 // A basis of span(vecs) whose first vectors (the lanes of one access phase)
 // reach distinct bank groups where the span allows.
 inline std::vector<uint32_t> bank_order(const std::vector<uint32_t>& vecs, int dtype) {
-  const int want = dtype == MLB_C128 ? 3 : 4;
+  const size_t want = dtype == MLB_C128 ? 3 : 4;
   std::vector<uint32_t> order;
-  Basis banks, chosen;
-  for (uint32_t mix = 1; mix < (1u << vecs.size()) && (int)order.size() < want; mix++) {
-    if (__builtin_popcount(mix) > 3) continue;
-    uint32_t t = 0;
-    for (size_t i = 0; i < vecs.size(); i++)
-      if (mix >> i & 1u) t ^= vecs[i];
-    if (!banks.reduce(bank_of(t, dtype)) || !chosen.reduce(t)) continue;
-    banks.add(bank_of(t, dtype));
-    chosen.add(t);
+  uint32_t bank[32], reached = 1;  // bit b: bank group b is a sum of the chosen vectors' (linear in them)
+  for (size_t i = 0; i < vecs.size(); i++) bank[i] = bank_of(vecs[i], dtype);
+  auto consider = [&](uint32_t t, uint32_t b) {
+    if (order.size() == want || (reached >> b & 1u)) return;
+    uint32_t more = reached;
+    for (uint32_t x = 0; x < 16; x++)
+      if (reached >> x & 1u) more |= 1u << (x ^ b);
+    reached = more;
     order.push_back(t);
+  };
+  // single vectors and sums of two and three, in the order of their sets as binary numbers
+  for (size_t i = 0; i < vecs.size() && order.size() < want; i++) {
+    consider(vecs[i], bank[i]);
+    for (size_t j = 0; j < i; j++) {
+      consider(vecs[i] ^ vecs[j], bank[i] ^ bank[j]);
+      for (size_t k = 0; k < j; k++) consider(vecs[i] ^ vecs[j] ^ vecs[k], bank[i] ^ bank[j] ^ bank[k]);
+    }
   }
+  Basis chosen;
+  for (uint32_t t : order) chosen.add(t);
   for (uint32_t t : vecs)
     if (chosen.add(t)) order.push_back(t);
   return order;
@@ -184,34 +208,44 @@ inline HeaSeg lower_segment(const std::vector<const Rot*>& rot, const Basis& B, 
 inline void plan(const std::vector<Rot>& rots, int n, int TB, int L, int dtype, std::vector<Pass>& out) {
   const int m = std::min(n, TB);
   L = std::min(L, m);
-  std::vector<int> rem(rots.size());
-  for (size_t i = 0; i < rem.size(); i++) rem[i] = (int)i;
-  const bool descending = !rots.empty() && rots.front().layer > rots.back().layer;
-  while (!rem.empty()) {
-    // two candidate orders, both topological: as given, and by bands of
-    // q + layer (a band is what a later band's rotations wait for)
+  // two candidate orders, both topological: as given, and by bands of
+  // q + layer (a band is what a later band's rotations wait for)
+  std::vector<int> rem[2];
+  for (size_t i = 0; i < rots.size(); i++) rem[0].push_back((int)i);
+  rem[1] = rem[0];
+  {
+    const bool descending = !rots.empty() && rots.front().layer > rots.back().layer;
+    auto key = [&](int i) { return rots[i].q + rots[i].layer; };
+    std::stable_sort(rem[1].begin(), rem[1].end(),
+                     [&](int a, int b) { return descending ? key(a) > key(b) : key(a) < key(b); });
+  }
+  while (!rem[0].empty()) {
     std::vector<int> best_take;
     Basis best_basis;
-    for (int form = 0; form < 2; form++) {
-      std::vector<int> order = rem;
-      if (form == 1) {
-        auto key = [&](int i) { return rots[i].q + rots[i].layer; };
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-          return descending ? key(a) > key(b) : key(a) < key(b);
-        });
-      }
+    for (const std::vector<int>& order : rem) {
       Basis V;
       for (int b = 0; b < L; b++) V.add(1ull << b);
-      std::vector<int> take, skipped;
+      // a rotation waits for the skipped ones that it does not commute with:
+      // it commutes with all where its functional vanishes on the span of
+      // their directions and theirs on its direction (both orders are
+      // topological, so that none of them comes after it in the sweep)
+      std::vector<int> take;
+      Basis dirs, funs;
       for (int i : order) {
-        bool ok = (int)take.size() < 3 * kMaxHeaSegs;
-        for (int j : skipped) ok = ok && !(j < i && conflict(rots[i], rots[j]));
+        if ((int)take.size() == 3 * kMaxHeaSegs || dirs.v.size() == (size_t)n || funs.v.size() == (size_t)n) break;
+        bool ok = true;
+        for (size_t j = 0; ok && j < dirs.v.size(); j++) ok = !parity(rots[i].fun & dirs.v[j]);
+        for (size_t j = 0; ok && j < funs.v.size(); j++) ok = !parity(funs.v[j] & rots[i].dir);
         if (ok && V.reduce(rots[i].dir)) {
           if ((int)V.v.size() < m) V.add(rots[i].dir);
           else ok = false;
         }
-        if (ok) take.push_back(i);
-        else skipped.push_back(i);
+        if (ok) {
+          take.push_back(i);
+        } else {
+          dirs.add(rots[i].dir);
+          funs.add(rots[i].fun);
+        }
       }
       if (take.size() > best_take.size()) {
         best_take = take;
@@ -265,10 +299,7 @@ inline void plan(const std::vector<Rot>& rots, int n, int TB, int L, int dtype, 
     std::vector<char> gone(rots.size(), 0);
     for (size_t i = 0; i < N; i++)
       if (done[i]) gone[best_take[i]] = 1;
-    std::vector<int> next;
-    for (int i : rem)
-      if (!gone[i]) next.push_back(i);
-    rem.swap(next);
+    for (std::vector<int>& r : rem) r.erase(std::remove_if(r.begin(), r.end(), [&](int i) { return gone[i]; }), r.end());
     out.push_back(std::move(P));
   }
 }
