@@ -154,17 +154,14 @@ __device__ __forceinline__ void inverse_norm(double t, Two& h) {
   h = {g, 0.5 * g * r};
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-}
-
 template <typename Real, bool BACK>
 __global__ void __launch_bounds__(HeaCfg<Real, BACK>::NT, HeaCfg<Real, BACK>::CTAS)
     k_hea(const typename Cplx<Real>::T* src, typename Cplx<Real>::T* psi, typename Cplx<Real>::T* lam,
           const __grid_constant__ HeaPass P, const HeaSeg* __restrict__ segs, const double2* __restrict__ cs,
           double* __restrict__ partials, int part_stride) {
   using A = typename Cplx<Real>::T;
-  constexpr int NT = HeaCfg<Real, BACK>::NT, TB = NT == 256 ? 8 : 7, kWarps = NT / 32;
+  constexpr int NT = HeaCfg<Real, BACK>::NT, TB = 7, kWarps = NT / 32;
+  static_assert(NT == 1 << TB);
   constexpr int UB = sizeof(A) == 16 ? 0 : 1;  // log2 of the amplitudes of a 16-byte unit
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t tile_bytes = (uint32_t)sizeof(A) << P.m;

@@ -56,6 +56,11 @@ __device__ __forceinline__ uint64_t pdep64(uint64_t j, uint64_t mask) {
 
 __device__ __forceinline__ int parity64(uint64_t x) { return __popcll(x) & 1; }
 
+// One 16-byte unit from global into shared memory, asynchronously.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
 // A kernel's dynamic shared-memory limit, raised once per device to the most
 // that any launch of it takes.  The limit belongs to the function and not to
 // a launch: set to one launch's own size, it would refuse a larger launch of

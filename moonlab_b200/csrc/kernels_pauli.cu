@@ -32,10 +32,6 @@ namespace {
 constexpr int kThreads = 256;       // two CTAs per SM: 16 warps at 128 registers
 constexpr int kMaxUnitSteps = 64;  // units of a tile per thread
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-}
-
 __device__ __forceinline__ double flip_sign(double c, uint32_t bit) {  // bit in 0/1
   return __hiloint2double(__double2hiint(c) ^ (int)(bit << 31), __double2loint(c));
 }

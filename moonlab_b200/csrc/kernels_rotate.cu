@@ -123,9 +123,7 @@ __global__ void __launch_bounds__(RotCfg<Real>::NT, RotCfg<Real>::CTAS)
   for (uint64_t tile = blockIdx.x; tile < P.num_tiles; tile += gridDim.x) {
     const uint64_t base = pdep64(tile, P.free_mask);
     for (uint32_t u = tid, j = 0; u < units; u += NT, j++)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sm0 + tile_swz16(u) * 16u),
-                   "l"(amp + (base | toff | joff[j]))
-                   : "memory");
+      cp_async16(sm0 + tile_swz16(u) * 16u, amp + (base | toff | joff[j]));
     for (int o = tid; o < num_ops; o += NT) {
       const RotOp& op = ops[o];
       TileOp<Real> w;

@@ -326,8 +326,7 @@ struct Lower {
   static bool lower(const DevPass& pass, int dtype, const std::vector<Gate>& ops, Program& out) {
     for (int max_var = kRotMaxVar; max_var >= 1; max_var--) {
       Program p;
-      long double scale = 1.0;
-      Lower(pass, dtype).build(ops, scale, true, p, max_var);
+      Lower(pass, dtype).build(ops, p, max_var);
       if (rot_shared_bytes(dtype, p.ops.size(), p.table.size()) > kRotMaxShared) continue;
       p.dev.entries = (uint32_t)p.table.size();
       out = std::move(p);
@@ -386,14 +385,14 @@ struct Lower {
     uint32_t reg = 0, zg = 0;
     uint64_t out = 0;
     bool c = false;
-    bool rest() const { return zg || out; }
   };
 
   using Rest = std::pair<uint32_t, uint64_t>;  // (group functional, outside functional)
 
-  // The program of `ops`.  `scale`: the factor owed by rotations so far, left
-  // for a later pass's table unless `settle`.  A table has up to 2^max_var variants.
-  void build(const std::vector<Gate>& ops, long double& scale, bool settle, Program& out, int max_var) {
+  // The program of `ops`; a table has up to 2^max_var variants where its ops
+  // allow.
+  void build(const std::vector<Gate>& ops, Program& out, int max_var) {
+    long double scale = 1.0L;  // owed by rotations so far
     items.reserve(3 * ops.size());
     for (const Gate& g : ops) add(*g.op, g.u);
     order();
@@ -416,7 +415,7 @@ struct Lower {
         if (it.pred.w[k] & ~before.w[k]) return false;
       return true;
     };
-    while (left || diags || (settle && scale != 1.0) || out.segs.empty()) {
+    while (left || diags || scale != 1.0L || out.segs.empty()) {
       // 1. the segment's directions and its rounds; a round's diagonals are
       // those its rotations wait for, `free` the others that could join
       hea::Basis W;
@@ -733,7 +732,7 @@ struct Lower {
         if (!open.empty())  // the table is paid for: others that may run now, with no variant more
           for (int i : r.free)
             if (!done.has(i) && !later_same(items[i]) && known(items[i])) join(i);
-        if (!open.empty() || scale < 0x1p-10 || (settle && scale != 1.0)) close(op);
+        if (!open.empty() || scale != 1.0L) close(op);
         else emit(op);
       }
       // what the registers hold now goes here; with no rotation left, all of it
@@ -746,7 +745,7 @@ struct Lower {
           for (int i : now)
             if (!done.has(i) && plain(items[i]) == (form == 0) && (form == 0 || left == 0 || (!open.empty() && known(items[i]))))
               join(i);
-        if (!open.empty() || (settle && !left && !diags && scale != 1.0)) close(RotOp{});
+        if (!open.empty()) close(RotOp{});
       } while (!left && diags);
       for (int i = 0; i < 4; i++) sg.alpha_out[i] = (uint16_t)hea::slot_bytes(cur[i], dtype);
       sg.op_end = (int)out.ops.size();
