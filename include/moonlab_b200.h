@@ -462,10 +462,11 @@ int  mlb_plan_ops(const mlb_op_t *ops, size_t num_ops, uint32_t num_qubits, int 
  * gate, 1 one generic 4x4 op in shared memory, 2 a dense 16x16 complex128
  * matrix on the FP64 tensor cores (dtype MLB_C128 with dense segments on,
  * as a state flushes by default).  A pass of one-qubit unitaries, CNOTs,
- * SWAPs and diagonals may run its ops as one rotation program instead of
- * these segments (complex128 from 13 qubits, complex64 from 21).  Segments
- * index the ops [op_begin, op_end) of the execution order.  Call with NULL buffers to learn the
- * sizes; a buffer too small gives MLB_ERR_INVALID_ARG. */
+ * SWAPs and diagonals runs its ops as one rotation program instead of these
+ * segments where that costs less (complex128 from 13 qubits, complex64 from
+ * 21; mlb_last_flush_rotation_passes counts them).  Segments index the ops
+ * [op_begin, op_end) of the execution order.  Call with NULL buffers to
+ * learn the sizes; a buffer too small gives MLB_ERR_INVALID_ARG. */
 typedef struct {
     uint8_t  high[16];
     uint8_t  num_low;
