@@ -425,7 +425,7 @@ int  mlb_last_flush_rotation_passes(const mlb_state_t *s, uint64_t *out);
  * identical with and without the cache.  0 entries (default) = off. */
 int  mlb_state_set_plan_cache(mlb_state_t *s, size_t entries);
 /* complex128 tiled mode: run each register segment that fits (4 register
- * qubits in a 13-qubit tile, at most 4 conditioning qubits outside them) as a
+ * qubits in a 12-qubit tile, at most 6 conditioning qubits outside them) as a
  * dense 16x16 complex matrix on the FP64 tensor cores (mma.sync f64), the
  * others gate by gate.  On (1) by default; 0 runs every segment gate by gate.
  * Queued ops are flushed first.  Results agree to rounding (~1e-15 per

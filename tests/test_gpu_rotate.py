@@ -38,7 +38,8 @@ def test_matches_the_oracle(gpu, n, count, seed):
     with StateVector(n) as sv:
         sv.run(g)
         got = sv.amplitudes()
-        assert sv.flush_stats()["dense_blocks"] > 0
+        st = sv.flush_stats()
+        assert st["rotation_passes"] == st["passes"]
     assert np.abs(got - B.port_run(n, g)).max() < 1e-12
 
 
@@ -51,6 +52,8 @@ def test_complex64_against_complex128(gpu, n):
         b.set_exec_mode("tiled")
         b.run(g)
         want, got = a.amplitudes(), b.amplitudes()
+        st = b.flush_stats()
+        assert a.flush_stats()["rotation_passes"] == 0 and st["rotation_passes"] == st["passes"]
     assert np.abs(got - want).max() < 2e-5
 
 
@@ -64,6 +67,7 @@ def test_pass_by_pass_choice(gpu, form):
         b.set_dense(False)
         b.run(g)
         x, y = a.amplitudes(), b.amplitudes()
+        assert a.flush_stats()["rotation_passes"] > 0 and b.flush_stats()["rotation_passes"] == 0
     assert np.abs(x - y).max() < 1e-12
 
 
@@ -71,7 +75,8 @@ def test_ops_of_both_kinds(gpu):
     """Ops that a program does not take, between ops that it takes."""
     n = 15
     rng = np.random.default_rng(9)
-    parts = [circuit(n, 60, 20 + k, TAKEN + [24, 25, 26]) for k in range(4)]
+    parts = [circuit(n, 60, 20 + k, TAKEN + [24, 25, 26]) for k in range(2)]
+    parts += [circuit(n, 600, 30 + k) for k in range(2)]
     m = rng.standard_normal((2, 2)) + 1j * rng.standard_normal((2, 2))  # not unitary
     with StateVector(n) as a, StateVector(n) as b:
         b.set_dense(False)
@@ -84,22 +89,24 @@ def test_ops_of_both_kinds(gpu):
                 if k == 2:
                     sv.apply_1q(4, m / np.linalg.norm(m))
         x, y = a.amplitudes(), b.amplitudes()
+        st = a.flush_stats()
+        assert 0 < st["rotation_passes"] < st["passes"]
     assert np.abs(x - y).max() < 1e-12
 
 
-@pytest.mark.parametrize("n,dtype,mode", [(13, "c128", "tiled"), (15, "c128", "tiled"), (21, "c64", "tiled"),
-                                          (21, "c64", "fused")])
-def test_controlled_zz(gpu, n, dtype, mode):
-    """ZZ under up to five controls, as ops of the C ABI (a program takes up
-    to three), on any qubits, against one kernel per gate."""
+@pytest.mark.parametrize("n,dtype,mode,most", [(13, "c128", "tiled", 3), (15, "c128", "tiled", 3), (15, "c128", "tiled", 5),
+                                               (21, "c64", "tiled", 3), (21, "c64", "fused", 5)])
+def test_controlled_zz(gpu, n, dtype, mode, most):
+    """ZZ under up to three controls, which a program takes, and up to five,
+    as ops of the C ABI on any qubits, against one kernel per gate."""
     rng = np.random.default_rng(n + len(mode))
     ops = (_lib.MlbOp * 30)()
     for i, o in enumerate(ops):
-        t, t2, *c = (int(q) for q in rng.permutation(n)[:2 + i % 6])
+        t, t2, *c = (int(q) for q in rng.permutation(n)[:2 + i % (most + 1)])
         o.kind, o.target, o.target2, o.cmask = 5, t, t2, sum(1 << q for q in c)
         for j, x in enumerate(np.exp(1j * rng.uniform(-np.pi, np.pi, 2))):
             o.m[2 * j], o.m[2 * j + 1] = x.real, x.imag
-    g = circuit(n, 40, 60 + n, [4, 7, 8, 9, 10])
+    g = circuit(n, 40 if mode == "fused" else 300, 60 + n, [4, 7, 8, 9, 10])
     with StateVector(n, dtype) as a, StateVector(n) as b:
         a.set_exec_mode(mode)
         b.set_exec_mode("eager")
@@ -108,6 +115,9 @@ def test_controlled_zz(gpu, n, dtype, mode):
             _lib.check(_lib.load().mlb_apply_ops(sv.handle, ops, len(ops)), "mlb_apply_ops")
             sv.run(g)
         x, y = a.amplitudes(), b.amplitudes()
+        st = a.flush_stats()
+    if most == 3:
+        assert st["rotation_passes"] == st["passes"]
     # the whole state's error: a fidelity of 1 - 1e-6 is 1.4e-3 on the fused path
     assert np.linalg.norm(x - y) < {"c128": 1e-12, "c64": 2e-3 if mode == "fused" else 2e-5}[dtype]
 
