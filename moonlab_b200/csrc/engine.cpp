@@ -829,21 +829,6 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
       }
     }
   }
-  // the segment matrices, in parallel over segments (~1 ms of host time each
-  // for 64 variants)
-  std::unique_ptr<double[]> frags(new double[nfrag]);
-  {
-    std::atomic<size_t> next{0};
-    auto work = [&]() {
-      for (size_t d; (d = next.fetch_add(1)) < dsegs.size();)
-        dense::fill_fragments(E->segs[dsrc[d]], E->dops.data(), dsegs[d], dplans[d], frags.get() + dsegs[d].frag_off);
-    };
-    const size_t nth = std::min<size_t>({host_cores(), (size_t)16, 1 + nfrag / (256 * 1024)});
-    std::vector<std::thread> pool;
-    for (size_t t = 1; t < nth; t++) pool.emplace_back(work);
-    work();
-    for (auto& t : pool) t.join();
-  }
   // one upload: ops, segments, dense segments, dense fragments, rotation programs
   size_t total = 0;
   auto room = [&](size_t bytes) {
@@ -875,7 +860,21 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   if (sb) std::memcpy(blob.get() + soff, dev_segs.data(), sb);
   if (!dsegs.empty()) {
     std::memcpy(blob.get() + doff, dsegs.data(), dsegs.size() * sizeof(DenseSegDev));
-    std::memcpy(blob.get() + foff, frags.get(), nfrag * sizeof(double));
+    // the segments' matrices, in place (11 MB for 400 random gates on 20
+    // qubits, half of them controlled rotations; through a buffer of their
+    // own the flush took 5.0 ms, not 2.9), in parallel over segments (~1 ms of
+    // host time each for 64 variants)
+    double* fr = reinterpret_cast<double*>(blob.get() + foff);
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+      for (size_t d; (d = next.fetch_add(1)) < dsegs.size();)
+        dense::fill_fragments(E->segs[dsrc[d]], E->dops.data(), dsegs[d], dplans[d], fr + dsegs[d].frag_off);
+    };
+    const size_t nth = std::min<size_t>({host_cores(), (size_t)16, 1 + nfrag / (256 * 1024)});
+    std::vector<std::thread> pool;
+    for (size_t t = 1; t < nth; t++) pool.emplace_back(work);
+    work();
+    for (auto& t : pool) t.join();
   }
   for (size_t k = 0; k < np; k++) {
     if (!is_rot[k]) continue;
