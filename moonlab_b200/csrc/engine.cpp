@@ -554,11 +554,12 @@ constexpr uint32_t kRotMinC128 = 13, kRotMinC64 = 21;
 // matrices of the dense segments, the programs' lowering); above, each pass
 // takes the form that the GPU runs faster.
 constexpr uint32_t kRotWholeC128 = 25;
+constexpr int kRotMostConditions = 64;  // more controlled diagonals, and more than rotations: pass by pass
 
 // What a pass costs in each form, in us, from counts that its plan has: least-
-// squares fits to 2000 passes of brickwork (depth 1 to 20, without and with
-// ZZ), QAOA, GHZ and RY circuits of 13 to 27 qubits (complex64: 18 to 24), each
-// run in both forms (a pass is 10 % off, rms).  `unit`: the pass's waves of
+// squares fits to 3000 passes of brickwork (depth 1 to 20, without and with
+// ZZ), QAOA, GHZ, RY, Trotter, Fourier and random circuits of 13 to 27 qubits
+// (complex64: 18 to 24), each run in both forms (a pass is 10 % off, rms).  `unit`: the pass's waves of
 // CTAs beside a 27-qubit state's.  Wall us of a flush on a full register, as
 // segments / as programs: complex128, 16 qubits, 2 layers 90 / 123, 20 layers
 // 1175 / 703; 20 qubits, 4 layers 189 / 303, 20 layers 1910 / 957, QAOA of 2
@@ -568,10 +569,11 @@ constexpr uint32_t kRotWholeC128 = 25;
 struct FormCost {
   double segments, program;  // with the host's part of the segments
   double lowering;           // the host's part of the program, one thread
+  bool fits;                 // the program probably does
 };
 FormCost form_cost(const mlb_state* s, const DevPass& pass, uint64_t tiles, const DevSegment* segs, int num_segs,
                    const DevOp* dops) {
-  int rotations = 0, diagonals = 0, moves = 0;
+  int rotations = 0, diagonals = 0, conditioned = 0, moves = 0;
   double fills = 0;  // ops times variants of the dense segments' matrices
   for (int k = 0; k < num_segs; k++) {
     const DevSegment& sg = segs[k];
@@ -585,20 +587,30 @@ FormCost form_cost(const mlb_state* s, const DevPass& pass, uint64_t tiles, cons
         case DOP_1Q_REAL: rotations++; break;
         case DOP_X:
         case DOP_SWAP: moves++; break;
-        default: diagonals++;
+        default: {
+          const int conditions = popc(dops[o].ocmask) + popc((uint64_t)dops[o].lcmask);
+          const int bits = popc(dops[o].omask) + popc((uint64_t)dops[o].lmask);
+          if (conditions || (dops[o].kind == DOP_PHASE && bits > 1)) conditioned++;
+          else diagonals++;
+        }
       }
   }
   const bool c128 = s->dtype == MLB_C128;
   const int bits = c128 ? kTileBitsC128 : 13, local = pass.L + pass.H;
   const uint64_t full = std::max<uint64_t>(1, tiles >> (bits - local)), wave = (uint64_t)s->num_sms * (c128 ? 3 : 2);
   const double unit = (double)((full + wave - 1) / wave * wave << bits) / (double)(1 << 27);
-  const double S = num_segs, K = rotations, D = diagonals, X = moves;
+  const double S = num_segs, K = rotations, D = diagonals, C = conditioned, X = moves;
+  // each conditioned diagonal brings functionals of its own: tables in more
+  // variants, and past some number, more than shared memory holds
+  const double lower = 0.8 * C + 0.025 * C * C;
+  const bool fits = C <= (c128 ? 64 : 128) || s->n <= 13;
   if (c128)
     return {9 + unit * (415 + 430 * S) + 2.3 * S + 0.188 * fills,
-            8.5 + unit * (470 + 125 * S + 42 * K + 17 * D + 13 * X), 1.3 * K + 1.5 * D + 0.35 * X + 1.6 * S};
+            8.5 + unit * (470 + 125 * S + 42 * K + 17 * D + 22 * C + 13 * X),
+            1.3 * K + 1.5 * D + lower + 0.35 * X + 1.6 * S, fits};
   // unfilled tiles (complex64, a last pass of few ops): 12.5 ns each
-  return {10 + unit * (220 + 170 * S + 54 * K + 103 * D + 55 * X) + 0.0125 * (double)(tiles - full),
-          10 + unit * (260 + 60 * S + 34 * K + 8 * D), 1.55 * K + 1.6 * D + 0.2 * X + 1.5 * S};
+  return {10 + unit * (220 + 170 * S + 54 * K + 103 * D + 55 * C + 55 * X) + 0.0125 * (double)(tiles - full),
+          10 + unit * (260 + 60 * S + 34 * K + 8 * D + 12 * C), 1.55 * K + 1.6 * D + lower + 0.2 * X + 1.5 * S, fits};
 }
 
 // The passes' rotation programs, lowered by threads of their own while the
@@ -730,8 +742,17 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   // the ops' own matrices (pushed ones, rounded for the other forms, cost
   // accuracy: 30 qubits, depth 40: <Z> 7.4e-13 off, not 3.7e-13).
   const bool rot_on = s->dtype == MLB_C64 ? s->n >= kRotMinC64 : s->dense_c128 && s->n >= kRotMinC128;
+  auto many_conditions = [&]() {  // the programs of some passes may not fit
+    int conditioned = 0, rotations = 0;
+    for (const mlb_op_t& o : ops) {
+      conditioned += (o.kind == MLB_OP_PHASE && popc(o.cmask) > 1) ||
+                     ((o.kind == MLB_OP_DIAG1 || o.kind == MLB_OP_ZZ) && o.cmask);
+      rotations += o.kind == MLB_OP_1Q;
+    }
+    return conditioned > kRotMostConditions && conditioned > rotations;
+  };
   const bool whole = rot_on && (s->dtype == MLB_C64 || s->n <= kRotWholeC128) &&
-                     std::all_of(ops.begin(), ops.end(), rot::covers);
+                     std::all_of(ops.begin(), ops.end(), rot::covers) && !many_conditions();
   const uint64_t allq = s->n >= 64 ? ~0ull : ((1ull << s->n) - 1ull);
   std::vector<rot::Unitary> units;
   Lowering low(s->dtype, ops, units);
@@ -749,7 +770,7 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
       return;
     const FormCost c =
         form_cost(s, pp.pass, tiles, segs.data() + pp.seg_begin, pp.seg_end - pp.seg_begin, dops.data());
-    const double mine = c.program + low.share() * c.lowering;
+    const double mine = c.fits ? c.program + low.share() * c.lowering : HUGE_VAL;
     if (!whole && mine >= c.segments) return;
     cost_segments += c.segments;
     cost_programs += mine;

@@ -222,6 +222,7 @@ struct Lower {
   std::vector<Item> items;
   Fun label[kRotBits];
   uint32_t dir[kRotBits];
+  bool full = false;  // the program outgrew shared memory: the rest is not planned
 
   Lower(const DevPass& pass, int dt) : P(pass), dtype(dt), m(pass.L + pass.H) {
     for (int& x : local_of) x = -1;
@@ -326,8 +327,7 @@ struct Lower {
   static bool lower(const DevPass& pass, int dtype, const std::vector<Gate>& ops, Program& out) {
     for (int max_var = kRotMaxVar; max_var >= 1; max_var--) {
       Program p;
-      Lower(pass, dtype).build(ops, p, max_var);
-      if (rot_shared_bytes(dtype, p.ops.size(), p.table.size()) > kRotMaxShared) continue;
+      if (!Lower(pass, dtype).build(ops, p, max_var)) continue;
       p.dev.entries = (uint32_t)p.table.size();
       out = std::move(p);
       return true;
@@ -390,8 +390,8 @@ struct Lower {
   using Rest = std::pair<uint32_t, uint64_t>;  // (group functional, outside functional)
 
   // The program of `ops`; a table has up to 2^max_var variants where its ops
-  // allow.
-  void build(const std::vector<Gate>& ops, Program& out, int max_var) {
+  // allow.  False: it does not fit shared memory.
+  bool build(const std::vector<Gate>& ops, Program& out, int max_var) {
     long double scale = 1.0L;  // owed by rotations so far
     items.reserve(3 * ops.size());
     for (const Gate& g : ops) add(*g.op, g.u);
@@ -416,6 +416,7 @@ struct Lower {
       return true;
     };
     while (left || diags || scale != 1.0L || out.segs.empty()) {
+      if (full) return false;
       // 1. the segment's directions and its rounds; a round's diagonals are
       // those its rotations wait for, `free` the others that could join
       hea::Basis W;
@@ -632,6 +633,13 @@ struct Lower {
       auto close = [&](RotOp op) {  // emits op with the open table
         const uint32_t nv = (uint32_t)var.size();
         const size_t at = out.table.size();
+        full = full || rot_shared_bytes(dtype, out.ops.size() + 1, at + ((size_t)16 << nv)) > kRotMaxShared;
+        if (full) {
+          var.clear();
+          open.clear();
+          scale = 1.0L;
+          return;
+        }
         out.table.resize(at + ((size_t)16 << nv));
         std::vector<cl> wide((size_t)16 << nv, cl(scale, 0.0L));
         scale = 1.0;
@@ -751,6 +759,7 @@ struct Lower {
       sg.op_end = (int)out.ops.size();
       out.segs.push_back(sg);
     }
+    if (full || rot_shared_bytes(dtype, out.ops.size(), out.table.size()) > kRotMaxShared) return false;
     D.num_ops = (int)out.ops.size();
     D.num_segs = (int)out.segs.size();
     for (int i = 0; i < m; i++) {
@@ -758,6 +767,7 @@ struct Lower {
       D.label_out[i] = label[i].out;
       if (label[i].c) D.label_const |= 1u << i;
     }
+    return true;
   }
 };
 

@@ -32,6 +32,14 @@ def circuit(n, count, seed, types=TAKEN):
     return g
 
 
+def qft(n):
+    recs = []
+    for q in range(n - 1, -1, -1):
+        recs.append((4, q, -1, 0, 0.0))
+        recs += [(23, q, k, 0, np.pi / (1 << (q - k))) for k in range(q - 1, -1, -1)]
+    return np.array(recs, dtype=GATE_DTYPE)
+
+
 @pytest.mark.parametrize("n,count,seed", [(13, 1, 1), (13, 300, 2), (14, 500, 3), (16, 400, 4), (18, 300, 5)])
 def test_matches_the_oracle(gpu, n, count, seed):
     g = circuit(n, count, seed)
@@ -129,6 +137,8 @@ def test_controlled_zz(gpu, n, dtype, mode, most):
     (20, "c128", "brickwork 20", 1), (20, "c128", "zz 6", 1), (24, "c128", "qaoa 2", 1), (25, "c128", "zz 4", 1),
     # pass by pass: some of either form
     (26, "c128", "brickwork 6", None), (26, "c128", "brickwork 14", None),
+    # many controlled phases: the passes that they crowd stay segments
+    (16, "c128", "qft 1", None), (20, "c128", "qft 1", None), (21, "c64", "qft 1", None),
     # registers below the programs' reach
     (12, "c128", "brickwork 20", 0), (20, "c64", "brickwork 20", 0),
     # complex64: a short circuit and a long one, and one whose last tile would hold few qubits
@@ -138,7 +148,8 @@ def test_form_that_costs_less(gpu, n, dtype, gates, programs):
     forms' kernels (one per gate)."""
     kind, depth = gates.split()
     depth = int(depth)
-    g = qaoa_circuit(n, depth, 3) if kind == "qaoa" else brickwork(n, depth, 3, zz_every=int(kind == "zz"))
+    g = (qaoa_circuit(n, depth, 3) if kind == "qaoa" else qft(n) if kind == "qft" else
+         brickwork(n, depth, 3, zz_every=int(kind == "zz")))
     if programs == 0 and n >= 13:  # the ops' own matrices, whatever was pushed forward on the way
         g = np.concatenate([g, circuit(n, 6, n, [4, 7])])
     with StateVector(n, dtype) as a, StateVector(n) as b:
