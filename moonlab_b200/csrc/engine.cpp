@@ -571,6 +571,9 @@ struct FormCost {
   double lowering;           // the host's part of the program, one thread
   bool fits;                 // the program probably does
 };
+// A controlled diagonal that reads so many functionals, beside one that reads
+// two: by its variants of a table.
+int condition_weight(int reads) { return reads == 2 ? 1 : reads == 3 ? 3 : 6; }
 FormCost form_cost(const mlb_state* s, const DevPass& pass, uint64_t tiles, const DevSegment* segs, int num_segs,
                    const DevOp* dops) {
   int rotations = 0, diagonals = 0, conditioned = 0, moves = 0;
@@ -588,9 +591,9 @@ FormCost form_cost(const mlb_state* s, const DevPass& pass, uint64_t tiles, cons
         case DOP_X:
         case DOP_SWAP: moves++; break;
         default: {
-          const int conditions = popc(dops[o].ocmask) + popc((uint64_t)dops[o].lcmask);
-          const int bits = popc(dops[o].omask) + popc((uint64_t)dops[o].lmask);
-          if (conditions || (dops[o].kind == DOP_PHASE && bits > 1)) conditioned++;
+          int reads = popc(dops[o].ocmask) + popc((uint64_t)dops[o].lcmask);
+          reads += dops[o].kind == DOP_PHASE ? popc(dops[o].omask) + popc((uint64_t)dops[o].lmask) : 1;
+          if (reads > 1) conditioned += condition_weight(reads);
           else diagonals++;
         }
       }
@@ -600,7 +603,7 @@ FormCost form_cost(const mlb_state* s, const DevPass& pass, uint64_t tiles, cons
   const uint64_t full = std::max<uint64_t>(1, tiles >> (bits - local)), wave = (uint64_t)s->num_sms * (c128 ? 3 : 2);
   const double unit = (double)((full + wave - 1) / wave * wave << bits) / (double)(1 << 27);
   const double S = num_segs, K = rotations, D = diagonals, C = conditioned, X = moves;
-  // each conditioned diagonal brings functionals of its own: tables in more
+  // each controlled diagonal brings functionals of its own: tables in more
   // variants, and past some number, more than shared memory holds
   const double lower = 0.8 * C + 0.025 * C * C;
   const bool fits = C <= (c128 ? 64 : 128) || s->n <= 13;
@@ -745,8 +748,9 @@ int flush_tiled(mlb_state* s, const std::vector<mlb_op_t>& ops, mlb_flush_stats_
   auto many_conditions = [&]() {  // the programs of some passes may not fit
     int conditioned = 0, rotations = 0;
     for (const mlb_op_t& o : ops) {
-      conditioned += (o.kind == MLB_OP_PHASE && popc(o.cmask) > 1) ||
-                     ((o.kind == MLB_OP_DIAG1 || o.kind == MLB_OP_ZZ) && o.cmask);
+      const bool keyed = o.kind == MLB_OP_DIAG1 || o.kind == MLB_OP_ZZ;
+      const int reads = popc(o.cmask) + keyed;
+      if ((keyed || o.kind == MLB_OP_PHASE) && reads > 1) conditioned += condition_weight(reads);
       rotations += o.kind == MLB_OP_1Q;
     }
     return conditioned > kRotMostConditions && conditioned > rotations;

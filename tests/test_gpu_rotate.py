@@ -108,20 +108,22 @@ def test_controlled_zz(gpu, n, dtype, mode, most):
     """ZZ under up to three controls, which a program takes, and up to five,
     as ops of the C ABI on any qubits, against one kernel per gate."""
     rng = np.random.default_rng(n + len(mode))
-    ops = (_lib.MlbOp * 30)()
+    ops = (_lib.MlbOp * 24)()
     for i, o in enumerate(ops):
         t, t2, *c = (int(q) for q in rng.permutation(n)[:2 + i % (most + 1)])
         o.kind, o.target, o.target2, o.cmask = 5, t, t2, sum(1 << q for q in c)
         for j, x in enumerate(np.exp(1j * rng.uniform(-np.pi, np.pi, 2))):
             o.m[2 * j], o.m[2 * j + 1] = x.real, x.imag
-    g = circuit(n, 40 if mode == "fused" else 300, 60 + n, [4, 7, 8, 9, 10])
+    parts = [circuit(n, 20 if mode == "fused" else 140, 60 + n + k, [4, 7, 8, 9, 10]) for k in range(5)]
     with StateVector(n, dtype) as a, StateVector(n) as b:
         a.set_exec_mode(mode)
         b.set_exec_mode("eager")
         for sv in (a, b):
-            sv.run(g)
-            _lib.check(_lib.load().mlb_apply_ops(sv.handle, ops, len(ops)), "mlb_apply_ops")
-            sv.run(g)
+            for k, g in enumerate(parts):
+                sv.run(g)
+                some = (_lib.MlbOp * 6)(*ops[6 * k:6 * k + 6]) if k < 4 else None
+                if some:
+                    _lib.check(_lib.load().mlb_apply_ops(sv.handle, some, 6), "mlb_apply_ops")
         x, y = a.amplitudes(), b.amplitudes()
         st = a.flush_stats()
     if most == 3:
@@ -138,7 +140,7 @@ def test_controlled_zz(gpu, n, dtype, mode, most):
     # pass by pass: some of either form
     (26, "c128", "brickwork 6", None), (26, "c128", "brickwork 14", None),
     # many controlled phases: the passes that they crowd stay segments
-    (16, "c128", "qft 1", None), (20, "c128", "qft 1", None), (21, "c64", "qft 1", None),
+    (16, "c128", "qft 1", None), (20, "c128", "qft 1", None),
     # registers below the programs' reach
     (12, "c128", "brickwork 20", 0), (20, "c64", "brickwork 20", 0),
     # complex64: a short circuit and a long one, and one whose last tile would hold few qubits
