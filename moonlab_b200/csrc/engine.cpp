@@ -556,24 +556,26 @@ constexpr uint32_t kRotMinC128 = 13, kRotMinC64 = 21;
 constexpr uint32_t kRotWholeC128 = 25;
 constexpr int kRotMostConditions = 64;  // more controlled diagonals, and more than rotations: pass by pass
 
+// A controlled diagonal that reads so many functionals, beside one that reads
+// two: by its variants of a table.
+int condition_weight(int reads) { return reads == 2 ? 1 : reads == 3 ? 3 : 6; }
+
 // What a pass costs in each form, in us, from counts that its plan has: least-
 // squares fits to 3000 passes of brickwork (depth 1 to 20, without and with
 // ZZ), QAOA, GHZ, RY, Trotter, Fourier and random circuits of 13 to 27 qubits
-// (complex64: 18 to 24), each run in both forms (a pass is 10 % off, rms).  `unit`: the pass's waves of
-// CTAs beside a 27-qubit state's.  Wall us of a flush on a full register, as
-// segments / as programs: complex128, 16 qubits, 2 layers 90 / 123, 20 layers
-// 1175 / 703; 20 qubits, 4 layers 189 / 303, 20 layers 1910 / 957, QAOA of 2
-// layers 1532 / 529; 25 qubits, 4 layers 1892 / 2647, with ZZ 4570 / 3498;
-// complex64, 21 qubits, QAOA of 1 layer 248 / 333, 20 layers 1183 / 1017; 24
-// qubits, 20 layers 7650 / 3927.  The cheaper form is taken in all but a few ties.
+// (complex64: 18 to 24), each run in both forms (a pass is 10 % off, rms).
+// `unit`: the pass's waves of CTAs beside a 27-qubit state's.  Wall us of a
+// flush on a full register, as segments / as programs: complex128, 16 qubits,
+// 2 layers 90 / 123, 20 layers 1175 / 703; 20 qubits, 4 layers 189 / 303, 20
+// layers 1910 / 957, QAOA of 2 layers 1532 / 529; 25 qubits, 4 layers 1892 /
+// 2647, with ZZ 4570 / 3498; complex64, 21 qubits, QAOA of 1 layer 248 / 333,
+// 20 layers 1183 / 1017; 24 qubits, 20 layers 7650 / 3927.  The cheaper form
+// is taken in all but a few ties.
 struct FormCost {
   double segments, program;  // with the host's part of the segments
   double lowering;           // the host's part of the program, one thread
   bool fits;                 // the program probably does
 };
-// A controlled diagonal that reads so many functionals, beside one that reads
-// two: by its variants of a table.
-int condition_weight(int reads) { return reads == 2 ? 1 : reads == 3 ? 3 : 6; }
 FormCost form_cost(const mlb_state* s, const DevPass& pass, uint64_t tiles, const DevSegment* segs, int num_segs,
                    const DevOp* dops) {
   int rotations = 0, diagonals = 0, conditioned = 0, moves = 0;
