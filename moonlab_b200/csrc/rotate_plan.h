@@ -393,6 +393,9 @@ struct Lower {
   // allow.  False: it does not fit shared memory.
   bool build(const std::vector<Gate>& ops, Program& out, int max_var) {
     long double scale = 1.0L;  // owed by rotations so far
+    // what a table's rounding took from the norm, given back by the next one: a
+    // table of one scale for all its entries rounds them all alike
+    long double owed = 1.0L;
     items.reserve(3 * ops.size());
     for (const Gate& g : ops) add(*g.op, g.u);
     order();
@@ -641,11 +644,11 @@ struct Lower {
           return;
         }
         out.table.resize(at + ((size_t)16 << nv));
-        std::vector<cl> wide((size_t)16 << nv, cl(scale, 0.0L));
+        std::vector<cl> wide((size_t)16 << nv, cl(scale * owed, 0.0L));
         scale = 1.0;
         struct Bit {
           uint32_t reg, v, c;  // patterns over the register index and the variant
-          uint32_t at(uint32_t k, uint32_t x) const { return ((reg >> k) ^ (v >> x) ^ c) & 1u; }
+          uint32_t row(uint32_t x) const { return (reg ^ (((v >> x) ^ c) & 1u ? 0xffffu : 0u)) & 0xffffu; }  // of variant x
         };
         auto pattern = [](uint32_t f) {
           uint32_t p = 0;
@@ -661,15 +664,26 @@ struct Lower {
           Bit cond[3];
           for (int c = 0; c < d.nc; c++) cond[c] = bit(d.cond[c]);
           const Bit key = d.keyed ? bit(d.key) : Bit{0, 0, 1};
-          for (uint32_t k = 0; k < 16; k++)
-            for (uint32_t x = 0; x < (1u << nv); x++) {
-              bool on = true;
-              for (int c = 0; c < d.nc; c++) on = on && cond[c].at(k, x);
-              cl& e = wide[16 * x + k];
-              if (on) e = mul(e, d.d[key.at(k, x)]);
-            }
+          for (uint32_t x = 0; x < (1u << nv); x++) {
+            uint32_t on = 0xffffu;
+            for (int c = 0; c < d.nc; c++) on &= cond[c].row(x);
+            for (int b = 0; b < 2; b++)
+              if (d.d[b] != cl(1.0L))
+                for (uint32_t m = on & (b ? key.row(x) : ~key.row(x)); m; m &= m - 1) {
+                  cl& e = wide[16 * x + (uint32_t)__builtin_ctz(m)];
+                  e = mul(e, d.d[b]);
+                }
+          }
         }
-        for (size_t k = 0; k < wide.size(); k++) out.table[at + k] = cd((double)wide[k].real(), (double)wide[k].imag());
+        long double off = 0.0L, sum = 0.0L;  // of the rounded entries' squares, halved; of the squares
+        for (size_t k = 0; k < wide.size(); k++) {
+          const cl w = wide[k];
+          const cd e = dtype == MLB_C128 ? cd((double)w.real(), (double)w.imag()) : cd((float)w.real(), (float)w.imag());
+          out.table[at + k] = e;
+          off += w.real() * (e.real() - w.real()) + w.imag() * (e.imag() - w.imag());
+          sum += norm(w);
+        }
+        owed = std::abs(off / sum) < 1e-6L ? 1.0L - off / sum : 1.0L;
         op.table = (uint32_t)at;
         op.nv = (uint8_t)nv;
         op.flags |= kRotTable;

@@ -177,3 +177,25 @@ def test_pushing_forward_costs_no_accuracy(host):
             errs.append(float(np.linalg.norm((got - exact).astype(complex))))
     own, pushed = np.sqrt(np.mean(np.square(errs).reshape(-1, 2), 0))
     assert pushed < 1.03 * own, (pushed, own)
+
+
+def test_tables_keep_the_norm(host):
+    """A table of one scale for all 16 entries rounds them all alike: what its
+    rounding takes from the norm is given back by the next one.  Layers of RY
+    and CNOT: the norm's drift, rms of 24 circuits, is 1.4e-16, 3.4e-16
+    without the correction; half as much again as the first is allowed."""
+    n, drift = 10, []
+    for seed in range(24):
+        rng = np.random.default_rng(seed)
+        ops = []
+        for k in range(14):
+            for q in range(n):
+                t = rng.uniform(-np.pi, np.pi)
+                ops.append(make(OP_1Q, q, -1, (), np.array([np.cos(t), -np.sin(t), np.sin(t), np.cos(t)]) + 0j))
+            ops += [make(OP_X, q + 1, -1, (q,)) for q in range(k & 1, n - 1, 2)]
+        a = np.zeros(1 << n, complex)
+        a[0] = 1
+        arr = (_lib.MlbOp * len(ops))(*ops)
+        assert host.host_run(arr, len(ops), n, (1 << n) - 1, _lib.MLB_C128, 1, a.ctypes.data) == 0
+        drift.append(float(np.linalg.norm(a.astype(np.clongdouble)) - 1))
+    assert np.sqrt(np.mean(np.square(drift))) < 2.2e-16
